@@ -35,120 +35,6 @@ __global__ void k_periodic(Geo g, double* __restrict__ b, int ncomp) {
   }
 }
 
-// ---- grid_interp.f -------------------------------------------------------
-
-// face_to_center (grid_interp.f:150-171), interior nodes.
-__global__ void k_face_to_center(Geo g, const double* __restrict__ v, double* __restrict__ vc) {
-  const long long N = n_interior(g);
-  const long long C = g.C, sx = 1, sy = g.nx, sz = (long long)g.nx * g.ny;
-  GRID_STRIDE(t, N) {
-    int i, j, k;
-    interior_ijk(g, t, i, j, k);
-    const long long o = nidx(g, i, j, k);
-    vc[o] = g.xr[i] * (v[o] - v[o - sx]) + v[o - sx];
-    vc[o + C] = g.yr[j] * (v[o + C] - v[o - sy + C]) + v[o - sy + C];
-    vc[o + 2 * C] = g.zr[k] * (v[o + 2 * C] - v[o - sz + 2 * C]) + v[o - sz + 2 * C];
-  }
-}
-
-// edge_to_center (grid_interp.f:22-57), interior nodes.
-__global__ void k_edge_to_center(Geo g, const double* __restrict__ bt, double* __restrict__ btc) {
-  const long long N = n_interior(g);
-  const long long C = g.C, sx = 1, sy = g.nx, sz = (long long)g.nx * g.ny;
-  GRID_STRIDE(t, N) {
-    int i, j, k;
-    interior_ijk(g, t, i, j, k);
-    const long long o = nidx(g, i, j, k);
-    const double yr = g.yr[j], xr = g.xr[i], zr = g.zr[k];
-    double b1, b2;
-    // component 1: y then z
-    b2 = bt[o - sy] + yr * (bt[o] - bt[o - sy]);
-    b1 = bt[o - sy - sz] + yr * (bt[o - sz] - bt[o - sy - sz]);
-    btc[o] = b1 + zr * (b2 - b1);
-    // component 2: x then z
-    const double* b = bt + C;
-    b2 = b[o - sx] + xr * (b[o] - b[o - sx]);
-    b1 = b[o - sx - sz] + xr * (b[o - sz] - b[o - sx - sz]);
-    btc[o + C] = b1 + zr * (b2 - b1);
-    // component 3: y then x
-    b = bt + 2 * C;
-    b2 = b[o - sy] + yr * (b[o] - b[o - sy]);
-    b1 = b[o - sx - sy] + yr * (b[o - sx] - b[o - sx - sy]);
-    btc[o + 2 * C] = b1 + xr * (b2 - b1);
-  }
-}
-
-// Face average cc_m = 0.5*(ct_m(node) + ct_m(node+e_m)) of crossf2
-// (gutsf.f:94-96) and edge_to_face (grid_interp.f:123-125), interior nodes.
-__global__ void k_face_avg(Geo g, const double* __restrict__ ct, double* __restrict__ cc) {
-  const long long N = n_interior(g);
-  const long long C = g.C, sy = g.nx, sz = (long long)g.nx * g.ny;
-  GRID_STRIDE(t, N) {
-    int i, j, k;
-    interior_ijk(g, t, i, j, k);
-    const long long o = nidx(g, i, j, k);
-    cc[o] = 0.5 * (ct[o] + ct[o + 1]);
-    cc[o + C] = 0.5 * (ct[o + C] + ct[o + sy + C]);
-    cc[o + 2 * C] = 0.5 * (ct[o + 2 * C] + ct[o + sz + 2 * C]);
-  }
-}
-
-// Cell-centre cross product of crossf2 (gutsf.f:65-76), interior nodes.
-__global__ void k_cross(Geo g, const double* __restrict__ aa, const double* __restrict__ btc,
-                        double* __restrict__ ct) {
-  const long long N = n_interior(g);
-  const long long C = g.C;
-  GRID_STRIDE(t, N) {
-    int i, j, k;
-    interior_ijk(g, t, i, j, k);
-    const long long o = nidx(g, i, j, k);
-    const double ax = aa[o], bx = btc[o], ay = aa[o + C], by = btc[o + C], az = aa[o + 2 * C],
-                 bz = btc[o + 2 * C];
-    ct[o] = ay * bz - az * by;
-    ct[o + C] = az * bx - ax * bz;
-    ct[o + 2 * C] = ax * by - ay * bx;
-  }
-}
-
-// ---- gutsf.f ---------------------------------------------------------------
-
-// curlB (gutsf.f:202-239), interior nodes.
-__global__ void k_curlB(Geo g, const double* __restrict__ b1, const double* __restrict__ np,
-                        double* __restrict__ aj, double alpha) {
-  const long long N = n_interior(g);
-  const long long C = g.C, sx = 1, sy = g.nx, sz = (long long)g.nx * g.ny;
-  GRID_STRIDE(t, N) {
-    int i, j, k;
-    interior_ijk(g, t, i, j, k);
-    const long long o = nidx(g, i, j, k);
-    const double n0 = np[o];
-    const double nt1 = 0.5 * (n0 + np[o + sx]);
-    const double nt2 = 0.5 * (n0 + np[o + sy]);
-    const double nt3 = 0.5 * (n0 + np[o + sz]);
-    const double* B1 = b1;
-    const double* B2 = b1 + C;
-    const double* B3 = b1 + 2 * C;
-    const double c1 = (B3[o] - B3[o - sy]) / g.dyc[j] + (B2[o - sz] - B2[o]) / g.dzc[k];
-    const double c2 = (B1[o] - B1[o - sz]) / g.dzc[k] + (B3[o - sx] - B3[o]) / g.dxc[i];
-    const double c3 = (B2[o] - B2[o - sx]) / g.dxc[i] + (B1[o - sy] - B1[o]) / g.dyc[j];
-    aj[o] = c1 / (nt1 * alpha);
-    aj[o + C] = c2 / (nt2 * alpha);
-    aj[o + 2 * C] = c3 / (nt3 * alpha);
-  }
-}
-
-// a = aj - up (gutsf.f:1059, 1261), interior nodes.
-__global__ void k_sub(Geo g, const double* __restrict__ aj, const double* __restrict__ up, double* __restrict__ a) {
-  const long long N = n_interior(g);
-  const long long C = g.C;
-  GRID_STRIDE(t, N) {
-    int i, j, k;
-    interior_ijk(g, t, i, j, k);
-    const long long o = nidx(g, i, j, k);
-    for (int m = 0; m < 3; ++m) a[o + C * m] = aj[o + C * m] - up[o + C * m];
-  }
-}
-
 // Pressure-gradient extension at faces (see oracle grad_pe_at).
 __device__ __forceinline__ double grad_pe_at(const Geo& g, const double* np, double gp, long long o, int i, int j,
                                              int k, int m) {
@@ -161,25 +47,6 @@ __device__ __forceinline__ double grad_pe_at(const Geo& g, const double* np, dou
   return gp * ((np[op] - np[o]) / dg) / nf;
 }
 
-// E = c + nu*aj (gutsf.f:1082, 1282), interior nodes.
-__global__ void k_e_from_c(Geo g, const double* __restrict__ c, const double* __restrict__ nu,
-                           const double* __restrict__ aj, const double* __restrict__ np, double gp,
-                           double* __restrict__ E) {
-  const long long N = n_interior(g);
-  const long long C = g.C;
-  GRID_STRIDE(t, N) {
-    int i, j, k;
-    interior_ijk(g, t, i, j, k);
-    const long long o = nidx(g, i, j, k);
-    const double nuo = nu[o];
-    for (int m = 0; m < 3; ++m) {
-      double e = c[o + C * m] + nuo * aj[o + C * m];
-      if (gp != 0.0) e = e - grad_pe_at(g, np, gp, o, i, j, k, m);
-      E[o + C * m] = e;
-    }
-  }
-}
-
 __global__ void k_grad_pe_face(Geo g, const double* __restrict__ np, double gp, double* __restrict__ gf) {
   const long long N = n_interior(g);
   const long long C = g.C;
@@ -189,35 +56,6 @@ __global__ void k_grad_pe_face(Geo g, const double* __restrict__ np, double gp, 
     const long long o = nidx(g, i, j, k);
     for (int m = 0; m < 3; ++m) gf[o + C * m] = grad_pe_at(g, np, gp, o, i, j, k, m);
   }
-}
-
-// curlE (gutsf.f:288-299) fused with b1p2 = base - coef*curlE
-// (predict_B gutsf.f:1158-1159 with coef = 2*dtsub; correct_B :1349-1350 with
-// coef = dtsub), interior nodes.
-__global__ void k_curlE_update(Geo g, const double* __restrict__ E, const double* __restrict__ base, double coef,
-                               double* __restrict__ b1p2) {
-  const long long N = n_interior(g);
-  const long long C = g.C, sx = 1, sy = g.nx, sz = (long long)g.nx * g.ny;
-  GRID_STRIDE(t, N) {
-    int i, j, k;
-    interior_ijk(g, t, i, j, k);
-    const long long o = nidx(g, i, j, k);
-    const double* E1 = E;
-    const double* E2 = E + C;
-    const double* E3 = E + 2 * C;
-    const double ce1 = (E3[o + sy] - E3[o]) / g.dyg[j] + (E2[o] - E2[o + sz]) / g.dzg[k];
-    const double ce2 = (E3[o] - E3[o + sx]) / g.dxg[i] + (E1[o + sz] - E1[o]) / g.dzg[k];
-    const double ce3 = (E1[o] - E1[o + sy]) / g.dyg[j] + (E2[o + sx] - E2[o]) / g.dxg[i];
-    b1p2[o] = base[o] - coef * ce1;
-    b1p2[o + C] = base[o + C] - coef * ce2;
-    b1p2[o + 2 * C] = base[o + 2 * C] - coef * ce3;
-  }
-}
-
-// btp1 = 0.5*(b1p2 + b1) over all nodes (gutsf.f:1210-1219).
-__global__ void k_half_sum(long long n, const double* __restrict__ a, const double* __restrict__ b,
-                           double* __restrict__ out) {
-  GRID_STRIDE(t, n) out[t] = 0.5 * (a[t] + b[t]);
 }
 
 // Whistler Courant time of check_time_step (gutsf.f:1785-1792) at every node.
@@ -404,29 +242,6 @@ __global__ void k_temperature(Geo g, const double* __restrict__ up2, const doubl
       a = a + d * d;
     }
     temp[o] = (1.0 / 3.0) * 1e6 * mion * sqrt(a);
-  }
-}
-
-// ct = S/np on interior nodes (the reference divides per particle by
-// np(node)*volb, gutsp.f:1704; the node factor is taken out of the sum).
-__global__ void k_ct_from_sums(Geo g, const double* __restrict__ S, const double* __restrict__ np,
-                               double* __restrict__ ct) {
-  const long long N = n_interior(g);
-  const long long C = g.C;
-  GRID_STRIDE(t, N) {
-    int i, j, k;
-    interior_ijk(g, t, i, j, k);
-    const long long o = nidx(g, i, j, k);
-    const double n = np[o];
-    // A node no particle reaches keeps ct = 0, as in the reference (its
-    // sums start at zero and nothing is added).
-    if (n == 0.0) {
-      ct[o] = 0.0; ct[o + C] = 0.0; ct[o + 2 * C] = 0.0;
-      continue;
-    }
-    ct[o] = S[o] / n;
-    ct[o + C] = S[o + C] / n;
-    ct[o + 2 * C] = S[o + 2 * C] / n;
   }
 }
 
@@ -648,37 +463,8 @@ __global__ void k_nonfinite(const double* __restrict__ x, long long n, unsigned 
 
 cudaError_t periodic3(const Geo& g, double* b, cudaStream_t st) { LAUNCH(k_periodic, n_ghost(g), g, b, 3); }
 cudaError_t periodic1(const Geo& g, double* b, cudaStream_t st) { LAUNCH(k_periodic, n_ghost(g), g, b, 1); }
-cudaError_t face_to_center_int(const Geo& g, const double* v, double* vc, cudaStream_t st) {
-  LAUNCH(k_face_to_center, n_interior(g), g, v, vc);
-}
-cudaError_t edge_to_center_int(const Geo& g, const double* bt, double* btc, cudaStream_t st) {
-  LAUNCH(k_edge_to_center, n_interior(g), g, bt, btc);
-}
-cudaError_t face_avg_int(const Geo& g, const double* ct, double* cc, cudaStream_t st) {
-  LAUNCH(k_face_avg, n_interior(g), g, ct, cc);
-}
-cudaError_t cross_int(const Geo& g, const double* aa, const double* btc, double* ct, cudaStream_t st) {
-  LAUNCH(k_cross, n_interior(g), g, aa, btc, ct);
-}
-cudaError_t curlB_int(const Geo& g, const double* b1, const double* np, double* aj, double alpha, cudaStream_t st) {
-  LAUNCH(k_curlB, n_interior(g), g, b1, np, aj, alpha);
-}
-cudaError_t sub_int(const Geo& g, const double* aj, const double* up, double* a, cudaStream_t st) {
-  LAUNCH(k_sub, n_interior(g), g, aj, up, a);
-}
-cudaError_t e_from_c_int(const Geo& g, const double* c, const double* nu, const double* aj, const double* np,
-                         double gp, double* E, cudaStream_t st) {
-  LAUNCH(k_e_from_c, n_interior(g), g, c, nu, aj, np, gp, E);
-}
 cudaError_t grad_pe_face_int(const Geo& g, const double* np, double gp, double* gf, cudaStream_t st) {
   LAUNCH(k_grad_pe_face, n_interior(g), g, np, gp, gf);
-}
-cudaError_t curlE_update_int(const Geo& g, const double* E, const double* base, double coef, double* b1p2,
-                             cudaStream_t st) {
-  LAUNCH(k_curlE_update, n_interior(g), g, E, base, coef, b1p2);
-}
-cudaError_t half_sum_all(const Geo& g, const double* a, const double* b, double* out, cudaStream_t st) {
-  LAUNCH(k_half_sum, 3 * g.C, 3 * g.C, a, b, out);
 }
 cudaError_t deltat_all(const Geo& g, const double* bt, const double* np, double alpha, double dx, double* dtn,
                        cudaStream_t st) {
@@ -714,9 +500,6 @@ cudaError_t scale_interior(const Geo& g, double* f, double a, cudaStream_t st) {
 cudaError_t temperature(const Geo& g, const double* up2, const double* upa, double mion, double* temp,
                         cudaStream_t st) {
   LAUNCH(k_temperature, g.C, g, up2, upa, mion, temp);
-}
-cudaError_t ct_from_sums(const Geo& g, const double* S, const double* np, double* ct, cudaStream_t st) {
-  LAUNCH(k_ct_from_sums, n_interior(g), g, S, np, ct);
 }
 cudaError_t get_Ep(const Geo& g, const PartDev& p, long long N, const double* ajc, const double* upc,
                    const double* btc, const double* gpc, double* Ep, int* err, cudaStream_t st) {

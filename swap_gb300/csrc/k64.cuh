@@ -21,18 +21,32 @@ struct PartDev {  // device mirrors of the particle arrays
 cudaError_t periodic3(const Geo& g, double* b, cudaStream_t st);
 cudaError_t periodic1(const Geo& g, double* b, cudaStream_t st);
 
-// grid_interp.f / gutsf.f operators on the interior nodes
-cudaError_t face_to_center_int(const Geo& g, const double* v, double* vc, cudaStream_t st);
-cudaError_t edge_to_center_int(const Geo& g, const double* bt, double* btc, cudaStream_t st);
-cudaError_t face_avg_int(const Geo& g, const double* ct, double* cc, cudaStream_t st);
-cudaError_t cross_int(const Geo& g, const double* aa, const double* btc, double* ct, cudaStream_t st);
-cudaError_t curlB_int(const Geo& g, const double* b1, const double* np, double* aj, double alpha, cudaStream_t st);
-cudaError_t sub_int(const Geo& g, const double* aj, const double* up, double* a, cudaStream_t st);
-cudaError_t e_from_c_int(const Geo& g, const double* c, const double* nu, const double* aj, const double* np,
-                         double grad_pe, double* E, cudaStream_t st);
-cudaError_t curlE_update_int(const Geo& g, const double* E, const double* base, double coef, double* b1p2,
-                             cudaStream_t st);
-cudaError_t half_sum_all(const Geo& g, const double* a, const double* b, double* out, cudaStream_t st);
+// The field operators (k64_field.cu).  fill: also write the ghost images of
+// the operator's B input, which the caller sees filled.  Every grid output
+// is stored with its ghost images unless noted.
+// curlB: aj at the interior (ghosts untouched); btc (may be null):
+// edge_to_center of b at the interior.
+cudaError_t curlB(const Geo& g, double* b, const double* np, double alpha, double* aj, double* btc, bool fill,
+                  cudaStream_t st);
+// ct = face_to_center(aj - up) x B at the centres, interior.  corr: b holds
+// curlB's btc, averaged to the faces and back; otherwise the edge field.
+cudaError_t cross_ct(const Geo& g, bool corr, const double* aj, const double* up, double* b, double* ct, bool fill,
+                     cudaStream_t st);
+// E = face average of ct + nu*aj (- the electron-pressure gradient).
+cudaError_t e_field(const Geo& g, const double* ct, const double* nu, const double* aj, const double* np, double gp,
+                    double* E, cudaStream_t st);
+// b1p2 = base - coef*curlE (skipped when null); half (may be null) =
+// 0.5*(b1p2 + b1) at the interior.
+cudaError_t b_advance(const Geo& g, const double* E, const double* base, double coef, double* b1p2, const double* b1,
+                      double* half, cudaStream_t st);
+// out = 0.5*(a + b) at the interior.
+cudaError_t half_sum(const Geo& g, const double* a, const double* b, double* out, cudaStream_t st);
+cudaError_t edge_to_center(const Geo& g, double* bt, double* btc, cudaStream_t st);
+// vc of v, and wc of w (null: v alone); the inputs' ghosts are filled.
+cudaError_t face_to_center(const Geo& g, double* v, double* vc, double* w, double* wc, cudaStream_t st);
+// up = face average of S/np (zero where np is zero).
+cudaError_t up_from_sums(const Geo& g, const double* S, const double* np, double* up, cudaStream_t st);
+
 cudaError_t deltat_all(const Geo& g, const double* bt, const double* np, double alpha, double dx, double* dtn,
                        cudaStream_t st);
 cudaError_t grad_pe_face_int(const Geo& g, const double* np, double grad_pe, double* gf, cudaStream_t st);
@@ -58,7 +72,6 @@ cudaError_t fix_to_double(long long n, Fix64 fix, double* out, cudaStream_t st);
 cudaError_t deposit_u(const Geo& g, const PartDev& p, long long N, double beta, int mode, const double* va,
                       const double* vb, double* out_v1, double* S, int* err, cudaStream_t st,
                       Fix64 fix = Fix64{nullptr, nullptr});
-cudaError_t ct_from_sums(const Geo& g, const double* S, const double* np, double* ct, cudaStream_t st);
 // update_rho deposit (folded into the interior), interior scaling, and the
 // temperature of get_temperature from the two face moments.
 cudaError_t deposit_rho(const Geo& g, const PartDev& p, long long N, double beta, double* mnp, int* err,

@@ -1,0 +1,431 @@
+// k64_field.cu -- the FP64 field operators of the drop-in (boundary.f,
+// grid_interp.f, gutsf.f), fused between the points where a stencil needs its
+// neighbours' results.
+//
+// Compiled with --fmad=false: every multiply and add is rounded in the
+// Fortran's order, so each entry's outputs equal the FP64 CPU restatement bit
+// for bit.
+//
+// What bounds them: GB300 retires two FP64 operations per SM and clock (a warp
+// instruction takes 16 clocks), so on grids of 10^5 nodes and more the
+// operators are bound by the FP64 pipe, not by HBM, and on small grids by the
+// number of launches.  Hence
+//  * one kernel per stencil dependency and no more: the periodic fills
+//    (boundary.f:9-52) are not passes of their own.  A kernel reads a ghost
+//    node at its interior image (wrapped index) and stores an output together
+//    with its ghost images.  A subcycle takes 9 launches instead of 44;
+//  * no value is computed twice: the neighbours' curl B, cross product and E
+//    are read back from memory rather than recomputed, because 8 bytes of HBM
+//    traffic cost a tenth of one FP64 operation;
+//  * divisions by a grid spacing are exact quotients from a stored reciprocal
+//    (quotient() below): one or three operations instead of about nine;
+//  * 32-bit index arithmetic (a 64-bit division by the row length is a long
+//    emulated sequence).
+// 128x64x64 nodes, one subcycle through the three entries curlB, predict_B,
+// correct_B: @SUB128@.
+#include "k64.cuh"
+
+namespace swapk {
+namespace {
+
+constexpr int TPB = 256;
+
+inline unsigned nblocks(long long n) {
+  const long long b = (n + TPB - 1) / TPB;
+  return (unsigned)(b < 1 ? 1 : b);
+}
+
+// x / d for a grid spacing d with r = 1/d rounded: exactly the rounded
+// quotient.  P2 (every spacing a power of two): r is exact, and x * r is x / d
+// with the same single rounding.  Otherwise Markstein's correction (P.
+// Markstein, IBM J. Res. Dev. 34, 1990): q = x*r, then q + (x - q*d)*r in
+// fused operations is the rounded quotient when r is the rounded reciprocal
+// and nothing underflows or overflows; x outside 2^-900..2^900 takes the
+// division.  (The host keeps r = 0 for a spacing outside 2^-60..2^60 or with
+// an all-ones significand, the exception of the theorem.)
+template <bool P2>
+__device__ __forceinline__ double quotient(double x, double d, double r) {
+  if (P2) return x * r;
+  const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
+  if (e - 123u > 1800u || r == 0.0) {
+    if (((unsigned)__double2hiint(x) << 1 | (unsigned)__double2loint(x)) == 0u && r != 0.0) return x * r;  // +-0
+    return x / d;
+  }
+  const double q = x * r;
+  return __fma_rn(__fma_rn(-q, d, x), r, q);
+}
+
+// Interior thread t -> node (i,j,k) and its offset.
+struct Node {
+  int i, j, k;
+  unsigned o;
+};
+__device__ __forceinline__ Node node_of(const Geo& g, unsigned t) {
+  const unsigned ix = (unsigned)g.nx - 2, iy = (unsigned)g.ny - 2;
+  const unsigned r = t / ix, r2 = r / iy;
+  Node n;
+  n.i = (int)(t - r * ix) + 2;
+  n.j = (int)(r - r2 * iy) + 2;
+  n.k = (int)r2 + 2;
+  n.o = (unsigned)(n.i - 1) + (unsigned)g.nx * ((unsigned)(n.j - 1) + (unsigned)g.ny * (unsigned)(n.k - 1));
+  return n;
+}
+
+// Offsets from an interior node to its neighbours, at the periodic image
+// where the neighbour is a ghost (boundary.f:21-22).
+struct Nbr {
+  int xm, xp, ym, yp, zm, zp;
+};
+__device__ __forceinline__ Nbr nbr_of(const Geo& g, const Node& n) {
+  const int sy = g.nx, sz = g.nx * g.ny;
+  Nbr b;
+  b.xm = n.i == 2 ? g.nx - 3 : -1;
+  b.xp = n.i == g.nx - 1 ? -(g.nx - 3) : 1;
+  b.ym = n.j == 2 ? (g.ny - 3) * sy : -sy;
+  b.yp = n.j == g.ny - 1 ? -(g.ny - 3) * sy : sy;
+  b.zm = n.k == 2 ? (g.nz - 3) * sz : -sz;
+  b.zp = n.k == g.nz - 1 ? -(g.nz - 3) * sz : sz;
+  return b;
+}
+
+// Whether the node has a ghost image, and the store of a value at every ghost
+// node whose image it is (the periodic fill, boundary.f:9-52).
+__device__ __forceinline__ bool on_edge(const Geo& g, const Node& n) {
+  return n.i == 2 || n.j == 2 || n.k == 2 || n.i == g.nx - 1 || n.j == g.ny - 1 || n.k == g.nz - 1;
+}
+__device__ __noinline__ void store_ghosts(int nx, int ny, int nz, long long C, int ncomp, double* f, int i, int j,
+                                          int k, double v0, double v1, double v2) {
+  for (int c = 0; c < 3; ++c) {
+    const int kk = c == 0 ? k : (c == 1 ? (k == 2 ? nz : 0) : (k == nz - 1 ? 1 : 0));
+    if (kk == 0) continue;
+    for (int b = 0; b < 3; ++b) {
+      const int jj = b == 0 ? j : (b == 1 ? (j == 2 ? ny : 0) : (j == ny - 1 ? 1 : 0));
+      if (jj == 0) continue;
+      for (int a = 0; a < 3; ++a) {
+        const int ii = a == 0 ? i : (a == 1 ? (i == 2 ? nx : 0) : (i == nx - 1 ? 1 : 0));
+        if (ii == 0 || (a == 0 && b == 0 && c == 0)) continue;
+        const long long o = (ii - 1) + (long long)nx * ((jj - 1) + (long long)ny * (kk - 1));
+        f[o] = v0;
+        if (ncomp == 3) {
+          f[o + C] = v1;
+          f[o + 2 * C] = v2;
+        }
+      }
+    }
+  }
+}
+__device__ __forceinline__ void ghosts3(const Geo& g, const Node& n, double* f, double v0, double v1, double v2) {
+  if (on_edge(g, n)) store_ghosts(g.nx, g.ny, g.nz, g.C, 3, f, n.i, n.j, n.k, v0, v1, v2);
+}
+
+// The ghost images of an array that the caller sees filled (its periodic()
+// in the reference) and this operator does not otherwise write.
+__device__ __forceinline__ void fill3(const Geo& g, const Node& n, double* f) {
+  if (on_edge(g, n))
+    store_ghosts(g.nx, g.ny, g.nz, g.C, 3, f, n.i, n.j, n.k, f[n.o], f[n.o + g.C], f[n.o + 2 * g.C]);
+}
+
+// ---- one node of each operator ------------------------------------------------
+
+// curlB (gutsf.f:202-239); the face densities' np is read as it stands (the
+// reference does not fill its ghosts here).
+template <bool P2>
+__device__ __forceinline__ void curlB_node(const Geo& g, const Node& n, const Nbr& d, const double* __restrict__ b,
+                                           const double* __restrict__ np, double alpha, double* __restrict__ aj) {
+  const long long C = g.C;
+  const unsigned o = n.o;
+  const double n0 = np[o];
+  const double nt1 = 0.5 * (n0 + np[o + 1]);
+  const double nt2 = 0.5 * (n0 + np[o + g.nx]);
+  const double nt3 = 0.5 * (n0 + np[o + g.nx * g.ny]);
+  const double *B1 = b, *B2 = b + C, *B3 = b + 2 * C;
+  const double dx = g.dxc[n.i], dy = g.dyc[n.j], dz = g.dzc[n.k];
+  const double rx = g.rdxc[n.i], ry = g.rdyc[n.j], rz = g.rdzc[n.k];
+  const double b1 = B1[o], b2 = B2[o], b3 = B3[o];
+  const double c1 = quotient<P2>(b3 - B3[o + d.ym], dy, ry) + quotient<P2>(B2[o + d.zm] - b2, dz, rz);
+  const double c2 = quotient<P2>(b1 - B1[o + d.zm], dz, rz) + quotient<P2>(B3[o + d.xm] - b3, dx, rx);
+  const double c3 = quotient<P2>(b2 - B2[o + d.xm], dx, rx) + quotient<P2>(B1[o + d.ym] - b1, dy, ry);
+  aj[o] = c1 / (nt1 * alpha);
+  aj[o + C] = c2 / (nt2 * alpha);
+  aj[o + 2 * C] = c3 / (nt3 * alpha);
+}
+
+// edge_to_center (grid_interp.f:22-57).
+__device__ __forceinline__ void e2c_node(const Geo& g, const Node& n, const Nbr& d, const double* __restrict__ bt,
+                                         double out[3]) {
+  const long long C = g.C;
+  const unsigned o = n.o;
+  const double xr = g.xr[n.i], yr = g.yr[n.j], zr = g.zr[n.k];
+  double a, b1, b2;
+  const double* b = bt;  // component 1: y then z
+  a = b[o + d.ym];
+  b2 = a + yr * (b[o] - a);
+  a = b[o + d.ym + d.zm];
+  b1 = a + yr * (b[o + d.zm] - a);
+  out[0] = b1 + zr * (b2 - b1);
+  b = bt + C;  // component 2: x then z
+  a = b[o + d.xm];
+  b2 = a + xr * (b[o] - a);
+  a = b[o + d.xm + d.zm];
+  b1 = a + xr * (b[o + d.zm] - a);
+  out[1] = b1 + zr * (b2 - b1);
+  b = bt + 2 * C;  // component 3: y then x
+  a = b[o + d.ym];
+  b2 = a + yr * (b[o] - a);
+  a = b[o + d.xm + d.ym];
+  b1 = a + yr * (b[o + d.xm] - a);
+  out[2] = b1 + xr * (b2 - b1);
+}
+
+// face_to_center (grid_interp.f:150-171) from a value and its lower neighbour.
+__device__ __forceinline__ double f2c(double r, double v, double vm) { return r * (v - vm) + vm; }
+
+// face_to_center(aj - up), B at the centres and the cross product of crossf2
+// (gutsf.f:1059-1075, 65-76).  Predictor (CORR false): b is the edge field,
+// taken to the centre here.  Corrector: b holds edge_to_center of it, taken
+// to the faces (grid_interp.f:123-125) and back to the centres
+// (gutsf.f:1268-1269).
+template <bool CORR>
+__device__ __forceinline__ void ct_node(const Geo& g, const Node& n, const Nbr& d, const double* __restrict__ aj,
+                                        const double* __restrict__ up, const double* __restrict__ b,
+                                        double* __restrict__ ct) {
+  const long long C = g.C;
+  const unsigned o = n.o;
+  const double xr = g.xr[n.i], yr = g.yr[n.j], zr = g.zr[n.k];
+  const double ax = f2c(xr, aj[o] - up[o], aj[o + d.xm] - up[o + d.xm]);
+  const double ay = f2c(yr, aj[o + C] - up[o + C], aj[o + C + d.ym] - up[o + C + d.ym]);
+  const double az = f2c(zr, aj[o + 2 * C] - up[o + 2 * C], aj[o + 2 * C + d.zm] - up[o + 2 * C + d.zm]);
+  double B[3];
+  if (!CORR) {
+    e2c_node(g, n, d, b, B);
+  } else {
+    const double x0 = b[o], y0 = b[o + C], z0 = b[o + 2 * C];
+    B[0] = f2c(xr, 0.5 * (x0 + b[o + d.xp]), 0.5 * (b[o + d.xm] + x0));
+    B[1] = f2c(yr, 0.5 * (y0 + b[o + C + d.yp]), 0.5 * (b[o + C + d.ym] + y0));
+    B[2] = f2c(zr, 0.5 * (z0 + b[o + 2 * C + d.zp]), 0.5 * (b[o + 2 * C + d.zm] + z0));
+  }
+  ct[o] = ay * B[2] - az * B[1];
+  ct[o + C] = az * B[0] - ax * B[2];
+  ct[o + 2 * C] = ax * B[1] - ay * B[0];
+}
+
+// Pressure-gradient extension at the face of component m (see the CPU
+// restatement's grad_pe_at); np's ghosts as they stand.
+__device__ __forceinline__ double grad_pe_at(const Geo& g, const double* np, double gp, const Node& n, int m) {
+  const unsigned o = n.o;
+  const unsigned op = o + (m == 0 ? 1u : (m == 1 ? (unsigned)g.nx : (unsigned)(g.nx * g.ny)));
+  const double dg = m == 0 ? g.dxg[n.i] : (m == 1 ? g.dyg[n.j] : g.dzg[n.k]);
+  const double nf = 0.5 * (np[o] + np[op]);
+  return gp * ((np[op] - np[o]) / dg) / nf;
+}
+
+// crossf2's face average (gutsf.f:94-96) and E = c + nu*aj (gutsf.f:1082,
+// 1282), with E's ghost images.
+__device__ __forceinline__ void e_node(const Geo& g, const Node& n, const Nbr& d, const double* __restrict__ ct,
+                                       const double* __restrict__ nu, const double* __restrict__ aj,
+                                       const double* __restrict__ np, double gp, double* __restrict__ E) {
+  const long long C = g.C;
+  const unsigned o = n.o;
+  const double nuo = nu[o];
+  double e[3];
+  e[0] = 0.5 * (ct[o] + ct[o + d.xp]) + nuo * aj[o];
+  e[1] = 0.5 * (ct[o + C] + ct[o + C + d.yp]) + nuo * aj[o + C];
+  e[2] = 0.5 * (ct[o + 2 * C] + ct[o + 2 * C + d.zp]) + nuo * aj[o + 2 * C];
+  if (gp != 0.0)
+    for (int m = 0; m < 3; ++m) e[m] = e[m] - grad_pe_at(g, np, gp, n, m);
+  E[o] = e[0];
+  E[o + C] = e[1];
+  E[o + 2 * C] = e[2];
+  ghosts3(g, n, E, e[0], e[1], e[2]);
+}
+
+// curlE (gutsf.f:288-299) and b1p2 = base - coef*curlE (predict_B
+// gutsf.f:1158-1159 with coef = 2*dtsub; correct_B :1349-1350 with coef =
+// dtsub), with b1p2's ghost images.  half: also the B at m+1/2 of get_Ep1
+// (gutsf.f:1210-1219), 0.5*(b1p2 + b1), at the interior nodes.
+template <bool P2>
+__device__ __forceinline__ void b_node(const Geo& g, const Node& n, const Nbr& d, const double* __restrict__ E,
+                                       const double* __restrict__ base, double coef, double* __restrict__ b1p2,
+                                       const double* __restrict__ b1, double* __restrict__ half) {
+  const long long C = g.C;
+  const unsigned o = n.o;
+  const double *E1 = E, *E2 = E + C, *E3 = E + 2 * C;
+  const double dx = g.dxg[n.i], dy = g.dyg[n.j], dz = g.dzg[n.k];
+  const double rx = g.rdxg[n.i], ry = g.rdyg[n.j], rz = g.rdzg[n.k];
+  const double e1 = E1[o], e2 = E2[o], e3 = E3[o];
+  const double ce1 = quotient<P2>(E3[o + d.yp] - e3, dy, ry) + quotient<P2>(e2 - E2[o + d.zp], dz, rz);
+  const double ce2 = quotient<P2>(e3 - E3[o + d.xp], dx, rx) + quotient<P2>(E1[o + d.zp] - e1, dz, rz);
+  const double ce3 = quotient<P2>(e1 - E1[o + d.yp], dy, ry) + quotient<P2>(E2[o + d.xp] - e2, dx, rx);
+  const double v0 = base[o] - coef * ce1;
+  const double v1 = base[o + C] - coef * ce2;
+  const double v2 = base[o + 2 * C] - coef * ce3;
+  if (b1p2) {
+    b1p2[o] = v0;
+    b1p2[o + C] = v1;
+    b1p2[o + 2 * C] = v2;
+    ghosts3(g, n, b1p2, v0, v1, v2);
+  }
+  if (half) {
+    half[o] = 0.5 * (v0 + b1[o]);
+    half[o + C] = 0.5 * (v1 + b1[o + C]);
+    half[o + 2 * C] = 0.5 * (v2 + b1[o + 2 * C]);
+  }
+}
+
+// ---- kernels --------------------------------------------------------------------
+
+#define NODES(n, d)                                                     \
+  const unsigned t_ = blockIdx.x * blockDim.x + threadIdx.x;            \
+  if (t_ >= (unsigned)n_interior(g)) return;                            \
+  const Node n = node_of(g, t_);                                        \
+  const Nbr d = nbr_of(g, n)
+
+// curlB; FILL: b's ghosts too (curlB begins with periodic(b)).  btc (not
+// null): edge_to_center of b at the interior nodes, for the corrector.
+template <bool P2>
+__global__ void __launch_bounds__(TPB) k_curlB(Geo g, double* b, const double* __restrict__ np, double alpha,
+                                               double* __restrict__ aj, double* __restrict__ btc, bool fill) {
+  NODES(n, d);
+  curlB_node<P2>(g, n, d, b, np, alpha, aj);
+  if (btc) {
+    double c[3];
+    e2c_node(g, n, d, b, c);
+    btc[n.o] = c[0];
+    btc[n.o + g.C] = c[1];
+    btc[n.o + 2 * g.C] = c[2];
+  }
+  if (fill) fill3(g, n, b);
+}
+
+template <bool CORR>
+__global__ void __launch_bounds__(TPB) k_ct(Geo g, const double* __restrict__ aj, const double* __restrict__ up,
+                                            double* b, double* __restrict__ ct, bool fill) {
+  NODES(n, d);
+  ct_node<CORR>(g, n, d, aj, up, b, ct);
+  if (fill) fill3(g, n, b);
+}
+
+__global__ void __launch_bounds__(TPB) k_E(Geo g, const double* __restrict__ ct, const double* __restrict__ nu,
+                                           const double* __restrict__ aj, const double* __restrict__ np, double gp,
+                                           double* __restrict__ E) {
+  NODES(n, d);
+  e_node(g, n, d, ct, nu, aj, np, gp, E);
+}
+
+template <bool P2>
+__global__ void __launch_bounds__(TPB) k_B(Geo g, const double* __restrict__ E, const double* __restrict__ base,
+                                           double coef, double* __restrict__ b1p2, const double* __restrict__ b1,
+                                           double* __restrict__ half) {
+  NODES(n, d);
+  b_node<P2>(g, n, d, E, base, coef, b1p2, b1, half);
+}
+
+// 0.5*(a + b) at the interior nodes (gutsf.f:1210-1219); the consumers read
+// ghosts at their images.
+__global__ void __launch_bounds__(TPB) k_half(Geo g, const double* __restrict__ a, const double* __restrict__ b,
+                                              double* __restrict__ out) {
+  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (unsigned)n_interior(g)) return;
+  const unsigned o = node_of(g, t).o;
+  for (int m = 0; m < 3; ++m) out[o + g.C * m] = 0.5 * (a[o + g.C * m] + b[o + g.C * m]);
+}
+
+// edge_to_center (grid_interp.f:10-62): bt's and btc's ghosts too.
+__global__ void __launch_bounds__(TPB) k_edge_to_center(Geo g, double* bt, double* __restrict__ btc) {
+  NODES(n, d);
+  double c[3];
+  e2c_node(g, n, d, bt, c);
+  btc[n.o] = c[0];
+  btc[n.o + g.C] = c[1];
+  btc[n.o + 2 * g.C] = c[2];
+  ghosts3(g, n, btc, c[0], c[1], c[2]);
+  fill3(g, n, bt);
+}
+
+// face_to_center (grid_interp.f:136-176) of v, and of w when given: the
+// ghosts of inputs and outputs too.
+__global__ void __launch_bounds__(TPB) k_face_to_center(Geo g, double* v, double* __restrict__ vc, double* w,
+                                                        double* __restrict__ wc) {
+  NODES(n, d);
+  const long long C = g.C;
+  const unsigned o = n.o;
+  const double xr = g.xr[n.i], yr = g.yr[n.j], zr = g.zr[n.k];
+  for (int q = 0; q < 2; ++q) {
+    double *in = q ? w : v, *out = q ? wc : vc;
+    if (!in) break;
+    const double c0 = f2c(xr, in[o], in[o + d.xm]);
+    const double c1 = f2c(yr, in[o + C], in[o + C + d.ym]);
+    const double c2 = f2c(zr, in[o + 2 * C], in[o + 2 * C + d.zm]);
+    out[o] = c0;
+    out[o + C] = c1;
+    out[o + 2 * C] = c2;
+    ghosts3(g, n, out, c0, c1, c2);
+    fill3(g, n, in);
+  }
+}
+
+// The end of update_up (gutsp.f:1825-1839): ct = S/np at the interior (zero
+// where no particle deposits, as in the reference) and its face average, with
+// up's ghosts.
+__device__ __forceinline__ double ct_at(const double* __restrict__ S, const double* __restrict__ np, unsigned o,
+                                        long long cm) {
+  const double n = np[o];
+  return n == 0.0 ? 0.0 : S[o + cm] / n;
+}
+__global__ void __launch_bounds__(TPB) k_up(Geo g, const double* __restrict__ S, const double* __restrict__ np,
+                                            double* __restrict__ up) {
+  NODES(n, d);
+  const long long C = g.C;
+  const unsigned o = n.o;
+  const double u0 = 0.5 * (ct_at(S, np, o, 0) + ct_at(S, np, o + d.xp, 0));
+  const double u1 = 0.5 * (ct_at(S, np, o, C) + ct_at(S, np, o + d.yp, C));
+  const double u2 = 0.5 * (ct_at(S, np, o, 2 * C) + ct_at(S, np, o + d.zp, 2 * C));
+  up[o] = u0;
+  up[o + C] = u1;
+  up[o + 2 * C] = u2;
+  ghosts3(g, n, up, u0, u1, u2);
+}
+
+}  // namespace
+
+// ---- launchers --------------------------------------------------------------------
+
+#define FL(kern, ...)                                                 \
+  do {                                                                \
+    kern<<<nblocks(n_interior(g)), TPB, 0, st>>>(__VA_ARGS__);        \
+    return cudaGetLastError();                                        \
+  } while (0)
+
+cudaError_t curlB(const Geo& g, double* b, const double* np, double alpha, double* aj, double* btc, bool fill,
+                  cudaStream_t st) {
+  if (g.spacing_p2) FL(k_curlB<true>, g, b, np, alpha, aj, btc, fill);
+  FL(k_curlB<false>, g, b, np, alpha, aj, btc, fill);
+}
+cudaError_t cross_ct(const Geo& g, bool corr, const double* aj, const double* up, double* b, double* ct, bool fill,
+                     cudaStream_t st) {
+  if (corr) FL(k_ct<true>, g, aj, up, b, ct, fill);
+  FL(k_ct<false>, g, aj, up, b, ct, fill);
+}
+cudaError_t e_field(const Geo& g, const double* ct, const double* nu, const double* aj, const double* np, double gp,
+                    double* E, cudaStream_t st) {
+  FL(k_E, g, ct, nu, aj, np, gp, E);
+}
+cudaError_t b_advance(const Geo& g, const double* E, const double* base, double coef, double* b1p2, const double* b1,
+                      double* half, cudaStream_t st) {
+  if (g.spacing_p2) FL(k_B<true>, g, E, base, coef, b1p2, b1, half);
+  FL(k_B<false>, g, E, base, coef, b1p2, b1, half);
+}
+cudaError_t half_sum(const Geo& g, const double* a, const double* b, double* out, cudaStream_t st) {
+  FL(k_half, g, a, b, out);
+}
+cudaError_t edge_to_center(const Geo& g, double* bt, double* btc, cudaStream_t st) {
+  FL(k_edge_to_center, g, bt, btc);
+}
+cudaError_t face_to_center(const Geo& g, double* v, double* vc, double* w, double* wc, cudaStream_t st) {
+  FL(k_face_to_center, g, v, vc, w, wc);
+}
+cudaError_t up_from_sums(const Geo& g, const double* S, const double* np, double* up, cudaStream_t st) {
+  FL(k_up, g, S, np, up);
+}
+
+}  // namespace swapk

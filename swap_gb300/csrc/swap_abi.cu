@@ -1,6 +1,7 @@
 // swap_abi.cu -- the extern "C" drop-in (include/swap_gpu.h): context,
 // registry of the caller's host arrays with device mirrors, and one entry per
 // reference subroutine built from the FP64 kernels in k64.cu.
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <string>
@@ -246,84 +247,83 @@ int periodic(swap_ctx* c, double* b) {
 
 // face_to_center (grid_interp.f:136-176)
 int face_to_center(swap_ctx* c, double* v, double* vc) {
-  KL("periodic", periodic3(c->g, v, c->st));
-  KL("face_to_center_int", face_to_center_int(c->g, v, vc, c->st));
-  KL("periodic", periodic3(c->g, vc, c->st));
+  KL("face_to_center", swapk::face_to_center(c->g, v, vc, nullptr, nullptr, c->st));
   return 0;
 }
 
 // edge_to_center (grid_interp.f:10-62)
 int edge_to_center(swap_ctx* c, double* bt, double* btc) {
-  KL("periodic", periodic3(c->g, bt, c->st));
-  KL("edge_to_center_int", edge_to_center_int(c->g, bt, btc, c->st));
-  KL("periodic", periodic3(c->g, btc, c->st));
-  return 0;
-}
-
-// edge_to_face (grid_interp.f:67-130): interior faces; ghosts of btmf are
-// left for the consumer's periodic() (face_to_center) as in the reference.
-int edge_to_face(swap_ctx* c, double* bt, double* btmf) {
-  KL("periodic", periodic3(c->g, bt, c->st));
-  KL("edge_to_center_int", edge_to_center_int(c->g, bt, c->s_btc2, c->st));
-  KL("periodic", periodic3(c->g, c->s_btc2, c->st));
-  KL("face_avg_int", face_avg_int(c->g, c->s_btc2, btmf, c->st));
-  return 0;
-}
-
-// crossf2 (gutsf.f:40-104); aa and btc arrive periodic from their producers.
-int crossf2(swap_ctx* c, double* aa, double* btc, double* cc) {
-  KL("cross_int", cross_int(c->g, aa, btc, c->s_ct, c->st));
-  KL("periodic", periodic3(c->g, c->s_ct, c->st));
-  KL("face_avg_int", face_avg_int(c->g, c->s_ct, cc, c->st));
-  KL("periodic", periodic3(c->g, cc, c->st));
+  KL("edge_to_center", swapk::edge_to_center(c->g, bt, btc, c->st));
   return 0;
 }
 
 // curlB (gutsf.f:178-244)
 int curlB(swap_ctx* c, double* bt, const double* np, double* aj) {
-  KL("periodic", periodic3(c->g, bt, c->st));
-  KL("curlB_int", curlB_int(c->g, bt, np, aj, c->prm.alpha, c->st));
-  return 0;
-}
-
-// E = crossf2(face_to_center(aj-up), btc) + nu*aj; periodic(E)
-int e_tail(swap_ctx* c, double* E, const double* aj, const double* np, const double* nu) {
-  TRY(crossf2(c, c->s_aa, c->s_btcl, c->s_c));
-  KL("e_from_c_int", e_from_c_int(c->g, c->s_c, nu, aj, np, c->prm.grad_pe, E, c->st));
-  KL("periodic", periodic3(c->g, E, c->st));
+  KL("curlB", swapk::curlB(c->g, bt, np, c->prm.alpha, aj, nullptr, true, c->st));
   return 0;
 }
 
 // get_E (gutsf.f:994-1110)
-int get_E(swap_ctx* c, double* E, double* bt, double* aj, const double* up, const double* np, const double* nu) {
-  KL("sub_int", sub_int(c->g, aj, up, c->s_a, c->st));
-  TRY(face_to_center(c, c->s_a, c->s_aa));
-  TRY(edge_to_center(c, bt, c->s_btcl));
-  return e_tail(c, E, aj, np, nu);
+int get_E(swap_ctx* c, double* E, double* bt, const double* aj, const double* up, const double* np,
+          const double* nu) {
+  KL("cross_ct", cross_ct(c->g, false, aj, up, bt, c->s_ct, true, c->st));
+  KL("e_field", e_field(c->g, c->s_ct, nu, aj, np, c->prm.grad_pe, E, c->st));
+  return 0;
 }
 
 // predict_B (gutsf.f:1115-1169)
 int predict_B(swap_ctx* c, double* b12, double* b1p2, double* bt, double* E, double* aj, double* up, double* np,
               double* nu, double dtsub) {
   TRY(get_E(c, E, bt, aj, up, np, nu));
-  KL("curlE_update_int", curlE_update_int(c->g, E, b12, 2.0 * dtsub, b1p2, c->st));
-  KL("periodic", periodic3(c->g, b1p2, c->st));
+  KL("b_advance", b_advance(c->g, E, b12, 2.0 * dtsub, b1p2, nullptr, nullptr, c->st));
   return 0;
 }
 
-// get_Ep1 (gutsf.f:1174-1304) + correct_B (gutsf.f:1309-1359)
+// get_Ep1 (gutsf.f:1174-1304) + correct_B (gutsf.f:1309-1359) from B at
+// m+1/2 (s_btp1, interior): writes aj, E and out.
+static int correct_from_half(swap_ctx* c, const double* b1, double* out, double* E, double* aj, const double* up,
+                             const double* np, const double* nu, double dtsub) {
+  KL("curlB", swapk::curlB(c->g, c->s_btp1, np, c->prm.alpha, aj, c->s_btc2, false, c->st));
+  KL("cross_ct", cross_ct(c->g, true, aj, up, c->s_btc2, c->s_ct, false, c->st));
+  KL("e_field", e_field(c->g, c->s_ct, nu, aj, np, c->prm.grad_pe, E, c->st));
+  KL("b_advance", b_advance(c->g, E, b1, dtsub, out, nullptr, nullptr, c->st));
+  return 0;
+}
+
 int correct_B(swap_ctx* c, double* b1, double* b1p2, double* E, double* aj, double* up, double* np, double* nu,
               double dtsub) {
-  double* btp1 = c->s_btp1;
-  KL("half_sum_all", half_sum_all(c->g, b1p2, b1, btp1, c->st));
-  TRY(curlB(c, btp1, np, aj));
-  KL("sub_int", sub_int(c->g, aj, up, c->s_a, c->st));
-  TRY(face_to_center(c, c->s_a, c->s_aa));
-  TRY(edge_to_face(c, btp1, c->s_btmf));
-  TRY(face_to_center(c, c->s_btmf, c->s_btcl));
-  TRY(e_tail(c, E, aj, np, nu));
-  KL("curlE_update_int", curlE_update_int(c->g, E, b1, dtsub, b1p2, c->st));
-  KL("periodic", periodic3(c->g, b1p2, c->st));
+  KL("half_sum", half_sum(c->g, b1p2, b1, c->s_btp1, c->st));
+  return correct_from_half(c, b1, b1p2, E, aj, up, np, nu, dtsub);
+}
+
+// n subcycles (maind.f:425-476) on arrays that stay on the device.  The same
+// values as n rounds of curlB, predict_B, correct_B, f_update_tlev; the
+// predicted B is only ever used at m+1/2, so it is stored there alone, and
+// the time levels change places instead of being copied: b12's memory takes
+// the new B, which becomes b1.  From the second subcycle on bt is b1.
+int subcycle_loop(swap_ctx* c, int n, double* b1, double* b12, double* b1p2, double* bt, double* E, double* aj,
+                  const double* up, const double* np, const double* nu, double dtsub) {
+  if (n <= 0) return 0;
+  double *now = b1, *old = b12;
+  for (int s = 0; s < n; ++s) {
+    double* b = s == 0 ? bt : now;
+    KL("curlB", swapk::curlB(c->g, b, np, c->prm.alpha, aj, nullptr, s == 0, c->st));
+    KL("cross_ct", cross_ct(c->g, false, aj, up, b, c->s_ct, false, c->st));
+    KL("e_field", e_field(c->g, c->s_ct, nu, aj, np, c->prm.grad_pe, E, c->st));
+    KL("b_advance", b_advance(c->g, E, old, 2.0 * dtsub, nullptr, now, c->s_btp1, c->st));
+    TRY(correct_from_half(c, now, old, E, aj, up, np, nu, dtsub));
+    std::swap(now, old);
+  }
+  const std::size_t bytes = 3 * (std::size_t)c->g.C * sizeof(double);
+  auto copy = [&](double* d, const double* from) {
+    return cudaMemcpyAsync(d, from, bytes, cudaMemcpyDeviceToDevice, c->st);
+  };
+  KL("cudaMemcpyAsync", copy(b1p2, now));
+  KL("cudaMemcpyAsync", copy(bt, now));
+  if (now != b1) {  // an odd count: the levels sit in each other's memory
+    KL("cudaMemcpyAsync", copy(b12, b1));
+    KL("cudaMemcpyAsync", copy(b1, b1p2));
+  }
   return 0;
 }
 
@@ -432,18 +432,14 @@ int update_up_mode(swap_ctx* c, int mode, const double* va, const double* vb, do
        deposit_u(c->g, c->part_view(), c->ntot(), c->prm.beta, mode, va, vb, out_v1, c->s_S, c->d_err, c->st));
   }
   if (c->fused) TRY(c->exchange(c->s_S, 3 * c->g.C, 8));  // MPI_ALLREDUCE, gutsp.f:1812-1822
-  KL("ct_from_sums", ct_from_sums(c->g, c->s_S, np, c->s_ct, c->st));
-  KL("periodic", periodic3(c->g, c->s_ct, c->st));
-  KL("face_avg_int", face_avg_int(c->g, c->s_ct, up, c->st));
-  KL("periodic", periodic3(c->g, up, c->st));
+  KL("up_from_sums", up_from_sums(c->g, c->s_S, np, up, c->st));
   return 0;
 }
 
 // get_Ep (gutsp.f:155-276)
 int get_Ep(swap_ctx* c, double* Ep, double* aj, const double* np, double* up, const double* btc) {
   TRY(need_weights(c));
-  TRY(face_to_center(c, aj, c->s_ajc));
-  TRY(face_to_center(c, up, c->s_upc));
+  KL("face_to_center", swapk::face_to_center(c->g, aj, c->s_ajc, up, c->s_upc, c->st));
   const double* gpc = nullptr;
   if (c->prm.grad_pe != 0.0) {
     KL("grad_pe_face_int", grad_pe_face_int(c->g, np, c->prm.grad_pe, c->s_gf, c->st));
@@ -535,7 +531,31 @@ extern "C" int swap_init(swap_ctx** out, const swap_dims* d, const swap_params* 
       return SWAP_ECUDA;
     }
   }
+  // reciprocals of the spacings (k64_field.cu quotient), 1-based like them
+  const double* rec[6];
+  bool p2 = true;
+  for (int a = 0; a < 6; ++a) {
+    const int n = ns[3 + a];
+    std::vector<double> h((std::size_t)n + 1, 0.0);
+    for (int q = 1; q <= n; ++q) {
+      const double v = arrs[3 + a][q - 1];
+      int e = 0;
+      const double m = std::frexp(v, &e);  // in [0.5, 1) for a normal positive v
+      const bool fits = v > 0.0 && std::isfinite(v) && e > -60 && e < 60;
+      if (fits && m != 1.0 - 0x1p-53) h[(std::size_t)q] = 1.0 / v;
+      if (q >= 2 && q <= n - 1) p2 = p2 && fits && m == 0.5;  // the stencils' nodes
+    }
+    double* r = c->dalloc(h.size());
+    if (!r || cudaMemcpy(r, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess) {
+      swap_finalize(c);
+      return SWAP_ECUDA;
+    }
+    rec[a] = r;
+  }
   Geo& g = c->g;
+  g.rdxg = rec[0]; g.rdyg = rec[1]; g.rdzg = rec[2];
+  g.rdxc = rec[3]; g.rdyc = rec[4]; g.rdzc = rec[5];
+  g.spacing_p2 = p2;
   g.nx = d->nx; g.ny = d->ny; g.nz = d->nz;
   g.C = (long long)d->nx * d->ny * d->nz;
   g.qx = dg[0]; g.qy = dg[1]; g.qz = dg[2];
@@ -550,8 +570,8 @@ extern "C" int swap_init(swap_ctx** out, const swap_dims* d, const swap_params* 
   c->h_qz.assign(co->qz, co->qz + d->nz);
   // grid scratch (the reference's /dummy/ a, c, ct and subroutine locals)
   const std::size_t C3 = 3 * (std::size_t)g.C;
-  double** bufs[] = {&c->s_a, &c->s_aa, &c->s_c, &c->s_ct, &c->s_btcl, &c->s_btc2, &c->s_btmf, &c->s_ajc,
-                     &c->s_upc, &c->s_btp1, &c->s_S, &c->s_gf, &c->s_gpc};
+  double** bufs[] = {&c->s_ct, &c->s_btc2, &c->s_btmf, &c->s_ajc, &c->s_upc, &c->s_btp1, &c->s_S, &c->s_gf,
+                     &c->s_gpc};
   for (double** b : bufs) {
     *b = c->dalloc(C3);
     if (!*b || cudaMemset(*b, 0, C3 * sizeof(double)) != cudaSuccess) {
@@ -1090,14 +1110,7 @@ int subcycles(swap_ctx* c, Bound& b) {
   TRY(ops::check_time_step(c, b.bt, b.np, &dtsub, &ntf));  // :423
   c->last_dtsub = dtsub;
   c->last_ntf = ntf;
-  const int n = (int)ntf;
-  for (int s = 0; s < n; ++s) {  // :425-476
-    TRY(ops::curlB(c, b.bt, b.np, b.aj));
-    TRY(ops::predict_B(c, b.b12, b.b1p2, b.bt, b.E, b.aj, b.up, b.np, b.nu, dtsub));
-    TRY(ops::correct_B(c, b.b1, b.b1p2, b.E, b.aj, b.up, b.np, b.nu, dtsub));
-    TRY(ops::f_update_tlev(c, b.b1, b.b12, b.b1p2, b.bt));
-  }
-  return SWAP_OK;
+  return ops::subcycle_loop(c, (int)ntf, b.b1, b.b12, b.b1p2, b.bt, b.E, b.aj, b.up, b.np, b.nu, dtsub);  // :425-476
 }
 
 // maind.f:479 and the sinks after it (res_chex, maind.f:484).

@@ -87,7 +87,7 @@ struct swap_ctx {
   long long weights_n = 0;
 
   // grid scratch: /dummy/ a, c, ct and subroutine locals
-  double *s_a = nullptr, *s_aa = nullptr, *s_c = nullptr, *s_ct = nullptr, *s_btcl = nullptr, *s_btc2 = nullptr;
+  double *s_ct = nullptr, *s_btc2 = nullptr;
   double *s_btmf = nullptr, *s_ajc = nullptr, *s_upc = nullptr, *s_btp1 = nullptr, *s_S = nullptr;
   double *s_gf = nullptr, *s_gpc = nullptr, *s_dtn = nullptr, *s_red = nullptr;
   // particle work arrays of the fused step (maind.f locals Ep, vplus, vminus)

@@ -19,6 +19,10 @@ struct Geo {
   const double *dxg, *dyg, *dzg;  // dx_grid ...
   const double *dxc, *dyc, *dzc;  // dx_cell ...
   const double *xr, *yr, *zr;     // xrat ...
+  // 1/spacing, rounded (0: divide instead); spacing_p2: every interior
+  // spacing is a power of two, its reciprocal exact (k64_field.cu quotient)
+  const double *rdxg, *rdyg, *rdzg, *rdxc, *rdyc, *rdzc;
+  bool spacing_p2;
   double dy;                      // module dy (gutsp.f:1404)
   double inv_dx, inv_dz;          // guesses for the cell search only
 };
