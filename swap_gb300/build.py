@@ -28,6 +28,7 @@ NVCC_COMMON = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O2
 UNITS = [
     ("k64.cu", ["--fmad=false"]),
     ("k64_field.cu", ["--fmad=false"]),
+    ("k64_pass.cu", ["--fmad=false"]),
     ("k32.cu", []),
     ("swap_abi.cu", []),
     ("swap_f32.cu", []),

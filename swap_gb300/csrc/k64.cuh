@@ -44,8 +44,12 @@ cudaError_t half_sum(const Geo& g, const double* a, const double* b, double* out
 cudaError_t edge_to_center(const Geo& g, double* bt, double* btc, cudaStream_t st);
 // vc of v, and wc of w (null: v alone); the inputs' ghosts are filled.
 cudaError_t face_to_center(const Geo& g, double* v, double* vc, double* w, double* wc, cudaStream_t st);
-// up = face average of S/np (zero where np is zero).
-cudaError_t up_from_sums(const Geo& g, const double* S, const double* np, double* up, cudaStream_t st);
+// up = face average of S/np (zero where np is zero); fill_np: np's ghosts too.
+cudaError_t up_from_sums(const Geo& g, const double* S, double* np, double* up, bool fill_np, cudaStream_t st);
+// The particle passes' gather table, [C][6]: face_to_center(aj - up) and, when
+// full, edge_to_center(bt), with btc and aj's ghosts.
+cudaError_t gather_kit(const Geo& g, bool full, double* aj, const double* up, const double* bt, double* btc,
+                       double* kit, cudaStream_t st);
 
 cudaError_t deltat_all(const Geo& g, const double* bt, const double* np, double alpha, double dx, double* dtn,
                        cudaStream_t st);
@@ -90,6 +94,21 @@ cudaError_t vp_final(const PartDev& p, long long N, double dt, const double* Ep,
 // move by the caller).
 cudaError_t move_half(const Geo& g, const PartDev& p, long long N, double dt, double* xp, const double* vp,
                       bool x_open, cudaStream_t st);
+
+// The particle half of a fused step in three passes (k64_pass.cu).
+struct PassArgs {
+  Geo g;
+  PartDev p;
+  long long N;
+  double dt, beta;
+  const double* kit;  // gather_kit's table
+  double* b3;         // (ni_max,3): B at each particle, pass 2 to pass 3
+  double *np, *S;     // raw deposit sums (zeroed by the caller); pass 2: S alone
+  int* err;
+  bool x_open;      // pass 3: the x axis does not wrap, and an ion outside deposits nothing
+  bool final_move;  // pass 3: also the half move of maind.f:479
+};
+cudaError_t particle_pass(int pass, const PassArgs& a, cudaStream_t st);
 
 // reductions (FP64)
 cudaError_t reduce_min(const double* x, long long n, double* d_partial, int nblk, cudaStream_t st);

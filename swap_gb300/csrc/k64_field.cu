@@ -18,12 +18,14 @@
 //    are read back from memory rather than recomputed, because 8 bytes of HBM
 //    traffic cost a tenth of one FP64 operation;
 //  * divisions by a grid spacing are exact quotients from a stored reciprocal
-//    (quotient() below): one or three operations instead of about nine;
+//    (quotient(), k64_dev.cuh): one or three operations instead of about nine;
 //  * 32-bit index arithmetic (a 64-bit division by the row length is a long
 //    emulated sequence).
 // 128x64x64 nodes, one subcycle through the three entries curlB, predict_B,
-// correct_B: @SUB128@.
+// correct_B: 1.04 -> 0.72 ms, of which on the
+// device 0.74 -> 0.36 ms (18x11x14: 0.355 -> 0.211 ms).
 #include "k64.cuh"
+#include "k64_dev.cuh"
 
 namespace swapk {
 namespace {
@@ -33,26 +35,6 @@ constexpr int TPB = 256;
 inline unsigned nblocks(long long n) {
   const long long b = (n + TPB - 1) / TPB;
   return (unsigned)(b < 1 ? 1 : b);
-}
-
-// x / d for a grid spacing d with r = 1/d rounded: exactly the rounded
-// quotient.  P2 (every spacing a power of two): r is exact, and x * r is x / d
-// with the same single rounding.  Otherwise Markstein's correction (P.
-// Markstein, IBM J. Res. Dev. 34, 1990): q = x*r, then q + (x - q*d)*r in
-// fused operations is the rounded quotient when r is the rounded reciprocal
-// and nothing underflows or overflows; x outside 2^-900..2^900 takes the
-// division.  (The host keeps r = 0 for a spacing outside 2^-60..2^60 or with
-// an all-ones significand, the exception of the theorem.)
-template <bool P2>
-__device__ __forceinline__ double quotient(double x, double d, double r) {
-  if (P2) return x * r;
-  const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
-  if (e - 123u > 1800u || r == 0.0) {
-    if (((unsigned)__double2hiint(x) << 1 | (unsigned)__double2loint(x)) == 0u && r != 0.0) return x * r;  // +-0
-    return x / d;
-  }
-  const double q = x * r;
-  return __fma_rn(__fma_rn(-q, d, x), r, q);
 }
 
 // Interior thread t -> node (i,j,k) and its offset.
@@ -372,8 +354,8 @@ __device__ __forceinline__ double ct_at(const double* __restrict__ S, const doub
   const double n = np[o];
   return n == 0.0 ? 0.0 : S[o + cm] / n;
 }
-__global__ void __launch_bounds__(TPB) k_up(Geo g, const double* __restrict__ S, const double* __restrict__ np,
-                                            double* __restrict__ up) {
+__global__ void __launch_bounds__(TPB) k_up(Geo g, const double* __restrict__ S, double* np,
+                                            double* __restrict__ up, bool fill_np) {
   NODES(n, d);
   const long long C = g.C;
   const unsigned o = n.o;
@@ -384,6 +366,45 @@ __global__ void __launch_bounds__(TPB) k_up(Geo g, const double* __restrict__ S,
   up[o + C] = u1;
   up[o + 2 * C] = u2;
   ghosts3(g, n, up, u0, u1, u2);
+  if (fill_np && on_edge(g, n)) store_ghosts(g.nx, g.ny, g.nz, g.C, 1, np, n.i, n.j, n.k, np[o], 0.0, 0.0);
+}
+
+// The particle passes' gather table, six doubles per node (ghosts included):
+// face_to_center(aj - up), and edge_to_center(bt) when FULL (otherwise the
+// table keeps it).  FULL also stores btc and fills aj's ghosts, as the
+// operators it stands for do (edge_to_center, get_Ep's face_to_center(aj)).
+template <bool FULL>
+__global__ void __launch_bounds__(TPB) k_kit(Geo g, double* aj, const double* __restrict__ up,
+                                             const double* __restrict__ bt, double* __restrict__ btc,
+                                             double* __restrict__ kit) {
+  NODES(n, d);
+  const long long C = g.C;
+  const unsigned o = n.o;
+  double v[6];
+  v[0] = f2c(g.xr[n.i], aj[o] - up[o], aj[o + d.xm] - up[o + d.xm]);
+  v[1] = f2c(g.yr[n.j], aj[o + C] - up[o + C], aj[o + C + d.ym] - up[o + C + d.ym]);
+  v[2] = f2c(g.zr[n.k], aj[o + 2 * C] - up[o + 2 * C], aj[o + 2 * C + d.zm] - up[o + 2 * C + d.zm]);
+  if (FULL) {
+    e2c_node(g, n, d, bt, v + 3);
+    btc[o] = v[3];
+    btc[o + C] = v[4];
+    btc[o + 2 * C] = v[5];
+    ghosts3(g, n, btc, v[3], v[4], v[5]);
+    fill3(g, n, aj);
+  }
+  const int nx = g.nx, ny = g.ny, nz = g.nz;
+  const int is[3] = {n.i, n.i == 2 ? nx : 0, n.i == nx - 1 ? 1 : 0};
+  const int js[3] = {n.j, n.j == 2 ? ny : 0, n.j == ny - 1 ? 1 : 0};
+  const int ks[3] = {n.k, n.k == 2 ? nz : 0, n.k == nz - 1 ? 1 : 0};
+  const int m = on_edge(g, n) ? 3 : 1;
+  for (int c = 0; c < m; ++c)
+    for (int b = 0; b < m; ++b)
+      for (int a = 0; a < m; ++a) {
+        if (!is[a] || !js[b] || !ks[c]) continue;
+        double* w = kit + 6 * nidx(g, is[a], js[b], ks[c]);
+#pragma unroll
+        for (int q = 0; q < (FULL ? 6 : 3); ++q) w[q] = v[q];
+      }
 }
 
 }  // namespace
@@ -424,8 +445,13 @@ cudaError_t edge_to_center(const Geo& g, double* bt, double* btc, cudaStream_t s
 cudaError_t face_to_center(const Geo& g, double* v, double* vc, double* w, double* wc, cudaStream_t st) {
   FL(k_face_to_center, g, v, vc, w, wc);
 }
-cudaError_t up_from_sums(const Geo& g, const double* S, const double* np, double* up, cudaStream_t st) {
-  FL(k_up, g, S, np, up);
+cudaError_t up_from_sums(const Geo& g, const double* S, double* np, double* up, bool fill_np, cudaStream_t st) {
+  FL(k_up, g, S, np, up, fill_np);
+}
+cudaError_t gather_kit(const Geo& g, bool full, double* aj, const double* up, const double* bt, double* btc,
+                       double* kit, cudaStream_t st) {
+  if (full) FL(k_kit<true>, g, aj, up, bt, btc, kit);
+  FL(k_kit<false>, g, aj, up, bt, btc, kit);
 }
 
 }  // namespace swapk

@@ -432,7 +432,7 @@ int update_up_mode(swap_ctx* c, int mode, const double* va, const double* vb, do
        deposit_u(c->g, c->part_view(), c->ntot(), c->prm.beta, mode, va, vb, out_v1, c->s_S, c->d_err, c->st));
   }
   if (c->fused) TRY(c->exchange(c->s_S, 3 * c->g.C, 8));  // MPI_ALLREDUCE, gutsp.f:1812-1822
-  KL("up_from_sums", up_from_sums(c->g, c->s_S, np, up, c->st));
+  KL("up_from_sums", up_from_sums(c->g, c->s_S, const_cast<double*>(np), up, false, c->st));
   return 0;
 }
 
@@ -556,6 +556,22 @@ extern "C" int swap_init(swap_ctx** out, const swap_dims* d, const swap_params* 
   g.rdxg = rec[0]; g.rdyg = rec[1]; g.rdzg = rec[2];
   g.rdxc = rec[3]; g.rdyc = rec[4]; g.rdzc = rec[5];
   g.spacing_p2 = p2;
+  {
+    bool uni = true;
+    double d[3], dg[3];
+    for (int a = 0; a < 3; ++a) {
+      d[a] = arrs[a][1] - arrs[a][0];
+      dg[a] = arrs[3 + a][0];
+      for (int q = 0; q + 1 < ns[a]; ++q) uni = uni && arrs[a][q + 1] - arrs[a][q] == d[a] && arrs[3 + a][q] == dg[a];
+    }
+    g.uniform = uni;
+    g.cell_q = d[0] * d[1] * d[2];
+    g.cell_g = dg[0] * dg[1] * dg[2];
+    g.inv_cell_q = 1.0 / g.cell_q;
+    int e = 0;
+    const double m = std::frexp(p->dy, &e);
+    g.rdy = p->dy > 0.0 && std::isfinite(p->dy) && e > -60 && e < 60 && m != 1.0 - 0x1p-53 ? 1.0 / p->dy : 0.0;
+  }
   g.nx = d->nx; g.ny = d->ny; g.nz = d->nz;
   g.C = (long long)d->nx * d->ny * d->nz;
   g.qx = dg[0]; g.qy = dg[1]; g.qz = dg[2];
@@ -570,15 +586,17 @@ extern "C" int swap_init(swap_ctx** out, const swap_dims* d, const swap_params* 
   c->h_qz.assign(co->qz, co->qz + d->nz);
   // grid scratch (the reference's /dummy/ a, c, ct and subroutine locals)
   const std::size_t C3 = 3 * (std::size_t)g.C;
-  double** bufs[] = {&c->s_ct, &c->s_btc2, &c->s_btmf, &c->s_ajc, &c->s_upc, &c->s_btp1, &c->s_S, &c->s_gf,
-                     &c->s_gpc};
+  double** bufs[] = {&c->s_ct, &c->s_btc2, &c->s_btmf, &c->s_btp1, &c->s_S, &c->s_gf, &c->s_gpc, &c->s_kit};
   for (double** b : bufs) {
-    *b = c->dalloc(C3);
-    if (!*b || cudaMemset(*b, 0, C3 * sizeof(double)) != cudaSuccess) {
+    const std::size_t n = b == &c->s_kit ? 2 * C3 : C3;
+    *b = c->dalloc(n);
+    if (!*b || cudaMemset(*b, 0, n * sizeof(double)) != cudaSuccess) {
       swap_finalize(c);
       return SWAP_ECUDA;
     }
   }
+  c->s_ajc = c->s_kit;
+  c->s_upc = c->s_kit + C3;
   c->s_dtn = c->dalloc((std::size_t)g.C);
   c->s_red = c->dalloc(8);
   int* e = nullptr;
@@ -1064,14 +1082,13 @@ int bound_inputs(swap_ctx* c, Bound& b) {
   TRY(c->use(c->h_aj, Access::InOut, &b.aj));
   TRY(c->use(c->h_E, Access::InOut, &b.E));
   TRY(c->use(c->h_nu, Access::In, &b.nu));
-  if (!c->w_Ep) {
-    const std::size_t n3 = 3 * (std::size_t)c->dims.ni_max + 2;
-    c->w_Ep = c->dalloc(n3);
-    c->w_vplus = c->dalloc(n3);
-    c->w_vminus = c->dalloc(n3);
-    if (!c->w_Ep || !c->w_vplus || !c->w_vminus) return c->fail(SWAP_ECUDA, "allocation of push work arrays");
-  }
   return SWAP_OK;
+}
+
+// One (ni_max,3) work array of the fused step, made on first use.
+int push_array(swap_ctx* c, double** w) {
+  if (!*w) *w = c->dalloc(3 * (std::size_t)c->dims.ni_max + 2);
+  return *w ? SWAP_OK : c->fail(SWAP_ECUDA, "allocation of push work arrays");
 }
 
 // Marks the deposits made in its scope as the fused step's (exchanged).
@@ -1081,9 +1098,67 @@ struct FusedScope {
   ~FusedScope() { c->fused = false; }
 };
 
-int step_pre(swap_ctx* c, Bound& b) {
+// Whether the step's particle half runs as the three passes of k64_pass.cu.
+// The operator-by-operator form stays for what the passes do not cover: the
+// exchange after each deposit (its count and order are the callers'
+// contract), the deterministic sums, which take each value on its own, and
+// the electron-pressure gather.
+bool use_passes(const swap_ctx* c) { return !c->xfn && !c->deterministic && c->prm.grad_pe == 0.0; }
+
+// maind.f:385-413, and with final_move also :479 (v does not change between
+// the two half moves, and nothing reads x).
+int step_passes(swap_ctx* c, Bound& b, bool final_move) {
+  TRY(push_array(c, &c->w_Ep));
+  PassArgs a{};
+  a.g = c->g;
+  a.p = c->part_view();
+  a.p.xp = b.xp;
+  a.p.vp = b.vp;
+  a.p.vp1 = b.vp1;
+  a.N = c->ntot();
+  a.dt = c->prm.dt;
+  a.beta = c->prm.beta;
+  a.kit = c->s_kit;
+  a.b3 = c->w_Ep;
+  a.np = b.np;
+  a.S = c->s_S;
+  a.err = c->d_err;
+  a.x_open = srcops::x_open(c);
+  a.final_move = final_move;
+  const std::size_t bC = (std::size_t)c->g.C * sizeof(double);
+  KL("cudaMemsetAsync", cudaMemsetAsync(b.np, 0, bC, c->st));
+  KL("cudaMemsetAsync", cudaMemsetAsync(c->s_S, 0, 3 * bC, c->st));
+  KL("pass1", particle_pass(1, a, c->st));                                      // :385-386, :399
+  KL("up_from_sums", up_from_sums(c->g, c->s_S, b.np, b.up, true, c->st));
+  TRY(ops::curlB(c, b.bt, b.np, b.aj));                                         // :395
+  KL("gather_kit", gather_kit(c->g, true, b.aj, b.up, b.bt, b.btc, c->s_kit, c->st));  // :398, :400
+  KL("cudaMemsetAsync", cudaMemsetAsync(c->s_S, 0, 3 * bC, c->st));
+  KL("pass2", particle_pass(2, a, c->st));                                      // :400-402
+  KL("up_from_sums", up_from_sums(c->g, c->s_S, b.np, b.up, false, c->st));
+  KL("gather_kit", gather_kit(c->g, false, b.aj, b.up, b.bt, b.btc, c->s_kit, c->st));  // :404
+  KL("cudaMemsetAsync", cudaMemsetAsync(b.np, 0, bC, c->st));
+  KL("cudaMemsetAsync", cudaMemsetAsync(c->s_S, 0, 3 * bC, c->st));
+  KL("pass3", particle_pass(3, a, c->st));                                      // :404-413
+  KL("up_from_sums", up_from_sums(c->g, c->s_S, b.np, b.up, true, c->st));
+  c->weights_valid = true;
+  c->weights_n = c->ntot();
+  return SWAP_OK;
+}
+
+// final_move: the caller goes on to step_post with it done (*moved).
+int step_pre(swap_ctx* c, Bound& b, bool final_move = false, bool* moved = nullptr) {
   FusedScope fs(c);
   TRY(srcops::step_begin(c, b.xp, b.vp, b.vp1));                            // sources
+  if (use_passes(c)) {
+    TRY(step_passes(c, b, final_move));
+    if (moved) *moved = final_move;
+    // an ion that left in the first half move goes on outwards in the second:
+    // one removal after both takes the same ions
+    return final_move ? SWAP_OK : srcops::after_move(c, b.xp, b.vp, b.vp1);
+  }
+  TRY(push_array(c, &c->w_Ep));
+  TRY(push_array(c, &c->w_vplus));
+  TRY(push_array(c, &c->w_vminus));
   TRY(ops::get_interp_weights(c, b.xp));                                     // maind.f:385
   TRY(ops::update_np(c, b.np));                                              // :386
   TRY(ops::update_up_mode(c, 0, b.vp, nullptr, nullptr, b.np, b.up));        // :387
@@ -1114,11 +1189,18 @@ int subcycles(swap_ctx* c, Bound& b) {
 }
 
 // maind.f:479 and the sinks after it (res_chex, maind.f:484).
-int step_post(swap_ctx* c, Bound& b) {
-  TRY(ops::move_ion_half(c, b.xp, b.vp));
+int step_post(swap_ctx* c, Bound& b, bool moved = false) {
+  if (!moved) TRY(ops::move_ion_half(c, b.xp, b.vp));
   TRY(srcops::after_move(c, b.xp, b.vp, b.vp1));
   TRY(srcops::step_end(c, b.xp, b.vp, b.vp1));
   return SWAP_OK;
+}
+
+int whole_step(swap_ctx* c, Bound& b) {
+  bool moved = false;
+  TRY(step_pre(c, b, true, &moved));
+  TRY(subcycles(c, b));
+  return step_post(c, b, moved);
 }
 
 }  // namespace
@@ -1151,9 +1233,7 @@ extern "C" int swap_ion_step(swap_ctx* c) {
   ENTRY;
   Bound b;
   TRY(bound_inputs(c, b));
-  TRY(step_pre(c, b));
-  TRY(subcycles(c, b));
-  TRY(step_post(c, b));
+  TRY(whole_step(c, b));
   return c->finish();
 }
 
@@ -1161,11 +1241,7 @@ extern "C" int swap_run(swap_ctx* c, int32_t nsteps) {
   ENTRY;
   Bound b;
   TRY(bound_inputs(c, b));
-  for (int s = 0; s < nsteps; ++s) {
-    TRY(step_pre(c, b));
-    TRY(subcycles(c, b));
-    TRY(step_post(c, b));
-  }
+  for (int s = 0; s < nsteps; ++s) TRY(whole_step(c, b));
   return c->finish();
 }
 

@@ -88,6 +88,7 @@ struct swap_ctx {
 
   // grid scratch: /dummy/ a, c, ct and subroutine locals
   double *s_ct = nullptr, *s_btc2 = nullptr;
+  double *s_kit = nullptr;  // the passes' gather table, 6 per node (s_ajc, s_upc: its halves, for the entries)
   double *s_btmf = nullptr, *s_ajc = nullptr, *s_upc = nullptr, *s_btp1 = nullptr, *s_S = nullptr;
   double *s_gf = nullptr, *s_gpc = nullptr, *s_dtn = nullptr, *s_red = nullptr;
   // particle work arrays of the fused step (maind.f locals Ep, vplus, vminus)

@@ -23,6 +23,11 @@ struct Geo {
   // spacing is a power of two, its reciprocal exact (k64_field.cu quotient)
   const double *rdxg, *rdyg, *rdzg, *rdxc, *rdyc, *rdzc;
   bool spacing_p2;
+  // uniform: every cell has the same spacings, bit for bit; cell_q and cell_g
+  // are then the products of a cell's node differences and of dx_grid ...
+  bool uniform;
+  double cell_q, cell_g, inv_cell_q;
+  double rdy;                     // 1/dy (0: divide)
   double dy;                      // module dy (gutsp.f:1404)
   double inv_dx, inv_dz;          // guesses for the cell search only
 };
