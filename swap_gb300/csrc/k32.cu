@@ -709,7 +709,7 @@ __device__ __forceinline__ void e2c(const G32& g, const float* bt, int i, int j,
 // (node o to o + e_m): grad_pe * (np(o+e_m) - np(o)) / d_m / n_face, n_face
 // the face average of np as in curlB.
 template <int m, class I = long long>
-__device__ __forceinline__ float gpe_face(const G32& g, const float* __restrict__ np, float gp, I o) {
+__device__ __forceinline__ float gpe_face(const G32& g, const float* np, float gp, I o) {
   const I s = m == 0 ? (I)1 : (m == 1 ? (I)g.nx : (I)g.nx * (I)g.ny);
   const float inv = m == 0 ? g.inv_dx : (m == 1 ? g.inv_dy : g.inv_dz);
   return gp * ((np[o + s] - np[o]) * inv) / (0.5f * (np[o] + np[o + s]));
@@ -773,59 +773,121 @@ constexpr int FBX = 32, FBY = 4;
   const int k = blockIdx.z + 2;                              \
   if (i > g.ncx + 1 || j > g.ncy + 1) return
 
-// Component m of aj = curl(dB)/(alpha * face-averaged np) at node (i,j,k)
-// (curlB, gutsf.f:202-239; curl b0 = 0 for the uniform b0).
-template <int m, class I = long long>
-__device__ __forceinline__ float aj_o(const G32& g, const float* __restrict__ b, const float* __restrict__ np,
-                                      float alpha, I o) {
-  const I C = (I)g.C, sx = 1, sy = (I)g.nx, sz = (I)g.nx * (I)g.ny;
-  const float* B1 = b;
-  const float* B2 = b + C;
-  const float* B3 = b + 2 * C;
-  float c;
-  I s;
-  if (m == 0) {
-    c = (B3[o] - B3[o - sy]) * g.inv_dy + (B2[o - sz] - B2[o]) * g.inv_dz;
-    s = sx;
-  } else if (m == 1) {
-    c = (B1[o] - B1[o - sz]) * g.inv_dz + (B3[o - sx] - B3[o]) * g.inv_dx;
-    s = sy;
-  } else {
-    c = (B2[o] - B2[o - sx]) * g.inv_dx + (B1[o - sy] - B1[o]) * g.inv_dy;
-    s = sz;
+// Neighbours by 32-bit offsets (3 C < 2^32), at the periodic image where the
+// neighbour is a ghost.  Every load of a node stands before its first store:
+// one round trip to memory per node, also on the boundary; and the ghost
+// images of all outputs are stored together.  (A separate path for boundary
+// nodes that mapped each neighbour's index and stored each output's images on
+// its own: 20 steps of 128x64x64 cells 46.9 ms against 42.9, of 256x128x128
+// cells 338 against 331; in the field loop below 307 us a step of 64x32x32
+// cells against 182.)
+
+struct Off {
+  int xm, xp, ym, yp, zm, zp;
+};
+__device__ __forceinline__ Off off_of(const G32& g, int i, int j, int k) {
+  const int sy = g.nx, sz = g.nx * g.ny;
+  Off d;
+  d.xm = i == 2 ? g.ncx - 1 : -1;
+  d.xp = i == g.nx - 1 ? 1 - g.ncx : 1;
+  d.ym = j == 2 ? (g.ncy - 1) * sy : -sy;
+  d.yp = j == g.ny - 1 ? (1 - g.ncy) * sy : sy;
+  d.zm = k == 2 ? (g.ncz - 1) * sz : -sz;
+  d.zp = k == g.nz - 1 ? (1 - g.ncz) * sz : sz;
+  return d;
+}
+
+// v[q] at the ghost images of node (i,j,k) in f[q] (at least 8 cells per axis:
+// one image per axis at most).
+template <int N>
+__device__ __forceinline__ void ghost_images(const G32& g, int i, int j, int k, float* const (&f)[N],
+                                             const float (&v)[N]) {
+  const int di = i == 2 ? g.ncx : (i == g.nx - 1 ? -g.ncx : 0), dj = j == 2 ? g.ncy : (j == g.ny - 1 ? -g.ncy : 0),
+            dk = k == 2 ? g.ncz : (k == g.nz - 1 ? -g.ncz : 0);
+  if (!(di | dj | dk)) return;
+  const long long o = nid(g, i, j, k);
+  const int x = di, y = dj * g.nx, z = dk * g.nx * g.ny;
+#pragma unroll 1
+  for (int c = 1; c < 8; ++c) {
+    if (((c & 1) && !x) || ((c & 2) && !y) || ((c & 4) && !z)) continue;
+    const long long t = o + ((c & 1) ? x : 0) + ((c & 2) ? y : 0) + ((c & 4) ? z : 0);
+#pragma unroll
+    for (int q = 0; q < N; ++q) f[q][t] = v[q];
   }
-  // the fast divide (two ulps): the denominator, a density times alpha, is
-  // far from the range where it loses accuracy
-  return __fdividef(c, 0.5f * (np[o] + np[o + s]) * alpha);
 }
 
-// Linear index of node (i+di, j+dj, k+dk) for |d| <= 1: by strides for a node
-// whose neighbours are all interior (INNER), else at the interior image.
-template <bool INNER>
-__device__ __forceinline__ long long nbr(const G32& g, long long o, int i, int j, int k, int di, int dj, int dk) {
-  if (INNER) return o + di + (long long)g.nx * (dj + (long long)g.ny * dk);
-  return nid(g, img(i + di, g.nx), img(j + dj, g.ny), img(k + dk, g.nz));
-}
-// a node at least one node away from every ghost plane
-__device__ __forceinline__ bool inner_node(const G32& g, int i, int j, int k) {
-  return i > 2 && i < g.nx - 1 && j > 2 && j < g.ny - 1 && k > 2 && k < g.nz - 1;
-}
-// store at an interior node, with its ghost images unless INNER
-template <bool INNER, class T>
-__device__ __forceinline__ void put(const G32& g, T* f, long long o, int i, int j, int k, T v) {
-  if (INNER) f[o] = v;
-  else store_img(g, f, i, j, k, v);
-}
-
-// curlB, face_to_center(aj - up) and the cross product of get_E (gutsf.f:
-// 1059-1075, crossf2 gutsf.f:65-76): writes aj and ct.  Predictor: B at
-// cell centres from edge_to_center of dB (grid_interp.f:35-51).  Corrector:
-// B at m+1/2 through edge_to_face then face_to_center (gutsf.f:1268-1269),
-// i.e. component m is the 1-2-1 average along axis m of edge_to_center.
-template <int m>
-__device__ __forceinline__ float aj_comp(const G32& g, const float* __restrict__ b, const float* __restrict__ np,
-                                         float alpha, int i, int j, int k) {
-  return aj_o<m>(g, b, np, alpha, nid(g, img(i, g.nx), img(j, g.ny), img(k, g.nz)));
+// curlB (gutsf.f:202-239; curl b0 = 0 for the uniform b0), face_to_center(aj -
+// up) and the cross product of get_E (gutsf.f:1059-1075, crossf2 gutsf.f:
+// 65-76): writes aj and ct.  Predictor: B at cell centres from edge_to_center
+// of dB (grid_interp.f:35-51).  Corrector: B at m+1/2 through edge_to_face
+// then face_to_center (gutsf.f:1268-1269), i.e. component m is the 1-2-1
+// average along axis m of edge_to_center.  The divide is the fast one (two
+// ulps): the denominator, a density times alpha, is far from the range where
+// it loses accuracy.
+template <bool CORR>
+__device__ __forceinline__ void aj_ct_node(const G32& g, const float* db, const float* np, const float* up,
+                                           const float* b0c, float alpha, float* aj, float* ct, int i, int j, int k) {
+  const Off d = off_of(g, i, j, k);
+  const long long C = g.C;
+  const unsigned o = (unsigned)nid(g, i, j, k);
+  const float *B1 = db, *B2 = db + C, *B3 = db + 2 * C, *u1 = up, *u2 = up + C, *u3 = up + 2 * C;
+  // B at the node and its lower neighbours: all that curl dB there and one
+  // step down each axis and the centred B need
+  const float b1 = B1[o], b1y = B1[o + d.ym], b1z = B1[o + d.zm], b1yz = B1[o + d.ym + d.zm];
+  const float b2 = B2[o], b2x = B2[o + d.xm], b2z = B2[o + d.zm], b2xz = B2[o + d.xm + d.zm];
+  const float b3 = B3[o], b3x = B3[o + d.xm], b3y = B3[o + d.ym], b3xy = B3[o + d.xm + d.ym];
+  const float n0 = np[o], nxm = np[o + d.xm], nxp = np[o + d.xp], nym = np[o + d.ym], nyp = np[o + d.yp],
+              nzm = np[o + d.zm], nzp = np[o + d.zp];
+  const float ux = u1[o], uxm = u1[o + d.xm], uy = u2[o], uym = u2[o + d.ym], uz = u3[o], uzm = u3[o + d.zm];
+  // the same four values one step down and up the component's own axis
+  float m[3][4], p[3][4];
+  if (CORR) {
+    const int e[3][3] = {{0, d.ym, d.zm}, {0, d.xm, d.zm}, {0, d.ym, d.xm}};
+    const int lo[3] = {d.xm, d.ym, d.zm}, hi[3] = {d.xp, d.yp, d.zp};
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const float* B = db + C * q;
+      const unsigned a = o + lo[q], b = o + hi[q];
+      m[q][0] = B[a]; m[q][1] = B[a + e[q][1]]; m[q][2] = B[a + e[q][2]]; m[q][3] = B[a + e[q][1] + e[q][2]];
+      p[q][0] = B[b]; p[q][1] = B[b + e[q][1]]; p[q][2] = B[b + e[q][2]]; p[q][3] = B[b + e[q][1] + e[q][2]];
+    }
+  }
+  const float c0x = b0c[0], c0y = b0c[1], c0z = b0c[2];
+  auto curl = [](float f, float fm, float gm, float h, float i1, float i2) { return (f - fm) * i1 + (gm - h) * i2; };
+  const float a1 = __fdividef(curl(b3, b3y, b2z, b2, g.inv_dy, g.inv_dz), 0.5f * (n0 + nxp) * alpha);
+  const float a2 = __fdividef(curl(b1, b1z, b3x, b3, g.inv_dz, g.inv_dx), 0.5f * (n0 + nyp) * alpha);
+  const float a3 = __fdividef(curl(b2, b2x, b1y, b1, g.inv_dx, g.inv_dy), 0.5f * (n0 + nzp) * alpha);
+  const float a1m = __fdividef(curl(b3x, b3xy, b2xz, b2x, g.inv_dy, g.inv_dz), 0.5f * (nxm + n0) * alpha);
+  const float a2m = __fdividef(curl(b1y, b1yz, b3xy, b3y, g.inv_dz, g.inv_dx), 0.5f * (nym + n0) * alpha);
+  const float a3m = __fdividef(curl(b2z, b2xz, b1yz, b1z, g.inv_dx, g.inv_dy), 0.5f * (nzm + n0) * alpha);
+  const float ax = 0.5f * ((a1 - ux) + (a1m - uxm));
+  const float ay = 0.5f * ((a2 - uy) + (a2m - uym));
+  const float az = 0.5f * ((a3 - uz) + (a3m - uzm));
+  // edge_to_center of the four values (node, step 1, step 2, both)
+  auto centre = [](float v, float v1, float v2, float v12) {
+    const float h2 = 0.5f * (v + v1), h1 = 0.5f * (v2 + v12);
+    return 0.5f * (h1 + h2);
+  };
+  float bx = centre(b1, b1y, b1z, b1yz), by = centre(b2, b2x, b2z, b2xz), bz = centre(b3, b3y, b3x, b3xy);
+  if (CORR) {
+    float lo[3], hi[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      lo[q] = centre(m[q][0], m[q][1], m[q][2], m[q][3]);
+      hi[q] = centre(p[q][0], p[q][1], p[q][2], p[q][3]);
+    }
+    bx = 0.25f * (lo[0] + 2.0f * bx + hi[0]);
+    by = 0.25f * (lo[1] + 2.0f * by + hi[1]);
+    bz = 0.25f * (lo[2] + 2.0f * bz + hi[2]);
+  }
+  bx += c0x;
+  by += c0y;
+  bz += c0z;
+  float* const f[6] = {aj, aj + C, aj + 2 * C, ct, ct + C, ct + 2 * C};
+  const float v[6] = {a1, a2, a3, ay * bz - az * by, az * bx - ax * bz, ax * by - ay * bx};
+#pragma unroll
+  for (int q = 0; q < 6; ++q) f[q][o] = v[q];
+  ghost_images(g, i, j, k, f, v);
 }
 
 template <bool CORR>
@@ -834,90 +896,15 @@ __global__ void __launch_bounds__(FBX * FBY) k_aj_ct(G32 g, const float* __restr
                                                      const float* __restrict__ b0c, float alpha,
                                                      float* __restrict__ aj, float* __restrict__ ct) {
   FIELD_NODE(i, j, k);
-  if (inner_node(g, i, j, k)) {
-    // every neighbour interior and no ghost image to store: strides, 32-bit
-    // offsets (3 C < 2^32), the same arithmetic as below
-    using U = unsigned;
-    const U C = (U)g.C, o = (U)nid(g, i, j, k), sy = (U)g.nx, sz = (U)g.nx * (U)g.ny;
-    const float a1 = aj_o<0, U>(g, db, np, alpha, o);
-    const float a2 = aj_o<1, U>(g, db, np, alpha, o);
-    const float a3 = aj_o<2, U>(g, db, np, alpha, o);
-    const float a1m = aj_o<0, U>(g, db, np, alpha, o - 1);
-    const float a2m = aj_o<1, U>(g, db, np, alpha, o - sy);
-    const float a3m = aj_o<2, U>(g, db, np, alpha, o - sz);
-    aj[o] = a1;
-    aj[o + C] = a2;
-    aj[o + 2 * C] = a3;
-    const float ax = 0.5f * ((a1 - up[o]) + (a1m - up[o - 1]));
-    const float ay = 0.5f * ((a2 - up[o + C]) + (a2m - up[o - sy + C]));
-    const float az = 0.5f * ((a3 - up[o + 2 * C]) + (a3m - up[o - sz + 2 * C]));
-    float bx, by, bz;
-    if (!CORR) {
-      e2c_o<U>(g, db, o, bx, by, bz);
-    } else {
-      float c1, c2, c3, m1, m2, m3, p1, p2, p3, d1, d2;
-      e2c_o<U>(g, db, o, c1, c2, c3);
-      e2c_o<U>(g, db, o - 1, m1, d1, d2);
-      e2c_o<U>(g, db, o + 1, p1, d1, d2);
-      e2c_o<U>(g, db, o - sy, d1, m2, d2);
-      e2c_o<U>(g, db, o + sy, d1, p2, d2);
-      e2c_o<U>(g, db, o - sz, d1, d2, m3);
-      e2c_o<U>(g, db, o + sz, d1, d2, p3);
-      bx = 0.25f * (m1 + 2.0f * c1 + p1);
-      by = 0.25f * (m2 + 2.0f * c2 + p2);
-      bz = 0.25f * (m3 + 2.0f * c3 + p3);
-    }
-    bx += b0c[0];
-    by += b0c[1];
-    bz += b0c[2];
-    ct[o] = ay * bz - az * by;
-    ct[o + C] = az * bx - ax * bz;
-    ct[o + 2 * C] = ax * by - ay * bx;
-    return;
-  }
-  const long long C = g.C, o = nid(g, i, j, k), sx = 1, sy = g.nx, sz = (long long)g.nx * g.ny;
-  const float a1 = aj_comp<0>(g, db, np, alpha, i, j, k);
-  const float a2 = aj_comp<1>(g, db, np, alpha, i, j, k);
-  const float a3 = aj_comp<2>(g, db, np, alpha, i, j, k);
-  const float a1m = aj_comp<0>(g, db, np, alpha, i - 1, j, k);
-  const float a2m = aj_comp<1>(g, db, np, alpha, i, j - 1, k);
-  const float a3m = aj_comp<2>(g, db, np, alpha, i, j, k - 1);
-  store_img(g, aj, i, j, k, a1);
-  store_img(g, aj + C, i, j, k, a2);
-  store_img(g, aj + 2 * C, i, j, k, a3);
-  const float ax = 0.5f * ((a1 - up[o]) + (a1m - up[o - sx]));
-  const float ay = 0.5f * ((a2 - up[o + C]) + (a2m - up[o - sy + C]));
-  const float az = 0.5f * ((a3 - up[o + 2 * C]) + (a3m - up[o - sz + 2 * C]));
-  float bx, by, bz;
-  if (!CORR) {
-    e2c(g, db, i, j, k, bx, by, bz);
-  } else {
-    float c1, c2, c3, m1, m2, m3, p1, p2, p3, d1, d2;
-    e2c(g, db, i, j, k, c1, c2, c3);
-    e2c(g, db, img(i - 1, g.nx), j, k, m1, d1, d2);
-    e2c(g, db, img(i + 1, g.nx), j, k, p1, d1, d2);
-    e2c(g, db, i, img(j - 1, g.ny), k, d1, m2, d2);
-    e2c(g, db, i, img(j + 1, g.ny), k, d1, p2, d2);
-    e2c(g, db, i, j, img(k - 1, g.nz), d1, d2, m3);
-    e2c(g, db, i, j, img(k + 1, g.nz), d1, d2, p3);
-    bx = 0.25f * (m1 + 2.0f * c1 + p1);
-    by = 0.25f * (m2 + 2.0f * c2 + p2);
-    bz = 0.25f * (m3 + 2.0f * c3 + p3);
-  }
-  bx += b0c[0];
-  by += b0c[1];
-  bz += b0c[2];
-  store_img(g, ct, i, j, k, ay * bz - az * by);
-  store_img(g, ct + C, i, j, k, az * bx - ax * bz);
-  store_img(g, ct + 2 * C, i, j, k, ax * by - ay * bx);
+  aj_ct_node<CORR>(g, db, np, up, b0c, alpha, aj, ct, i, j, k);
 }
 
 // Component m of E = face average of ct + nu*aj at node (i,j,k) (gutsf.f:
 // 94-96, 1082), less the electron-pressure face gradient gpf when given
 // (the isothermal extension of the commented "- gradP", gutsf.f:1083,1283).
 template <int m>
-__device__ __forceinline__ float e_o(const G32& g, const float* __restrict__ ct, const float* __restrict__ nu,
-                                     const float* __restrict__ aj, const float* __restrict__ gpf, long long o) {
+__device__ __forceinline__ float e_o(const G32& g, const float* ct, const float* nu,
+                                     const float* aj, const float* gpf, long long o) {
   const long long C = g.C;
   const long long s = m == 0 ? 1 : (m == 1 ? (long long)g.nx : (long long)g.nx * g.ny);
   const float e = 0.5f * (ct[o + C * m] + ct[o + s + C * m]) + nu[o] * aj[o + C * m];
@@ -950,50 +937,71 @@ __device__ __forceinline__ void df_sub_mul(float bh, float bl, float ch, float c
 // (predict_B gutsf.f:1158-1159 with coef = 2 dtsub on b12; correct_B
 // gutsf.f:1349-1350 with coef = dtsub on b1) in double-float; dB of the
 // result in FP32.  Predictor: only dB at m+1/2 = (dB_new + dB1)/2
-// (gutsf.f:1210-1219), the one use of the predicted B.  WRITE_E: store E
-// (the step's last corrector).
-template <bool PRED, bool WRITE_E, bool INNER>
-__device__ __forceinline__ void bstep_node(const G32& g, const float* __restrict__ ct, const float* __restrict__ nu,
-                                           const float* __restrict__ aj, const float* __restrict__ gpf,
-                                           const float* __restrict__ bh,
-                                           const float* __restrict__ bl, float ch, float cl,
-                                           const float* __restrict__ b0c, float* __restrict__ oh,
-                                           float* __restrict__ ol, float* __restrict__ dbo,
-                                           const float* __restrict__ db1, float* __restrict__ dbtp1,
-                                           float* __restrict__ E, float* __restrict__ e_acc, int i, int j, int k) {
-  const long long C = g.C, o = nid(g, i, j, k);
-  const long long ox = nbr<INNER>(g, o, i, j, k, 1, 0, 0), oy = nbr<INNER>(g, o, i, j, k, 0, 1, 0),
-                  oz = nbr<INNER>(g, o, i, j, k, 0, 0, 1);
-  const float e1 = e_o<0>(g, ct, nu, aj, gpf, o);
-  const float e2 = e_o<1>(g, ct, nu, aj, gpf, o);
-  const float e3 = e_o<2>(g, ct, nu, aj, gpf, o);
-  const float e1y = e_o<0>(g, ct, nu, aj, gpf, oy), e1z = e_o<0>(g, ct, nu, aj, gpf, oz);
-  const float e2x = e_o<1>(g, ct, nu, aj, gpf, ox), e2z = e_o<1>(g, ct, nu, aj, gpf, oz);
-  const float e3x = e_o<2>(g, ct, nu, aj, gpf, ox), e3y = e_o<2>(g, ct, nu, aj, gpf, oy);
+// (gutsf.f:1210-1219), the one use of the predicted B: the corrector rewrites
+// B and dB from b1.  WRITE_E: store E (the step's last corrector).  e_acc: the
+// sum of the correctors' E over a step, the surrogate's target.
+template <bool PRED, bool WRITE_E>
+__device__ __forceinline__ void bstep_node(const G32& g, const float* ct, const float* nu, const float* aj,
+                                           const float* gpf, const float* bh, const float* bl, float ch, float cl,
+                                           const float* b0c, float* oh, float* ol, float* dbo, const float* db1,
+                                           float* dbtp1, float* E, float* e_acc, int i, int j, int k) {
+  const Off d = off_of(g, i, j, k);
+  const long long C = g.C;
+  const unsigned o = (unsigned)nid(g, i, j, k), ox = o + d.xp, oy = o + d.yp, oz = o + d.zp;
+  const float *c1 = ct, *c2 = ct + C, *c3 = ct + 2 * C, *j1 = aj, *j2 = aj + C, *j3 = aj + 2 * C;
+  const float n0 = nu[o], nx = nu[ox], ny = nu[oy], nz = nu[oz];
+  float e1 = 0.5f * (c1[o] + c1[ox]) + n0 * j1[o], e1y = 0.5f * (c1[oy] + c1[oy + d.xp]) + ny * j1[oy],
+        e1z = 0.5f * (c1[oz] + c1[oz + d.xp]) + nz * j1[oz];
+  float e2 = 0.5f * (c2[o] + c2[oy]) + n0 * j2[o], e2x = 0.5f * (c2[ox] + c2[ox + d.yp]) + nx * j2[ox],
+        e2z = 0.5f * (c2[oz] + c2[oz + d.yp]) + nz * j2[oz];
+  float e3 = 0.5f * (c3[o] + c3[oz]) + n0 * j3[o], e3x = 0.5f * (c3[ox] + c3[ox + d.zp]) + nx * j3[ox],
+        e3y = 0.5f * (c3[oy] + c3[oy + d.zp]) + ny * j3[oy];
+  float h[3], l[3], c0[3], old[3];
+#pragma unroll
+  for (int m = 0; m < 3; ++m) {
+    h[m] = bh[o + C * m];
+    l[m] = bl[o + C * m];
+    c0[m] = b0c[m];
+    old[m] = PRED ? db1[o + C * m] : 0.0f;
+  }
+  if (gpf) {
+    const float *g1 = gpf, *g2 = gpf + C, *g3 = gpf + 2 * C;
+    e1 -= g1[o]; e1y -= g1[oy]; e1z -= g1[oz];
+    e2 -= g2[o]; e2x -= g2[ox]; e2z -= g2[oz];
+    e3 -= g3[o]; e3x -= g3[ox]; e3y -= g3[oy];
+  }
   const float ce[3] = {(e3y - e3) * g.inv_dy + (e2 - e2z) * g.inv_dz,
                        (e3 - e3x) * g.inv_dx + (e1z - e1) * g.inv_dz,
                        (e1 - e1y) * g.inv_dy + (e2x - e2) * g.inv_dx};
+  constexpr int N = (PRED ? 3 : 9) + (WRITE_E ? 3 : 0);
+  float* f[N];
+  float v[N];
 #pragma unroll
   for (int m = 0; m < 3; ++m) {
     float rh, rl;
-    df_sub_mul(bh[o + C * m], bl[o + C * m], ch, cl, ce[m], rh, rl);
-    const float d = __fadd_rn(__fsub_rn(rh, b0c[m]), rl);
+    df_sub_mul(h[m], l[m], ch, cl, ce[m], rh, rl);
+    const float b = __fadd_rn(__fsub_rn(rh, c0[m]), rl);
     if (PRED) {
-      // the predicted B enters the corrector only through dB at m+1/2:
-      // the corrector rewrites B and dB from b1
-      put<INNER>(g, dbtp1 + C * m, o, i, j, k, 0.5f * (d + db1[o + C * m]));
+      f[m] = dbtp1 + C * m;
+      v[m] = 0.5f * (b + old[m]);
     } else {
-      put<INNER>(g, oh + C * m, o, i, j, k, rh);
-      put<INNER>(g, ol + C * m, o, i, j, k, rl);
-      put<INNER>(g, dbo + C * m, o, i, j, k, d);
+      f[m] = oh + C * m;
+      v[m] = rh;
+      f[3 + m] = ol + C * m;
+      v[3 + m] = rl;
+      f[6 + m] = dbo + C * m;
+      v[6 + m] = b;
     }
   }
   if (WRITE_E) {
-    put<INNER>(g, E, o, i, j, k, e1);
-    put<INNER>(g, E + C, o, i, j, k, e2);
-    put<INNER>(g, E + 2 * C, o, i, j, k, e3);
+    f[N - 3] = E; f[N - 2] = E + C; f[N - 1] = E + 2 * C;
+    v[N - 3] = e1; v[N - 2] = e2; v[N - 1] = e3;
   }
-  if (e_acc) {  // the sum of the correctors' E over a step: the surrogate's target
+#pragma unroll
+  for (int q = 0; q < N; ++q) f[q][o] = v[q];
+  float* const(&cf)[N] = f;
+  ghost_images(g, i, j, k, cf, v);
+  if (e_acc) {
     e_acc[o] += e1;
     e_acc[o + C] += e2;
     e_acc[o + 2 * C] += e3;
@@ -1011,12 +1019,118 @@ __global__ void __launch_bounds__(FBX * FBY) k_bstep(G32 g, const float* __restr
                                                      float* __restrict__ dbtp1, float* __restrict__ E,
                                                      float* __restrict__ e_acc) {
   FIELD_NODE(i, j, k);
-  if (inner_node(g, i, j, k))
-    bstep_node<PRED, WRITE_E, true>(g, ct, nu, aj, gpf, bh, bl, ch, cl, b0c, oh, ol, dbo, db1, dbtp1, E, e_acc, i, j,
-                                    k);
-  else
-    bstep_node<PRED, WRITE_E, false>(g, ct, nu, aj, gpf, bh, bl, ch, cl, b0c, oh, ol, dbo, db1, dbtp1, E, e_acc, i,
-                                     j, k);
+  bstep_node<PRED, WRITE_E>(g, ct, nu, aj, gpf, bh, bl, ch, cl, b0c, oh, ol, dbo, db1, dbtp1, E, e_acc, i, j, k);
+}
+
+// ---- the whole field step of a small grid in one launch ----
+//
+// Below FIELD_LOOP_NODES the subcycles' kernels are bound by their launches
+// and the latency of a few loads, not by work.  So the 40 half-kernels of ten
+// subcycles run as phases of one kernel whose blocks meet at a barrier
+// between them (bounded waits).  The same node functions on the same
+// operands.  Two forms.  CLUSTER: one cluster of FIELD_CLUSTER blocks, which
+// meet at the hardware's cluster barrier (0.24 us) -- up to FIELD_CLUSTER *
+// LOOP_TPB nodes.  Otherwise a cooperative launch with a counter in memory
+// (1.2 us at 152 blocks), at most one block per SM, so that the loops of two
+// contexts on one GPU are resident side by side.
+// A step of 8 ions per cell, loop against launches, in ms: 1.5k nodes 0.234
+// against 0.325, 33k 0.314 against 0.342, 65k 0.341 against 0.408, 131k 0.533
+// against 0.524, 262k 0.887 against 0.791 (one block per SM then hides less
+// latency than full occupancy does): hence FIELD_LOOP_NODES.
+constexpr int LOOP_TPB = 512;
+
+struct LoopBarrier {
+  unsigned* bar;  // [0] arrivals, [1] blocks that are through
+  unsigned polls;
+  unsigned target;
+  bool ok;
+  // Every block's stores before it are visible to every block after it;
+  // false: the wait ran out (the caller returns).
+  template <bool CLUSTER>
+  __device__ __forceinline__ bool sync() {
+    if (CLUSTER) {
+      asm volatile(
+          "barrier.cluster.arrive.release.aligned;\n"
+          "barrier.cluster.wait.acquire.aligned;" ::
+              : "memory");
+      return true;
+    }
+    target += gridDim.x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      atomicAdd(bar, 1u);
+      unsigned v, n = 0;
+      do {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+      } while (v < target && n++ < polls);
+      __threadfence();
+      ok = v >= target;
+    }
+    return !__syncthreads_or(threadIdx.x == 0 && !ok);
+  }
+  // The last block to finish leaves the counters at zero for the next launch.
+  __device__ __forceinline__ void done() {
+    if (threadIdx.x == 0) {
+      __threadfence();
+      if (atomicAdd(bar + 1, 1u) == gridDim.x - 1) {
+        bar[0] = 0u;
+        bar[1] = 0u;
+        __threadfence();
+      }
+    }
+  }
+};
+
+template <bool CLUSTER>
+__global__ void __launch_bounds__(LOOP_TPB, 2) k_field_loop(G32 g, FieldLoop f) {
+  // uniform over the grid (both words are a snapshot that nothing writes
+  // now): a failed pass or a Courant violation leaves the state as it is
+  if (*f.failed != 0 || (double)*f.courant <= f.courant_floor) return;
+  LoopBarrier bar{f.bar, f.polls, 0u, true};
+  const unsigned n = (unsigned)n_int(g), t0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  float *b1h = f.b1h, *b1l = f.b1l, *b12h = f.b12h, *b12l = f.b12l, *bph = f.bph, *bpl = f.bpl, *db1 = f.db1,
+        *dbp = f.dbp;
+  auto each = [&](auto&& node) {
+    for (unsigned t = t0; t < n; t += step) {
+      int i, j, k;
+      interior_of(g, t, i, j, k);
+      node(i, j, k);
+    }
+    return bar.template sync<CLUSTER>();
+  };
+  for (int s = 0; s < f.n; ++s) {
+    if (!each([&](int i, int j, int k) {
+          aj_ct_node<false>(g, db1, f.np, f.up, f.b0c, f.alpha, f.aj, f.ct, i, j, k);
+        }))
+      break;
+    if (!each([&](int i, int j, int k) {
+          bstep_node<true, false>(g, f.ct, f.nu, f.aj, f.gpf, b12h, b12l, f.ch2, f.cl2, f.b0c, bph, bpl, dbp, db1,
+                                  f.dbt, f.E, nullptr, i, j, k);
+        }))
+      break;
+    if (!each([&](int i, int j, int k) {
+          aj_ct_node<true>(g, f.dbt, f.np, f.up, f.b0c, f.alpha, f.aj, f.ct, i, j, k);
+        }))
+      break;
+    const bool last = s + 1 == f.n;
+    if (!each([&](int i, int j, int k) {
+          if (last)
+            bstep_node<false, true>(g, f.ct, f.nu, f.aj, f.gpf, b1h, b1l, f.ch, f.cl, f.b0c, bph, bpl, dbp, nullptr,
+                                    nullptr, f.E, f.e_acc, i, j, k);
+          else
+            bstep_node<false, false>(g, f.ct, f.nu, f.aj, f.gpf, b1h, b1l, f.ch, f.cl, f.b0c, bph, bpl, dbp, nullptr,
+                                     nullptr, f.E, f.e_acc, i, j, k);
+        }))
+      break;
+    // f_update_tlev (gutsf.f:10-35): b12 <- b1, b1 <- b1p2
+    float* q = b12h; b12h = b1h; b1h = bph; bph = q;
+    q = b12l; b12l = b1l; b1l = bpl; bpl = q;
+    q = db1; db1 = dbp; dbp = q;
+  }
+  if (CLUSTER) return;
+  if (!bar.ok && threadIdx.x == 0) set_err(f.err, KERR_WAIT);
+  bar.done();
 }
 
 // B_new = base - coef * curl E for a given E (with ghost images), in
@@ -1760,6 +1874,33 @@ cudaError_t b_step(const G32& g, bool pred, bool write_e, const float* ct, const
   RET((k_bstep<false, false><<<grid, blk, 0, st>>>(g, ct, nu, aj, gpf, bh, bl, ch, cl, b0c, oh, ol, dbo, db1, dbtp1, E,
                                                    e_acc)));
 }
+bool field_loop_fits(const G32& g) { return n_int(g) <= FIELD_LOOP_NODES; }
+
+cudaError_t field_loop(const G32& g, const FieldLoop& f, cudaStream_t st) {
+  const long long need = (n_int(g) + LOOP_TPB - 1) / LOOP_TPB;
+  if (need <= FIELD_CLUSTER) {  // always the whole cluster: fewer warps share an SM's load path
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(FIELD_CLUSTER);
+    cfg.blockDim = dim3((unsigned)((n_int(g) / FIELD_CLUSTER + 31) / 32 * 32));
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = FIELD_CLUSTER;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_field_loop<true>, g, f);
+  }
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  G32 gg = g;
+  FieldLoop ff = f;
+  void* args[] = {&gg, &ff};
+  return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&k_field_loop<false>),
+                                     dim3((unsigned)(need < sms ? need : sms)), dim3(LOOP_TPB), args, 0, st);
+}
 cudaError_t b_step_given_e(const G32& g, const float* E, const float* bh, const float* bl, double coef,
                            const float* b0c, float* oh, float* ol, float* dbo, cudaStream_t st) {
   const dim3 grid((g.ncx + FBX - 1) / FBX, (g.ncy + FBY - 1) / FBY, g.ncz), blk(FBX, FBY);
@@ -1799,8 +1940,7 @@ cudaError_t join_df(long long n, const float* h, const float* l, double* a, cuda
 }
 cudaError_t courant_min(const G32& g, const float* dbt, const float* b0c, const float* np, float alpha, float dx,
                         float* dtn, float* d_min, cudaStream_t st) {
-  const unsigned init = 0x7f7fffffu;  // FLT_MAX
-  cudaError_t e = cudaMemcpyAsync(d_min, &init, sizeof(init), cudaMemcpyHostToDevice, st);
+  cudaError_t e = cudaMemsetAsync(d_min, 0x7f, sizeof(unsigned), st);  // 3.39e38
   if (e != cudaSuccess) return e;
   const unsigned nb = nblk(g.C) < 152u * 8u ? nblk(g.C) : 152u * 8u;
   RET((k_courant<<<nb, TPB, 0, st>>>(g, dbt, b0c, np, alpha, dx, dtn, reinterpret_cast<unsigned*>(d_min))));

@@ -200,6 +200,28 @@ cudaError_t aj_ct(const G32& g, bool corr, const float* db, const float* np, con
 cudaError_t b_step(const G32& g, bool pred, bool write_e, const float* ct, const float* nu, const float* aj,
                    const float* gpf, const float* bh, const float* bl, double coef, const float* b0c, float* oh,
                    float* ol, float* dbo, const float* db1, float* dbtp1, float* E, float* e_acc, cudaStream_t st);
+// The n subcycles of a small grid in one launch (field_loop_fits), from and
+// to the buffers that n rounds of the two launchers above would use.  Nothing
+// is done when *failed is set or *courant (the smallest Courant time) <=
+// courant_floor: the caller looks at both.  Neither word may change meanwhile.
+constexpr long long FIELD_LOOP_NODES = 3 << 15;
+constexpr int FIELD_CLUSTER = 8;  // the portable cluster size
+struct FieldLoop {
+  int n;
+  const float *np, *up, *nu, *gpf, *b0c;
+  float *b1h, *b1l, *b12h, *b12l, *bph, *bpl;  // B levels, double-float
+  float *db1, *dbp, *dbt;                      // dB of b1, b1p2 and at m+1/2
+  float *aj, *ct, *E, *e_acc;
+  float alpha, ch, cl, ch2, cl2;  // dtsub and 2 dtsub in double-float
+  const float* courant;
+  double courant_floor;
+  const int* failed;
+  int* err;  // set to KERR_WAIT when a barrier's wait runs out
+  unsigned* bar;  // two counters, zero between launches
+  unsigned polls;
+};
+bool field_loop_fits(const G32& g);
+cudaError_t field_loop(const G32& g, const FieldLoop& f, cudaStream_t st);
 // The surrogate's field advance: B_new = base - coef * curl E for a given E.
 cudaError_t b_step_given_e(const G32& g, const float* E, const float* bh, const float* bl, double coef,
                            const float* b0c, float* oh, float* ol, float* dbo, cudaStream_t st);

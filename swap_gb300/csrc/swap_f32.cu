@@ -86,12 +86,23 @@ struct F32State {
   cudaEvent_t ev_sort = nullptr;
   int64_t* h_n = nullptr;
   bool sort_pending = false;
+  // the smallest Courant time and the error word of the step, in pinned
+  // memory once ev_look has passed
+  struct Look {
+    float min;
+    int err;
+  };
+  Look* h_look = nullptr;
+  cudaEvent_t ev_look = nullptr;
+  unsigned* loop_bar = nullptr;  // the field loop's barrier counters
   ~F32State() {
     if (side) cudaStreamSynchronize(side);
     if (ev_main) cudaEventDestroy(ev_main);
     if (ev_side) cudaEventDestroy(ev_side);
     if (ev_sort) cudaEventDestroy(ev_sort);
     if (h_n) cudaFreeHost(h_n);
+    if (ev_look) cudaEventDestroy(ev_look);
+    if (h_look) cudaFreeHost(h_look);
     if (side) cudaStreamDestroy(side);
     srcops::stage_free(stage);
     for (void* p : owned) cudaFree(p);
@@ -163,6 +174,8 @@ static int check_err(swap_ctx* c) {
   CU(cudaStreamSynchronize(c->st));
   if (herr) {
     cudaMemset(c->d_err, 0, sizeof(int));
+    if (F32State* s = f32(c))  // a barrier that gave up leaves its counters part-way
+      if (s->loop_bar) cudaMemset(s->loop_bar, 0, 2 * sizeof(unsigned));
     if (herr == swapk::KERR_DOMAIN) return c->fail(SWAP_EDOMAIN, "a particle lies outside the grid");
     if (herr == swapk::KERR_CAPACITY) return c->fail(SWAP_ECAPACITY, "Ni_max exceeded by new ions");
     if (herr == swapk::KERR_MOVE)
@@ -383,11 +396,15 @@ extern "C" int swap_f32_begin(swap_ctx* c) {
   s->d_min = s->alloc<float>(4);
   s->dtn = s->alloc<float>(C);
   s->acc = s->alloc<double>(4);
+  s->loop_bar = s->alloc<unsigned>(2);
+  CU(cudaEventCreateWithFlags(&s->ev_look, cudaEventDisableTiming));
+  CU(cudaMallocHost(&s->h_look, sizeof(F32State::Look)));
   if (!s->start || !s->start_new || !s->count || !s->sums || !s->dirrank || !s->dep || !s->pre || !s->partial || !s->kit ||
       !s->np || !s->S || !s->up || !s->aj || !s->ct || !s->E || !s->nu || !s->db1 || !s->db1p2 || !s->dbtp1 ||
-      !s->b0 || !s->b1.l || !s->b12.l || !s->b1p2.l || !s->b0c || !s->d_min || !s->acc || !s->dtn || !s->far.idx ||
+      !s->b0 || !s->b1.l || !s->b12.l || !s->b1p2.l || !s->b0c || !s->d_min || !s->acc || !s->dtn || !s->loop_bar || !s->far.idx ||
       !s->far.key || !s->far.dcell || !s->far.o || !s->far.q || !s->far.n || !s->far.total)
     return c->fail(SWAP_ECUDA, "FP32 grid allocation failed");
+  CU(cudaMemsetAsync(s->loop_bar, 0, 2 * sizeof(unsigned), c->st));
   CU(cudaMemsetAsync(s->far.n, 0, sizeof(int), c->st));
   CU(cudaMemsetAsync(s->far.total, 0, sizeof(unsigned long long), c->st));
   CU(cudaMemsetAsync(s->np, 0, C * sizeof(float), c->st));
@@ -471,15 +488,40 @@ static int subcycles(swap_ctx* c, F32State* s, float* e_acc = nullptr) {
   // reference's ordered halving (once per violating node, k innermost) is
   // replayed on the host from the node values.
   KL("f32_courant", courant_min(g, s->db1, s->b0c, s->np, (float)c->prm.alpha, g.dx, s->dtn, s->d_min, c->st));
-  float mn = 0;
-  int herr = 0;
-  CU(cudaMemcpyAsync(&mn, s->d_min, sizeof(float), cudaMemcpyDeviceToHost, c->st));
-  CU(cudaMemcpyAsync(&herr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->st));
-  CU(cudaStreamSynchronize(c->st));
+  // a snapshot of the error word beside it: the sort on the second stream may
+  // still set the word itself
+  CU(cudaMemcpyAsync(s->d_min + 1, c->d_err, sizeof(int), cudaMemcpyDeviceToDevice, c->st));
+  CU(cudaMemcpyAsync(s->h_look, s->d_min, sizeof(F32State::Look), cudaMemcpyDeviceToHost, c->st));
+  CU(cudaEventRecord(s->ev_look, c->st));
+  // a small grid's subcycles go out before the host has looked: the kernel
+  // itself leaves the state alone in the two cases below
+  const bool looped = field_loop_fits(g);
+  if (looped) {
+    FieldLoop f{};
+    f.n = c->prm.ntsub;
+    f.np = s->np; f.up = s->up; f.nu = s->nu; f.gpf = s->gpf; f.b0c = s->b0c;
+    f.b1h = s->b1.h; f.b1l = s->b1.l; f.b12h = s->b12.h; f.b12l = s->b12.l; f.bph = s->b1p2.h; f.bpl = s->b1p2.l;
+    f.db1 = s->db1; f.dbp = s->db1p2; f.dbt = s->dbtp1;
+    f.aj = s->aj; f.ct = s->ct; f.E = s->E; f.e_acc = e_acc;
+    f.alpha = (float)c->prm.alpha;
+    f.ch = (float)dtsub; f.cl = (float)(dtsub - (double)f.ch);
+    f.ch2 = (float)(2.0 * dtsub); f.cl2 = (float)(2.0 * dtsub - (double)f.ch2);
+    f.courant = s->d_min;
+    f.courant_floor = 2.0 * dtsub;
+    f.failed = reinterpret_cast<const int*>(s->d_min + 1);
+    f.err = c->d_err;
+    f.bar = s->loop_bar;
+    f.polls = c->wait_polls;
+    KL("f32_field_loop", field_loop(g, f, c->st));
+  }
+  CU(cudaEventSynchronize(s->ev_look));
+  const float mn = s->h_look->min;
+  const int herr = s->h_look->err;
   // a pass that failed (a wait that gave up, an ion outside the grid) ends
   // the step here, before its moments reach the fields
   if (herr) return check_err(c);
-  if ((double)mn <= 2.0 * dtsub) {
+  const bool mn_above = !((double)mn <= 2.0 * dtsub);
+  if (!mn_above) {
     std::vector<float> h((std::size_t)g.C);
     CU(cudaMemcpy(h.data(), s->dtn, h.size() * sizeof(float), cudaMemcpyDeviceToHost));
     for (int i = 0; i < g.nx; ++i)
@@ -494,6 +536,14 @@ static int subcycles(swap_ctx* c, F32State* s, float* e_acc = nullptr) {
   s->last_dtsub = dtsub;
   s->last_ntf = ntf;
   const int n = (int)ntf;
+  if (looped && mn_above) {  // done by the loop kernel
+    for (int it = 0; it < n; ++it) {
+      std::swap(s->b12, s->b1);
+      std::swap(s->b1, s->b1p2);
+      std::swap(s->db1, s->db1p2);
+    }
+    return SWAP_OK;
+  }
   const float alpha = (float)c->prm.alpha;
   for (int it = 0; it < n; ++it) {
     const bool last = it == n - 1;
