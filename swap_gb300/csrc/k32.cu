@@ -600,110 +600,56 @@ __global__ void __launch_bounds__(TPB_PASS, PASS == 3 ? 7 : 8) k_pass(G32 g, Par
 // offset (p+1+O)%4 and in the one before at offset +4 when that is < T
 // (O = 1 for the 7-node tiles, whose origin is one node lower).  The density
 // is stored with its ghost images (boundary.f:167-206 fused in).
-template <int T>
-__global__ void k_node_sum(G32 g, const void* __restrict__ partial, int nq, int exact, float* __restrict__ np,
-                           float* __restrict__ S) {
+// All of a node's tile values (up to 8 tiles times NQ moments) are loaded
+// before the first is added: a loop over the tiles that are there left one
+// load in flight per node (256x128x128 cells, ms per step: 0.57 -> 0.36).
+template <int T, int NQ, bool EXACT>
+__global__ void k_node_sum(G32 g, const void* __restrict__ partial, float* __restrict__ np, float* __restrict__ S) {
   constexpr int O = T == TN ? 1 : 0, TNOD = T * T * T;
+  using V = typename std::conditional<EXACT, long long, float>::type;
   GSTRIDE(t, n_int(g)) {
-    int P, Q, R;
-    interior_of(g, t, P, Q, R);
-    P -= 2;
-    Q -= 2;
-    R -= 2;
-    int bx[2], ox[2], by[2], oy[2], bz[2], oz[2], nxc = 1, nyc = 1, nzc = 1;
-    bx[0] = (P + 1 + O) >> 2; ox[0] = (P + 1 + O) & 3;
-    if (bx[0] >= g.nbx) bx[0] -= g.nbx;
-    if (ox[0] + 4 < T) { bx[1] = bx[0] == 0 ? g.nbx - 1 : bx[0] - 1; ox[1] = ox[0] + 4; nxc = 2; }
-    by[0] = (Q + 1 + O) >> 2; oy[0] = (Q + 1 + O) & 3;
-    if (by[0] >= g.nby) by[0] -= g.nby;
-    if (oy[0] + 4 < T) { by[1] = by[0] == 0 ? g.nby - 1 : by[0] - 1; oy[1] = oy[0] + 4; nyc = 2; }
-    bz[0] = (R + 1 + O) >> 2; oz[0] = (R + 1 + O) & 3;
-    if (bz[0] >= g.nbz) bz[0] -= g.nbz;
-    if (oz[0] + 4 < T) { bz[1] = bz[0] == 0 ? g.nbz - 1 : bz[0] - 1; oz[1] = oz[0] + 4; nzc = 2; }
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    long long fix[4] = {0, 0, 0, 0};  // exact: the fixed-point sums (units of 2^-32)
-    for (int a = 0; a < nxc; ++a)
-      for (int bb = 0; bb < nyc; ++bb)
-        for (int cc = 0; cc < nzc; ++cc) {
-          const long long brick = bx[a] + (long long)g.nbx * (by[bb] + (long long)g.nby * bz[cc]);
-          const long long at = brick * (4 * TNOD) + ox[a] + T * (oy[bb] + T * oz[cc]);
-          if (exact) {
-            const long long* src = static_cast<const long long*>(partial) + at;
-            for (int q = 4 - nq; q < 4; ++q) fix[q] += src[q * TNOD];
-          } else {
-            const float* src = static_cast<const float*>(partial) + at;
-            for (int q = 4 - nq; q < 4; ++q) acc[q] += src[q * TNOD];
-          }
-        }
-    if (exact)  // the one rounding of the exact sum
-      for (int q = 0; q < 4; ++q) acc[q] = (float)((double)fix[q] * FIX_INV);
-    const long long o = pid(g, P, Q, R);
-    if (nq == 4) store_img(g, np, P + 2, Q + 2, R + 2, acc[0]);  // np with its ghost images
-    S[o] = acc[1];
-    S[o + g.C] = acc[2];
-    S[o + 2 * g.C] = acc[3];
+    int i, j, k;
+    interior_of(g, t, i, j, k);
+    const int P = i - 2, Q = j - 2, R = k - 2;
+    // per axis: the tile that starts below the node, and the one before it
+    // when it reaches this far
+    const int ox = (P + 1 + O) & 3, oy = (Q + 1 + O) & 3, oz = (R + 1 + O) & 3;
+    int bx = (P + 1 + O) >> 2, by = (Q + 1 + O) >> 2, bz = (R + 1 + O) >> 2;
+    if (bx >= g.nbx) bx -= g.nbx;
+    if (by >= g.nby) by -= g.nby;
+    if (bz >= g.nbz) bz -= g.nbz;
+    const int bx1 = bx == 0 ? g.nbx - 1 : bx - 1, by1 = by == 0 ? g.nby - 1 : by - 1, bz1 = bz == 0 ? g.nbz - 1 : bz - 1;
+    V v[8][NQ];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const bool there = (!(c & 1) || ox + 4 < T) && (!(c & 2) || oy + 4 < T) && (!(c & 4) || oz + 4 < T);
+      const long long brick =
+          (c & 1 ? bx1 : bx) + (long long)g.nbx * ((c & 2 ? by1 : by) + (long long)g.nby * (c & 4 ? bz1 : bz));
+      const V* src = static_cast<const V*>(partial) + brick * (4 * TNOD) + (ox + (c & 1 ? 4 : 0)) +
+                     T * ((oy + (c & 2 ? 4 : 0)) + T * (oz + (c & 4 ? 4 : 0)));
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) v[c][q] = there ? src[(4 - NQ + q) * TNOD] : (V)0;
+    }
+    float acc[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      V s = v[0][q];
+      // (plain form: the order of the tiles is x outermost)
+#pragma unroll
+      for (int r = 1; r < 8; ++r) s += v[(r >> 2 & 1) | (r & 2) | (r & 1) << 2][q];
+      acc[q] = EXACT ? (float)((double)s * FIX_INV) : (float)s;  // exact: the one rounding of the sum
+    }
+    const long long o = nid(g, i, j, k);
+    if (NQ == 4) store_img(g, np, i, j, k, acc[0]);  // np with its ghost images
+    S[o] = acc[NQ - 3];
+    S[o + g.C] = acc[NQ - 2];
+    S[o + 2 * g.C] = acc[NQ - 1];
   }
 }
 
 // ---------------------------------------------------------------------------
 // fields (interior nodes, ghost images written by the producer)
 // ---------------------------------------------------------------------------
-
-// ct = S/np at the interior image; up_m = 0.5*(ct_m(node) + ct_m(node+e_m))
-// (gutsp.f:1825-1836); np and up with ghost images.
-// (The fast divide, two ulps: n is a density, far from where it loses accuracy.)
-__device__ __forceinline__ float ct_o(const float* np, const float* S, long long o, long long cm) {
-  const float n = np[o];
-  return n == 0.0f ? 0.0f : __fdividef(S[o + cm], n);
-}
-__device__ __forceinline__ float ct_at(const G32& g, const float* np, const float* S, int i, int j, int k, int m) {
-  return ct_o(np, S, nid(g, img(i, g.nx), img(j, g.ny), img(k, g.nz)), g.C * m);
-}
-
-__global__ void k_ct_up(G32 g, float* __restrict__ np, const float* __restrict__ S, float* __restrict__ up) {
-  GSTRIDE(t, n_int(g)) {
-    int i, j, k;
-    interior_of(g, t, i, j, k);
-    if (i > 2 && j > 2 && k > 2 && i < g.nx - 1 && j < g.ny - 1 && k < g.nz - 1) {
-      // the +1 neighbours interior and no ghost image to store: strides
-      const long long C = g.C, o = nid(g, i, j, k), sy = g.nx, sz = (long long)g.nx * g.ny;
-      up[o] = 0.5f * (ct_o(np, S, o, 0) + ct_o(np, S, o + 1, 0));
-      up[o + C] = 0.5f * (ct_o(np, S, o, C) + ct_o(np, S, o + sy, C));
-      up[o + 2 * C] = 0.5f * (ct_o(np, S, o, 2 * C) + ct_o(np, S, o + sz, 2 * C));
-      continue;
-    }
-    const float ux = 0.5f * (ct_at(g, np, S, i, j, k, 0) + ct_at(g, np, S, i + 1, j, k, 0));
-    const float uy = 0.5f * (ct_at(g, np, S, i, j, k, 1) + ct_at(g, np, S, i, j + 1, k, 1));
-    const float uz = 0.5f * (ct_at(g, np, S, i, j, k, 2) + ct_at(g, np, S, i, j, k + 1, 2));
-    store_img(g, up, i, j, k, ux);
-    store_img(g, up + g.C, i, j, k, uy);
-    store_img(g, up + 2 * g.C, i, j, k, uz);
-  }
-}
-
-// Cell-centre B from the edge field (edge_to_center, grid_interp.f:35-51)
-// with xrat = yrat = zrat = 1/2 (uniform grid), at an interior node.
-// I: the offset type, 32-bit unsigned where every offset of the call fits
-template <class I = long long>
-__device__ __forceinline__ void e2c_o(const G32& g, const float* bt, I o, float& c1, float& c2, float& c3) {
-  const I C = (I)g.C, sx = 1, sy = (I)g.nx, sz = (I)g.nx * (I)g.ny;
-  float b1, b2;
-  b2 = 0.5f * (bt[o] + bt[o - sy]);
-  b1 = 0.5f * (bt[o - sz] + bt[o - sy - sz]);
-  c1 = 0.5f * (b1 + b2);
-  const float* B = bt + C;
-  b2 = 0.5f * (B[o] + B[o - sx]);
-  b1 = 0.5f * (B[o - sz] + B[o - sx - sz]);
-  c2 = 0.5f * (b1 + b2);
-  B = bt + 2 * C;
-  b2 = 0.5f * (B[o] + B[o - sy]);
-  b1 = 0.5f * (B[o - sx] + B[o - sx - sy]);
-  c3 = 0.5f * (b1 + b2);
-}
-__device__ __forceinline__ void e2c(const G32& g, const float* bt, int i, int j, int k, float& c1, float& c2,
-                                    float& c3) {
-  e2c_o(g, bt, nid(g, i, j, k), c1, c2, c3);
-}
 
 // The isothermal electron-pressure gradient at the face of component m
 // (node o to o + e_m): grad_pe * (np(o+e_m) - np(o)) / d_m / n_face, n_face
@@ -713,50 +659,6 @@ __device__ __forceinline__ float gpe_face(const G32& g, const float* np, float g
   const I s = m == 0 ? (I)1 : (m == 1 ? (I)g.nx : (I)g.nx * (I)g.ny);
   const float inv = m == 0 ? g.inv_dx : (m == 1 ? g.inv_dy : g.inv_dz);
   return gp * ((np[o + s] - np[o]) * inv) / (0.5f * (np[o] + np[o + s]));
-}
-
-// Gather kit per physical node: (ajc - upc, btc) with ajc/upc =
-// face_to_center (grid_interp.f:163-170) and btc = edge_to_center of
-// dB plus the centred b0.
-__global__ void k_kit(G32 g, const float* __restrict__ aj, const float* __restrict__ up,
-                      const float* __restrict__ dbt, const float* __restrict__ b0c, const float* __restrict__ np,
-                      float gp, float4* __restrict__ kit, float4* __restrict__ kitg) {
-  GSTRIDE(t, n_int(g)) {
-    int i, j, k;
-    interior_of(g, t, i, j, k);
-    const long long C = g.C, o = nid(g, i, j, k), sx = 1, sy = g.nx, sz = (long long)g.nx * g.ny;
-    if (kitg)  // the pressure gradient centred like aj (face_to_center), for get_Ep
-      kitg[t] = make_float4(0.5f * (gpe_face<0>(g, np, gp, o) + gpe_face<0>(g, np, gp, o - sx)),
-                            0.5f * (gpe_face<1>(g, np, gp, o) + gpe_face<1>(g, np, gp, o - sy)),
-                            0.5f * (gpe_face<2>(g, np, gp, o) + gpe_face<2>(g, np, gp, o - sz)), 0.0f);
-    const float ax = 0.5f * ((aj[o] - up[o]) + (aj[o - sx] - up[o - sx]));
-    const float ay = 0.5f * ((aj[o + C] - up[o + C]) + (aj[o - sy + C] - up[o - sy + C]));
-    const float az = 0.5f * ((aj[o + 2 * C] - up[o + 2 * C]) + (aj[o - sz + 2 * C] - up[o - sz + 2 * C]));
-    float c1, c2, c3;
-    e2c(g, dbt, i, j, k, c1, c2, c3);
-    kit[2 * t] = make_float4(ax, ay, az, c1 + b0c[0]);
-    kit[2 * t + 1] = make_float4(c2 + b0c[1], c3 + b0c[2], 0.0f, 0.0f);
-  }
-}
-
-// curlB (gutsf.f:202-239) on dB with uniform spacing; curl(b0) = 0.
-__global__ void k_curlB(G32 g, const float* __restrict__ b, const float* __restrict__ np, float alpha,
-                        float* __restrict__ aj) {
-  GSTRIDE(t, n_int(g)) {
-    int i, j, k;
-    interior_of(g, t, i, j, k);
-    const long long C = g.C, o = nid(g, i, j, k), sx = 1, sy = g.nx, sz = (long long)g.nx * g.ny;
-    const float n0 = np[o];
-    const float* B1 = b;
-    const float* B2 = b + C;
-    const float* B3 = b + 2 * C;
-    const float c1 = (B3[o] - B3[o - sy]) * g.inv_dy + (B2[o - sz] - B2[o]) * g.inv_dz;
-    const float c2 = (B1[o] - B1[o - sz]) * g.inv_dz + (B3[o - sx] - B3[o]) * g.inv_dx;
-    const float c3 = (B2[o] - B2[o - sx]) * g.inv_dx + (B1[o - sy] - B1[o]) * g.inv_dy;
-    store_img(g, aj, i, j, k, c1 / (0.5f * (n0 + np[o + sx]) * alpha));
-    store_img(g, aj + C, i, j, k, c2 / (0.5f * (n0 + np[o + sy]) * alpha));
-    store_img(g, aj + 2 * C, i, j, k, c3 / (0.5f * (n0 + np[o + sz]) * alpha));
-  }
 }
 
 // ---- the field subcycle: two fused kernels per half step ----
@@ -816,6 +718,139 @@ __device__ __forceinline__ void ghost_images(const G32& g, int i, int j, int k, 
   }
 }
 
+// dB at a node and its lower neighbours: what curl dB there and one step down
+// each axis and the centred B need.
+struct Stencil {
+  float b1, b1y, b1z, b1yz, b2, b2x, b2z, b2xz, b3, b3x, b3y, b3xy;
+};
+__device__ __forceinline__ Stencil stencil_of(const G32& g, const float* db, unsigned o, const Off& d) {
+  const float *B1 = db, *B2 = db + g.C, *B3 = db + 2 * g.C;
+  return Stencil{B1[o], B1[o + d.ym], B1[o + d.zm], B1[o + d.ym + d.zm], B2[o], B2[o + d.xm], B2[o + d.zm],
+                 B2[o + d.xm + d.zm], B3[o], B3[o + d.xm], B3[o + d.ym], B3[o + d.xm + d.ym]};
+}
+// Component m of curl dB (gutsf.f:202-239) at the node, and (curl_down) one
+// step down axis m.
+__device__ __forceinline__ float curl_term(float f, float fm, float gm, float h, float i1, float i2) {
+  return (f - fm) * i1 + (gm - h) * i2;
+}
+template <int m>
+__device__ __forceinline__ float curl_at(const G32& g, const Stencil& s) {
+  if (m == 0) return curl_term(s.b3, s.b3y, s.b2z, s.b2, g.inv_dy, g.inv_dz);
+  if (m == 1) return curl_term(s.b1, s.b1z, s.b3x, s.b3, g.inv_dz, g.inv_dx);
+  return curl_term(s.b2, s.b2x, s.b1y, s.b1, g.inv_dx, g.inv_dy);
+}
+template <int m>
+__device__ __forceinline__ float curl_down(const G32& g, const Stencil& s) {
+  if (m == 0) return curl_term(s.b3x, s.b3xy, s.b2xz, s.b2x, g.inv_dy, g.inv_dz);
+  if (m == 1) return curl_term(s.b1y, s.b1yz, s.b3xy, s.b3y, g.inv_dz, g.inv_dx);
+  return curl_term(s.b2z, s.b2xz, s.b1yz, s.b1z, g.inv_dx, g.inv_dy);
+}
+// Cell-centre B from the edge field's values at the node, one step down two
+// axes, and both (edge_to_center, grid_interp.f:35-51, with ratios 1/2).
+__device__ __forceinline__ float centre(float v, float v1, float v2, float v12) {
+  const float h2 = 0.5f * (v + v1), h1 = 0.5f * (v2 + v12);
+  return 0.5f * (h1 + h2);
+}
+
+// ct = S/np (zero where no ion deposits; the fast divide, two ulps: n is a
+// density, far from where it loses accuracy).
+__device__ __forceinline__ float ct_of(float s, float n) { return n == 0.0f ? 0.0f : __fdividef(s, n); }
+
+// update_up's face average (gutsp.f:1825-1836) of ct, with ghost images, and
+// the whistler Courant time of check_time_step (gutsf.f:1782-1792) per node,
+// ghosts included, with its smallest value.  look[0]: that value (set large
+// before); look[1]: the error word as it stands (see field_loop).
+__global__ void __launch_bounds__(TPB) k_up_courant(G32 g, const float* __restrict__ np, const float* __restrict__ S,
+                                                    const float* __restrict__ db, const float* __restrict__ b0c,
+                                                    float alpha, float dx, float* __restrict__ up,
+                                                    float* __restrict__ dtn, unsigned* look, const int* err) {
+  float mn = 3.0e38f;
+  if (blockIdx.x == 0 && threadIdx.x == 0) look[1] = (unsigned)*err;
+  GSTRIDE(t, n_int(g)) {
+    int i, j, k;
+    interior_of(g, t, i, j, k);
+    const Off d = off_of(g, i, j, k);
+    const long long C = g.C;
+    const unsigned o = (unsigned)nid(g, i, j, k);
+    const float *s1 = S, *s2 = S + C, *s3 = S + 2 * C;
+    const float n = np[o], nx = np[o + d.xp], ny = np[o + d.yp], nz = np[o + d.zp];
+    const float a0 = s1[o], a1 = s1[o + d.xp], c0 = s2[o], c1 = s2[o + d.yp], e0 = s3[o], e1 = s3[o + d.zp];
+    const float b1 = db[o] + b0c[0], b2 = db[o + C] + b0c[1], b3 = db[o + 2 * C] + b0c[2];
+    const float btot = sqrtf(b1 * b1 + b2 * b2 + b3 * b3);
+    const float ak = 2.0f / dx;
+    const float q1 = ak * ak * btot / (alpha * n);
+    const float q2 = (ak * btot) * (ak * btot) / (alpha * n);
+    const float womega = 0.5f * (q1 + sqrtf(q1 * q1 + 4.0f * q2));
+    const float dt = dx / (womega / ak);
+    mn = fminf(mn, dt > 0.0f ? dt : 0.0f);
+    float* const f[4] = {up, up + C, up + 2 * C, dtn};
+    const float v[4] = {0.5f * (ct_of(a0, n) + ct_of(a1, nx)), 0.5f * (ct_of(c0, n) + ct_of(c1, ny)),
+                        0.5f * (ct_of(e0, n) + ct_of(e1, nz)), dt};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) f[q][o] = v[q];
+    ghost_images(g, i, j, k, f, v);
+  }
+  // one atomic per block (a grid of a few per SM): atomics from every warp to
+  // the one address serialise in L2
+  __shared__ float s_mn[TPB / 32];
+  for (int off = 16; off > 0; off >>= 1) mn = fminf(mn, __shfl_down_sync(0xffffffffu, mn, off));
+  if ((threadIdx.x & 31) == 0) s_mn[threadIdx.x >> 5] = mn;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) mn = fminf(mn, s_mn[w]);
+    atomicMin(look, __float_as_uint(mn));
+  }
+}
+
+// The passes' gather kit per physical node, from the moment sums and dB
+// alone: (ajc - upc, btc) with aj of curlB (gutsf.f:202-239) and up of
+// update_up (gutsp.f:1825-1836) at the node and one step down each axis,
+// face_to_center (grid_interp.f:163-170) of their difference, and
+// edge_to_center of dB plus the centred b0.  (256x128x128 cells, ms per
+// step with k_up_courant: 0.33; as up, curlB, kit and the Courant time in
+// kernels of their own with their arrays in between: 0.47.)
+// kitg (may be null): the pressure gradient centred like aj, for get_Ep.
+// Thread 0 also resets the far list's count and the Courant word, which the
+// rest of the step writes.
+__global__ void __launch_bounds__(TPB) k_kit(G32 g, const float* __restrict__ S, const float* __restrict__ db,
+                                             const float* __restrict__ b0c, const float* __restrict__ np, float alpha,
+                                             float gp, float4* __restrict__ kit, float4* __restrict__ kitg, int* far_n,
+                                             unsigned* look) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    *far_n = 0;
+    look[0] = 0x7f7fffffu;  // FLT_MAX
+  }
+  GSTRIDE(t, n_int(g)) {
+    int i, j, k;
+    interior_of(g, t, i, j, k);
+    const Off d = off_of(g, i, j, k);
+    const long long C = g.C;
+    const unsigned o = (unsigned)nid(g, i, j, k);
+    const Stencil s = stencil_of(g, db, o, d);
+    const float n0 = np[o], nxm = np[o + d.xm], nxp = np[o + d.xp], nym = np[o + d.ym], nyp = np[o + d.yp],
+                nzm = np[o + d.zm], nzp = np[o + d.zp];
+    const float *s1 = S, *s2 = S + C, *s3 = S + 2 * C;
+    const float x0 = ct_of(s1[o], n0), xm = ct_of(s1[o + d.xm], nxm), xp = ct_of(s1[o + d.xp], nxp);
+    const float y0 = ct_of(s2[o], n0), ym = ct_of(s2[o + d.ym], nym), yp = ct_of(s2[o + d.yp], nyp);
+    const float z0 = ct_of(s3[o], n0), zm = ct_of(s3[o + d.zm], nzm), zp = ct_of(s3[o + d.zp], nzp);
+    const float ux = 0.5f * (x0 + xp), uxm = 0.5f * (xm + x0), uy = 0.5f * (y0 + yp), uym = 0.5f * (ym + y0),
+                uz = 0.5f * (z0 + zp), uzm = 0.5f * (zm + z0);
+    const float a1 = curl_at<0>(g, s) / (0.5f * (n0 + nxp) * alpha), a1m = curl_down<0>(g, s) / (0.5f * (nxm + n0) * alpha);
+    const float a2 = curl_at<1>(g, s) / (0.5f * (n0 + nyp) * alpha), a2m = curl_down<1>(g, s) / (0.5f * (nym + n0) * alpha);
+    const float a3 = curl_at<2>(g, s) / (0.5f * (n0 + nzp) * alpha), a3m = curl_down<2>(g, s) / (0.5f * (nzm + n0) * alpha);
+    kit[2 * t] = make_float4(0.5f * ((a1 - ux) + (a1m - uxm)), 0.5f * ((a2 - uy) + (a2m - uym)),
+                             0.5f * ((a3 - uz) + (a3m - uzm)), centre(s.b1, s.b1y, s.b1z, s.b1yz) + b0c[0]);
+    kit[2 * t + 1] = make_float4(centre(s.b2, s.b2x, s.b2z, s.b2xz) + b0c[1],
+                                 centre(s.b3, s.b3y, s.b3x, s.b3xy) + b0c[2], 0.0f, 0.0f);
+    if (kitg) {
+      const unsigned sy = (unsigned)g.nx, sz = (unsigned)(g.nx * g.ny);
+      kitg[t] = make_float4(0.5f * (gpe_face<0>(g, np, gp, o) + gpe_face<0>(g, np, gp, o - 1u)),
+                            0.5f * (gpe_face<1>(g, np, gp, o) + gpe_face<1>(g, np, gp, o - sy)),
+                            0.5f * (gpe_face<2>(g, np, gp, o) + gpe_face<2>(g, np, gp, o - sz)), 0.0f);
+    }
+  }
+}
+
 // curlB (gutsf.f:202-239; curl b0 = 0 for the uniform b0), face_to_center(aj -
 // up) and the cross product of get_E (gutsf.f:1059-1075, crossf2 gutsf.f:
 // 65-76): writes aj and ct.  Predictor: B at cell centres from edge_to_center
@@ -830,12 +865,8 @@ __device__ __forceinline__ void aj_ct_node(const G32& g, const float* db, const 
   const Off d = off_of(g, i, j, k);
   const long long C = g.C;
   const unsigned o = (unsigned)nid(g, i, j, k);
-  const float *B1 = db, *B2 = db + C, *B3 = db + 2 * C, *u1 = up, *u2 = up + C, *u3 = up + 2 * C;
-  // B at the node and its lower neighbours: all that curl dB there and one
-  // step down each axis and the centred B need
-  const float b1 = B1[o], b1y = B1[o + d.ym], b1z = B1[o + d.zm], b1yz = B1[o + d.ym + d.zm];
-  const float b2 = B2[o], b2x = B2[o + d.xm], b2z = B2[o + d.zm], b2xz = B2[o + d.xm + d.zm];
-  const float b3 = B3[o], b3x = B3[o + d.xm], b3y = B3[o + d.ym], b3xy = B3[o + d.xm + d.ym];
+  const float *u1 = up, *u2 = up + C, *u3 = up + 2 * C;
+  const Stencil s = stencil_of(g, db, o, d);
   const float n0 = np[o], nxm = np[o + d.xm], nxp = np[o + d.xp], nym = np[o + d.ym], nyp = np[o + d.yp],
               nzm = np[o + d.zm], nzp = np[o + d.zp];
   const float ux = u1[o], uxm = u1[o + d.xm], uy = u2[o], uym = u2[o + d.ym], uz = u3[o], uzm = u3[o + d.zm];
@@ -853,22 +884,17 @@ __device__ __forceinline__ void aj_ct_node(const G32& g, const float* db, const 
     }
   }
   const float c0x = b0c[0], c0y = b0c[1], c0z = b0c[2];
-  auto curl = [](float f, float fm, float gm, float h, float i1, float i2) { return (f - fm) * i1 + (gm - h) * i2; };
-  const float a1 = __fdividef(curl(b3, b3y, b2z, b2, g.inv_dy, g.inv_dz), 0.5f * (n0 + nxp) * alpha);
-  const float a2 = __fdividef(curl(b1, b1z, b3x, b3, g.inv_dz, g.inv_dx), 0.5f * (n0 + nyp) * alpha);
-  const float a3 = __fdividef(curl(b2, b2x, b1y, b1, g.inv_dx, g.inv_dy), 0.5f * (n0 + nzp) * alpha);
-  const float a1m = __fdividef(curl(b3x, b3xy, b2xz, b2x, g.inv_dy, g.inv_dz), 0.5f * (nxm + n0) * alpha);
-  const float a2m = __fdividef(curl(b1y, b1yz, b3xy, b3y, g.inv_dz, g.inv_dx), 0.5f * (nym + n0) * alpha);
-  const float a3m = __fdividef(curl(b2z, b2xz, b1yz, b1z, g.inv_dx, g.inv_dy), 0.5f * (nzm + n0) * alpha);
+  const float a1 = __fdividef(curl_at<0>(g, s), 0.5f * (n0 + nxp) * alpha);
+  const float a2 = __fdividef(curl_at<1>(g, s), 0.5f * (n0 + nyp) * alpha);
+  const float a3 = __fdividef(curl_at<2>(g, s), 0.5f * (n0 + nzp) * alpha);
+  const float a1m = __fdividef(curl_down<0>(g, s), 0.5f * (nxm + n0) * alpha);
+  const float a2m = __fdividef(curl_down<1>(g, s), 0.5f * (nym + n0) * alpha);
+  const float a3m = __fdividef(curl_down<2>(g, s), 0.5f * (nzm + n0) * alpha);
   const float ax = 0.5f * ((a1 - ux) + (a1m - uxm));
   const float ay = 0.5f * ((a2 - uy) + (a2m - uym));
   const float az = 0.5f * ((a3 - uz) + (a3m - uzm));
-  // edge_to_center of the four values (node, step 1, step 2, both)
-  auto centre = [](float v, float v1, float v2, float v12) {
-    const float h2 = 0.5f * (v + v1), h1 = 0.5f * (v2 + v12);
-    return 0.5f * (h1 + h2);
-  };
-  float bx = centre(b1, b1y, b1z, b1yz), by = centre(b2, b2x, b2z, b2xz), bz = centre(b3, b3y, b3x, b3xy);
+  float bx = centre(s.b1, s.b1y, s.b1z, s.b1yz), by = centre(s.b2, s.b2x, s.b2z, s.b2xz),
+        bz = centre(s.b3, s.b3y, s.b3x, s.b3xy);
   if (CORR) {
     float lo[3], hi[3];
 #pragma unroll
@@ -1291,34 +1317,6 @@ __global__ void k_split_df(long long n, const double* __restrict__ a, float* __r
 __global__ void k_join_df(long long n, const float* __restrict__ h, const float* __restrict__ l,
                           double* __restrict__ a) {
   GSTRIDE(t, n) a[t] = (double)h[t] + (double)l[t];
-}
-
-// Whistler Courant time at every node, ghosts included, as check_time_step
-// loops over them (gutsf.f:1782-1792), plus the smallest value.
-__global__ void k_courant(G32 g, const float* __restrict__ dbt, const float* __restrict__ b0c,
-                          const float* __restrict__ np, float alpha, float dx, float* __restrict__ dtn, unsigned* out) {
-  float mn = 3.0e38f;
-  GSTRIDE(o, g.C) {
-    const float b1 = dbt[o] + b0c[0], b2 = dbt[o + g.C] + b0c[1], b3 = dbt[o + 2 * g.C] + b0c[2];
-    const float btot = sqrtf(b1 * b1 + b2 * b2 + b3 * b3);
-    const float ak = 2.0f / dx;
-    const float a1 = ak * ak * btot / (alpha * np[o]);
-    const float a2 = (ak * btot) * (ak * btot) / (alpha * np[o]);
-    const float womega = 0.5f * (a1 + sqrtf(a1 * a1 + 4.0f * a2));
-    const float d = dx / (womega / ak);
-    dtn[o] = d;
-    mn = fminf(mn, d > 0.0f ? d : 0.0f);
-  }
-  // one atomic per block (a grid of a few per SM): atomics from every warp to
-  // the one address serialise in L2
-  __shared__ float s_mn[TPB / 32];
-  for (int off = 16; off > 0; off >>= 1) mn = fminf(mn, __shfl_down_sync(0xffffffffu, mn, off));
-  if ((threadIdx.x & 31) == 0) s_mn[threadIdx.x >> 5] = mn;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) mn = fminf(mn, s_mn[w]);
-    atomicMin(out, __float_as_uint(mn));
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1822,18 +1820,26 @@ cudaError_t pass(int which, const G32& g, const Part& p, const Species& sp, cons
   return launch_pass<3, false, false>(PASS_ARGS);
 #undef PASS_ARGS
 }
-cudaError_t node_sum(const G32& g, int pass, const void* partial, int nq, bool exact, float* np, float* S,
-                     cudaStream_t st) {
-  const unsigned nb = nblk((long long)g.ncx * g.ncy * g.ncz);
-  if (pass_tile(pass) == TN) RET((k_node_sum<TN><<<nb, TPB, 0, st>>>(g, partial, nq, exact ? 1 : 0, np, S)));
-  RET((k_node_sum<TN_IN><<<nb, TPB, 0, st>>>(g, partial, nq, exact ? 1 : 0, np, S)));
+cudaError_t node_sum(const G32& g, int pass, const void* partial, bool exact, float* np, float* S, cudaStream_t st) {
+  const unsigned nb = nblk(n_int(g));
+  // pass 2 deposits no density
+  if (pass == 3 && exact) RET((k_node_sum<TN, 4, true><<<nb, TPB, 0, st>>>(g, partial, np, S)));
+  if (pass == 3) RET((k_node_sum<TN, 4, false><<<nb, TPB, 0, st>>>(g, partial, np, S)));
+  if (pass == 2 && exact) RET((k_node_sum<TN_IN, 3, true><<<nb, TPB, 0, st>>>(g, partial, np, S)));
+  if (pass == 2) RET((k_node_sum<TN_IN, 3, false><<<nb, TPB, 0, st>>>(g, partial, np, S)));
+  if (exact) RET((k_node_sum<TN_IN, 4, true><<<nb, TPB, 0, st>>>(g, partial, np, S)));
+  RET((k_node_sum<TN_IN, 4, false><<<nb, TPB, 0, st>>>(g, partial, np, S)));
 }
-cudaError_t ct_and_up(const G32& g, const float* np, const float* S, float* up, cudaStream_t st) {
-  RET((k_ct_up<<<nblk((long long)g.ncx * g.ncy * g.ncz), TPB, 0, st>>>(g, const_cast<float*>(np), S, up)));
+cudaError_t up_courant(const G32& g, const float* np, const float* S, const float* db, const float* b0c, float alpha,
+                       float dx, float* up, float* dtn, float* look, const int* err, cudaStream_t st) {
+  const unsigned nb = nblk(n_int(g)) < 152u * 8u ? nblk(n_int(g)) : 152u * 8u;
+  RET((k_up_courant<<<nb, TPB, 0, st>>>(g, np, S, db, b0c, alpha, dx, up, dtn, reinterpret_cast<unsigned*>(look),
+                                        err)));
 }
-cudaError_t build_kit(const G32& g, const float* aj, const float* up, const float* dbt, const float* b0c,
-                      const float* np, float gp, float4* kit, float4* kitg, cudaStream_t st) {
-  RET((k_kit<<<nblk((long long)g.ncx * g.ncy * g.ncz), TPB, 0, st>>>(g, aj, up, dbt, b0c, np, gp, kit, kitg)));
+cudaError_t build_kit(const G32& g, const float* S, const float* db, const float* b0c, const float* np, float alpha,
+                      float gp, float4* kit, float4* kitg, int* far_n, float* look, cudaStream_t st) {
+  RET((k_kit<<<nblk(n_int(g)), TPB, 0, st>>>(g, S, db, b0c, np, alpha, gp, kit, kitg, far_n,
+                                             reinterpret_cast<unsigned*>(look))));
 }
 __global__ void k_gpe(G32 g, const float* __restrict__ np, float gp, float* __restrict__ gpf) {
   GSTRIDE(t, n_int(g)) {
@@ -1847,9 +1853,6 @@ __global__ void k_gpe(G32 g, const float* __restrict__ np, float gp, float* __re
 }
 cudaError_t gpe_faces(const G32& g, const float* np, float gp, float* gpf, cudaStream_t st) {
   RET((k_gpe<<<nblk(n_int(g)), TPB, 0, st>>>(g, np, gp, gpf)));
-}
-cudaError_t curlB32(const G32& g, const float* dbt, const float* np, float alpha, float* aj, cudaStream_t st) {
-  RET((k_curlB<<<nblk((long long)g.ncx * g.ncy * g.ncz), TPB, 0, st>>>(g, dbt, np, alpha, aj)));
 }
 cudaError_t aj_ct(const G32& g, bool corr, const float* db, const float* np, const float* up, const float* b0c,
                   float alpha, float* aj, float* ct, cudaStream_t st) {
@@ -1937,13 +1940,6 @@ cudaError_t split_df(long long n, const double* a, float* h, float* l, cudaStrea
 }
 cudaError_t join_df(long long n, const float* h, const float* l, double* a, cudaStream_t st) {
   RET((k_join_df<<<nblk(n), TPB, 0, st>>>(n, h, l, a)));
-}
-cudaError_t courant_min(const G32& g, const float* dbt, const float* b0c, const float* np, float alpha, float dx,
-                        float* dtn, float* d_min, cudaStream_t st) {
-  cudaError_t e = cudaMemsetAsync(d_min, 0x7f, sizeof(unsigned), st);  // 3.39e38
-  if (e != cudaSuccess) return e;
-  const unsigned nb = nblk(g.C) < 152u * 8u ? nblk(g.C) : 152u * 8u;
-  RET((k_courant<<<nb, TPB, 0, st>>>(g, dbt, b0c, np, alpha, dx, dtn, reinterpret_cast<unsigned*>(d_min))));
 }
 // ---------------------------------------------------------------------------
 // ions that moved more than one cell in a step (pass 3's far list)

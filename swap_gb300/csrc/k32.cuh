@@ -176,19 +176,21 @@ cudaError_t far_scatter(const G32& g, const FarList& far, const int32_t* ncount,
                         const Part& src, const Part& dst, long long cap, int* err, cudaStream_t st);
 // Sum the brick partial tiles into np and S (interior nodes, (nx,ny,nz) layout).
 // pass: the pass (1-3) whose tiles `partial` holds
-cudaError_t node_sum(const G32& g, int pass, const void* partial, int nq, bool exact, float* np, float* S,
-                     cudaStream_t st);
+cudaError_t node_sum(const G32& g, int pass, const void* partial, bool exact, float* np, float* S, cudaStream_t st);
 
 // ---- fields ----
-cudaError_t ct_and_up(const G32& g, const float* np, const float* S, float* up, cudaStream_t st);
-// kitg (may be null): the electron-pressure face gradient of np (grad_pe
-// gp) centred per node, for the passes' gathered E.
-cudaError_t build_kit(const G32& g, const float* aj, const float* up, const float* dbt, const float* b0c,
-                      const float* np, float gp, float4* kit, float4* kitg, cudaStream_t st);
+// up from the node sums (pass 3's), and the Courant time per node (dtn).
+// look[0]: its smallest value; look[1]: the error word before the field step.
+cudaError_t up_courant(const G32& g, const float* np, const float* S, const float* db, const float* b0c, float alpha,
+                       float dx, float* up, float* dtn, float* look, const int* err, cudaStream_t st);
+// The passes' gather table from the node sums and dB.  kitg (may be null): the
+// electron-pressure face gradient of np (grad_pe gp) centred per node.  Also
+// resets *far_n and look[0].
+cudaError_t build_kit(const G32& g, const float* S, const float* db, const float* b0c, const float* np, float alpha,
+                      float gp, float4* kit, float4* kitg, int* far_n, float* look, cudaStream_t st);
 // gpf: the electron-pressure gradient at every face (with ghost images),
 // which E subtracts (the isothermal extension of gutsf.f:1083,1283).
 cudaError_t gpe_faces(const G32& g, const float* np, float gp, float* gpf, cudaStream_t st);
-cudaError_t curlB32(const G32& g, const float* dbt, const float* np, float alpha, float* aj, cudaStream_t st);
 // One half of a field subcycle in two fused kernels: aj and the cross
 // product ct (predictor: B from dB; corrector: B at m+1/2), then E on the
 // fly, curlE and B_new = base - coef*curlE in double-float (hi, lo float
@@ -245,8 +247,6 @@ cudaError_t grid_e_to_voxels(const G32& g, const float* E, float f, const float*
 // FP64 <-> double-float (hi + lo).
 cudaError_t split_df(long long n, const double* a, float* h, float* l, cudaStream_t st);
 cudaError_t join_df(long long n, const float* h, const float* l, double* a, cudaStream_t st);
-cudaError_t courant_min(const G32& g, const float* dbt, const float* b0c, const float* np, float alpha, float dx,
-                        float* dtn, float* d_min, cudaStream_t st);
 
 // ---- sort ----
 // Sort words and the direction-major counts dep[dir * nkeys + key] without pass 3.

@@ -54,7 +54,7 @@ struct F32State {
   float* b0c = nullptr;  // 3 floats: the uniform b0
   uint8_t* order = nullptr;  // source-key order table of the incremental sort
   float* dtn = nullptr;  // per-node Courant time
-  float* d_min = nullptr;
+  float* d_min = nullptr;  // its smallest value and a snapshot of the error word
   double* acc = nullptr;
   double last_dtsub = 0, last_ntf = 0;
   std::vector<void*> owned;
@@ -468,15 +468,11 @@ extern "C" int swap_f32_begin(swap_ctx* c) {
   return check_err(c);
 }
 
-// Deposit finish: node sums -> np (+ghosts) and up (maind.f:386-387 etc.).
-static int finish_deposit(swap_ctx* c, F32State* s, int pass, int nq) {
-  KL("f32_node_sum", node_sum(s->g, pass, s->partial, nq, s->exact, s->np, s->S, c->st));
-  // the rank sum of the raw node sums (MPI_ALLREDUCE, gutsp.f:1503,1812-1822);
-  // pass 2 deposits no density
-  if (nq == 4) TRY(c->exchange(s->np, s->np_span, 4));
-  else TRY(c->exchange(s->S, 3 * s->g.C, 4));
-  KL("f32_ct_up", ct_and_up(s->g, s->np, s->S, s->up, c->st));
-  return SWAP_OK;
+// A pass's node sums and their rank sum (MPI_ALLREDUCE, gutsp.f:1503,
+// 1812-1822); pass 2 deposits no density.
+static int deposit_sums(swap_ctx* c, F32State* s, int pass) {
+  KL("f32_node_sum", node_sum(s->g, pass, s->partial, s->exact, s->np, s->S, c->st));
+  return pass == 2 ? c->exchange(s->S, 3 * s->g.C, 4) : c->exchange(s->np, s->np_span, 4);
 }
 
 static int subcycles(swap_ctx* c, F32State* s, float* e_acc = nullptr) {
@@ -487,10 +483,8 @@ static int subcycles(swap_ctx* c, F32State* s, float* e_acc = nullptr) {
   // the smallest leaves dtsub alone nothing changes, otherwise the
   // reference's ordered halving (once per violating node, k innermost) is
   // replayed on the host from the node values.
-  KL("f32_courant", courant_min(g, s->db1, s->b0c, s->np, (float)c->prm.alpha, g.dx, s->dtn, s->d_min, c->st));
-  // a snapshot of the error word beside it: the sort on the second stream may
-  // still set the word itself
-  CU(cudaMemcpyAsync(s->d_min + 1, c->d_err, sizeof(int), cudaMemcpyDeviceToDevice, c->st));
+  // (formed with up after pass 3, with a snapshot of the error word beside
+  // them: the sort on the second stream may still set the word itself)
   CU(cudaMemcpyAsync(s->h_look, s->d_min, sizeof(F32State::Look), cudaMemcpyDeviceToHost, c->st));
   CU(cudaEventRecord(s->ev_look, c->st));
   // a small grid's subcycles go out before the host has looked: the kernel
@@ -809,15 +803,17 @@ static int one_step_body(swap_ctx* c, F32State* s) {
   const StepParams sp = step_params(c, s);
   const Part& p = s->buf[s->cur];
   KL("f32_P1", pass(1, g, p, s->sp, sp, s->start, s->kit, s->partial, nullptr, nullptr, c->d_err, s->exact, c->st));  // :385-387,399
-  TRY(finish_deposit(c, s, 1, 4));
-  KL("f32_curlB", curlB32(g, s->db1, s->np, (float)c->prm.alpha, s->aj, c->st));  // :395
-  KL("f32_kit", build_kit(g, s->aj, s->up, s->db1, s->b0c, s->np, s->gp, s->kit, s->kitg, c->st));  // :398, :183-184
+  TRY(deposit_sums(c, s, 1));
+  auto kit = [&] {  // :395, :398-400 (curlB, edge_to_center, up and get_Ep's face_to_center)
+    return build_kit(g, s->S, s->db1, s->b0c, s->np, (float)c->prm.alpha, s->gp, s->kit, s->kitg, s->far.n, s->d_min,
+                     c->st);
+  };
+  KL("f32_kit", kit());
   KL("f32_P2", pass(2, g, p, s->sp, sp, s->start, s->kit, s->partial, nullptr, nullptr, c->d_err, s->exact, c->st,
                     nullptr, s->kitg));  // :400-402
-  TRY(finish_deposit(c, s, 2, 3));
-  KL("f32_kit", build_kit(g, s->aj, s->up, s->db1, s->b0c, s->np, s->gp, s->kit, s->kitg, c->st));  // :404
+  TRY(deposit_sums(c, s, 2));
+  KL("f32_kit", kit());  // :404
   // :404-413, the final half move of :479 and res_chex; prepares the sort
-  CU(cudaMemsetAsync(s->far.n, 0, sizeof(int), c->st));
   KL("f32_P3", pass(3, g, p, s->sp, sp, s->start, s->kit, s->partial, s->dirrank, s->dep, c->d_err, s->exact,
                     c->st, &s->far, s->kitg));
   KL("f32_far_deposit", far_deposit(g, s->far, s->partial, s->exact, c->d_err, c->st));
@@ -832,7 +828,9 @@ static int one_step_body(swap_ctx* c, F32State* s) {
   // the sort on the second stream, beside the moments' sums and the field
   // subcycles: it reads pass 3's outputs and the staging, they the grids
   TRY(sort_step(c, s, c->src_step + 1, true, &pre, true));
-  TRY(finish_deposit(c, s, 3, 4));
+  TRY(deposit_sums(c, s, 3));
+  KL("f32_up_courant", up_courant(g, s->np, s->S, s->db1, s->b0c, (float)c->prm.alpha, g.dx, s->up, s->dtn, s->d_min,
+                                  c->d_err, c->st));
   if (s->gpf) KL("f32_gpe", gpe_faces(g, s->np, s->gp, s->gpf, c->st));  // E's pressure term at the new np
   TRY(field_step(c, s));                                                          // :420-476
   TRY(sort_join(c, s));
