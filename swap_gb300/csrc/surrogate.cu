@@ -90,6 +90,7 @@ struct ConvArgs {
   __nv_bfloat16* Y;                    // [V][COUT] activations out (may be null)
   __nv_bfloat16* Z;                    // [V][COUT] pre-activations out (may be null)
   float* Yf;                           // [V][ldf] FP32 out (may be null)
+  const __nv_bfloat16* Zb;             // [V][COUT] pre-activations of a data gradient (may be null)
   int ldf, nstore;                     // FP32 row length and channels stored
   int gelu;                            // apply GELU for Y
   int* err;
@@ -105,6 +106,50 @@ __device__ __forceinline__ float tanh_hw(float x) {
 constexpr float GELU_K0 = 0.7978845608028654f, GELU_K1 = 0.044715f;
 __device__ __forceinline__ float gelu(float x) {
   return 0.5f * x * (1.0f + tanh_hw(GELU_K0 * fmaf(GELU_K1 * x, x * x, x)));
+}
+
+__device__ __forceinline__ float gelu_grad(float x) {
+  const float t = tanh_hw(GELU_K0 * fmaf(GELU_K1 * x, x * x, x));
+  return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * GELU_K0 * fmaf(3.0f * GELU_K1, x * x, 1.0f);
+}
+
+__device__ __forceinline__ uint4 pack_bf16(const float* v) {
+  alignas(16) __nv_bfloat16 h[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) h[e] = __float2bfloat16(v[e]);
+  return *reinterpret_cast<const uint4*>(h);
+}
+
+// The epilogue's stores of N channels from c0 on of voxel vo (COUT per voxel,
+// the bias added): whatever of Z, Y and Yf is asked for; with Zb the value is
+// an output gradient, and Y is it times GELU'(Zb).
+template <int COUT, int N = COUT>
+__device__ __forceinline__ void conv_store(const ConvArgs& a, long long vo, int c0, const float (&acc)[N]) {
+  if (a.Z) {
+#pragma unroll
+    for (int c = 0; c < N; c += 8) *reinterpret_cast<uint4*>(a.Z + vo * COUT + c0 + c) = pack_bf16(acc + c);
+  }
+  if (a.Y) {
+#pragma unroll
+    for (int c = 0; c < N; c += 8) {
+      float v[8];
+      if (a.Zb) {
+        const uint4 zb = *reinterpret_cast<const uint4*>(a.Zb + vo * COUT + c0 + c);
+        const __nv_bfloat16* z = reinterpret_cast<const __nv_bfloat16*>(&zb);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = acc[c + e] * gelu_grad(__bfloat162float(z[e]));
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = a.gelu ? gelu(acc[c + e]) : acc[c + e];
+      }
+      *reinterpret_cast<uint4*>(a.Y + vo * COUT + c0 + c) = pack_bf16(v);
+    }
+  }
+  if (a.Yf) {
+#pragma unroll
+    for (int c = 0; c < N; ++c)
+      if (c0 + c < a.nstore) a.Yf[vo * a.ldf + c0 + c] = acc[c];
+  }
 }
 
 template <int CIN, int COUT>
@@ -187,29 +232,7 @@ __global__ void __launch_bounds__(128) k_conv3(ConvArgs a) {
     const long long vo = tile * 128 + warp * 32 + lane;
 #pragma unroll
     for (int c = 0; c < COUT; ++c) acc[c] += sbias[c];
-    if (a.Z) {
-#pragma unroll
-      for (int c = 0; c < COUT; c += 8) {
-        alignas(16) __nv_bfloat16 h[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) h[e] = __float2bfloat16(acc[c + e]);
-        *reinterpret_cast<uint4*>(a.Z + vo * COUT + c) = *reinterpret_cast<const uint4*>(h);
-      }
-    }
-    if (a.Y) {
-#pragma unroll
-      for (int c = 0; c < COUT; c += 8) {
-        alignas(16) __nv_bfloat16 h[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) h[e] = __float2bfloat16(a.gelu ? gelu(acc[c + e]) : acc[c + e]);
-        *reinterpret_cast<uint4*>(a.Y + vo * COUT + c) = *reinterpret_cast<const uint4*>(h);
-      }
-    }
-    if (a.Yf) {
-#pragma unroll
-      for (int c = 0; c < COUT; ++c)
-        if (c < a.nstore) a.Yf[vo * a.ldf + c] = acc[c];
-    }
+    conv_store<COUT>(a, vo, 0, acc);
     tc05::fence_before_sync();
     __syncthreads();  // accumulator reads done before the next tile's MMAs
     tc05::fence_after_sync();
@@ -293,29 +316,7 @@ __global__ void __launch_bounds__(256) k_conv3r(ConvArgs a, int ychunk) {
     const long long vo = v0 + q * 32 + lane;
 #pragma unroll
     for (int c = 0; c < HC; ++c) acc[c] += sbias[c0 + c];
-    if (a.Z) {
-#pragma unroll
-      for (int c = 0; c < HC; c += 8) {
-        alignas(16) __nv_bfloat16 h[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) h[e] = __float2bfloat16(acc[c + e]);
-        *reinterpret_cast<uint4*>(a.Z + vo * COUT + c0 + c) = *reinterpret_cast<const uint4*>(h);
-      }
-    }
-    if (a.Y) {
-#pragma unroll
-      for (int c = 0; c < HC; c += 8) {
-        alignas(16) __nv_bfloat16 h[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) h[e] = __float2bfloat16(a.gelu ? gelu(acc[c + e]) : acc[c + e]);
-        *reinterpret_cast<uint4*>(a.Y + vo * COUT + c0 + c) = *reinterpret_cast<const uint4*>(h);
-      }
-    }
-    if (a.Yf) {
-#pragma unroll
-      for (int c = 0; c < HC; ++c)
-        if (c0 + c < a.nstore) a.Yf[vo * a.ldf + c0 + c] = acc[c];
-    }
+    conv_store<COUT, HC>(a, vo, c0, acc);
   };
   constexpr uint32_t idesc = tc05::idesc_bf16_f32(128, COUT);
   const uint64_t adesc0 = tc05::desc_noswizzle(tc05::smem_u32(sR), PLANE, 128);
@@ -399,6 +400,147 @@ __global__ void __launch_bounds__(256) k_conv3r(ConvArgs a, int ychunk) {
   if (warp == 0) tc05::tmem_free(tslot, 64);
 }
 
+// The whole-row form, for rows of x that divide a tile (nx of 1, 2, 4 ... 64
+// with 128 % nx == 0): a tile is 128 / nx rows, so a tap's shift along x is a
+// rotation inside the tile's own rows.  Per (dy, dz) every thread loads one
+// voxel's channels and stores them three times, rotated by dx: 9 loads per
+// voxel instead of 27, all of a plane's (three dy) in registers one stage
+// ahead, and 9 taps per barrier.  (k_conv3, below, loads each tap as it
+// needs it: one load in flight per thread and a barrier per tap.  A 16 -> 16
+// layer of 64^3 voxels: 108 us there, 30 us here.)
+// Three stages (dz) per tile in two operand buffers; two accumulators let the
+// epilogue of a tile run beside the next tile's products.  The taps are
+// multiplied in the same order as in the other forms: the same bits.
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(128) k_conv3t(ConvArgs a) {
+  static_assert(CIN % 16 == 0 && (COUT == 16 || COUT == 32), "operand shapes");
+  constexpr int KG = CIN / 8, WBYTES = 27 * COUT * CIN * 2, ABYTES = 128 * CIN * 2, SBYTES = 9 * ABYTES;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t* sW = smem;
+  uint8_t* sA = smem + WBYTES;
+  __shared__ uint64_t mbar[2];
+  __shared__ uint32_t tslot;
+  __shared__ float sbias[COUT];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  for (int i = tid; i < 27 * COUT * KG; i += 128) {
+    const int t = i / (COUT * KG), r = i % (COUT * KG), n = r / KG, k = 8 * (r % KG);
+    *reinterpret_cast<uint4*>(sW + t * (COUT * CIN * 2) + tc05::core_offset(n, k, COUT)) =
+        reinterpret_cast<const uint4*>(a.W)[i];
+  }
+  if (tid < COUT) sbias[tid] = a.bias ? a.bias[tid] : 0.0f;
+  if (warp == 0) tc05::tmem_alloc(&tslot, 64);
+  if (tid == 0) {
+    tc05::mbar_init(&mbar[0], 1);
+    tc05::mbar_init(&mbar[1], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  tc05::fence_before_sync();
+  __syncthreads();
+  tc05::fence_after_sync();
+  const uint32_t tmem = tslot;
+  const int nx = a.nx, ny = a.ny, nz = a.nz, rows = 128 / nx;
+  const int x = tid % nx, row = tid / nx;
+  // where this thread's voxel goes as the neighbour at dx = -1, 0, 1
+  int dst[3];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const int xo = x - (q - 1);
+    dst[q] = row * nx + (xo < 0 ? xo + nx : (xo >= nx ? xo - nx : xo));
+  }
+  constexpr uint32_t idesc = tc05::idesc_bf16_f32(128, COUT);
+  const uint64_t adesc0 = tc05::desc_noswizzle(tc05::smem_u32(sA), 16 * 128, 128);
+  const uint64_t bdesc0 = tc05::desc_noswizzle(tc05::smem_u32(sW), (COUT / 8) * 128, 128);
+  const int ntiles = (int)(a.V / 128);
+  uint4 reg[3][KG];
+  auto load = [&](int tile, int dz) {  // the three dy of plane z + dz - 1
+    const int r = tile * rows + row, y = r % ny, z = r / ny;
+    int zz = z + dz - 1;
+    zz = zz < 0 ? zz + nz : (zz >= nz ? zz - nz : zz);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      int yy = y + d - 1;
+      yy = yy < 0 ? yy + ny : (yy >= ny ? yy - ny : yy);
+      const uint4* src = reinterpret_cast<const uint4*>(a.X + ((long long)(zz * ny + yy) * nx + x) * CIN);
+#pragma unroll
+      for (int q = 0; q < KG; ++q) reg[d][q] = src[q];
+    }
+  };
+  auto epilogue = [&](int tile, int b) {
+    float acc[COUT];
+    const uint32_t taddr = tmem + (uint32_t)(b * 32) + ((uint32_t)(warp * 32) << 16);
+    if constexpr (COUT == 32) tc05::tmem_ld32(taddr, acc);
+    else tc05::tmem_ld16(taddr, acc);
+    const long long vo = (long long)tile * 128 + warp * 32 + lane;
+#pragma unroll
+    for (int c = 0; c < COUT; ++c) acc[c] += sbias[c];
+    conv_store<COUT>(a, vo, 0, acc);
+  };
+  bool ok = true;
+  int stage = 0, acc = 0, prev = -1;
+  if ((int)blockIdx.x < ntiles) load(blockIdx.x, 0);
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, acc ^= 1) {
+    for (int dz = 0; dz < 3; ++dz, ++stage) {
+      const int b = stage & 1;
+      // the products of the stage before last are done: its buffer is free
+      if (stage >= 2) ok &= tc05::mbar_wait(&mbar[b], (uint32_t)(stage / 2 - 1) & 1u, WAIT_LIMIT);
+      uint8_t* buf = sA + b * SBYTES;
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+#pragma unroll
+          for (int kg = 0; kg < KG; ++kg)
+            *reinterpret_cast<uint4*>(buf + (3 * d + q) * ABYTES + tc05::core_offset(dst[q], 8 * kg, 128)) = reg[d][kg];
+      tc05::fence_async_smem();
+      tc05::fence_before_sync();
+      __syncthreads();
+      tc05::fence_after_sync();
+      if (tid == 0) {
+#pragma unroll
+        for (int t = 0; t < 9; ++t)
+#pragma unroll
+          for (int kk = 0; kk < KG / 2; ++kk) {
+            const uint32_t aoff = (uint32_t)(b * SBYTES + t * ABYTES + kk * 2 * (16 * 128));
+            const uint32_t boff = (uint32_t)((9 * dz + t) * (COUT * CIN * 2) + kk * 2 * ((COUT / 8) * 128));
+            tc05::mma_bf16(tmem + acc * 32, adesc0 + (aoff >> 4), bdesc0 + (boff >> 4), idesc,
+                           dz > 0 || t > 0 || kk > 0);
+          }
+        tc05::mma_commit(&mbar[b]);
+      }
+      // the next stage's loads
+      if (dz < 2) load(tile, dz + 1);
+      else if (tile + (int)gridDim.x < ntiles) load(tile + gridDim.x, 0);
+      // the last tile's products were waited for above, in its last stage's
+      // buffer: two stages ago
+      if (dz == 1 && prev >= 0) {
+        tc05::fence_after_sync();
+        epilogue(prev, acc ^ 1);
+        tc05::fence_before_sync();
+      }
+    }
+    prev = tile;
+  }
+  if (prev >= 0) {  // the last tile: both of its latest stages
+    for (int s = stage - 2; s < stage; ++s) ok &= tc05::mbar_wait(&mbar[s & 1], (uint32_t)(s / 2) & 1u, WAIT_LIMIT);
+    tc05::fence_after_sync();
+    epilogue(prev, acc ^ 1);
+  }
+  if (!ok) atomicCAS(a.err, 0, SWAP_EWAIT);
+  tc05::fence_before_sync();
+  __syncthreads();
+  if (warp == 0) tc05::tmem_free(tmem, 64);
+}
+
+template <int CIN, int COUT>
+cudaError_t launch_conv3t(const ConvArgs& a, int nsm, cudaStream_t st) {
+  const int smem = 27 * COUT * CIN * 2 + 2 * 9 * 128 * CIN * 2;
+  cudaError_t e = cudaFuncSetAttribute(k_conv3t<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  const long long ntiles = a.V / 128, most = (CIN == 16 ? 2LL : 1LL) * nsm;  // blocks that fit in shared memory
+  k_conv3t<CIN, COUT><<<(unsigned)(ntiles < most ? ntiles : most), 128, smem, st>>>(a);
+  return cudaGetLastError();
+}
+
 template <int CIN, int COUT>
 cudaError_t launch_conv3r(const ConvArgs& a, int nsm, cudaStream_t st) {
   constexpr int KG = CIN / 8, RP = KG == 2 ? 132 : 130;
@@ -422,6 +564,7 @@ cudaError_t launch_conv3r(const ConvArgs& a, int nsm, cudaStream_t st) {
 template <int CIN, int COUT>
 cudaError_t launch_conv3(const ConvArgs& a, int nsm, cudaStream_t st) {
   if (a.nx % 128 == 0) return launch_conv3r<CIN, COUT>(a, nsm, st);
+  if (128 % a.nx == 0) return launch_conv3t<CIN, COUT>(a, nsm, st);
   const int smem = 27 * COUT * CIN * 2 + 2 * 128 * CIN * 2;
   cudaError_t e = cudaFuncSetAttribute(k_conv3<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
@@ -536,11 +679,6 @@ constexpr LayerDims LCOUT = layer_dims(false);  // last layer: 3 output channels
 constexpr int NIN = 14, NOUT = 3;
 static_assert(NIN <= 16, "the first layer's input is padded to 16 channels");
 
-__device__ __forceinline__ float gelu_grad(float x) {
-  const float t = tanh_hw(GELU_K0 * fmaf(GELU_K1 * x, x * x, x));
-  return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * GELU_K0 * fmaf(3.0f * GELU_K1, x * x, 1.0f);
-}
-
 // Normalised BF16 inputs [V][16] from FP32 [V][NIN].
 __global__ void k_norm_inputs(long long V, const float* __restrict__ in, const float* __restrict__ mean,
                               const float* __restrict__ inv_std, __nv_bfloat16* __restrict__ x) {
@@ -654,13 +792,6 @@ __global__ void k_loss_curl(int nx, int ny, int nz, const float* __restrict__ ou
   }
   for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
   if ((threadIdx.x & 31) == 0) atomicAdd(acc, s);
-}
-
-// dZ = dY * GELU'(Z) as BF16 [V][C].
-__global__ void k_gelu_back(long long n, const float* __restrict__ dy, const __nv_bfloat16* __restrict__ z,
-                            __nv_bfloat16* __restrict__ dz) {
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
-    dz[t] = __float2bfloat16(dy[t] * gelu_grad(__bfloat162float(z[t])));
 }
 
 // Weight gradient of a periodic conv layer on the CUDA cores:
@@ -833,6 +964,144 @@ __global__ void __launch_bounds__(128) k_conv3_dw_tc(int nx, int ny, int nz, lon
   if (warp == 0) tc05::tmem_free(tmem, 32);
 }
 
+// Weight and bias gradients by lines, for rows of x that are whole groups of
+// 16 voxels.  The voxels are K, and a voxel's channel vector is 16 contiguous
+// bytes per 8 channels in memory already: as the M-major A operand (and the
+// N-major B of dZ) it goes to shared memory as it is, with 16-byte
+// asynchronous copies, where k_conv3_dw_tc transposes every value into the
+// K-major layout with a 2-byte store, per tap.  A stage holds the nine lines
+// (dy, dz) around SEG voxels of a row, one voxel longer at either end: the
+// three taps along x read them one voxel (16 bytes) apart.  The rows of a
+// product are (line, channel); a tenth line of ones makes one row of dx = 0
+// the bias gradient.  Rows past it are products with whatever lies there, and
+// are not read.  One block per SM (NST stages in flight) adds its sums with
+// FP32 atomics.
+// 16 -> 16 channels, 64^3 voxels, with the bias: 165 us transposing, 59 us.
+template <int CIN, int COUT>
+struct DwLines {
+  static constexpr int KG = CIN / 8, SEG = 64, PLANE = (SEG + 4) * 16, LINE = KG * PLANE;
+  static constexpr int NB = (9 * CIN + 127) / 128;       // products of 128 rows that cover the lines
+  static constexpr int ABYTES = 10 * LINE, BPLANE = SEG * 16, BBYTES = (COUT / 8) * BPLANE;
+  static constexpr int NST = CIN == 16 ? 4 : 3;
+  static constexpr int TAIL = (NB * (128 / CIN) - 10) * LINE;  // read past the last stage's lines
+  static constexpr int SMEM = NST * (ABYTES + BBYTES) + TAIL;
+  static constexpr int COLS = 3 * NB * COUT <= 128 ? 128 : (3 * NB * COUT <= 256 ? 256 : 512);
+};
+constexpr int DW_TPB = 9 * 32;  // a warp per line
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(DW_TPB) k_conv3_dw_lines(int nx, int ny, int nz, const __nv_bfloat16* __restrict__ X,
+                                                        const __nv_bfloat16* __restrict__ dZ, float* __restrict__ gW,
+                                                        float* __restrict__ gb, int units_per_block, int* err) {
+  using D = DwLines<CIN, COUT>;
+  constexpr int KG = D::KG, SEG = D::SEG, NB = D::NB, NST = D::NST;
+  extern __shared__ __align__(1024) uint8_t smem[];  // NST A stages, then NST B stages, then the tail
+  uint8_t* const sB = smem + NST * D::ABYTES;
+  __shared__ uint64_t mbar[NST];
+  __shared__ uint32_t tslot;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  for (int i = tid; i < NST * D::LINE / 4; i += DW_TPB)  // the lines of ones
+    *reinterpret_cast<uint32_t*>(smem + (i / (D::LINE / 4)) * D::ABYTES + 9 * D::LINE + (i % (D::LINE / 4)) * 4) =
+        0x3f803f80u;
+  if (warp == 0) tc05::tmem_alloc(&tslot, D::COLS);
+  if (tid == 0) {
+    for (int q = 0; q < NST; ++q) tc05::mbar_init(&mbar[q], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  tc05::fence_before_sync();
+  __syncthreads();
+  tc05::fence_after_sync();
+  const uint32_t tmem = tslot;
+  // both operands with the channels contiguous (bits 15 and 16)
+  constexpr uint32_t idesc = tc05::idesc_bf16_f32(128, COUT) | (1u << 15) | (1u << 16);
+  const int segs = (nx + SEG - 1) / SEG;
+  const long long nunits = (long long)segs * ny * nz, u0 = (long long)blockIdx.x * units_per_block;
+  const int n = (int)(nunits - u0 < units_per_block ? nunits - u0 : units_per_block);
+  auto seg_len = [&](int seg) { return nx - seg * SEG < SEG ? nx - seg * SEG : SEG; };
+  auto load = [&](int i) {  // unit u0 + i into stage i % NST
+    const long long u = u0 + i;
+    const int seg = (int)(u % segs), y = (int)(u / segs % ny), z = (int)(u / ((long long)segs * ny));
+    const int x0 = seg * SEG, len = seg_len(seg), per = (len + 2) * KG;
+    uint8_t* A = smem + (i % NST) * D::ABYTES;
+    uint8_t* B = sB + (i % NST) * D::BBYTES;
+    // warp l copies line l, and its share of dZ
+    int yy = y + warp % 3 - 1, zz = z + warp / 3 - 1;
+    yy = yy < 0 ? yy + ny : (yy >= ny ? yy - ny : yy);
+    zz = zz < 0 ? zz + nz : (zz >= nz ? zz - nz : zz);
+    const __nv_bfloat16* row = X + (long long)(zz * ny + yy) * nx * CIN;
+    uint8_t* dst = A + warp * D::LINE;
+    for (int it = lane; it < per; it += 32) {
+      const int p = it % KG, q = it / KG;
+      int x = x0 - 1 + q;
+      x = x < 0 ? x + nx : (x >= nx ? x - nx : x);
+      tc05::cp_async16(dst + p * D::PLANE + q * 16, row + x * CIN + 8 * p);
+    }
+    const __nv_bfloat16* drow = dZ + ((long long)(z * ny + y) * nx + x0) * COUT;
+    for (int it = tid; it < len * (COUT / 8); it += DW_TPB) {
+      const int p = it % (COUT / 8), q = it / (COUT / 8);
+      tc05::cp_async16(B + p * D::BPLANE + q * 16, drow + q * COUT + 8 * p);
+    }
+  };
+  bool ok = true;
+  for (int i = 0; i < NST - 1; ++i) {
+    if (i < n) load(i);
+    tc05::cp_async_commit();
+  }
+  for (int i = 0; i < n; ++i) {
+    tc05::cp_async_wait<NST - 2>();
+    tc05::fence_async_smem();
+    tc05::fence_before_sync();
+    __syncthreads();
+    tc05::fence_after_sync();
+    if (tid == 0) {
+      const int len = seg_len((int)((u0 + i) % segs));
+      // M- and N-major: 8 voxels (K) 128 bytes apart, 8 channels a plane apart
+      const uint64_t ad = tc05::desc_noswizzle(tc05::smem_u32(smem + (i % NST) * D::ABYTES), 128, D::PLANE);
+      const uint64_t bd = tc05::desc_noswizzle(tc05::smem_u32(sB + (i % NST) * D::BBYTES), 128, D::BPLANE);
+      for (int kk = 0; kk < len / 16; ++kk)
+#pragma unroll
+        for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+          for (int mb = 0; mb < NB; ++mb)
+            tc05::mma_bf16(tmem + (dx * NB + mb) * COUT,
+                           ad + ((mb * (128 / CIN) * D::LINE + (16 * kk + dx) * 16) >> 4), bd + ((16 * kk * 16) >> 4),
+                           idesc, i > 0 || kk > 0);
+      tc05::mma_commit(&mbar[i % NST]);
+    }
+    // stage i - 1's products are done: its buffer takes unit i - 1 + NST
+    if (i > 0) ok &= tc05::mbar_wait(&mbar[(i - 1) % NST], (uint32_t)((i - 1) / NST) & 1u, WAIT_LIMIT);
+    tc05::fence_after_sync();
+    if (i > 0 ? i - 1 + NST < n : NST - 1 < n) load(i - 1 + NST);
+    tc05::cp_async_commit();
+  }
+  if (n > 0) ok &= tc05::mbar_wait(&mbar[(n - 1) % NST], (uint32_t)((n - 1) / NST) & 1u, WAIT_LIMIT);
+  tc05::cp_async_wait_all();
+  tc05::fence_after_sync();
+  if (n > 0 && warp < 4) {  // the accumulator's 128 rows
+    const int r = warp * 32 + lane, ci = r % CIN;
+#pragma unroll 1
+    for (int q = 0; q < 3 * NB; ++q) {
+      const int dx = q / NB, line = (q % NB) * (128 / CIN) + r / CIN;
+      float acc[COUT];
+      const uint32_t taddr = tmem + (uint32_t)(q * COUT) + ((uint32_t)(warp * 32) << 16);
+      if constexpr (COUT == 32) tc05::tmem_ld32(taddr, acc);
+      else tc05::tmem_ld16(taddr, acc);
+      if (!ok) continue;
+      if (line < 9) {
+        float* w = gW + (long long)(3 * line + dx) * COUT * CIN + ci;
+#pragma unroll
+        for (int co = 0; co < COUT; ++co) atomicAdd(w + co * CIN, acc[co]);
+      } else if (line == 9 && ci == 0 && dx == 0) {
+#pragma unroll
+        for (int co = 0; co < COUT; ++co) atomicAdd(gb + co, acc[co]);
+      }
+    }
+  }
+  if (!ok) atomicCAS(err, 0, SWAP_EWAIT);
+  tc05::fence_before_sync();
+  __syncthreads();
+  if (warp == 0) tc05::tmem_free(tmem, D::COLS);
+}
+
 // gb[co] += sum_v dZ[v][co].
 template <int COUT>
 __global__ void __launch_bounds__(256) k_bias_grad(long long V, const __nv_bfloat16* __restrict__ dZ,
@@ -900,6 +1169,17 @@ cudaError_t conv3_dw(int nx, int ny, int nz, long long V, const __nv_bfloat16* X
     k_conv3_dw<CIN, COUT><<<grid, 256, 0, st>>>(nx, ny, nz, V, X, dZ, gW, gb, vchunk);
     return cudaGetLastError();
   }
+  if (nx % 16 == 0) {
+    using D = DwLines<CIN, COUT>;
+    cudaError_t e = cudaFuncSetAttribute(k_conv3_dw_lines<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         D::SMEM);
+    if (e != cudaSuccess) return e;
+    const long long units = (long long)((nx + D::SEG - 1) / D::SEG) * ny * nz;
+    const long long per = (units + 151) / 152;
+    k_conv3_dw_lines<CIN, COUT><<<(unsigned)((units + per - 1) / per), DW_TPB, D::SMEM, st>>>(nx, ny, nz, X, dZ, gW, gb,
+                                                                                          (int)per, err);
+    return cudaGetLastError();
+  }
   // voxel chunks of a multiple of 64 (V is a multiple of 128), about 152 x 4
   // blocks over all tap groups
   constexpr int TPG = 128 / CIN, NG = (27 + TPG - 1) / TPG;
@@ -957,7 +1237,7 @@ struct swap_surrogate {
   __nv_bfloat16 *Z[NL - 1] = {}, *Y[NL - 1] = {};  // [V][32]
   float* out = nullptr;                    // [V][3]
   __nv_bfloat16* d16 = nullptr;            // [V][16]
-  float* dy = nullptr;                     // [V][32]
+  float* dy = nullptr;                     // [V][6], the curl loss's e and curl e
   __nv_bfloat16 *dzA = nullptr, *dzB = nullptr;  // [V][32]
   float* acc = nullptr;
   int* err = nullptr;
@@ -1016,7 +1296,7 @@ int ensure_shape(swap_surrogate* net, int nx, int ny, int nz) {
   }
   net->out = static_cast<float*>(take(V * NOUT * 4));
   net->d16 = static_cast<__nv_bfloat16*>(take(V * 16 * 2));
-  net->dy = static_cast<float*>(take(V * (HID > 6 ? HID : 6) * 4));  // also the curl loss's scratch (6 V)
+  net->dy = static_cast<float*>(take(V * 6 * 4));
   net->dzA = static_cast<__nv_bfloat16*>(take(V * HID * 2));
   net->dzB = static_cast<__nv_bfloat16*>(take(V * HID * 2));
   if (net->work.size() != 2 * (NL - 1) + 6) {  // x0, Z and Y per hidden layer, out, d16, dy, dzA, dzB
@@ -1080,17 +1360,15 @@ int backward(swap_surrogate* net, cudaStream_t st) {
   SCU((conv3_dw<HID, 16>(nx, ny, nz, V, net->Y[L - 1], net->d16, net->gw[L], net->gb[L], net->err, net->dw_cores,
                           st)));
   ConvArgs a = conv_args(net);
-  a.Y = nullptr; a.Z = nullptr; a.bias = nullptr; a.gelu = 0; a.ldf = HID; a.nstore = HID; a.Yf = net->dy;
-  // last layer -> the one before: the data gradient, then through its GELU
-  a.X = net->d16; a.W = net->wt[L];
-  SCU(conv3(16, HID, a, st));
+  a.Z = nullptr; a.bias = nullptr; a.Yf = nullptr;
+  // last layer -> the one before: the data gradient, through its GELU as it is stored
   __nv_bfloat16 *dz = net->dzA, *dz_next = net->dzB;
-  k_gelu_back<<<nblk(V * HID), 256, 0, st>>>(V * HID, net->dy, net->Z[L - 1], dz);
+  a.X = net->d16; a.W = net->wt[L]; a.Y = dz; a.Zb = net->Z[L - 1];
+  SCU(conv3(16, HID, a, st));
   for (int l = L - 1; l >= 1; --l) {  // layer l -> l - 1
     SCU((conv3_dw<HID, HID>(nx, ny, nz, V, net->Y[l - 1], dz, net->gw[l], net->gb[l], net->err, net->dw_cores, st)));
-    a.X = dz; a.W = net->wt[l];
+    a.X = dz; a.W = net->wt[l]; a.Y = dz_next; a.Zb = net->Z[l - 1];
     SCU(conv3(HID, HID, a, st));
-    k_gelu_back<<<nblk(V * HID), 256, 0, st>>>(V * HID, net->dy, net->Z[l - 1], dz_next);
     std::swap(dz, dz_next);
   }
   SCU((conv3_dw<16, HID>(nx, ny, nz, V, net->x0, dz, net->gw[0], net->gb[0], net->err, net->dw_cores, st)));
@@ -1132,7 +1410,7 @@ int adam_step(swap_surrogate* net, float lr, cudaStream_t st) {
 int loss_grad(swap_surrogate* net, const float* tgt, float gnorm, double* sq, cudaStream_t st) {
   SCU(cudaMemsetAsync(net->acc, 0, 2 * sizeof(float), st));
   const bool curl = net->curl_w > 0.0f && net->kref2 > 0.0;
-  if (curl) {  // e and curl e in the (free until the backward pass) dy buffer
+  if (curl) {
     float *e = net->dy, *kap = net->dy + 3 * net->V;
     k_err3<<<nblk(net->V), 256, 0, st>>>(net->V, net->out, tgt, net->on, e);
     k_curl3<<<nblk(net->V), 256, 0, st>>>(net->nx, net->ny, net->nz, e, kap, net->acc + 1);
