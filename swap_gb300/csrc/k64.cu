@@ -5,7 +5,10 @@
 // everything except the atomic deposit sums reproduces the FP64 CPU
 // restatement bit for bit.  One thread per node (interior nodes for the
 // stencils) or per particle.
+#include <cmath>
+
 #include "k64.cuh"
+#include "k64_dev.cuh"
 
 namespace swapk {
 namespace {
@@ -79,21 +82,13 @@ __global__ void k_deltat(Geo g, const double* __restrict__ bt, const double* __r
 // get_interp_weights (gutsp.f:1391-1432).
 __global__ void k_weights(Geo g, PartDev p, long long N, int* err) {
   GRID_STRIDE(l, N) {
-    const double x = p.xp[l], y = p.xp[l + p.NM], z = p.xp[l + 2 * p.NM];
-    const int i = cell_search(g.qx, g.nx, x, g.inv_dx);
-    const int j = (int)floor(y / g.dy);
-    const int k = cell_search(g.qz, g.nz, z, g.inv_dz);
+    int i, j, k;
+    double w[8];
+    if (!weights_at(g, p.xp[l], p.xp[l + p.NM], p.xp[l + 2 * p.NM], i, j, k, w)) set_err(err, KERR_DOMAIN);
     p.ijk[l] = i;
     p.ijk[l + p.NM] = j;
     p.ijk[l + 2 * p.NM] = k;
-    if (i < 1 || j < 1 || j >= g.ny || k < 1) {
-      set_err(err, KERR_DOMAIN);
-      for (int c = 0; c < 8; ++c) p.wght[l + c * p.NM] = 0.0;
-      p.ijk[l] = 1; p.ijk[l + p.NM] = 1; p.ijk[l + 2 * p.NM] = 1;
-      continue;
-    }
-    double w[8];
-    weights8(g, i, j, k, x, y, z, w);
+#pragma unroll
     for (int c = 0; c < 8; ++c) p.wght[l + c * p.NM] = w[c];
   }
 }
@@ -111,7 +106,6 @@ __device__ __forceinline__ void corners(const Geo& g, int i, int j, int k, long 
   nd[4] = o + sy; nd[5] = o + 1 + sy; nd[6] = o + sy + sz; nd[7] = o + 1 + sy + sz;
 }
 
-// update_np deposit (gutsp.f:1461-1493) into the folded node.
 // One value into a deterministic fixed-point sum (Fix64); a value out of
 // range or not finite is flagged instead (the conversions saturate).
 __device__ __forceinline__ void fix_add(const Fix64& f, long long t, double x, unsigned& bad) {
@@ -132,9 +126,89 @@ __global__ void k_fix_to_double(long long n, Fix64 f, double* __restrict__ out) 
   }
 }
 
-template <bool DET>
-__global__ void k_deposit_np(Geo g, PartDev p, long long N, double beta, double* __restrict__ np, Fix64 fx,
-                             int* err) {
+// The velocity a particle deposits, by mode (see deposit_u).
+__device__ __forceinline__ void deposit_velocity(const PartDev& p, long long l, int mode, const double* va,
+                                                 const double* vb, double* out_v1, double v[3]) {
+  const double sq = mode >= 3 ? sqrt(p.mrat[l]) : 1.0;
+  for (int m = 0; m < 3; ++m) {
+    const double a = va[l + m * p.NM];
+    if (mode == 0) v[m] = a;
+    else if (mode == 1) v[m] = 1.5 * a - 0.5 * vb[l + m * p.NM];  // gutsp.f:144
+    else if (mode == 2) {
+      v[m] = 0.5 * (a + vb[l + m * p.NM]);  // gutsp.f:422
+      out_v1[l + m * p.NM] = v[m];
+    } else {
+      const double mv = a / sq;  // get_temperature's mvp (gutsp.f:2291)
+      v[m] = mode == 3 ? mv * mv : mv;
+    }
+  }
+}
+
+// update_np's deposit (gutsp.f:1461-1493) and update_up's (gutsp.f:1676-1800)
+// without the per-node 1/np factor, which up_from_sums applies once per node,
+// into the folded nodes.  The warp's ions are summed by cell first
+// (warp_deposit): one FP64 operation per ion, moment and corner and one
+// reduction per cell, where an atomic per ion and value was bound by L2's
+// rate (276k ions in 31k cells, us: np 18 -> 15, u 40 -> 30).
+__global__ void __launch_bounds__(128, 6) k_deposit_np(Geo g, PartDev p, long long N, double beta,
+                                                       double* __restrict__ np, int* err) {
+  __shared__ Red s_red[4];
+  __shared__ BlockConst s_bc;
+  if (threadIdx.x == 0) s_bc.set(g, beta, p.beta_p[0]);
+  __syncthreads();
+  const long long l = blockIdx.x * 128LL + threadIdx.x;
+  bool live = l < N;
+  int i = 1, j = 1, k = 1;
+  double w[8], fn = 0.0, fu;
+  if (live) {
+    i = p.ijk[l];
+    j = p.ijk[l + p.NM];
+    k = p.ijk[l + 2 * p.NM];
+    live = cell_ok(g, i, j, k);
+    if (!live) set_err(err, KERR_DOMAIN);
+  }
+  if (live) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) w[c] = p.wght[l + c * p.NM];
+    density_factors(g, beta, p.beta_p[l], s_bc, i, j, k, fn, fu);
+  }
+  warp_deposit1(g, s_red[threadIdx.x >> 5], live, i, j, k, w, fn, np);
+}
+
+__global__ void __launch_bounds__(128, 6) k_deposit_u(Geo g, PartDev p, long long N, double beta, int mode,
+                                                      const double* __restrict__ va, const double* __restrict__ vb,
+                                                      double* __restrict__ out_v1, double* __restrict__ S, int* err) {
+  __shared__ Red s_red[4];
+  __shared__ BlockConst s_bc;
+  if (threadIdx.x == 0) s_bc.set(g, beta, p.beta_p[0]);
+  __syncthreads();
+  const long long l = blockIdx.x * 128LL + threadIdx.x;
+  bool live = l < N;
+  int i = 1, j = 1, k = 1;
+  double w[8], m[4];
+  if (live) {
+    double v[3];
+    deposit_velocity(p, l, mode, va, vb, out_v1, v);
+    i = p.ijk[l];
+    j = p.ijk[l + p.NM];
+    k = p.ijk[l + 2 * p.NM];
+    live = cell_ok(g, i, j, k);
+    if (live) {
+#pragma unroll
+      for (int c = 0; c < 8; ++c) w[c] = p.wght[l + c * p.NM];
+      const double fu = flow_factor(g, beta, p.beta_p[l], s_bc, i, j, k);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) m[1 + q] = v[q] * fu;
+    } else {
+      set_err(err, KERR_DOMAIN);
+    }
+  }
+  warp_deposit<false>(g, s_red[threadIdx.x >> 5], live, i, j, k, w, m, nullptr, S);
+}
+
+// The same deposits in deterministic fixed point: each value on its own, so
+// that a sum depends on no grouping.
+__global__ void k_deposit_np_fix(Geo g, PartDev p, long long N, double beta, Fix64 fx, int* err) {
   unsigned bad = 0;
   GRID_STRIDE(l, N) {
     const int i = p.ijk[l], j = p.ijk[l + p.NM], k = p.ijk[l + 2 * p.NM];
@@ -145,38 +219,19 @@ __global__ void k_deposit_np(Geo g, PartDev p, long long N, double beta, double*
     const double volb = 1.0 / (g.dxg[i] * g.dyg[j] * g.dzg[k] * beta * p.beta_p[l]);
     long long tg[8];
     corner_targets(g, i, j, k, tg);
-    for (int c = 0; c < 8; ++c) {
-      if (tg[c] < 0) continue;
-      if (DET) fix_add(fx, tg[c], p.wght[l + c * p.NM] * volb, bad);
-      else atomicAdd(np + tg[c], p.wght[l + c * p.NM] * volb);
-    }
+    for (int c = 0; c < 8; ++c)
+      if (tg[c] >= 0) fix_add(fx, tg[c], p.wght[l + c * p.NM] * volb, bad);
   }
-  if (DET && bad) set_err(err, KERR_RANGE);
+  if (bad) set_err(err, KERR_RANGE);
 }
 
-// update_up deposit (gutsp.f:1676-1800) without the per-node 1/np factor,
-// which ct_from_sums applies once per node: sum v*w/volb.
-template <bool DET>
-__global__ void k_deposit_u(Geo g, PartDev p, long long N, double beta, int mode, const double* __restrict__ va,
-                            const double* __restrict__ vb, double* __restrict__ out_v1, double* __restrict__ S,
-                            Fix64 fx, int* err) {
+__global__ void k_deposit_u_fix(Geo g, PartDev p, long long N, double beta, int mode, const double* __restrict__ va,
+                                const double* __restrict__ vb, double* __restrict__ out_v1, Fix64 fx, int* err) {
   const long long C = g.C;
   unsigned bad = 0;
   GRID_STRIDE(l, N) {
     double v[3];
-    const double sq = mode >= 3 ? sqrt(p.mrat[l]) : 1.0;
-    for (int m = 0; m < 3; ++m) {
-      const double a = va[l + m * p.NM];
-      if (mode == 0) v[m] = a;
-      else if (mode == 1) v[m] = 1.5 * a - 0.5 * vb[l + m * p.NM];  // gutsp.f:144
-      else if (mode == 2) {
-        v[m] = 0.5 * (a + vb[l + m * p.NM]);  // gutsp.f:422
-        out_v1[l + m * p.NM] = v[m];
-      } else {
-        const double mv = a / sq;  // get_temperature's mvp (gutsp.f:2291)
-        v[m] = mode == 3 ? mv * mv : mv;
-      }
-    }
+    deposit_velocity(p, l, mode, va, vb, out_v1, v);
     const int i = p.ijk[l], j = p.ijk[l + p.NM], k = p.ijk[l + 2 * p.NM];
     if (!cell_ok(g, i, j, k)) {
       set_err(err, KERR_DOMAIN);
@@ -190,18 +245,10 @@ __global__ void k_deposit_u(Geo g, PartDev p, long long N, double beta, int mode
     for (int c = 0; c < 8; ++c) {
       if (tg[c] < 0) continue;
       const double w = p.wght[l + c * p.NM] * ivolb;
-      if (DET) {
-        fix_add(fx, tg[c], v[0] * w, bad);
-        fix_add(fx, tg[c] + C, v[1] * w, bad);
-        fix_add(fx, tg[c] + 2 * C, v[2] * w, bad);
-      } else {
-        atomicAdd(S + tg[c], v[0] * w);
-        atomicAdd(S + tg[c] + C, v[1] * w);
-        atomicAdd(S + tg[c] + 2 * C, v[2] * w);
-      }
+      for (int m = 0; m < 3; ++m) fix_add(fx, tg[c] + m * C, v[m] * w, bad);
     }
   }
-  if (DET && bad) set_err(err, KERR_RANGE);
+  if (bad) set_err(err, KERR_RANGE);
 }
 
 // update_rho deposit (gutsp.f:1543-1567): (w/mrat)/volb.
@@ -453,6 +500,27 @@ __global__ void k_nonfinite(const double* __restrict__ x, long long n, unsigned 
 
 }  // namespace
 
+void set_cell_constants(Geo& g, const double* qx, const double* qy, const double* qz, const double* dxg,
+                        const double* dyg, const double* dzg) {
+  const double* q[3] = {qx, qy, qz};
+  const double* s[3] = {dxg, dyg, dzg};
+  const int n[3] = {g.nx, g.ny, g.nz};
+  double d[3], dg[3];
+  g.uniform = true;
+  for (int a = 0; a < 3; ++a) {
+    d[a] = q[a][1] - q[a][0];
+    dg[a] = s[a] ? s[a][0] : d[a];
+    for (int i = 0; i + 1 < n[a]; ++i)
+      g.uniform = g.uniform && q[a][i + 1] - q[a][i] == d[a] && (!s[a] || s[a][i] == dg[a]);
+  }
+  g.cell_q = d[0] * d[1] * d[2];
+  g.cell_g = dg[0] * dg[1] * dg[2];
+  g.inv_cell_q = 1.0 / g.cell_q;
+  int e = 0;
+  const double m = std::frexp(g.dy, &e);  // in [0.5, 1) for a normal positive dy
+  g.rdy = g.dy > 0.0 && std::isfinite(g.dy) && e > -60 && e < 60 && m != 1.0 - 0x1p-53 ? 1.0 / g.dy : 0.0;
+}
+
 // ---- launchers -------------------------------------------------------------------
 
 #define LAUNCH(kern, n, ...)                                     \
@@ -477,14 +545,16 @@ cudaError_t interp_weights(const Geo& g, const PartDev& p, long long N, int* err
 cudaError_t deposit_np(const Geo& g, const PartDev& p, long long N, double beta, double* np, int* err,
                        cudaStream_t st, Fix64 fix) {
   if (N <= 0) return cudaSuccess;
-  if (fix.h) LAUNCH(k_deposit_np<true>, N, g, p, N, beta, np, fix, err);
-  LAUNCH(k_deposit_np<false>, N, g, p, N, beta, np, fix, err);
+  if (fix.h) LAUNCH(k_deposit_np_fix, N, g, p, N, beta, fix, err);
+  k_deposit_np<<<(unsigned)((N + 127) / 128), 128, 0, st>>>(g, p, N, beta, np, err);
+  return cudaGetLastError();
 }
 cudaError_t deposit_u(const Geo& g, const PartDev& p, long long N, double beta, int mode, const double* va,
                       const double* vb, double* out_v1, double* S, int* err, cudaStream_t st, Fix64 fix) {
   if (N <= 0) return cudaSuccess;
-  if (fix.h) LAUNCH(k_deposit_u<true>, N, g, p, N, beta, mode, va, vb, out_v1, S, fix, err);
-  LAUNCH(k_deposit_u<false>, N, g, p, N, beta, mode, va, vb, out_v1, S, fix, err);
+  if (fix.h) LAUNCH(k_deposit_u_fix, N, g, p, N, beta, mode, va, vb, out_v1, fix, err);
+  k_deposit_u<<<(unsigned)((N + 127) / 128), 128, 0, st>>>(g, p, N, beta, mode, va, vb, out_v1, S, err);
+  return cudaGetLastError();
 }
 cudaError_t fix_to_double(long long n, Fix64 fix, double* out, cudaStream_t st) {
   LAUNCH(k_fix_to_double, n, n, fix, out);

@@ -17,6 +17,11 @@ struct PartDev {  // device mirrors of the particle arrays
   long long NM;   // leading dimension ni_max
 };
 
+// Host: the uniform-grid constants and 1/dy of g (nx, ny, nz and dy set) from
+// the host's node coordinates and, when given, dx_grid ... (else cell_g = cell_q).
+void set_cell_constants(Geo& g, const double* qx, const double* qy, const double* qz, const double* dxg,
+                        const double* dyg, const double* dzg);
+
 // boundary.f
 cudaError_t periodic3(const Geo& g, double* b, cudaStream_t st);
 cudaError_t periodic1(const Geo& g, double* b, cudaStream_t st);

@@ -33,8 +33,12 @@ __device__ __forceinline__ long long ordered(double x) {
   return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
 }
 
-// cell_search (swap_dev.cuh) with integer comparisons and an FP32 guess: the
-// same index for every x, 0 when x is outside (q(1), q(n)] or not a number.
+// Cell search of get_interp_weights (gutsp.f:1396-1401): the index i with
+// q(i) < x <= q(i+1), i.e. one less than the first node with x <= q(node), 0
+// when x is outside (q(1), q(n)] or not a number.  An FP32 guess from the
+// uniform spacing is corrected against the node array itself by integer
+// comparisons, so the result is the reference's linear search for any
+// monotone q.
 __device__ __forceinline__ int find_cell(const double* __restrict__ q, int n, double x, float q1, float inv_d) {
   const long long xb = ordered(x);
   int i = (int)((__double2float_rn(x) - q1) * inv_d) + 1;
@@ -42,6 +46,182 @@ __device__ __forceinline__ int find_cell(const double* __restrict__ q, int n, do
   while (i > 1 && !(xb > ordered(q[i]))) --i;
   while (i < n - 1 && xb > ordered(q[i + 1])) ++i;
   return xb > ordered(q[i]) && xb <= ordered(q[i + 1]) ? i : 0;
+}
+
+// Cell and corner weights of a position (get_interp_weights, gutsp.f:1391-
+// 1432), in the reference's order (000,100,001,101,010,110,011,111 over
+// x,z,y) and with its products' rounding (their common factors formed once;
+// on a uniform grid the cell's inverse volume is given).  Units compiled with
+// --fmad=false round every product like the Fortran.  Outside the grid:
+// false, cell (1,1,1) and weights of zero.
+__device__ __forceinline__ bool weights_at(const Geo& g, double x, double y, double z, int& i, int& j, int& k,
+                                           double (&w)[8]) {
+  i = find_cell(g.qx, g.nx, x, (float)g.qx[1], (float)g.inv_dx);
+  k = find_cell(g.qz, g.nz, z, (float)g.qz[1], (float)g.inv_dz);
+  j = __double2int_rz(quotient<false>(y, g.dy, g.rdy));  // floor for y >= 0; any y below is outside either way
+  if (!(i >= 1 && j >= 1 && j < g.ny && k >= 1)) {
+    i = j = k = 1;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) w[c] = 0.0;
+    return false;
+  }
+  const double qx = g.qx[i], qxp = g.qx[i + 1], qy = g.qy[j], qyp = g.qy[j + 1], qz = g.qz[k], qzp = g.qz[k + 1];
+  const double vol = g.uniform ? g.inv_cell_q : 1.0 / ((qxp - qx) * (qyp - qy) * (qzp - qz));
+  const double x1 = fabs(x - qx), x2 = fabs(x - qxp), y1 = fabs(y - qy), y2 = fabs(y - qyp), z1 = fabs(z - qz),
+               z2 = fabs(z - qzp);
+  const double x2y2 = x2 * y2, x1y2 = x1 * y2, x2y1 = x2 * y1, x1y1 = x1 * y1;
+  w[0] = x2y2 * z2 * vol;
+  w[1] = x1y2 * z2 * vol;
+  w[2] = x2y2 * z1 * vol;
+  w[3] = x1y2 * z1 * vol;
+  w[4] = x2y1 * z2 * vol;
+  w[5] = x1y1 * z2 * vol;
+  w[6] = x2y1 * z1 * vol;
+  w[7] = x1y1 * z1 * vol;
+  return true;
+}
+
+__device__ __forceinline__ double volume_factor(double cell, double beta, double bp) {
+  return 1.0 / (cell * beta * bp);
+}
+
+// The density factors of one beta_p on a uniform grid, kept per block (most
+// runs have one or two values): update_np's volb and update_up's 1/volb.
+struct BlockConst {
+  double bp, inv_n, inv_u;
+  __device__ __forceinline__ void set(const Geo& g, double beta, double b) {
+    bp = b;
+    inv_n = volume_factor(g.cell_g, beta, b);
+    inv_u = volume_factor(g.cell_q, beta, b);
+  }
+};
+
+// update_np's 1/(dx_grid dy_grid dz_grid beta beta_p) and update_up's inverse
+// volb for a particle of cell (i,j,k).
+__device__ __forceinline__ void density_factors(const Geo& g, double beta, double bp, const BlockConst& bc, int i,
+                                                int j, int k, double& fn, double& fu) {
+  if (!g.uniform) {
+    fn = volume_factor(g.dxg[i] * g.dyg[j] * g.dzg[k], beta, bp);
+    fu = volume_factor((g.qx[i + 1] - g.qx[i]) * (g.qy[j + 1] - g.qy[j]) * (g.qz[k + 1] - g.qz[k]), beta, bp);
+  } else if (__double_as_longlong(bp) == __double_as_longlong(bc.bp)) {
+    fn = bc.inv_n;
+    fu = bc.inv_u;
+  } else {
+    fu = volume_factor(g.cell_q, beta, bp);
+    fn = g.cell_g == g.cell_q ? fu : volume_factor(g.cell_g, beta, bp);
+  }
+}
+
+// update_up's factor alone, from the node coordinates.
+__device__ __forceinline__ double flow_factor(const Geo& g, double beta, double bp, const BlockConst& bc, int i, int j,
+                                              int k) {
+  if (!g.uniform)
+    return volume_factor((g.qx[i + 1] - g.qx[i]) * (g.qy[j + 1] - g.qy[j]) * (g.qz[k + 1] - g.qz[k]), beta, bp);
+  return __double_as_longlong(bp) == __double_as_longlong(bc.bp) ? bc.inv_u : volume_factor(g.cell_q, beta, bp);
+}
+
+// ---- the deposits of one warp ----
+
+constexpr int RED_ROW = 34;  // doubles per row: 8 rows a lane group reads at once start on different banks
+
+struct Red {
+  double v[12][RED_ROW];        // 8 weights, 4 moments; columns = the warp's ions grouped by cell
+  unsigned long long cell[32];  // i | j << 21 | k << 42 per column; ~0 for none
+};
+
+// The column of each lane's ion with the warp's ions grouped by cell, and (the
+// same in every lane) a bit per column that ends a group.
+__device__ __forceinline__ int group_by_cell(unsigned node, unsigned& ends) {
+  const int lane = threadIdx.x & 31;
+  const unsigned peers = __match_any_sync(0xffffffffu, node);
+  const int leader = __ffs(peers) - 1;
+  const int mine = lane == leader ? __popc(peers) : 0;
+  int incl = mine;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  const int base = __shfl_sync(0xffffffffu, incl - mine, leader);
+  // the column before each group's first ends another group
+  ends = (__reduce_or_sync(0xffffffffu, lane == leader ? 1u << base : 0u) >> 1) | 0x80000000u;
+  return base + __popc(peers & ((1u << lane) - 1u));
+}
+
+// Adds a sum at corner c (x, z, y from the lowest bit) of a packed cell.
+__device__ __forceinline__ void add_at_corner(const Geo& g, double* arr, unsigned long long cell, int c, double v) {
+  const int i = (int)(cell & 0x1fffffu) + (c & 1), j = (int)(cell >> 21 & 0x1fffffu) + (c >> 2),
+            k = (int)(cell >> 42) + (c >> 1 & 1);
+  const long long t = fold_target(g, i, j, k);
+  if (t >= 0) atomicAdd(arr + t, v);
+}
+
+// Adds the warp's ions to the node sums: lane (moment, corner) forms the
+// products of its row pair over the columns and adds each group's sum.  w:
+// the corner weights; m: the density and velocity moments.  NP false: the
+// velocity moments alone.
+template <bool NP>
+__device__ __forceinline__ void warp_deposit(const Geo& g, Red& s, bool live, int i, int j, int k,
+                                             const double (&w)[8], const double (&m)[4], double* __restrict__ np,
+                                             double* __restrict__ S) {
+  const int lane = threadIdx.x & 31;
+  unsigned ends;
+  const int pos = group_by_cell(live ? (unsigned)nidx(g, i, j, k) : 0xffffffffu, ends);
+#pragma unroll
+  for (int c = 0; c < 8; ++c) s.v[c][pos] = live ? w[c] : 0.0;
+#pragma unroll
+  for (int q = NP ? 0 : 1; q < 4; ++q) s.v[8 + q][pos] = live ? m[q] : 0.0;
+  s.cell[pos] = live ? (unsigned long long)i | (unsigned long long)j << 21 | (unsigned long long)k << 42 : ~0ull;
+  __syncwarp();
+  const int cv = lane & 7, qv = lane >> 3;
+  const bool adds = NP || qv != 0;
+  const double2* wr = reinterpret_cast<const double2*>(s.v[cv]);
+  const double2* mr = reinterpret_cast<const double2*>(s.v[8 + (adds ? qv : 1)]);
+  double* const arr = qv == 0 ? np : S + (qv - 1) * g.C;
+  auto flush = [&](int r, double acc) {
+    const unsigned long long c = s.cell[r];
+    if (c != ~0ull && adds) add_at_corner(g, arr, c, cv, acc);
+  };
+  double acc = 0.0;
+#pragma unroll
+  for (int r = 0; r < 16; ++r) {
+    const double2 a = wr[r], b = mr[r];
+    acc = __fma_rn(a.x, b.x, acc);
+    if (ends >> (2 * r) & 1u) {
+      flush(2 * r, acc);
+      acc = 0.0;
+    }
+    acc = __fma_rn(a.y, b.y, acc);
+    if (ends >> (2 * r + 1) & 1u) {
+      flush(2 * r + 1, acc);
+      acc = 0.0;
+    }
+  }
+  __syncwarp();
+}
+
+// One moment alone: lane (quarter, corner) takes eight of the columns.
+__device__ __forceinline__ void warp_deposit1(const Geo& g, Red& s, bool live, int i, int j, int k,
+                                              const double (&w)[8], double m, double* __restrict__ out) {
+  const int lane = threadIdx.x & 31;
+  unsigned ends;
+  const int pos = group_by_cell(live ? (unsigned)nidx(g, i, j, k) : 0xffffffffu, ends);
+#pragma unroll
+  for (int c = 0; c < 8; ++c) s.v[c][pos] = live ? w[c] : 0.0;
+  s.v[8][pos] = live ? m : 0.0;
+  s.cell[pos] = live ? (unsigned long long)i | (unsigned long long)j << 21 | (unsigned long long)k << 42 : ~0ull;
+  __syncwarp();
+  const int cv = lane & 7, r0 = lane & 24;
+  double acc = 0.0;
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    acc = __fma_rn(s.v[cv][r0 + r], s.v[8][r0 + r], acc);
+    if (r == 7 || (ends >> (r0 + r) & 1u)) {
+      const unsigned long long c = s.cell[r0 + r];
+      if (c != ~0ull) add_at_corner(g, out, c, cv, acc);
+      acc = 0.0;
+    }
+  }
+  __syncwarp();
 }
 
 }  // namespace swapk

@@ -30,10 +30,15 @@
 namespace swapk {
 namespace {
 
-constexpr int TPB = 256;
+constexpr int TPB = 128;  // most threads of a block
 
+// Threads per block: a warp instruction of the FP64 pipe holds its SM for 16
+// clocks, so small grids are spread over all 152 SMs a warp at a time (2772
+// nodes in 11 blocks of 256 took 8.5 us for curl B, in 87 of 32 6.9),
+// and middling ones in blocks small enough to even out the SMs' shares.
+inline unsigned threads_for(long long n) { return n <= 152 * 64 ? 32u : (n <= 152 * 64 * 64 ? 64u : 128u); }
 inline unsigned nblocks(long long n) {
-  const long long b = (n + TPB - 1) / TPB;
+  const long long t = threads_for(n), b = (n + t - 1) / t;
   return (unsigned)(b < 1 ? 1 : b);
 }
 
@@ -75,22 +80,30 @@ __device__ __forceinline__ Nbr nbr_of(const Geo& g, const Node& n) {
 __device__ __forceinline__ bool on_edge(const Geo& g, const Node& n) {
   return n.i == 2 || n.j == 2 || n.k == 2 || n.i == g.nx - 1 || n.j == g.ny - 1 || n.k == g.nz - 1;
 }
+// ncomp components (v0, v1, v2) of f; one image per axis and side, both sides
+// on an axis of a single cell.
 __device__ __noinline__ void store_ghosts(int nx, int ny, int nz, long long C, int ncomp, double* f, int i, int j,
                                           int k, double v0, double v1, double v2) {
+  const int sy = nx, sz = nx * ny;
+  f += (i - 1) + (long long)nx * ((j - 1) + (long long)ny * (k - 1));
+  // offset to the image beyond the far end (node 2) and the near end (node n-1)
+  const int x[3] = {0, i == 2 ? nx - 2 : 0, i == nx - 1 ? 2 - nx : 0};
+  const int y[3] = {0, j == 2 ? (ny - 2) * sy : 0, j == ny - 1 ? (2 - ny) * sy : 0};
+  const int z[3] = {0, k == 2 ? (nz - 2) * sz : 0, k == nz - 1 ? (2 - nz) * sz : 0};
+#pragma unroll
   for (int c = 0; c < 3; ++c) {
-    const int kk = c == 0 ? k : (c == 1 ? (k == 2 ? nz : 0) : (k == nz - 1 ? 1 : 0));
-    if (kk == 0) continue;
+    if (c && !z[c]) continue;
+#pragma unroll
     for (int b = 0; b < 3; ++b) {
-      const int jj = b == 0 ? j : (b == 1 ? (j == 2 ? ny : 0) : (j == ny - 1 ? 1 : 0));
-      if (jj == 0) continue;
+      if (b && !y[b]) continue;
+#pragma unroll
       for (int a = 0; a < 3; ++a) {
-        const int ii = a == 0 ? i : (a == 1 ? (i == 2 ? nx : 0) : (i == nx - 1 ? 1 : 0));
-        if (ii == 0 || (a == 0 && b == 0 && c == 0)) continue;
-        const long long o = (ii - 1) + (long long)nx * ((jj - 1) + (long long)ny * (kk - 1));
-        f[o] = v0;
+        if ((a && !x[a]) || a + b + c == 0) continue;
+        double* t = f + (x[a] + y[b] + z[c]);
+        t[0] = v0;
         if (ncomp == 3) {
-          f[o + C] = v1;
-          f[o + 2 * C] = v2;
+          t[C] = v1;
+          t[2 * C] = v2;
         }
       }
     }
@@ -413,7 +426,7 @@ __global__ void __launch_bounds__(TPB) k_kit(Geo g, double* aj, const double* __
 
 #define FL(kern, ...)                                                 \
   do {                                                                \
-    kern<<<nblocks(n_interior(g)), TPB, 0, st>>>(__VA_ARGS__);        \
+    kern<<<nblocks(n_interior(g)), threads_for(n_interior(g)), 0, st>>>(__VA_ARGS__);        \
     return cudaGetLastError();                                        \
   } while (0)
 

@@ -34,137 +34,19 @@ namespace swapk {
 namespace {
 
 constexpr int TPB = 128, WARPS = TPB / 32;
-constexpr int ROW = 34;  // doubles per row: 8 rows a lane group reads at once start on different banks
-
-struct Red {
-  double v[12][ROW];            // 8 weights, 4 moments; columns = the warp's ions grouped by cell
-  unsigned long long cell[32];  // i | j << 21 | k << 42 per column; ~0 for none
-};
-
-__device__ __forceinline__ unsigned long long pack(int i, int j, int k) {
-  return (unsigned long long)i | (unsigned long long)j << 21 | (unsigned long long)k << 42;
-}
-
-// Adds the warp's ions to the node sums.  w: the corner weights in the
-// reference's order (x, z, y from the lowest bit); m: the density and
-// velocity moments.  NP false: the velocity moments alone.
-template <bool NP>
-__device__ __forceinline__ void warp_deposit(const Geo& g, Red& s, bool live, unsigned node, unsigned long long cell,
-                                             const double (&w)[8], const double (&m)[4], double* __restrict__ np,
-                                             double* __restrict__ S) {
-  const int lane = threadIdx.x & 31;
-  const unsigned peers = __match_any_sync(0xffffffffu, live ? node : 0xffffffffu);
-  const int leader = __ffs(peers) - 1;
-  int incl = lane == leader ? __popc(peers) : 0;
-  const int mine = incl;
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += y;
-  }
-  const int base = __shfl_sync(0xffffffffu, incl - mine, leader);
-  const int pos = base + __popc(peers & ((1u << lane) - 1u));
-  // the column after each group is another group's first
-  const unsigned heads = __reduce_or_sync(0xffffffffu, lane == leader ? 1u << base : 0u);
-  const unsigned ends = (heads >> 1) | 0x80000000u;
-#pragma unroll
-  for (int c = 0; c < 8; ++c) s.v[c][pos] = live ? w[c] : 0.0;
-#pragma unroll
-  for (int q = NP ? 0 : 1; q < 4; ++q) s.v[8 + q][pos] = live ? m[q] : 0.0;
-  s.cell[pos] = live ? cell : ~0ull;
-  __syncwarp();
-  const int cv = lane & 7, qv = lane >> 3;
-  const bool adds = NP || qv != 0;
-  const double2* wr = reinterpret_cast<const double2*>(s.v[cv]);
-  const double2* mr = reinterpret_cast<const double2*>(s.v[8 + (adds ? qv : 1)]);
-  double* const arr = qv == 0 ? np : S + (qv - 1) * g.C;
-  auto flush = [&](int r, double acc) {
-    const unsigned long long c = s.cell[r];
-    if (c == ~0ull || !adds) return;
-    const int i = (int)(c & 0x1fffffu) + (cv & 1), j = (int)(c >> 21 & 0x1fffffu) + (cv >> 2),
-              k = (int)(c >> 42) + (cv >> 1 & 1);
-    const long long t = fold_target(g, i, j, k);
-    if (t >= 0) atomicAdd(arr + t, acc);
-  };
-  double acc = 0.0;
-#pragma unroll
-  for (int r = 0; r < 16; ++r) {
-    const double2 a = wr[r], b = mr[r];
-    acc = __fma_rn(a.x, b.x, acc);
-    if (ends >> (2 * r) & 1u) {
-      flush(2 * r, acc);
-      acc = 0.0;
-    }
-    acc = __fma_rn(a.y, b.y, acc);
-    if (ends >> (2 * r + 1) & 1u) {
-      flush(2 * r + 1, acc);
-      acc = 0.0;
-    }
-  }
-  __syncwarp();
-}
-
-// Constants of the block: the guess of the cell search, and the density
-// factors of the first particle's beta_p (most runs have one or two).
-struct BlockConst {
-  double bp, inv_n, inv_u;  // update_np's volb and update_up's 1/volb for bp
-};
-
-__device__ __forceinline__ double volume_factor(double cell, double beta, double bp) {
-  return 1.0 / (cell * beta * bp);
-}
 
 // Cell and weights at a position (get_interp_weights), stored like the
 // reference's COMMON blocks; false when the position is outside the grid.
 __device__ __forceinline__ bool locate(const PassArgs& a, long long l, double x, double y, double z, int& i, int& j,
                                        int& k, double (&w)[8]) {
-  const Geo& g = a.g;
   const PartDev& p = a.p;
-  i = find_cell(g.qx, g.nx, x, (float)g.qx[1], (float)g.inv_dx);
-  k = find_cell(g.qz, g.nz, z, (float)g.qz[1], (float)g.inv_dz);
-  j = __double2int_rz(quotient<false>(y, g.dy, g.rdy));  // floor for y >= 0; any y below is outside either way
-  const bool ok = i >= 1 && j >= 1 && j < g.ny && k >= 1;
-  if (!ok) i = j = k = 1;
+  const bool ok = weights_at(a.g, x, y, z, i, j, k, w);
   p.ijk[l] = i;
   p.ijk[l + p.NM] = j;
   p.ijk[l + 2 * p.NM] = k;
-  if (!ok) {
-#pragma unroll
-    for (int c = 0; c < 8; ++c) p.wght[l + c * p.NM] = w[c] = 0.0;
-    return false;
-  }
-  const double qx = g.qx[i], qxp = g.qx[i + 1], qy = g.qy[j], qyp = g.qy[j + 1], qz = g.qz[k], qzp = g.qz[k + 1];
-  const double vol = g.uniform ? g.inv_cell_q : 1.0 / ((qxp - qx) * (qyp - qy) * (qzp - qz));
-  const double x1 = fabs(x - qx), x2 = fabs(x - qxp), y1 = fabs(y - qy), y2 = fabs(y - qyp), z1 = fabs(z - qz),
-               z2 = fabs(z - qzp);
-  const double x2y2 = x2 * y2, x1y2 = x1 * y2, x2y1 = x2 * y1, x1y1 = x1 * y1;
-  w[0] = x2y2 * z2 * vol;
-  w[1] = x1y2 * z2 * vol;
-  w[2] = x2y2 * z1 * vol;
-  w[3] = x1y2 * z1 * vol;
-  w[4] = x2y1 * z2 * vol;
-  w[5] = x1y1 * z2 * vol;
-  w[6] = x2y1 * z1 * vol;
-  w[7] = x1y1 * z1 * vol;
 #pragma unroll
   for (int c = 0; c < 8; ++c) p.wght[l + c * p.NM] = w[c];
-  return true;
-}
-
-// update_np's 1/(dx_grid dy_grid dz_grid beta beta_p) and update_up's inverse volb.
-__device__ __forceinline__ void density_factors(const PassArgs& a, const BlockConst& bc, long long l, int i, int j,
-                                                int k, double& fn, double& fu) {
-  const Geo& g = a.g;
-  const double bp = a.p.beta_p[l];
-  if (!g.uniform) {
-    fn = volume_factor(g.dxg[i] * g.dyg[j] * g.dzg[k], a.beta, bp);
-    fu = volume_factor((g.qx[i + 1] - g.qx[i]) * (g.qy[j + 1] - g.qy[j]) * (g.qz[k + 1] - g.qz[k]), a.beta, bp);
-  } else if (__double_as_longlong(bp) == __double_as_longlong(bc.bp)) {
-    fn = bc.inv_n;
-    fu = bc.inv_u;
-  } else {
-    fu = volume_factor(g.cell_q, a.beta, bp);
-    fn = g.cell_g == g.cell_q ? fu : volume_factor(g.cell_g, a.beta, bp);
-  }
+  return ok;
 }
 
 // The half move of move_ion_half along one axis with its one wrap (gutsp.f:473-510).
@@ -185,12 +67,7 @@ __global__ void __launch_bounds__(TPB, 4) k_pass(PassArgs a) {
   const Geo& g = a.g;
   const PartDev& p = a.p;
   const long long NM = p.NM;
-  if (threadIdx.x == 0) {
-    const double bp = p.beta_p[0];
-    s_bc.bp = bp;
-    s_bc.inv_n = volume_factor(g.cell_g, a.beta, bp);
-    s_bc.inv_u = volume_factor(g.cell_q, a.beta, bp);
-  }
+  if (threadIdx.x == 0) s_bc.set(g, a.beta, p.beta_p[0]);
   __syncthreads();
   Red& red = s_red[threadIdx.x >> 5];
   const long long step = (long long)gridDim.x * TPB;
@@ -208,7 +85,7 @@ __global__ void __launch_bounds__(TPB, 4) k_pass(PassArgs a) {
       live = locate(a, l, p.xp[l], p.xp[l + NM], p.xp[l + 2 * NM], i, j, k, w);
       if (!live) set_err(a.err, KERR_DOMAIN);
       double fn, fu;
-      density_factors(a, s_bc, l, i, j, k, fn, fu);
+      density_factors(g, a.beta, p.beta_p[l], s_bc, i, j, k, fn, fu);
       m[0] = fn;
       const double f1 = 1.5 * fu, f2 = -0.5 * fu;
 #pragma unroll
@@ -269,10 +146,8 @@ __global__ void __launch_bounds__(TPB, 4) k_pass(PassArgs a) {
         const double c = __fma_rn(vm[q1], B[q2], -(vm[q2] * B[q1]));
         vn[q] = ad * __fma_rn(kd, B[q], __fma_rn(dt, c, om * vm[q]));
       }
-      double fn, fu;
       if (PASS == 2) {  // improve_up (gutsp.f:422)
-        density_factors(a, s_bc, l, i, j, k, fn, fu);
-        const double f = 0.5 * fu;
+        const double f = 0.5 * flow_factor(g, a.beta, p.beta_p[l], s_bc, i, j, k);
 #pragma unroll
         for (int q = 0; q < 3; ++q) m[1 + q] = f * (vn[q] + vm[q]);
       } else {
@@ -298,7 +173,8 @@ __global__ void __launch_bounds__(TPB, 4) k_pass(PassArgs a) {
         } else {
           live = locate(a, l, x, y, z, i, j, k, w);
           if (!live) set_err(a.err, KERR_DOMAIN);
-          density_factors(a, s_bc, l, i, j, k, fn, fu);
+          double fn, fu;
+          density_factors(g, a.beta, p.beta_p[l], s_bc, i, j, k, fn, fu);
           m[0] = fn;
 #pragma unroll
           for (int q = 0; q < 3; ++q) m[1 + q] = fu * vn[q];
@@ -313,7 +189,7 @@ __global__ void __launch_bounds__(TPB, 4) k_pass(PassArgs a) {
         p.xp[l + 2 * NM] = z;
       }
     }
-    warp_deposit<PASS != 2>(g, red, live, (unsigned)nidx(g, i, j, k), pack(i, j, k), w, m, a.np, a.S);
+    warp_deposit<PASS != 2>(g, red, live, i, j, k, w, m, a.np, a.S);
   }
 }
 

@@ -172,7 +172,11 @@ int swap_ctx::begin() {
 // Finish an entry: wait for the stream, read the kernel error flag, and mark
 // every output device-current.
 int swap_ctx::finish() {
-  cudaError_t e = cudaStreamSynchronize(st);
+  // the error word rides on the entry's own wait (a copy of its own after it
+  // was a second round trip, 10 us of a 20 us entry)
+  cudaError_t e = cudaMemcpyAsync(h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, st);
+  const cudaError_t e2 = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) e = e2;
   if (e != cudaSuccess) return cuda_fail(e, "stream");
   for (Mirror* m : touched) {
     m->dev_valid = true;
@@ -184,9 +188,7 @@ int swap_ctx::finish() {
     m->dev_valid = false;
   }
   touched_host.clear();
-  int herr = 0;
-  e = cudaMemcpy(&herr, d_err, sizeof(int), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return cuda_fail(e, "error flag");
+  const int herr = *h_err;
   if (herr) {
     cudaMemset(d_err, 0, sizeof(int));
     if (herr == KERR_DOMAIN) return fail(SWAP_EDOMAIN, "a particle lies outside the grid");
@@ -556,22 +558,6 @@ extern "C" int swap_init(swap_ctx** out, const swap_dims* d, const swap_params* 
   g.rdxg = rec[0]; g.rdyg = rec[1]; g.rdzg = rec[2];
   g.rdxc = rec[3]; g.rdyc = rec[4]; g.rdzc = rec[5];
   g.spacing_p2 = p2;
-  {
-    bool uni = true;
-    double d[3], dg[3];
-    for (int a = 0; a < 3; ++a) {
-      d[a] = arrs[a][1] - arrs[a][0];
-      dg[a] = arrs[3 + a][0];
-      for (int q = 0; q + 1 < ns[a]; ++q) uni = uni && arrs[a][q + 1] - arrs[a][q] == d[a] && arrs[3 + a][q] == dg[a];
-    }
-    g.uniform = uni;
-    g.cell_q = d[0] * d[1] * d[2];
-    g.cell_g = dg[0] * dg[1] * dg[2];
-    g.inv_cell_q = 1.0 / g.cell_q;
-    int e = 0;
-    const double m = std::frexp(p->dy, &e);
-    g.rdy = p->dy > 0.0 && std::isfinite(p->dy) && e > -60 && e < 60 && m != 1.0 - 0x1p-53 ? 1.0 / p->dy : 0.0;
-  }
   g.nx = d->nx; g.ny = d->ny; g.nz = d->nz;
   g.C = (long long)d->nx * d->ny * d->nz;
   g.qx = dg[0]; g.qy = dg[1]; g.qz = dg[2];
@@ -579,6 +565,7 @@ extern "C" int swap_init(swap_ctx** out, const swap_dims* d, const swap_params* 
   g.dxc = dg[6]; g.dyc = dg[7]; g.dzc = dg[8];
   g.xr = dg[9]; g.yr = dg[10]; g.zr = dg[11];
   g.dy = p->dy;
+  set_cell_constants(g, co->qx, co->qy, co->qz, co->dx_grid, co->dy_grid, co->dz_grid);
   g.inv_dx = 1.0 / (co->qx[1] - co->qx[0]);
   g.inv_dz = 1.0 / (co->qz[1] - co->qz[0]);
   c->h_qx.assign(co->qx, co->qx + d->nx);
@@ -606,6 +593,11 @@ extern "C" int swap_init(swap_ctx** out, const swap_dims* d, const swap_params* 
   }
   c->owned.push_back(e);
   c->d_err = e;
+  if (cudaMallocHost(&c->h_err, sizeof(int)) != cudaSuccess) {
+    c->h_err = nullptr;
+    swap_finalize(c);
+    return SWAP_ECUDA;
+  }
   if (cudaMemset(e, 0, sizeof(int)) != cudaSuccess || cudaEventCreate(&c->t0) != cudaSuccess ||
       cudaEventCreate(&c->t1) != cudaSuccess) {
     swap_finalize(c);
@@ -624,6 +616,7 @@ extern "C" int swap_finalize(swap_ctx* c) {
   for (auto& kv : c->reg) cudaFree(kv.second.dev);
   for (void* p : c->owned) cudaFree(p);
   if (c->stage32) cudaFree(c->stage32);
+  if (c->h_err) cudaFreeHost(c->h_err);
   if (c->t0) cudaEventDestroy(c->t0);
   if (c->t1) cudaEventDestroy(c->t1);
   c->prof_free();
@@ -798,21 +791,22 @@ extern "C" int swap_get_interp_weights(swap_ctx* c, const double* xp) {
   TRY(need_particle_scalars(c));
   TRY(c->use(xp, Access::In, &dxp));
   TRY(ops::get_interp_weights(c, dxp));
-  int r = c->finish();
-  if (r == SWAP_OK && c->h_ijkp) {  // the COMMON ijkp mirror now holds new indices
-    Mirror* m = c->find(c->h_ijkp);
+  Mirror* m = c->h_ijkp ? c->find(c->h_ijkp) : nullptr;
+  cudaError_t e = cudaSuccess;
+  if (m) {  // the COMMON ijkp mirror takes the new indices
     const std::size_t NM = (std::size_t)c->dims.ni_max;
-    cudaError_t e = cudaSuccess;
     for (int k = 0; k < 3 && e == cudaSuccess && c->ntot() > 0; ++k)
       e = cudaMemcpyAsync(static_cast<int32_t*>(m->dev) + k * NM, c->d_ijk + k * NM, (std::size_t)c->ntot() * 4,
                           cudaMemcpyDeviceToDevice, c->st);
-    const cudaError_t e2 = cudaStreamSynchronize(c->st);  // also after a failed copy: nothing stays queued
-    if (e == cudaSuccess) e = e2;
-    if (e != cudaSuccess) return c->cuda_fail(e, "ijkp mirror");
+  }
+  const int r = c->finish();  // also after a failed copy: nothing stays queued
+  if (r) return r;
+  if (e != cudaSuccess) return c->cuda_fail(e, "ijkp mirror");
+  if (m) {
     m->dev_valid = true;
     m->host_valid = false;
   }
-  return r;
+  return SWAP_OK;
 }
 
 extern "C" int swap_update_np(swap_ctx* c, double* np) {

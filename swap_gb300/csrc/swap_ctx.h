@@ -41,6 +41,7 @@ struct swap_ctx {
   swapk::Geo g{};
   cudaStream_t st = nullptr;
   int* d_err = nullptr;
+  int* h_err = nullptr;  // its value at the last finish(), pinned
   std::string err;
 
   // registry of bound host arrays

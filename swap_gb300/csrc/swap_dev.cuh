@@ -87,40 +87,6 @@ __device__ __forceinline__ void set_err(int* err, int code) {
   if (err) atomicCAS(err, 0, code);
 }
 
-// Cell search of get_interp_weights (gutsp.f:1396-1401): the index i with
-// q(i) < x <= q(i+1), i.e. one less than the first node with x <= q(node).
-// A guess from the uniform spacing is corrected against the node array
-// itself, so the result equals the reference's linear search for any
-// monotone q.  Returns 0 (invalid) when x <= q(1) or x > q(n).
-__device__ __forceinline__ int cell_search(const double* __restrict__ q, int n, double x, double inv_d) {
-  if (!(x > q[1]) || x > q[n]) return 0;
-  int i = (int)((x - q[1]) * inv_d) + 1;
-  i = i < 1 ? 1 : (i > n - 1 ? n - 1 : i);
-  while (i > 1 && !(x > q[i])) --i;
-  while (i < n - 1 && x > q[i + 1]) ++i;
-  return i;
-}
-
-// The eight interpolation weights of a particle at (x,y,z) in cell (i,j,k),
-// in the reference's order (000,100,001,101,010,110,011,111 over x,z,y;
-// gutsp.f:1414-1429).  Units compiled with --fmad=false round every product
-// like the Fortran.
-__device__ __forceinline__ void weights8(const Geo& g, int i, int j, int k, double x, double y, double z,
-                                         double w[8]) {
-  const double vol = 1.0 / ((g.qx[i + 1] - g.qx[i]) * (g.qy[j + 1] - g.qy[j]) * (g.qz[k + 1] - g.qz[k]));
-  const double x1 = fabs(x - g.qx[i]), x2 = fabs(x - g.qx[i + 1]);
-  const double y1 = fabs(y - g.qy[j]), y2 = fabs(y - g.qy[j + 1]);
-  const double z1 = fabs(z - g.qz[k]), z2 = fabs(z - g.qz[k + 1]);
-  w[0] = x2 * y2 * z2 * vol;
-  w[1] = x1 * y2 * z2 * vol;
-  w[2] = x2 * y2 * z1 * vol;
-  w[3] = x1 * y2 * z1 * vol;
-  w[4] = x2 * y1 * z2 * vol;
-  w[5] = x1 * y1 * z2 * vol;
-  w[6] = x2 * y1 * z1 * vol;
-  w[7] = x1 * y1 * z1 * vol;
-}
-
 // Deposit target of a raw corner after the periodic fold (gutsp.f:1496-1498,
 // 1803-1805) and the ghost overwrite of periodic_scalar/periodic: plane 1 goes
 // to plane n-1, plane n is discarded.  Returns -1 for a discarded corner.
