@@ -242,13 +242,13 @@ class Hybrid:
         return cnt.value
 
     def sync_to_host(self, arr=None):
-        self._check(self.lib.swap_sync_to_host(self.ctx, None if arr is None else arr.ctypes.data_as(C.c_void_p)))
+        self._check(self.lib.swap_sync_to_host(self.ctx, None if arr is None else abi.addr(arr)))
 
     def sync_to_device(self, arr=None):
-        self._check(self.lib.swap_sync_to_device(self.ctx, None if arr is None else arr.ctypes.data_as(C.c_void_p)))
+        self._check(self.lib.swap_sync_to_device(self.ctx, None if arr is None else abi.addr(arr)))
 
     def mark_host_dirty(self, arr=None):
-        self._check(self.lib.swap_mark_host_dirty(self.ctx, None if arr is None else arr.ctypes.data_as(C.c_void_p)))
+        self._check(self.lib.swap_mark_host_dirty(self.ctx, None if arr is None else abi.addr(arr)))
 
     def set_host_direct(self, on: bool):
         """Let the FP32 form's conversions read and write the FP64 particle arrays in host memory."""
