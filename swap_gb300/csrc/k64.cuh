@@ -30,9 +30,11 @@ cudaError_t periodic1(const Geo& g, double* b, cudaStream_t st);
 // the operator's B input, which the caller sees filled.  Every grid output
 // is stored with its ghost images unless noted.
 // curlB: aj at the interior (ghosts untouched); btc (may be null):
-// edge_to_center of b at the interior.
-cudaError_t curlB(const Geo& g, double* b, const double* np, double alpha, double* aj, double* btc, bool fill,
-                  cudaStream_t st);
+// edge_to_center of b at the interior.  den (may be null): face_density's.
+cudaError_t curlB(const Geo& g, double* b, const double* np, const double* den, double alpha, double* aj,
+                  double* btc, bool fill, cudaStream_t st);
+// Per component the face density times alpha and its reciprocal, [6][C], interior.
+cudaError_t face_density(const Geo& g, const double* np, double alpha, double* den, cudaStream_t st);
 // ct = face_to_center(aj - up) x B at the centres, interior.  corr: b holds
 // curlB's btc, averaged to the faces and back; otherwise the edge field.
 cudaError_t cross_ct(const Geo& g, bool corr, const double* aj, const double* up, double* b, double* ct, bool fill,

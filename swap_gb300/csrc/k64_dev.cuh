@@ -5,24 +5,37 @@
 
 namespace swapk {
 
-// x / d for a grid spacing d with r = 1/d rounded: exactly the rounded
-// quotient.  P2 (every spacing a power of two): r is exact, and x * r is x / d
-// with the same single rounding.  Otherwise Markstein's correction (P.
-// Markstein, IBM J. Res. Dev. 34, 1990): q = x*r, then q + (x - q*d)*r in
-// fused operations is the rounded quotient when r is the rounded reciprocal
-// and nothing underflows or overflows; x outside 2^-900..2^900 takes the
-// division.  (The host keeps r = 0 for a spacing outside 2^-60..2^60 or with
-// an all-ones significand, the exception of the theorem.)
-template <bool P2>
+// How a quotient by a grid spacing is formed (Geo::spacing, set by the host).
+enum Spacing : int {
+  SPACING_ANY = 0,
+  SPACING_P2 = 1,    // every spacing a power of two: its reciprocal is exact
+  SPACING_UNIT = 2,  // every spacing one (lengths in cells): nothing to do
+};
+
+// x / d with r = 1/d rounded: exactly the rounded quotient.  A power of two: x
+// * r is x / d with the same single rounding.  Otherwise Markstein's
+// correction (P. Markstein, IBM J. Res. Dev. 34, 1990): q = x*r, then q + (x -
+// q*d)*r in fused operations is the rounded quotient when r is the rounded
+// reciprocal and nothing underflows or overflows: three operations instead of
+// about nine.  x outside 2^-900..2^900 takes the division; reciprocal() is 0
+// where the theorem does not hold (d outside 2^-60..2^60, or with an all-ones
+// significand) and d is divided by.
+template <int SP>
 __device__ __forceinline__ double quotient(double x, double d, double r) {
-  if (P2) return x * r;
+  if (SP == SPACING_UNIT) return x;
+  if (SP == SPACING_P2) return x * r;
   const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
-  if (e - 123u > 1800u || r == 0.0) {
-    if (((unsigned)__double2hiint(x) << 1 | (unsigned)__double2loint(x)) == 0u && r != 0.0) return x * r;  // +-0
-    return x / d;
+  if (e - 123u > 1800u || __double_as_longlong(r) == 0) {
+    const bool zero = ((unsigned)__double2hiint(x) << 1 | (unsigned)__double2loint(x)) == 0u;
+    return zero && __double_as_longlong(r) != 0 ? x * r : x / d;
   }
   const double q = x * r;
   return __fma_rn(__fma_rn(-q, d, x), r, q);
+}
+__device__ __forceinline__ double reciprocal(double d) {
+  const unsigned hi = (unsigned)__double2hiint(d), e = hi >> 20;  // the sign bit puts a negative d out of range
+  const bool ones = (hi & 0xfffffu) == 0xfffffu && (unsigned)__double2loint(d) == 0xffffffffu;
+  return e - 963u <= 120u && !ones ? 1.0 / d : 0.0;
 }
 
 // The bits of a double as an integer that orders like it (NaN beyond the
@@ -58,7 +71,7 @@ __device__ __forceinline__ bool weights_at(const Geo& g, double x, double y, dou
                                            double (&w)[8]) {
   i = find_cell(g.qx, g.nx, x, (float)g.qx[1], (float)g.inv_dx);
   k = find_cell(g.qz, g.nz, z, (float)g.qz[1], (float)g.inv_dz);
-  j = __double2int_rz(quotient<false>(y, g.dy, g.rdy));  // floor for y >= 0; any y below is outside either way
+  j = __double2int_rz(quotient<SPACING_ANY>(y, g.dy, g.rdy));  // floor for y >= 0; any y below is outside either way
   if (!(i >= 1 && j >= 1 && j < g.ny && k >= 1)) {
     i = j = k = 1;
 #pragma unroll

@@ -124,25 +124,40 @@ __device__ __forceinline__ void fill3(const Geo& g, const Node& n, double* f) {
 
 // curlB (gutsf.f:202-239); the face densities' np is read as it stands (the
 // reference does not fill its ghosts here).
-template <bool P2>
-__device__ __forceinline__ void curlB_node(const Geo& g, const Node& n, const Nbr& d, const double* __restrict__ b,
-                                           const double* __restrict__ np, double alpha, double* __restrict__ aj) {
+// den (may be null): the divisors and their reciprocals (face_density).
+__device__ __forceinline__ void face_densities(const Geo& g, const double* np, double alpha, unsigned o,
+                                               double (&f)[3]) {
+  const double n0 = np[o];
+  f[0] = 0.5 * (n0 + np[o + 1]) * alpha;
+  f[1] = 0.5 * (n0 + np[o + g.nx]) * alpha;
+  f[2] = 0.5 * (n0 + np[o + g.nx * g.ny]) * alpha;
+}
+template <int SP>
+__device__ __forceinline__ void curlB_node(const Geo& g, const Node& n, const Nbr& d, const double* b,
+                                           const double* np, const double* den, double alpha, double* aj) {
   const long long C = g.C;
   const unsigned o = n.o;
-  const double n0 = np[o];
-  const double nt1 = 0.5 * (n0 + np[o + 1]);
-  const double nt2 = 0.5 * (n0 + np[o + g.nx]);
-  const double nt3 = 0.5 * (n0 + np[o + g.nx * g.ny]);
   const double *B1 = b, *B2 = b + C, *B3 = b + 2 * C;
   const double dx = g.dxc[n.i], dy = g.dyc[n.j], dz = g.dzc[n.k];
   const double rx = g.rdxc[n.i], ry = g.rdyc[n.j], rz = g.rdzc[n.k];
   const double b1 = B1[o], b2 = B2[o], b3 = B3[o];
-  const double c1 = quotient<P2>(b3 - B3[o + d.ym], dy, ry) + quotient<P2>(B2[o + d.zm] - b2, dz, rz);
-  const double c2 = quotient<P2>(b1 - B1[o + d.zm], dz, rz) + quotient<P2>(B3[o + d.xm] - b3, dx, rx);
-  const double c3 = quotient<P2>(b2 - B2[o + d.xm], dx, rx) + quotient<P2>(B1[o + d.ym] - b1, dy, ry);
-  aj[o] = c1 / (nt1 * alpha);
-  aj[o + C] = c2 / (nt2 * alpha);
-  aj[o + 2 * C] = c3 / (nt3 * alpha);
+  const double c1 = quotient<SP>(b3 - B3[o + d.ym], dy, ry) + quotient<SP>(B2[o + d.zm] - b2, dz, rz);
+  const double c2 = quotient<SP>(b1 - B1[o + d.zm], dz, rz) + quotient<SP>(B3[o + d.xm] - b3, dx, rx);
+  const double c3 = quotient<SP>(b2 - B2[o + d.xm], dx, rx) + quotient<SP>(B1[o + d.ym] - b1, dy, ry);
+  if (den) {
+    const double a1 = quotient<SPACING_ANY>(c1, den[o], den[o + 3 * C]);
+    const double a2 = quotient<SPACING_ANY>(c2, den[o + C], den[o + 4 * C]);
+    const double a3 = quotient<SPACING_ANY>(c3, den[o + 2 * C], den[o + 5 * C]);
+    aj[o] = a1;
+    aj[o + C] = a2;
+    aj[o + 2 * C] = a3;
+  } else {
+    double f[3];
+    face_densities(g, np, alpha, o, f);
+    aj[o] = c1 / f[0];
+    aj[o + C] = c2 / f[1];
+    aj[o + 2 * C] = c3 / f[2];
+  }
 }
 
 // edge_to_center (grid_interp.f:22-57).
@@ -238,7 +253,7 @@ __device__ __forceinline__ void e_node(const Geo& g, const Node& n, const Nbr& d
 // gutsf.f:1158-1159 with coef = 2*dtsub; correct_B :1349-1350 with coef =
 // dtsub), with b1p2's ghost images.  half: also the B at m+1/2 of get_Ep1
 // (gutsf.f:1210-1219), 0.5*(b1p2 + b1), at the interior nodes.
-template <bool P2>
+template <int SP>
 __device__ __forceinline__ void b_node(const Geo& g, const Node& n, const Nbr& d, const double* __restrict__ E,
                                        const double* __restrict__ base, double coef, double* __restrict__ b1p2,
                                        const double* __restrict__ b1, double* __restrict__ half) {
@@ -248,9 +263,9 @@ __device__ __forceinline__ void b_node(const Geo& g, const Node& n, const Nbr& d
   const double dx = g.dxg[n.i], dy = g.dyg[n.j], dz = g.dzg[n.k];
   const double rx = g.rdxg[n.i], ry = g.rdyg[n.j], rz = g.rdzg[n.k];
   const double e1 = E1[o], e2 = E2[o], e3 = E3[o];
-  const double ce1 = quotient<P2>(E3[o + d.yp] - e3, dy, ry) + quotient<P2>(e2 - E2[o + d.zp], dz, rz);
-  const double ce2 = quotient<P2>(e3 - E3[o + d.xp], dx, rx) + quotient<P2>(E1[o + d.zp] - e1, dz, rz);
-  const double ce3 = quotient<P2>(e1 - E1[o + d.yp], dy, ry) + quotient<P2>(E2[o + d.xp] - e2, dx, rx);
+  const double ce1 = quotient<SP>(E3[o + d.yp] - e3, dy, ry) + quotient<SP>(e2 - E2[o + d.zp], dz, rz);
+  const double ce2 = quotient<SP>(e3 - E3[o + d.xp], dx, rx) + quotient<SP>(E1[o + d.zp] - e1, dz, rz);
+  const double ce3 = quotient<SP>(e1 - E1[o + d.yp], dy, ry) + quotient<SP>(E2[o + d.xp] - e2, dx, rx);
   const double v0 = base[o] - coef * ce1;
   const double v1 = base[o + C] - coef * ce2;
   const double v2 = base[o + 2 * C] - coef * ce3;
@@ -277,11 +292,12 @@ __device__ __forceinline__ void b_node(const Geo& g, const Node& n, const Nbr& d
 
 // curlB; FILL: b's ghosts too (curlB begins with periodic(b)).  btc (not
 // null): edge_to_center of b at the interior nodes, for the corrector.
-template <bool P2>
-__global__ void __launch_bounds__(TPB) k_curlB(Geo g, double* b, const double* __restrict__ np, double alpha,
+template <int SP>
+__global__ void __launch_bounds__(TPB) k_curlB(Geo g, double* b, const double* __restrict__ np,
+                                               const double* __restrict__ den, double alpha,
                                                double* __restrict__ aj, double* __restrict__ btc, bool fill) {
   NODES(n, d);
-  curlB_node<P2>(g, n, d, b, np, alpha, aj);
+  curlB_node<SP>(g, n, d, b, np, den, alpha, aj);
   if (btc) {
     double c[3];
     e2c_node(g, n, d, b, c);
@@ -290,6 +306,22 @@ __global__ void __launch_bounds__(TPB) k_curlB(Geo g, double* b, const double* _
     btc[n.o + 2 * g.C] = c[2];
   }
   if (fill) fill3(g, n, b);
+}
+
+// The divisors of curlB and their reciprocals: once per field step, where each
+// of its 20 curls divided anew (nine operations a quotient).
+__global__ void __launch_bounds__(TPB) k_face_density(Geo g, const double* __restrict__ np, double alpha,
+                                                      double* __restrict__ den) {
+  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (unsigned)n_interior(g)) return;
+  const unsigned o = node_of(g, t).o;
+  double f[3];
+  face_densities(g, np, alpha, o, f);
+#pragma unroll
+  for (int m = 0; m < 3; ++m) {
+    den[o + g.C * m] = f[m];
+    den[o + g.C * (3 + m)] = reciprocal(f[m]);
+  }
 }
 
 template <bool CORR>
@@ -307,12 +339,12 @@ __global__ void __launch_bounds__(TPB) k_E(Geo g, const double* __restrict__ ct,
   e_node(g, n, d, ct, nu, aj, np, gp, E);
 }
 
-template <bool P2>
+template <int SP>
 __global__ void __launch_bounds__(TPB) k_B(Geo g, const double* __restrict__ E, const double* __restrict__ base,
                                            double coef, double* __restrict__ b1p2, const double* __restrict__ b1,
                                            double* __restrict__ half) {
   NODES(n, d);
-  b_node<P2>(g, n, d, E, base, coef, b1p2, b1, half);
+  b_node<SP>(g, n, d, E, base, coef, b1p2, b1, half);
 }
 
 // 0.5*(a + b) at the interior nodes (gutsf.f:1210-1219); the consumers read
@@ -430,10 +462,14 @@ __global__ void __launch_bounds__(TPB) k_kit(Geo g, double* aj, const double* __
     return cudaGetLastError();                                        \
   } while (0)
 
-cudaError_t curlB(const Geo& g, double* b, const double* np, double alpha, double* aj, double* btc, bool fill,
-                  cudaStream_t st) {
-  if (g.spacing_p2) FL(k_curlB<true>, g, b, np, alpha, aj, btc, fill);
-  FL(k_curlB<false>, g, b, np, alpha, aj, btc, fill);
+cudaError_t curlB(const Geo& g, double* b, const double* np, const double* den, double alpha, double* aj,
+                  double* btc, bool fill, cudaStream_t st) {
+  if (g.spacing == SPACING_UNIT) FL(k_curlB<SPACING_UNIT>, g, b, np, den, alpha, aj, btc, fill);
+  if (g.spacing == SPACING_P2) FL(k_curlB<SPACING_P2>, g, b, np, den, alpha, aj, btc, fill);
+  FL(k_curlB<SPACING_ANY>, g, b, np, den, alpha, aj, btc, fill);
+}
+cudaError_t face_density(const Geo& g, const double* np, double alpha, double* den, cudaStream_t st) {
+  FL(k_face_density, g, np, alpha, den);
 }
 cudaError_t cross_ct(const Geo& g, bool corr, const double* aj, const double* up, double* b, double* ct, bool fill,
                      cudaStream_t st) {
@@ -446,8 +482,9 @@ cudaError_t e_field(const Geo& g, const double* ct, const double* nu, const doub
 }
 cudaError_t b_advance(const Geo& g, const double* E, const double* base, double coef, double* b1p2, const double* b1,
                       double* half, cudaStream_t st) {
-  if (g.spacing_p2) FL(k_B<true>, g, E, base, coef, b1p2, b1, half);
-  FL(k_B<false>, g, E, base, coef, b1p2, b1, half);
+  if (g.spacing == SPACING_UNIT) FL(k_B<SPACING_UNIT>, g, E, base, coef, b1p2, b1, half);
+  if (g.spacing == SPACING_P2) FL(k_B<SPACING_P2>, g, E, base, coef, b1p2, b1, half);
+  FL(k_B<SPACING_ANY>, g, E, base, coef, b1p2, b1, half);
 }
 cudaError_t half_sum(const Geo& g, const double* a, const double* b, double* out, cudaStream_t st) {
   FL(k_half, g, a, b, out);

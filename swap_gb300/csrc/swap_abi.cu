@@ -261,7 +261,7 @@ int edge_to_center(swap_ctx* c, double* bt, double* btc) {
 
 // curlB (gutsf.f:178-244)
 int curlB(swap_ctx* c, double* bt, const double* np, double* aj) {
-  KL("curlB", swapk::curlB(c->g, bt, np, c->prm.alpha, aj, nullptr, true, c->st));
+  KL("curlB", swapk::curlB(c->g, bt, np, nullptr, c->prm.alpha, aj, nullptr, true, c->st));
   return 0;
 }
 
@@ -284,8 +284,8 @@ int predict_B(swap_ctx* c, double* b12, double* b1p2, double* bt, double* E, dou
 // get_Ep1 (gutsf.f:1174-1304) + correct_B (gutsf.f:1309-1359) from B at
 // m+1/2 (s_btp1, interior): writes aj, E and out.
 static int correct_from_half(swap_ctx* c, const double* b1, double* out, double* E, double* aj, const double* up,
-                             const double* np, const double* nu, double dtsub) {
-  KL("curlB", swapk::curlB(c->g, c->s_btp1, np, c->prm.alpha, aj, c->s_btc2, false, c->st));
+                             const double* np, const double* den, const double* nu, double dtsub) {
+  KL("curlB", swapk::curlB(c->g, c->s_btp1, np, den, c->prm.alpha, aj, c->s_btc2, false, c->st));
   KL("cross_ct", cross_ct(c->g, true, aj, up, c->s_btc2, c->s_ct, false, c->st));
   KL("e_field", e_field(c->g, c->s_ct, nu, aj, np, c->prm.grad_pe, E, c->st));
   KL("b_advance", b_advance(c->g, E, b1, dtsub, out, nullptr, nullptr, c->st));
@@ -295,7 +295,7 @@ static int correct_from_half(swap_ctx* c, const double* b1, double* out, double*
 int correct_B(swap_ctx* c, double* b1, double* b1p2, double* E, double* aj, double* up, double* np, double* nu,
               double dtsub) {
   KL("half_sum", half_sum(c->g, b1p2, b1, c->s_btp1, c->st));
-  return correct_from_half(c, b1, b1p2, E, aj, up, np, nu, dtsub);
+  return correct_from_half(c, b1, b1p2, E, aj, up, np, nullptr, nu, dtsub);
 }
 
 // n subcycles (maind.f:425-476) on arrays that stay on the device.  The same
@@ -306,14 +306,18 @@ int correct_B(swap_ctx* c, double* b1, double* b1p2, double* E, double* aj, doub
 int subcycle_loop(swap_ctx* c, int n, double* b1, double* b12, double* b1p2, double* bt, double* E, double* aj,
                   const double* up, const double* np, const double* nu, double dtsub) {
   if (n <= 0) return 0;
+  // the face densities do not change meanwhile: their products with alpha and
+  // the reciprocals once, in the particle passes' table (free now)
+  double* den = c->s_kit;
+  KL("face_density", face_density(c->g, np, c->prm.alpha, den, c->st));
   double *now = b1, *old = b12;
   for (int s = 0; s < n; ++s) {
     double* b = s == 0 ? bt : now;
-    KL("curlB", swapk::curlB(c->g, b, np, c->prm.alpha, aj, nullptr, s == 0, c->st));
+    KL("curlB", swapk::curlB(c->g, b, np, den, c->prm.alpha, aj, nullptr, s == 0, c->st));
     KL("cross_ct", cross_ct(c->g, false, aj, up, b, c->s_ct, false, c->st));
     KL("e_field", e_field(c->g, c->s_ct, nu, aj, np, c->prm.grad_pe, E, c->st));
     KL("b_advance", b_advance(c->g, E, old, 2.0 * dtsub, nullptr, now, c->s_btp1, c->st));
-    TRY(correct_from_half(c, now, old, E, aj, up, np, nu, dtsub));
+    TRY(correct_from_half(c, now, old, E, aj, up, np, den, nu, dtsub));
     std::swap(now, old);
   }
   const std::size_t bytes = 3 * (std::size_t)c->g.C * sizeof(double);
@@ -535,7 +539,7 @@ extern "C" int swap_init(swap_ctx** out, const swap_dims* d, const swap_params* 
   }
   // reciprocals of the spacings (k64_field.cu quotient), 1-based like them
   const double* rec[6];
-  bool p2 = true;
+  bool p2 = true, unit = true;
   for (int a = 0; a < 6; ++a) {
     const int n = ns[3 + a];
     std::vector<double> h((std::size_t)n + 1, 0.0);
@@ -545,7 +549,10 @@ extern "C" int swap_init(swap_ctx** out, const swap_dims* d, const swap_params* 
       const double m = std::frexp(v, &e);  // in [0.5, 1) for a normal positive v
       const bool fits = v > 0.0 && std::isfinite(v) && e > -60 && e < 60;
       if (fits && m != 1.0 - 0x1p-53) h[(std::size_t)q] = 1.0 / v;
-      if (q >= 2 && q <= n - 1) p2 = p2 && fits && m == 0.5;  // the stencils' nodes
+      if (q >= 2 && q <= n - 1) {  // the stencils' nodes
+        p2 = p2 && fits && m == 0.5;
+        unit = unit && v == 1.0;
+      }
     }
     double* r = c->dalloc(h.size());
     if (!r || cudaMemcpy(r, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess) {
@@ -557,7 +564,7 @@ extern "C" int swap_init(swap_ctx** out, const swap_dims* d, const swap_params* 
   Geo& g = c->g;
   g.rdxg = rec[0]; g.rdyg = rec[1]; g.rdzg = rec[2];
   g.rdxc = rec[3]; g.rdyc = rec[4]; g.rdzc = rec[5];
-  g.spacing_p2 = p2;
+  g.spacing = unit ? 2 : (p2 ? 1 : 0);  // Spacing, k64_dev.cuh
   g.nx = d->nx; g.ny = d->ny; g.nz = d->nz;
   g.C = (long long)d->nx * d->ny * d->nz;
   g.qx = dg[0]; g.qy = dg[1]; g.qz = dg[2];

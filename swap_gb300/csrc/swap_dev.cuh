@@ -19,10 +19,10 @@ struct Geo {
   const double *dxg, *dyg, *dzg;  // dx_grid ...
   const double *dxc, *dyc, *dzc;  // dx_cell ...
   const double *xr, *yr, *zr;     // xrat ...
-  // 1/spacing, rounded (0: divide instead); spacing_p2: every interior
-  // spacing is a power of two, its reciprocal exact (k64_field.cu quotient)
+  // 1/spacing, rounded (0: divide instead), and what all interior spacings
+  // have in common (Spacing, k64_dev.cuh)
   const double *rdxg, *rdyg, *rdzg, *rdxc, *rdyc, *rdzc;
-  bool spacing_p2;
+  int spacing;
   // uniform: every cell has the same spacings, bit for bit; cell_q and cell_g
   // are then the products of a cell's node differences and of dx_grid ...
   bool uniform;
