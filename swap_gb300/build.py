@@ -30,6 +30,7 @@ UNITS = [
     ("k64_field.cu", ["--fmad=false"]),
     ("k64_pass.cu", ["--fmad=false"]),
     ("k32.cu", []),
+    ("grid_loop.cu", []),
     ("swap_abi.cu", []),
     ("swap_f32.cu", []),
     ("swap_prof.cu", []),

@@ -2,6 +2,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "grid_loop.cuh"
 #include "k32.cuh"
 #include "philox.h"
 #include "swap_dev.cuh"
@@ -1057,63 +1058,19 @@ __global__ void __launch_bounds__(FBX * FBY) k_bstep(G32 g, const float* __restr
 // operands.  Two forms.  CLUSTER: one cluster of FIELD_CLUSTER blocks, which
 // meet at the hardware's cluster barrier (0.24 us) -- up to FIELD_CLUSTER *
 // LOOP_TPB nodes.  Otherwise a cooperative launch with a counter in memory
-// (1.2 us at 152 blocks), at most one block per SM, so that the loops of two
-// contexts on one GPU are resident side by side.
+// (1.2 us at 152 blocks; grid_loop.cuh).
 // A step of 8 ions per cell, loop against launches, in ms: 1.5k nodes 0.234
 // against 0.325, 33k 0.314 against 0.342, 65k 0.341 against 0.408, 131k 0.533
 // against 0.524, 262k 0.887 against 0.791 (one block per SM then hides less
 // latency than full occupancy does): hence FIELD_LOOP_NODES.
 constexpr int LOOP_TPB = 512;
 
-struct LoopBarrier {
-  unsigned* bar;  // [0] arrivals, [1] blocks that are through
-  unsigned polls;
-  unsigned target;
-  bool ok;
-  // Every block's stores before it are visible to every block after it;
-  // false: the wait ran out (the caller returns).
-  template <bool CLUSTER>
-  __device__ __forceinline__ bool sync() {
-    if (CLUSTER) {
-      asm volatile(
-          "barrier.cluster.arrive.release.aligned;\n"
-          "barrier.cluster.wait.acquire.aligned;" ::
-              : "memory");
-      return true;
-    }
-    target += gridDim.x;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      __threadfence();
-      atomicAdd(bar, 1u);
-      unsigned v, n = 0;
-      do {
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-      } while (v < target && n++ < polls);
-      __threadfence();
-      ok = v >= target;
-    }
-    return !__syncthreads_or(threadIdx.x == 0 && !ok);
-  }
-  // The last block to finish leaves the counters at zero for the next launch.
-  __device__ __forceinline__ void done() {
-    if (threadIdx.x == 0) {
-      __threadfence();
-      if (atomicAdd(bar + 1, 1u) == gridDim.x - 1) {
-        bar[0] = 0u;
-        bar[1] = 0u;
-        __threadfence();
-      }
-    }
-  }
-};
-
 template <bool CLUSTER>
 __global__ void __launch_bounds__(LOOP_TPB, 2) k_field_loop(G32 g, FieldLoop f) {
   // uniform over the grid (both words are a snapshot that nothing writes
   // now): a failed pass or a Courant violation leaves the state as it is
   if (*f.failed != 0 || (double)*f.courant <= f.courant_floor) return;
-  LoopBarrier bar{f.bar, f.polls, 0u, true};
+  loop::Barrier bar{f.bar, f.polls, 0u, true};
   const unsigned n = (unsigned)n_int(g), t0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
   float *b1h = f.b1h, *b1l = f.b1l, *b12h = f.b12h, *b12l = f.b12l, *bph = f.bph, *bpl = f.bpl, *db1 = f.db1,
         *dbp = f.dbp;
@@ -1894,15 +1851,10 @@ cudaError_t field_loop(const G32& g, const FieldLoop& f, cudaStream_t st) {
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k_field_loop<true>, g, f);
   }
-  int dev = 0, sms = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e != cudaSuccess) return e;
   G32 gg = g;
   FieldLoop ff = f;
   void* args[] = {&gg, &ff};
-  return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&k_field_loop<false>),
-                                     dim3((unsigned)(need < sms ? need : sms)), dim3(LOOP_TPB), args, 0, st);
+  return loop::launch(reinterpret_cast<const void*>(&k_field_loop<false>), need, LOOP_TPB, args, st);
 }
 cudaError_t b_step_given_e(const G32& g, const float* E, const float* bh, const float* bl, double coef,
                            const float* b0c, float* oh, float* ol, float* dbo, cudaStream_t st) {

@@ -61,10 +61,13 @@ __global__ void k_grad_pe_face(Geo g, const double* __restrict__ np, double gp, 
   }
 }
 
-// Whistler Courant time of check_time_step (gutsf.f:1785-1792) at every node.
+// Whistler Courant time of check_time_step (gutsf.f:1785-1792) at every node,
+// and the bits of the smallest (non-negative doubles order like them), one
+// atomic per block.
 __global__ void k_deltat(Geo g, const double* __restrict__ bt, const double* __restrict__ np, double alpha,
-                         double dx, double* __restrict__ dtn) {
+                         double dx, double* __restrict__ dtn, unsigned long long* least) {
   const long long C = g.C;
+  double mn = 1.0e306;
   GRID_STRIDE(o, C) {
     const double ak = 2. / dx;
     const double b1 = bt[o], b2 = bt[o + C], b3 = bt[o + 2 * C];
@@ -73,7 +76,17 @@ __global__ void k_deltat(Geo g, const double* __restrict__ bt, const double* __r
     const double a2 = (ak * btot) * (ak * btot) / (alpha * (np[o]));
     const double womega = 0.5 * (a1 + sqrt(a1 * a1 + 4.0 * a2));
     const double phi = womega / ak;
-    dtn[o] = dx / phi;
+    const double dt = dx / phi;
+    dtn[o] = dt;
+    mn = fmin(mn, dt);
+  }
+  __shared__ double s_mn[TPB / 32];
+  for (int o = 16; o > 0; o >>= 1) mn = fmin(mn, __shfl_down_sync(0xffffffffu, mn, o));
+  if ((threadIdx.x & 31) == 0) s_mn[threadIdx.x >> 5] = mn;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) mn = fmin(mn, s_mn[w]);
+    atomicMin(least, (unsigned long long)__double_as_longlong(mn > 0.0 ? mn : 0.0));
   }
 }
 
@@ -424,14 +437,6 @@ __device__ __forceinline__ double block_sum(double v) {
   return r;  // valid in thread 0
 }
 
-// Non-negative doubles order like their bit patterns.
-__global__ void k_min_nonneg(const double* __restrict__ x, long long n, unsigned long long* out) {
-  double m = 1.0e308;
-  GRID_STRIDE(t, n) m = fmin(m, x[t]);
-  for (int o = 16; o > 0; o >>= 1) m = fmin(m, __shfl_down_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMin(out, (unsigned long long)__double_as_longlong(m > 0.0 ? m : 0.0));
-}
-
 __global__ void k_energy_particles(PartDev p, long long N, double beta, const double* __restrict__ vp,
                                    double* acc) {
   double s = 0.0;
@@ -535,8 +540,10 @@ cudaError_t grad_pe_face_int(const Geo& g, const double* np, double gp, double* 
   LAUNCH(k_grad_pe_face, n_interior(g), g, np, gp, gf);
 }
 cudaError_t deltat_all(const Geo& g, const double* bt, const double* np, double alpha, double dx, double* dtn,
-                       cudaStream_t st) {
-  LAUNCH(k_deltat, g.C, g, bt, np, alpha, dx, dtn);
+                       unsigned long long* least, cudaStream_t st) {
+  const cudaError_t e = cudaMemsetAsync(least, 0x7f, sizeof(*least), st);  // 1.4e306
+  if (e != cudaSuccess) return e;
+  LAUNCH(k_deltat, g.C, g, bt, np, alpha, dx, dtn, least);
 }
 cudaError_t interp_weights(const Geo& g, const PartDev& p, long long N, int* err, cudaStream_t st) {
   if (N <= 0) return cudaSuccess;
@@ -591,12 +598,6 @@ cudaError_t move_half(const Geo& g, const PartDev& p, long long N, double dt, do
                       bool x_open, cudaStream_t st) {
   if (N <= 0) return cudaSuccess;
   LAUNCH(k_move_half, N, g, p, N, dt, xp, vp, x_open);
-}
-cudaError_t reduce_min(const double* x, long long n, double* d_out, int, cudaStream_t st) {
-  const unsigned long long init = (unsigned long long)0x7fefffffffffffffULL;  // DBL_MAX bits
-  cudaError_t e = cudaMemcpyAsync(d_out, &init, sizeof(init), cudaMemcpyHostToDevice, st);
-  if (e != cudaSuccess) return e;
-  LAUNCH(k_min_nonneg, n, x, n, reinterpret_cast<unsigned long long*>(d_out));
 }
 cudaError_t energy_parts(const Geo& g, const PartDev& p, long long N, double beta, double alpha, const double* vp,
                          const double* b0, const double* b1, const double* E, double* d_acc4, cudaStream_t st) {

@@ -46,6 +46,23 @@ cudaError_t e_field(const Geo& g, const double* ct, const double* nu, const doub
 // 0.5*(b1p2 + b1) at the interior.
 cudaError_t b_advance(const Geo& g, const double* E, const double* base, double coef, double* b1p2, const double* b1,
                       double* half, cudaStream_t st);
+// n subcycles of a small grid in one launch (field_loop_fits): as n rounds of
+// the launchers above with b1 and b12 changing places after each.  Nothing is
+// done when *courant (a double's bits) <= courant_floor: the caller looks too.
+constexpr long long FIELD_LOOP_NODES = 5 << 15;
+struct FieldLoop64 {
+  int n;
+  double *bt, *b1, *b12, *half, *btc, *ct, *E, *aj;
+  const double *up, *np, *nu, *den;
+  double gp, alpha, dtsub;
+  const unsigned long long* courant;
+  double courant_floor;
+  int* err;       // KERR_WAIT when a barrier's wait runs out
+  unsigned* bar;  // two counters, zero between launches
+  unsigned polls;
+};
+bool field_loop_fits(const Geo& g);
+cudaError_t field_loop(const Geo& g, const FieldLoop64& f, cudaStream_t st);
 // out = 0.5*(a + b) at the interior.
 cudaError_t half_sum(const Geo& g, const double* a, const double* b, double* out, cudaStream_t st);
 cudaError_t edge_to_center(const Geo& g, double* bt, double* btc, cudaStream_t st);
@@ -58,8 +75,9 @@ cudaError_t up_from_sums(const Geo& g, const double* S, double* np, double* up, 
 cudaError_t gather_kit(const Geo& g, bool full, double* aj, const double* up, const double* bt, double* btc,
                        double* kit, cudaStream_t st);
 
+// The Courant time per node, and the bits of the smallest into *least.
 cudaError_t deltat_all(const Geo& g, const double* bt, const double* np, double alpha, double dx, double* dtn,
-                       cudaStream_t st);
+                       unsigned long long* least, cudaStream_t st);
 cudaError_t grad_pe_face_int(const Geo& g, const double* np, double grad_pe, double* gf, cudaStream_t st);
 
 // gutsp.f particle operators
@@ -118,7 +136,6 @@ struct PassArgs {
 cudaError_t particle_pass(int pass, const PassArgs& a, cudaStream_t st);
 
 // reductions (FP64)
-cudaError_t reduce_min(const double* x, long long n, double* d_partial, int nblk, cudaStream_t st);
 cudaError_t energy_parts(const Geo& g, const PartDev& p, long long N, double beta, double alpha, const double* vp,
                          const double* b0, const double* b1, const double* E, double* d_acc4, cudaStream_t st);
 cudaError_t divb_max(const Geo& g, const double* b, double* d_max, cudaStream_t st);

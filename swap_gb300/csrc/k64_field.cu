@@ -25,6 +25,7 @@
 // correct_B: 1.04 -> 0.72 ms, of which on the
 // device 0.74 -> 0.36 ms (18x11x14: 0.355 -> 0.211 ms).
 #include "k64.cuh"
+#include "grid_loop.cuh"
 #include "k64_dev.cuh"
 
 namespace swapk {
@@ -161,7 +162,7 @@ __device__ __forceinline__ void curlB_node(const Geo& g, const Node& n, const Nb
 }
 
 // edge_to_center (grid_interp.f:22-57).
-__device__ __forceinline__ void e2c_node(const Geo& g, const Node& n, const Nbr& d, const double* __restrict__ bt,
+__device__ __forceinline__ void e2c_node(const Geo& g, const Node& n, const Nbr& d, const double* bt,
                                          double out[3]) {
   const long long C = g.C;
   const unsigned o = n.o;
@@ -196,9 +197,9 @@ __device__ __forceinline__ double f2c(double r, double v, double vm) { return r 
 // to the faces (grid_interp.f:123-125) and back to the centres
 // (gutsf.f:1268-1269).
 template <bool CORR>
-__device__ __forceinline__ void ct_node(const Geo& g, const Node& n, const Nbr& d, const double* __restrict__ aj,
-                                        const double* __restrict__ up, const double* __restrict__ b,
-                                        double* __restrict__ ct) {
+__device__ __forceinline__ void ct_node(const Geo& g, const Node& n, const Nbr& d, const double* aj,
+                                        const double* up, const double* b,
+                                        double* ct) {
   const long long C = g.C;
   const unsigned o = n.o;
   const double xr = g.xr[n.i], yr = g.yr[n.j], zr = g.zr[n.k];
@@ -231,9 +232,9 @@ __device__ __forceinline__ double grad_pe_at(const Geo& g, const double* np, dou
 
 // crossf2's face average (gutsf.f:94-96) and E = c + nu*aj (gutsf.f:1082,
 // 1282), with E's ghost images.
-__device__ __forceinline__ void e_node(const Geo& g, const Node& n, const Nbr& d, const double* __restrict__ ct,
-                                       const double* __restrict__ nu, const double* __restrict__ aj,
-                                       const double* __restrict__ np, double gp, double* __restrict__ E) {
+__device__ __forceinline__ void e_node(const Geo& g, const Node& n, const Nbr& d, const double* ct,
+                                       const double* nu, const double* aj,
+                                       const double* np, double gp, double* E) {
   const long long C = g.C;
   const unsigned o = n.o;
   const double nuo = nu[o];
@@ -254,9 +255,9 @@ __device__ __forceinline__ void e_node(const Geo& g, const Node& n, const Nbr& d
 // dtsub), with b1p2's ghost images.  half: also the B at m+1/2 of get_Ep1
 // (gutsf.f:1210-1219), 0.5*(b1p2 + b1), at the interior nodes.
 template <int SP>
-__device__ __forceinline__ void b_node(const Geo& g, const Node& n, const Nbr& d, const double* __restrict__ E,
-                                       const double* __restrict__ base, double coef, double* __restrict__ b1p2,
-                                       const double* __restrict__ b1, double* __restrict__ half) {
+__device__ __forceinline__ void b_node(const Geo& g, const Node& n, const Nbr& d, const double* E,
+                                       const double* base, double coef, double* b1p2,
+                                       const double* b1, double* half) {
   const long long C = g.C;
   const unsigned o = n.o;
   const double *E1 = E, *E2 = E + C, *E3 = E + 2 * C;
@@ -452,9 +453,80 @@ __global__ void __launch_bounds__(TPB) k_kit(Geo g, double* aj, const double* __
       }
 }
 
+// ---- the whole field step of a small grid in one launch ----
+//
+// The eight kernels of a subcycle as phases of one cooperative kernel, whose
+// blocks meet at a barrier (1.2 us) instead of in a launch: below
+// FIELD_LOOP_NODES a phase's FP64 work is about as long as a launch and the
+// ramp of its loads.  The same node functions on the same operands: the same
+// bits.  A step of 4 ions per cell, loop against launches, in ms: 960 nodes
+// 0.42 against 0.54, 33k 0.58 against 0.76, 65k 0.84 against 0.98, 131k 1.48
+// against 1.53, 262k 2.63 against 2.54 (16 warps per SM then hide less than a
+// full SM): hence FIELD_LOOP_NODES.
+constexpr int LOOP_TPB = 512;
+template <int SP>
+__global__ void __launch_bounds__(LOOP_TPB) k_field_loop(Geo g, FieldLoop64 f) {
+  // the same in every block: a Courant violation leaves the state as it is
+  if (__longlong_as_double((long long)*f.courant) <= f.courant_floor) return;
+  loop::Barrier bar{f.bar, f.polls, 0u, true};
+  const unsigned nodes = (unsigned)n_interior(g), t0 = blockIdx.x * blockDim.x + threadIdx.x,
+                 step = gridDim.x * blockDim.x;
+  auto each = [&](auto&& node) {
+    for (unsigned t = t0; t < nodes; t += step) {
+      const Node n = node_of(g, t);
+      node(n, nbr_of(g, n));
+    }
+    return bar.sync<false>();
+  };
+  double *now = f.b1, *old = f.b12;
+  for (int s = 0; s < f.n; ++s) {
+    double* b = s == 0 ? f.bt : now;
+    const bool on =
+        each([&](const Node& n, const Nbr& d) {
+          curlB_node<SP>(g, n, d, b, f.np, f.den, f.alpha, f.aj);
+          if (s == 0) fill3(g, n, b);
+        }) &&
+        each([&](const Node& n, const Nbr& d) { ct_node<false>(g, n, d, f.aj, f.up, b, f.ct); }) &&
+        each([&](const Node& n, const Nbr& d) { e_node(g, n, d, f.ct, f.nu, f.aj, f.np, f.gp, f.E); }) &&
+        each([&](const Node& n, const Nbr& d) {
+          b_node<SP>(g, n, d, f.E, old, 2.0 * f.dtsub, nullptr, now, f.half);
+        }) &&
+        each([&](const Node& n, const Nbr& d) {
+          curlB_node<SP>(g, n, d, f.half, f.np, f.den, f.alpha, f.aj);
+          double c[3];
+          e2c_node(g, n, d, f.half, c);
+          f.btc[n.o] = c[0];
+          f.btc[n.o + g.C] = c[1];
+          f.btc[n.o + 2 * g.C] = c[2];
+        }) &&
+        each([&](const Node& n, const Nbr& d) { ct_node<true>(g, n, d, f.aj, f.up, f.btc, f.ct); }) &&
+        each([&](const Node& n, const Nbr& d) { e_node(g, n, d, f.ct, f.nu, f.aj, f.np, f.gp, f.E); }) &&
+        each([&](const Node& n, const Nbr& d) { b_node<SP>(g, n, d, f.E, now, f.dtsub, old, nullptr, nullptr); });
+    if (!on) break;
+    double* q = now;
+    now = old;
+    old = q;
+  }
+  if (!bar.ok && threadIdx.x == 0) set_err(f.err, KERR_WAIT);
+  bar.done();
+}
+
 }  // namespace
 
 // ---- launchers --------------------------------------------------------------------
+
+bool field_loop_fits(const Geo& g) { return n_interior(g) <= FIELD_LOOP_NODES; }
+cudaError_t field_loop(const Geo& g, const FieldLoop64& f, cudaStream_t st) {
+  Geo gg = g;
+  FieldLoop64 ff = f;
+  void* args[] = {&gg, &ff};
+  const void* k = g.spacing == SPACING_UNIT ? reinterpret_cast<const void*>(&k_field_loop<SPACING_UNIT>)
+                  : g.spacing == SPACING_P2 ? reinterpret_cast<const void*>(&k_field_loop<SPACING_P2>)
+                                            : reinterpret_cast<const void*>(&k_field_loop<SPACING_ANY>);
+  // the nodes evenly over the SMs, a block on each
+  const long long n = n_interior(g), per = ((n + 151) / 152 + 31) / 32 * 32, t = per < LOOP_TPB ? per : LOOP_TPB;
+  return loop::launch(k, (n + t - 1) / t, (int)t, args, st);
+}
 
 #define FL(kern, ...)                                                 \
   do {                                                                \

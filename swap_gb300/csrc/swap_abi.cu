@@ -1,6 +1,7 @@
 // swap_abi.cu -- the extern "C" drop-in (include/swap_gpu.h): context,
 // registry of the caller's host arrays with device mirrors, and one entry per
 // reference subroutine built from the FP64 kernels in k64.cu.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -9,6 +10,7 @@
 #include <vector>
 
 #include "../../include/swap_gpu.h"
+#include "grid_loop.cuh"
 #include "k64.cuh"
 #include "swap_ctx.h"
 #include "swap_ops.h"
@@ -174,7 +176,7 @@ int swap_ctx::begin() {
 int swap_ctx::finish() {
   // the error word rides on the entry's own wait (a copy of its own after it
   // was a second round trip, 10 us of a 20 us entry)
-  cudaError_t e = cudaMemcpyAsync(h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, st);
+  cudaError_t e = cudaMemcpyAsync(&pinned->err, d_err, sizeof(int), cudaMemcpyDeviceToHost, st);
   const cudaError_t e2 = cudaStreamSynchronize(st);
   if (e == cudaSuccess) e = e2;
   if (e != cudaSuccess) return cuda_fail(e, "stream");
@@ -188,9 +190,10 @@ int swap_ctx::finish() {
     m->dev_valid = false;
   }
   touched_host.clear();
-  const int herr = *h_err;
+  const int herr = pinned->err;
   if (herr) {
     cudaMemset(d_err, 0, sizeof(int));
+    cudaMemset(loop_bar, 0, 2 * sizeof(unsigned));  // a barrier that gave up leaves its counters part-way
     if (herr == KERR_DOMAIN) return fail(SWAP_EDOMAIN, "a particle lies outside the grid");
     if (herr == KERR_MOVE) return fail(SWAP_EMOVE, "a particle moved more than one cell in one step");
     if (herr == KERR_WAIT) return fail(SWAP_EWAIT, "a device wait reached its iteration limit");
@@ -298,27 +301,49 @@ int correct_B(swap_ctx* c, double* b1, double* b1p2, double* E, double* aj, doub
   return correct_from_half(c, b1, b1p2, E, aj, up, np, nullptr, nu, dtsub);
 }
 
-// n subcycles (maind.f:425-476) on arrays that stay on the device.  The same
-// values as n rounds of curlB, predict_B, correct_B, f_update_tlev; the
-// predicted B is only ever used at m+1/2, so it is stored there alone, and
-// the time levels change places instead of being copied: b12's memory takes
-// the new B, which becomes b1.  From the second subcycle on bt is b1.
-int subcycle_loop(swap_ctx* c, int n, double* b1, double* b12, double* b1p2, double* bt, double* E, double* aj,
-                  const double* up, const double* np, const double* nu, double dtsub) {
-  if (n <= 0) return 0;
+// The subcycles of a fused step (maind.f:420-476) on arrays that stay on the
+// device: the values of check_time_step and rounds of curlB, predict_B,
+// correct_B and f_update_tlev.  The predicted B is only ever used at m+1/2,
+// so it is stored there alone, and the time levels change places instead of
+// being copied: b12's memory takes the new B, which becomes b1.  From the
+// second subcycle on bt is b1.
+int courant_begin(swap_ctx* c, const double* bt, const double* np);
+int courant_end(swap_ctx* c, double* dtsub, double* ntf);
+int field_step(swap_ctx* c, double* b1, double* b12, double* b1p2, double* bt, double* E, double* aj,
+               const double* up, const double* np, const double* nu, double* dtsub, double* ntf) {
+  TRY(courant_begin(c, bt, np));
   // the face densities do not change meanwhile: their products with alpha and
   // the reciprocals once, in the particle passes' table (free now)
   double* den = c->s_kit;
   KL("face_density", face_density(c->g, np, c->prm.alpha, den, c->st));
+  const bool looped = field_loop_fits(c->g);
+  if (looped) {  // goes out before the host has looked: it looks for itself
+    FieldLoop64 f{};
+    f.n = (int)*ntf;
+    f.bt = bt; f.b1 = b1; f.b12 = b12; f.half = c->s_btp1; f.btc = c->s_btc2; f.ct = c->s_ct; f.E = E; f.aj = aj;
+    f.up = up; f.np = np; f.nu = nu; f.den = den;
+    f.gp = c->prm.grad_pe; f.alpha = c->prm.alpha; f.dtsub = *dtsub;
+    f.courant = reinterpret_cast<const unsigned long long*>(c->s_red);
+    f.courant_floor = 2.0 * *dtsub;
+    f.err = c->d_err; f.bar = c->loop_bar; f.polls = std::max(c->wait_polls, loop::MIN_POLLS);
+    KL("field_loop", field_loop(c->g, f, c->st));
+  }
+  const double ntf0 = *ntf;
+  TRY(courant_end(c, dtsub, ntf));
+  const int n = (int)*ntf;
   double *now = b1, *old = b12;
-  for (int s = 0; s < n; ++s) {
-    double* b = s == 0 ? bt : now;
-    KL("curlB", swapk::curlB(c->g, b, np, den, c->prm.alpha, aj, nullptr, s == 0, c->st));
-    KL("cross_ct", cross_ct(c->g, false, aj, up, b, c->s_ct, false, c->st));
-    KL("e_field", e_field(c->g, c->s_ct, nu, aj, np, c->prm.grad_pe, E, c->st));
-    KL("b_advance", b_advance(c->g, E, old, 2.0 * dtsub, nullptr, now, c->s_btp1, c->st));
-    TRY(correct_from_half(c, now, old, E, aj, up, np, den, nu, dtsub));
-    std::swap(now, old);
+  if (looped && *ntf == ntf0) {
+    if (n & 1) std::swap(now, old);
+  } else {
+    for (int s = 0; s < n; ++s) {
+      double* b = s == 0 ? bt : now;
+      KL("curlB", swapk::curlB(c->g, b, np, den, c->prm.alpha, aj, nullptr, s == 0, c->st));
+      KL("cross_ct", cross_ct(c->g, false, aj, up, b, c->s_ct, false, c->st));
+      KL("e_field", e_field(c->g, c->s_ct, nu, aj, np, c->prm.grad_pe, E, c->st));
+      KL("b_advance", b_advance(c->g, E, old, 2.0 * *dtsub, nullptr, now, c->s_btp1, c->st));
+      TRY(correct_from_half(c, now, old, E, aj, up, np, den, nu, *dtsub));
+      std::swap(now, old);
+    }
   }
   const std::size_t bytes = 3 * (std::size_t)c->g.C * sizeof(double);
   auto copy = [&](double* d, const double* from) {
@@ -346,13 +371,16 @@ int f_update_tlev(swap_ctx* c, double* b1, double* b12, double* b1p2, double* bt
 // formed on the device; when even the smallest leaves the current dtsub
 // alone (the normal case) nothing changes.  Otherwise the reference's
 // ordered, per-node halving is replayed on the host from the node values.
-int check_time_step(swap_ctx* c, const double* bt, const double* np, double* dtsub, double* ntf) {
-  KL("deltat_all", deltat_all(c->g, bt, np, c->prm.alpha, c->prm.dx, c->s_dtn, c->st));
-  KL("reduce_min", reduce_min(c->s_dtn, c->g.C, c->s_red, 0, c->st));
-  double mn = 0;
-  KL("cudaMemcpyAsync", cudaMemcpyAsync(&mn, c->s_red, sizeof(double), cudaMemcpyDeviceToHost, c->st));
-  CU(cudaStreamSynchronize(c->st));
-  if (mn > 2.0 * *dtsub) return 0;
+int courant_begin(swap_ctx* c, const double* bt, const double* np) {
+  KL("deltat_all", deltat_all(c->g, bt, np, c->prm.alpha, c->prm.dx, c->s_dtn,
+                              reinterpret_cast<unsigned long long*>(c->s_red), c->st));
+  CU(cudaMemcpyAsync(&c->pinned->courant, c->s_red, sizeof(double), cudaMemcpyDeviceToHost, c->st));
+  CU(cudaEventRecord(c->ev_look, c->st));
+  return 0;
+}
+int courant_end(swap_ctx* c, double* dtsub, double* ntf) {
+  CU(cudaEventSynchronize(c->ev_look));
+  if (c->pinned->courant > 2.0 * *dtsub) return 0;
   std::vector<double> dtn((std::size_t)c->g.C);
   CU(cudaMemcpy(dtn.data(), c->s_dtn, dtn.size() * sizeof(double), cudaMemcpyDeviceToHost));
   const Geo& g = c->g;
@@ -366,6 +394,10 @@ int check_time_step(swap_ctx* c, const double* bt, const double* np, double* dts
       }
   if (*ntf > 1.0e6) return c->fail(SWAP_ESUBCYCLE, "subcycle count overflow in check_time_step");
   return 0;
+}
+int check_time_step(swap_ctx* c, const double* bt, const double* np, double* dtsub, double* ntf) {
+  TRY(courant_begin(c, bt, np));
+  return courant_end(c, dtsub, ntf);
 }
 
 // get_interp_weights (gutsp.f:1378-1435)
@@ -600,8 +632,10 @@ extern "C" int swap_init(swap_ctx** out, const swap_dims* d, const swap_params* 
   }
   c->owned.push_back(e);
   c->d_err = e;
-  if (cudaMallocHost(&c->h_err, sizeof(int)) != cudaSuccess) {
-    c->h_err = nullptr;
+  c->loop_bar = reinterpret_cast<unsigned*>(c->dalloc(1));
+  if (cudaMallocHost(&c->pinned, sizeof(*c->pinned)) != cudaSuccess) c->pinned = nullptr;
+  if (!c->pinned || !c->loop_bar || cudaMemset(c->loop_bar, 0, 2 * sizeof(unsigned)) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->ev_look, cudaEventDisableTiming) != cudaSuccess) {
     swap_finalize(c);
     return SWAP_ECUDA;
   }
@@ -623,7 +657,8 @@ extern "C" int swap_finalize(swap_ctx* c) {
   for (auto& kv : c->reg) cudaFree(kv.second.dev);
   for (void* p : c->owned) cudaFree(p);
   if (c->stage32) cudaFree(c->stage32);
-  if (c->h_err) cudaFreeHost(c->h_err);
+  if (c->pinned) cudaFreeHost(c->pinned);
+  if (c->ev_look) cudaEventDestroy(c->ev_look);
   if (c->t0) cudaEventDestroy(c->t0);
   if (c->t1) cudaEventDestroy(c->t1);
   c->prof_free();
@@ -1183,10 +1218,10 @@ int step_pre(swap_ctx* c, Bound& b, bool final_move = false, bool* moved = nullp
 int subcycles(swap_ctx* c, Bound& b) {
   double dtsub = c->prm.dt / (double)c->prm.ntsub;  // maind.f:420 (dtsub_init, inputs.f:142)
   double ntf = (double)c->prm.ntsub;                // :421
-  TRY(ops::check_time_step(c, b.bt, b.np, &dtsub, &ntf));  // :423
+  TRY(ops::field_step(c, b.b1, b.b12, b.b1p2, b.bt, b.E, b.aj, b.up, b.np, b.nu, &dtsub, &ntf));  // :423-476
   c->last_dtsub = dtsub;
   c->last_ntf = ntf;
-  return ops::subcycle_loop(c, (int)ntf, b.b1, b.b12, b.b1p2, b.bt, b.E, b.aj, b.up, b.np, b.nu, dtsub);  // :425-476
+  return SWAP_OK;
 }
 
 // maind.f:479 and the sinks after it (res_chex, maind.f:484).

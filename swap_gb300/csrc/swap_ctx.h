@@ -41,7 +41,15 @@ struct swap_ctx {
   swapk::Geo g{};
   cudaStream_t st = nullptr;
   int* d_err = nullptr;
-  int* h_err = nullptr;  // its value at the last finish(), pinned
+  // what the host reads back, in page-locked memory: the error word at the
+  // last finish(), the smallest Courant time once ev_look has passed
+  struct Pinned {
+    double courant;
+    int err;
+  };
+  Pinned* pinned = nullptr;
+  cudaEvent_t ev_look = nullptr;
+  unsigned* loop_bar = nullptr;  // barrier counters of the field loop
   std::string err;
 
   // registry of bound host arrays

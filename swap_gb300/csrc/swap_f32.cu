@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "../../include/swap_gpu.h"
+#include "grid_loop.cuh"
 #include "k32.cuh"
 #include "swap_dev.cuh"
 #include "swap_ctx.h"
@@ -505,7 +506,7 @@ static int subcycles(swap_ctx* c, F32State* s, float* e_acc = nullptr) {
     f.failed = reinterpret_cast<const int*>(s->d_min + 1);
     f.err = c->d_err;
     f.bar = s->loop_bar;
-    f.polls = c->wait_polls;
+    f.polls = std::max(c->wait_polls, loop::MIN_POLLS);
     KL("f32_field_loop", field_loop(g, f, c->st));
   }
   CU(cudaEventSynchronize(s->ev_look));

@@ -47,11 +47,14 @@ def test_operators_equal_the_oracle(cells, d):
     h.close()
 
 
-@pytest.mark.parametrize("ntsub", [1, 2, 5])
-def test_subcycles_equal_the_entries(ntsub):
-    """The fused loop leaves every array as the per-subroutine entries do."""
-    h, _ = _pair((9, 5, 6), (0.7, 1.3, 0.9), ntsub)
-    r, _ = _pair((9, 5, 6), (0.7, 1.3, 0.9), ntsub)
+@pytest.mark.parametrize("d", [(1.0, 1.0, 1.0), (0.7, 1.3, 0.9)])
+@pytest.mark.parametrize("cells,ntsub", [((9, 5, 6), 1), ((9, 5, 6), 2), ((1, 3, 2), 3), ((40, 30, 5), 5),
+                                         ((64, 64, 40), 2), ((64, 64, 41), 3)])
+def test_subcycles_equal_the_entries(cells, ntsub, d):
+    """The fused field step (one launch up to 163840 nodes, then one per
+    operator) leaves every array as the per-subroutine entries do."""
+    h, _ = _pair(cells, d, ntsub)
+    r, _ = _pair(cells, d, ntsub)
     h._check(h.lib.swap_field_subcycles(h.ctx))
     dtsub = r.cfg.dt / ntsub
     for _ in range(ntsub):
@@ -65,3 +68,19 @@ def test_subcycles_equal_the_entries(ntsub):
         assert np.array_equal(getattr(h, n), getattr(r, n)), n
     h.close()
     r.close()
+
+
+def test_courant_violation_takes_the_replayed_count():
+    """Above the Courant limit dtsub is halved on the host (gutsf.f:1776-1822);
+    the loop launched ahead of that look leaves the state alone."""
+    cfg = config(0, cells=(9, 5, 6), ppc=8, seed=4, ntsub=2, dt=2.0)  # dtsub of about twice the Courant time
+    x = Hybrid(cfg, ni_max=cfg.n_particles)
+    x.load_maxwellian()
+    y = oracle_for(x)
+    x.ion_step()
+    x.sync_to_host()
+    y.ion_step()
+    for n in ("b1", "b12", "E", "np"):
+        a, b = getattr(x, n), getattr(y, n)
+        assert np.max(np.abs(a - b)) <= 1e-12 * np.max(np.abs(b)), n
+    x.close()
