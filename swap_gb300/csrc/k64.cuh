@@ -132,8 +132,9 @@ struct PassArgs {
   int* err;
   bool x_open;      // pass 3: the x axis does not wrap, and an ion outside deposits nothing
   bool final_move;  // pass 3: also the half move of maind.f:479
+  double half_dt, quarter_dt2, half_dt2;  // set by particle_pass
 };
-cudaError_t particle_pass(int pass, const PassArgs& a, cudaStream_t st);
+cudaError_t particle_pass(int pass, PassArgs a, cudaStream_t st);
 
 // reductions (FP64)
 cudaError_t energy_parts(const Geo& g, const PartDev& p, long long N, double beta, double alpha, const double* vp,

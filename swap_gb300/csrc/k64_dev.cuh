@@ -32,6 +32,17 @@ __device__ __forceinline__ double quotient(double x, double d, double r) {
   const double q = x * r;
   return __fma_rn(__fma_rn(-q, d, x), r, q);
 }
+// 1/x to the last bit or two for x in [2^-500, 2^500]: the hardware's
+// approximation (20 bits or more) and two Newton-Raphson steps, four FP64
+// operations where a division takes about nine.
+__device__ __forceinline__ double fast_reciprocal(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  r = __fma_rn(__fma_rn(-x, r, 1.0), r, r);
+  return __fma_rn(__fma_rn(-x, r, 1.0), r, r);
+}
+__device__ __forceinline__ bool is_one(double x) { return __double_as_longlong(x) == 0x3ff0000000000000LL; }
+
 __device__ __forceinline__ double reciprocal(double d) {
   const unsigned hi = (unsigned)__double2hiint(d), e = hi >> 20;  // the sign bit puts a negative d out of range
   const bool ones = (hi & 0xfffffu) == 0xfffffu && (unsigned)__double2loint(d) == 0xffffffffu;
@@ -71,7 +82,9 @@ __device__ __forceinline__ bool weights_at(const Geo& g, double x, double y, dou
                                            double (&w)[8]) {
   i = find_cell(g.qx, g.nx, x, (float)g.qx[1], (float)g.inv_dx);
   k = find_cell(g.qz, g.nz, z, (float)g.qz[1], (float)g.inv_dz);
-  j = __double2int_rz(quotient<SPACING_ANY>(y, g.dy, g.rdy));  // floor for y >= 0; any y below is outside either way
+  // floor for y >= 0 (any y below is outside either way); a spacing of one
+  // needs no quotient
+  j = __double2int_rz(is_one(g.rdy) ? y : quotient<SPACING_ANY>(y, g.dy, g.rdy));
   if (!(i >= 1 && j >= 1 && j < g.ny && k >= 1)) {
     i = j = k = 1;
 #pragma unroll
@@ -83,14 +96,18 @@ __device__ __forceinline__ bool weights_at(const Geo& g, double x, double y, dou
   const double x1 = fabs(x - qx), x2 = fabs(x - qxp), y1 = fabs(y - qy), y2 = fabs(y - qyp), z1 = fabs(z - qz),
                z2 = fabs(z - qzp);
   const double x2y2 = x2 * y2, x1y2 = x1 * y2, x2y1 = x2 * y1, x1y1 = x1 * y1;
-  w[0] = x2y2 * z2 * vol;
-  w[1] = x1y2 * z2 * vol;
-  w[2] = x2y2 * z1 * vol;
-  w[3] = x1y2 * z1 * vol;
-  w[4] = x2y1 * z2 * vol;
-  w[5] = x1y1 * z2 * vol;
-  w[6] = x2y1 * z1 * vol;
-  w[7] = x1y1 * z1 * vol;
+  w[0] = x2y2 * z2;
+  w[1] = x1y2 * z2;
+  w[2] = x2y2 * z1;
+  w[3] = x1y2 * z1;
+  w[4] = x2y1 * z2;
+  w[5] = x1y1 * z2;
+  w[6] = x2y1 * z1;
+  w[7] = x1y1 * z1;
+  if (!is_one(vol)) {  // (a unit cell: the products are the weights)
+#pragma unroll
+    for (int c = 0; c < 8; ++c) w[c] = w[c] * vol;
+  }
   return true;
 }
 
@@ -185,28 +202,57 @@ __device__ __forceinline__ void warp_deposit(const Geo& g, Red& s, bool live, in
   for (int q = NP ? 0 : 1; q < 4; ++q) s.v[8 + q][pos] = live ? m[q] : 0.0;
   s.cell[pos] = live ? (unsigned long long)i | (unsigned long long)j << 21 | (unsigned long long)k << 42 : ~0ull;
   __syncwarp();
-  const int cv = lane & 7, qv = lane >> 3;
-  const bool adds = NP || qv != 0;
-  const double2* wr = reinterpret_cast<const double2*>(s.v[cv]);
-  const double2* mr = reinterpret_cast<const double2*>(s.v[8 + (adds ? qv : 1)]);
-  double* const arr = qv == 0 ? np : S + (qv - 1) * g.C;
-  auto flush = [&](int r, double acc) {
-    const unsigned long long c = s.cell[r];
-    if (c != ~0ull && adds) add_at_corner(g, arr, c, cv, acc);
-  };
-  double acc = 0.0;
+  const int cv = lane & 7;
+  if (NP) {
+    const int qv = lane >> 3;
+    const double2* wr = reinterpret_cast<const double2*>(s.v[cv]);
+    const double2* mr = reinterpret_cast<const double2*>(s.v[8 + qv]);
+    double* const arr = qv == 0 ? np : S + (qv - 1) * g.C;
+    auto flush = [&](int r, double acc) {
+      const unsigned long long c = s.cell[r];
+      if (c != ~0ull) add_at_corner(g, arr, c, cv, acc);
+    };
+    double acc = 0.0;
 #pragma unroll
-  for (int r = 0; r < 16; ++r) {
-    const double2 a = wr[r], b = mr[r];
-    acc = __fma_rn(a.x, b.x, acc);
-    if (ends >> (2 * r) & 1u) {
-      flush(2 * r, acc);
-      acc = 0.0;
+    for (int r = 0; r < 16; ++r) {
+      const double2 a = wr[r], b = mr[r];
+      acc = __fma_rn(a.x, b.x, acc);
+      if (ends >> (2 * r) & 1u) {
+        flush(2 * r, acc);
+        acc = 0.0;
+      }
+      acc = __fma_rn(a.y, b.y, acc);
+      if (ends >> (2 * r + 1) & 1u) {
+        flush(2 * r + 1, acc);
+        acc = 0.0;
+      }
     }
-    acc = __fma_rn(a.y, b.y, acc);
-    if (ends >> (2 * r + 1) & 1u) {
-      flush(2 * r + 1, acc);
-      acc = 0.0;
+  } else {
+    // 24 pairs of rows for 32 lanes: lane < 24 takes columns 0-23 of its
+    // pair, lane 24 + corner columns 24-31 of the corner's three pairs; 24
+    // operations each where a pair per lane takes 32
+    const bool tail = lane >= 24;
+    const double* wr = s.v[cv] + (tail ? 24 : 0);
+    double acc = 0.0;
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {  // eight columns at a time
+      const int q = tail ? b : lane >> 3, r0 = tail ? 0 : 8 * b;
+      const double* mr = s.v[9 + q] + (tail ? 24 : 0);
+      const unsigned e8 = ends >> (tail ? 24 : 8 * b) & 0xffu;
+#pragma unroll
+      for (int r = 0; r < 8; r += 2) {
+        const double2 x = *reinterpret_cast<const double2*>(wr + r0 + r), y = *reinterpret_cast<const double2*>(mr + r0 + r);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          acc = __fma_rn(h ? x.y : x.x, h ? y.y : y.x, acc);
+          // a group ends, or this lane's columns do
+          if ((e8 >> (r + h) & 1u) || (r + h == 7 && (b == 2 || tail))) {
+            const unsigned long long c = s.cell[(tail ? 24 : 8 * b) + r + h];
+            if (c != ~0ull) add_at_corner(g, S + q * g.C, c, cv, acc);
+            acc = 0.0;
+          }
+        }
+      }
     }
   }
   __syncwarp();

@@ -11,7 +11,7 @@
 //
 // What bounds them: GB300's FP64 pipe, two operations per SM and clock (a
 // warp instruction takes 16 clocks, 527e9 a second measured), so what counts is the number
-// of FP64 operations per ion, about 350 here against 930 for the operators
+// of FP64 operations per ion, about 340 here against 930 for the operators
 // one by one:
 //  * fused multiply-adds wherever the sum's rounding is free;
 //  * the difference aj - up is gathered (three components), not both fields;
@@ -25,8 +25,9 @@
 //    (__match_any_sync), so a cell's sum leaves as one reduction per value:
 //    L2 takes about 200e9 FP64 reductions a second, and 24 + 8 per ion were
 //    the deposits' bound.
-// 8.4M ions, 128x64x64 cells, ms per step for the particle half: 1.21 + 2.07 + 2.73 = 6.0 (pass
-// 1, 2, 3) against 17.3 for the operators one by one.
+// 8.4M ions, 128x64x64 cells, ms per step for the particle half: 1.17 + 1.87 +
+// 2.59 = 5.6 (pass 1, 2, 3; the FP64 pipe 88 to 92% busy) against 17.3 for the
+// operators one by one.
 #include "k64.cuh"
 #include "k64_dev.cuh"
 
@@ -122,24 +123,27 @@ __global__ void __launch_bounds__(TPB, 4) k_pass(PassArgs a) {
         if (PASS == 2) a.b3[l + q * NM] = B[q];
         else B[q] = a.b3[l + q * NM];
       }
-      const double mr = p.mrat[l], dt = a.dt, h = 0.5 * dt;
+      const double mr = p.mrat[l], dt = a.dt;
       double v[3], E[3];
 #pragma unroll
       for (int q = 0; q < 3; ++q) v[q] = p.vp[l + q * NM];
-      // Ep = ((aj - up) x B) mrat (gutsp.f:260-270)
-      E[0] = __fma_rn(A[1], B[2], -(A[2] * B[1])) * mr;
-      E[1] = __fma_rn(A[2], B[0], -(A[0] * B[2])) * mr;
-      E[2] = __fma_rn(A[0], B[1], -(A[1] * B[0])) * mr;
+      // (aj - up) x B; Ep is mrat times it (gutsp.f:260-270)
+      E[0] = __fma_rn(A[1], B[2], -(A[2] * B[1]));
+      E[1] = __fma_rn(A[2], B[0], -(A[0] * B[2]));
+      E[2] = __fma_rn(A[0], B[1], -(A[1] * B[0]));
+      double h = a.half_dt;
+      if (!is_one(mr)) {
+        h *= mr;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) B[q] *= mr;
+      }
       // v- and the rotation of get_vplus_vminus (gutsp.f:302-397)
       double vm[3], vn[3];
 #pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        vm[q] = __fma_rn(h, E[q], v[q]);
-        B[q] = B[q] * mr;
-      }
-      const double t = 0.25 * dt * dt * __fma_rn(B[0], B[0], __fma_rn(B[1], B[1], B[2] * B[2]));
-      const double ad = 1.0 / (1.0 + t), om = 1.0 - t;
-      const double kd = 0.5 * dt * dt * __fma_rn(vm[0], B[0], __fma_rn(vm[1], B[1], vm[2] * B[2]));
+      for (int q = 0; q < 3; ++q) vm[q] = __fma_rn(h, E[q], v[q]);
+      const double t = a.quarter_dt2 * __fma_rn(B[0], B[0], __fma_rn(B[1], B[1], B[2] * B[2]));
+      const double ad = fast_reciprocal(1.0 + t), om = 1.0 - t;
+      const double kd = a.half_dt2 * __fma_rn(vm[0], B[0], __fma_rn(vm[1], B[1], vm[2] * B[2]));
 #pragma unroll
       for (int q = 0; q < 3; ++q) {
         const int q1 = (q + 1) % 3, q2 = (q + 2) % 3;
@@ -195,10 +199,13 @@ __global__ void __launch_bounds__(TPB, 4) k_pass(PassArgs a) {
 
 }  // namespace
 
-cudaError_t particle_pass(int pass, const PassArgs& a, cudaStream_t st) {
+cudaError_t particle_pass(int pass, PassArgs a, cudaStream_t st) {
   if (a.N <= 0) return cudaSuccess;
   // four blocks of 128 an SM hide the latencies; more blocks than that at
   // once only repeat the block's set-up
+  a.half_dt = 0.5 * a.dt;
+  a.quarter_dt2 = 0.25 * a.dt * a.dt;
+  a.half_dt2 = 0.5 * a.dt * a.dt;
   const long long need = (a.N + TPB - 1) / TPB, most = 152LL * 4 * 8;
   const unsigned nb = (unsigned)(need < most ? need : most);
   if (pass == 1) k_pass<1><<<nb, TPB, 0, st>>>(a);

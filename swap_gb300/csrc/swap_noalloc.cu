@@ -86,7 +86,7 @@ using swapk::Geo;
 // into S = sum v*w/volb at folded nodes, a warp's ions summed by cell first:
 // bound by the FP64 pipe (about 75 operations an ion) instead of by the L2
 // reductions of 24 values an ion.  3.9M ions, 96x80x64 cells, the whole call:
-// 0.93 -> 0.64 ms.
+// 0.93 -> 0.55 ms.
 __global__ void __launch_bounds__(128, 6) k_na_deposit(Geo g, const double* __restrict__ xp,
                                                        const double* __restrict__ vp,
                                                        const double* __restrict__ beta_p, long long N, long long NM,
