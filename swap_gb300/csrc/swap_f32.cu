@@ -79,29 +79,28 @@ struct F32State {
 
   // the next step's new ions are staged on a second stream while this step's
   // fields advance (the staging draws in FP64, the field kernels stream HBM)
+  // The step's sort runs on the second stream too, beside the field
+  // subcycles (it reads only pass 3's outputs and the staging): ev_sort its
+  // end, h_look->n the new ion count it copies.  All made on first use and
+  // handed on when swap_f32_begin replaces the state.
   cudaStream_t side = nullptr;
-  cudaEvent_t ev_main = nullptr, ev_side = nullptr;
-  // the step's sort runs on the second stream too, beside the field
-  // subcycles (it reads only pass 3's outputs and the staging): its end, and
-  // the new ion count it copies to pinned host memory
-  cudaEvent_t ev_sort = nullptr;
-  int64_t* h_n = nullptr;
-  bool sort_pending = false;
-  // the smallest Courant time and the error word of the step, in pinned
-  // memory once ev_look has passed
+  cudaEvent_t ev_main = nullptr, ev_side = nullptr, ev_sort = nullptr;
+  // what the host looks at, page-locked: the smallest Courant time and the
+  // error word of the step once ev_look has passed, the count after ev_sort
   struct Look {
     float min;
     int err;
+    int64_t n;
   };
   Look* h_look = nullptr;
   cudaEvent_t ev_look = nullptr;
+  bool sort_pending = false;
   unsigned* loop_bar = nullptr;  // the field loop's barrier counters
   ~F32State() {
     if (side) cudaStreamSynchronize(side);
     if (ev_main) cudaEventDestroy(ev_main);
     if (ev_side) cudaEventDestroy(ev_side);
     if (ev_sort) cudaEventDestroy(ev_sort);
-    if (h_n) cudaFreeHost(h_n);
     if (ev_look) cudaEventDestroy(ev_look);
     if (h_look) cudaFreeHost(h_look);
     if (side) cudaStreamDestroy(side);
@@ -198,6 +197,7 @@ struct PreStaged {
   long long n_host = 0, n_max = 0;
   const int64_t* n_dev = nullptr;
 };
+static int side_stream(swap_ctx* c, F32State* s);
 static int sort_step(swap_ctx* c, F32State* s, long long src_step, bool prepared = false,
                      const PreStaged* pre = nullptr, bool on_side = false);
 
@@ -226,6 +226,13 @@ extern "C" int swap_f32_begin(swap_ctx* c) {
     for (std::size_t q = old->pool_next; q < old->pool.size(); ++q) s->pool.push_back(old->pool[q]);
     old->owned.clear();
     old->pool.clear();
+    if (old->side) CU(cudaStreamSynchronize(old->side));
+    std::swap(s->side, old->side);
+    std::swap(s->ev_main, old->ev_main);
+    std::swap(s->ev_side, old->ev_side);
+    std::swap(s->ev_sort, old->ev_sort);
+    std::swap(s->ev_look, old->ev_look);
+    std::swap(s->h_look, old->h_look);
     swap_f32_free(c);
   }
   c->f32_state = s;
@@ -398,8 +405,7 @@ extern "C" int swap_f32_begin(swap_ctx* c) {
   s->dtn = s->alloc<float>(C);
   s->acc = s->alloc<double>(4);
   s->loop_bar = s->alloc<unsigned>(2);
-  CU(cudaEventCreateWithFlags(&s->ev_look, cudaEventDisableTiming));
-  CU(cudaMallocHost(&s->h_look, sizeof(F32State::Look)));
+  TRY(side_stream(c, s));
   if (!s->start || !s->start_new || !s->count || !s->sums || !s->dirrank || !s->dep || !s->pre || !s->partial || !s->kit ||
       !s->np || !s->S || !s->up || !s->aj || !s->ct || !s->E || !s->nu || !s->db1 || !s->db1p2 || !s->dbtp1 ||
       !s->b0 || !s->b1.l || !s->b12.l || !s->b1p2.l || !s->b0c || !s->d_min || !s->acc || !s->dtn || !s->loop_bar || !s->far.idx ||
@@ -486,7 +492,7 @@ static int subcycles(swap_ctx* c, F32State* s, float* e_acc = nullptr) {
   // replayed on the host from the node values.
   // (formed with up after pass 3, with a snapshot of the error word beside
   // them: the sort on the second stream may still set the word itself)
-  CU(cudaMemcpyAsync(s->h_look, s->d_min, sizeof(F32State::Look), cudaMemcpyDeviceToHost, c->st));
+  CU(cudaMemcpyAsync(s->h_look, s->d_min, sizeof(float) + sizeof(int), cudaMemcpyDeviceToHost, c->st));
   CU(cudaEventRecord(s->ev_look, c->st));
   // a small grid's subcycles go out before the host has looked: the kernel
   // itself leaves the state alone in the two cases below
@@ -593,7 +599,7 @@ static int sort_join(swap_ctx* c, F32State* s) {
   CU(cudaStreamWaitEvent(c->st, s->ev_sort, 0));
   if (s->src_on) {
     CU(cudaEventSynchronize(s->ev_sort));
-    const int64_t n = *s->h_n;
+    const int64_t n = s->h_look->n;
     if (n > c->dims.ni_max) return c->fail(SWAP_ECAPACITY, "Ni_max exceeded by new ions");
     s->N = n;
   }
@@ -632,7 +638,7 @@ static int sort_body(swap_ctx* c, F32State* s, long long src_step, bool prepared
   std::swap(s->start, s->start_new);
   s->cur = 1 - s->cur;
   if (on_side) {  // the count, for sort_join
-    if (s->src_on) CU(cudaMemcpyAsync(s->h_n, s->start + g.nkeys, sizeof(int64_t), cudaMemcpyDeviceToHost, c->st));
+    if (s->src_on) CU(cudaMemcpyAsync(&s->h_look->n, s->start + g.nkeys, sizeof(int64_t), cudaMemcpyDeviceToHost, c->st));
     return SWAP_OK;
   }
   if (s->src_on) {  // the count changed: the host needs it for the next launches
@@ -760,14 +766,15 @@ static int field_step(swap_ctx* c, F32State* s) {
   return SWAP_OK;
 }
 
-// The second stream, its events and the pinned count, made once.
+// The second stream, the events and the page-locked look, made once.
 static int side_stream(swap_ctx* c, F32State* s) {
   if (s->side) return SWAP_OK;
   CU(cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking));
   CU(cudaEventCreateWithFlags(&s->ev_main, cudaEventDisableTiming));
   CU(cudaEventCreateWithFlags(&s->ev_side, cudaEventDisableTiming));
   CU(cudaEventCreateWithFlags(&s->ev_sort, cudaEventDisableTiming));
-  CU(cudaMallocHost(&s->h_n, sizeof(int64_t)));
+  CU(cudaEventCreateWithFlags(&s->ev_look, cudaEventDisableTiming));
+  CU(cudaMallocHost(&s->h_look, sizeof(F32State::Look)));
   return SWAP_OK;
 }
 
