@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -404,8 +405,8 @@ __global__ void __launch_bounds__(256) k_conv3r(ConvArgs a, int ychunk) {
 // with 128 % nx == 0): a tile is 128 / nx rows, so a tap's shift along x is a
 // rotation inside the tile's own rows.  Per (dy, dz) every thread loads one
 // voxel's channels and stores them three times, rotated by dx: 9 loads per
-// voxel instead of 27, all of a plane's (three dy) in registers one stage
-// ahead, and 9 taps per barrier.  (k_conv3, below, loads each tap as it
+// voxel instead of 27, a plane's (three dy) in registers two stages ahead,
+// and 9 taps per barrier.  (k_conv3, below, loads each tap as it
 // needs it: one load in flight per thread and a barrier per tap.  A 16 -> 16
 // layer of 64^3 voxels: 108 us there, 30 us here.)
 // Three stages (dz) per tile in two operand buffers; two accumulators let the
@@ -451,8 +452,11 @@ __global__ void __launch_bounds__(128) k_conv3t(ConvArgs a) {
   const uint64_t adesc0 = tc05::desc_noswizzle(tc05::smem_u32(sA), 16 * 128, 128);
   const uint64_t bdesc0 = tc05::desc_noswizzle(tc05::smem_u32(sW), (COUT / 8) * 128, 128);
   const int ntiles = (int)(a.V / 128);
-  uint4 reg[3][KG];
-  auto load = [&](int tile, int dz) {  // the three dy of plane z + dz - 1
+  uint4 reg[2][3][KG];  // the loads of the two stages ahead
+  // stage s of this block is (tile, dz) = (blockIdx.x + s / 3 * gridDim.x, s % 3)
+  auto load = [&](uint4 (&to)[3][KG], int st) {  // the three dy of plane z + dz - 1
+    const int tile = (int)blockIdx.x + st / 3 * (int)gridDim.x, dz = st % 3;
+    if (tile >= ntiles) return;
     const int r = tile * rows + row, y = r % ny, z = r / ny;
     int zz = z + dz - 1;
     zz = zz < 0 ? zz + nz : (zz >= nz ? zz - nz : zz);
@@ -462,7 +466,7 @@ __global__ void __launch_bounds__(128) k_conv3t(ConvArgs a) {
       yy = yy < 0 ? yy + ny : (yy >= ny ? yy - ny : yy);
       const uint4* src = reinterpret_cast<const uint4*>(a.X + ((long long)(zz * ny + yy) * nx + x) * CIN);
 #pragma unroll
-      for (int q = 0; q < KG; ++q) reg[d][q] = src[q];
+      for (int q = 0; q < KG; ++q) to[d][q] = src[q];
     }
   };
   auto epilogue = [&](int tile, int b) {
@@ -476,54 +480,54 @@ __global__ void __launch_bounds__(128) k_conv3t(ConvArgs a) {
     conv_store<COUT>(a, vo, 0, acc);
   };
   bool ok = true;
-  int stage = 0, acc = 0, prev = -1;
-  if ((int)blockIdx.x < ntiles) load(blockIdx.x, 0);
-  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, acc ^= 1) {
-    for (int dz = 0; dz < 3; ++dz, ++stage) {
-      const int b = stage & 1;
-      // the products of the stage before last are done: its buffer is free
-      if (stage >= 2) ok &= tc05::mbar_wait(&mbar[b], (uint32_t)(stage / 2 - 1) & 1u, WAIT_LIMIT);
-      uint8_t* buf = sA + b * SBYTES;
+  const int mine = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0, nstages = 3 * mine;
+  auto run = [&](uint4 (&from)[3][KG], int st) {
+    const int b = st & 1, dz = st % 3, acc = (st / 3) & 1;
+    // the products of the stage before last are done: its buffer is free
+    if (st >= 2) ok &= tc05::mbar_wait(&mbar[b], (uint32_t)(st / 2 - 1) & 1u, WAIT_LIMIT);
+    uint8_t* buf = sA + b * SBYTES;
 #pragma unroll
-      for (int d = 0; d < 3; ++d)
+    for (int d = 0; d < 3; ++d)
 #pragma unroll
-        for (int q = 0; q < 3; ++q)
+      for (int q = 0; q < 3; ++q)
 #pragma unroll
-          for (int kg = 0; kg < KG; ++kg)
-            *reinterpret_cast<uint4*>(buf + (3 * d + q) * ABYTES + tc05::core_offset(dst[q], 8 * kg, 128)) = reg[d][kg];
-      tc05::fence_async_smem();
-      tc05::fence_before_sync();
-      __syncthreads();
-      tc05::fence_after_sync();
-      if (tid == 0) {
-#pragma unroll
-        for (int t = 0; t < 9; ++t)
-#pragma unroll
-          for (int kk = 0; kk < KG / 2; ++kk) {
-            const uint32_t aoff = (uint32_t)(b * SBYTES + t * ABYTES + kk * 2 * (16 * 128));
-            const uint32_t boff = (uint32_t)((9 * dz + t) * (COUT * CIN * 2) + kk * 2 * ((COUT / 8) * 128));
-            tc05::mma_bf16(tmem + acc * 32, adesc0 + (aoff >> 4), bdesc0 + (boff >> 4), idesc,
-                           dz > 0 || t > 0 || kk > 0);
-          }
-        tc05::mma_commit(&mbar[b]);
-      }
-      // the next stage's loads
-      if (dz < 2) load(tile, dz + 1);
-      else if (tile + (int)gridDim.x < ntiles) load(tile + gridDim.x, 0);
-      // the last tile's products were waited for above, in its last stage's
-      // buffer: two stages ago
-      if (dz == 1 && prev >= 0) {
-        tc05::fence_after_sync();
-        epilogue(prev, acc ^ 1);
-        tc05::fence_before_sync();
-      }
-    }
-    prev = tile;
-  }
-  if (prev >= 0) {  // the last tile: both of its latest stages
-    for (int s = stage - 2; s < stage; ++s) ok &= tc05::mbar_wait(&mbar[s & 1], (uint32_t)(s / 2) & 1u, WAIT_LIMIT);
+        for (int kg = 0; kg < KG; ++kg)
+          *reinterpret_cast<uint4*>(buf + (3 * d + q) * ABYTES + tc05::core_offset(dst[q], 8 * kg, 128)) = from[d][kg];
+    tc05::fence_async_smem();
+    tc05::fence_before_sync();
+    __syncthreads();
     tc05::fence_after_sync();
-    epilogue(prev, acc ^ 1);
+    if (tid == 0) {
+#pragma unroll
+      for (int t = 0; t < 9; ++t)
+#pragma unroll
+        for (int kk = 0; kk < KG / 2; ++kk) {
+          const uint32_t aoff = (uint32_t)(b * SBYTES + t * ABYTES + kk * 2 * (16 * 128));
+          const uint32_t boff = (uint32_t)((9 * dz + t) * (COUT * CIN * 2) + kk * 2 * ((COUT / 8) * 128));
+          tc05::mma_bf16(tmem + acc * 32, adesc0 + (aoff >> 4), bdesc0 + (boff >> 4), idesc,
+                         dz > 0 || t > 0 || kk > 0);
+        }
+      tc05::mma_commit(&mbar[b]);
+    }
+    load(from, st + 2);
+    // the tile before: its last stage's products were waited for above
+    if (dz == 1 && st >= 3) {
+      tc05::fence_after_sync();
+      epilogue((int)blockIdx.x + (st / 3 - 1) * (int)gridDim.x, acc ^ 1);
+      tc05::fence_before_sync();
+    }
+  };
+  load(reg[0], 0);
+  load(reg[1], 1);
+  for (int st = 0; st < nstages; st += 2) {
+    run(reg[0], st);
+    if (st + 1 < nstages) run(reg[1], st + 1);
+  }
+  if (mine > 0) {  // the last tile: both of its latest stages
+    for (int st = nstages - 2; st < nstages; ++st)
+      ok &= tc05::mbar_wait(&mbar[st & 1], (uint32_t)(st / 2) & 1u, WAIT_LIMIT);
+    tc05::fence_after_sync();
+    epilogue((int)blockIdx.x + (mine - 1) * (int)gridDim.x, (mine - 1) & 1);
   }
   if (!ok) atomicCAS(a.err, 0, SWAP_EWAIT);
   tc05::fence_before_sync();
@@ -697,6 +701,20 @@ struct OutNorm {
   float mean[3], std[3];
 };
 
+// Adds the block's sum of s to *acc: one atomic per block of a small grid
+// (loss_blocks), where one per warp queued up at the one address (64^3 voxels:
+// 16 us a kernel).
+__device__ __forceinline__ void add_block_sum(float s, float* acc) {
+  __shared__ float sh[8];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) s += sh[w];
+    atomicAdd(acc, s);
+  }
+}
+
 // Loss 0.5*mean (out - (tgt - mean)/std)^2 over V*3 values, its gradient as
 // BF16 [V][16] (channels 3..15 zero); the sum of squares goes to *acc.
 __global__ void k_loss(long long V, const float* __restrict__ out, const float* __restrict__ tgt, OutNorm on,
@@ -716,8 +734,7 @@ __global__ void k_loss(long long V, const float* __restrict__ out, const float* 
     dst[0] = reinterpret_cast<const uint4*>(h)[0];
     dst[1] = reinterpret_cast<const uint4*>(h)[1];
   }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) atomicAdd(acc, s);
+  add_block_sum(s, acc);
 }
 
 // The B error a prediction makes is dt curl(E error) (B advances as
@@ -733,20 +750,20 @@ __global__ void k_err3(long long V, const float* __restrict__ out, const float* 
       e[v * NOUT + c] = (out ? fmaf(out[v * NOUT + c], on.std[c], on.mean[c]) : 0.0f) - tgt[v * NOUT + c];
 }
 
-__device__ __forceinline__ long long vox(int i, int j, int k, int nx, int ny, int nz) {
+__device__ __forceinline__ unsigned vox(int i, int j, int k, int nx, int ny, int nz) {
   i = i < 0 ? i + nx : (i >= nx ? i - nx : i);
   j = j < 0 ? j + ny : (j >= ny ? j - ny : j);
   k = k < 0 ? k + nz : (k >= nz ? k - nz : k);
-  return (long long)i + (long long)nx * ((long long)j + (long long)ny * k);
+  return (unsigned)(i + nx * (j + ny * k));
 }
 
 // kap = curl e (forward differences): kap_x = Dy e3 - Dz e2, kap_y = Dz e1 -
 // Dx e3, kap_z = Dx e2 - Dy e1; the sum of |kap|^2 into *acc.
 __global__ void k_curl3(int nx, int ny, int nz, const float* __restrict__ e, float* __restrict__ kap, float* acc) {
-  const long long V = (long long)nx * ny * nz;
+  const unsigned V = (unsigned)(nx * ny * nz);  // the work buffers hold far fewer than 2^31 voxels
   float s = 0.0f;
-  for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < V; v += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(v % nx), j = (int)((v / nx) % ny), k = (int)(v / ((long long)nx * ny));
+  for (unsigned v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
+    const int r = (int)(v / (unsigned)nx), i = (int)v - r * nx, k = r / ny, j = r - k * ny;
     const float* o = e + v * 3;
     const float* px = e + vox(i + 1, j, k, nx, ny, nz) * 3;
     const float* py = e + vox(i, j + 1, k, nx, ny, nz) * 3;
@@ -757,8 +774,7 @@ __global__ void k_curl3(int nx, int ny, int nz, const float* __restrict__ e, flo
     kap[v * 3] = kx; kap[v * 3 + 1] = ky; kap[v * 3 + 2] = kz;
     s += kx * kx + ky * ky + kz * kz;
   }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) atomicAdd(acc, s);
+  add_block_sum(s, acc);
 }
 
 // The plain loss of k_loss plus lam * std_c * (curl^T kap)_c in the output
@@ -766,10 +782,10 @@ __global__ void k_curl3(int nx, int ny, int nz, const float* __restrict__ e, flo
 __global__ void k_loss_curl(int nx, int ny, int nz, const float* __restrict__ out, const float* __restrict__ tgt,
                             OutNorm on, float gscale, float lam, const float* __restrict__ kap,
                             __nv_bfloat16* __restrict__ d16, float* acc) {
-  const long long V = (long long)nx * ny * nz;
+  const unsigned V = (unsigned)(nx * ny * nz);  // the work buffers hold far fewer than 2^31 voxels
   float s = 0.0f;
-  for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < V; v += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(v % nx), j = (int)((v / nx) % ny), k = (int)(v / ((long long)nx * ny));
+  for (unsigned v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
+    const int r = (int)(v / (unsigned)nx), i = (int)v - r * nx, k = r / ny, j = r - k * ny;
     const float* o = kap + v * 3;
     const float* mx = kap + vox(i - 1, j, k, nx, ny, nz) * 3;
     const float* my = kap + vox(i, j - 1, k, nx, ny, nz) * 3;
@@ -790,8 +806,7 @@ __global__ void k_loss_curl(int nx, int ny, int nz, const float* __restrict__ ou
     dst[0] = reinterpret_cast<const uint4*>(h)[0];
     dst[1] = reinterpret_cast<const uint4*>(h)[1];
   }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) atomicAdd(acc, s);
+  add_block_sum(s, acc);
 }
 
 // Weight gradient of a periodic conv layer on the CUDA cores:
@@ -976,7 +991,7 @@ __global__ void __launch_bounds__(128) k_conv3_dw_tc(int nx, int ny, int nz, lon
 // the bias gradient.  Rows past it are products with whatever lies there, and
 // are not read.  One block per SM (NST stages in flight) adds its sums with
 // FP32 atomics.
-// 16 -> 16 channels, 64^3 voxels, with the bias: 165 us transposing, 59 us.
+// 16 -> 16 channels, 64^3 voxels, with the bias: 165 us transposing, 45 us.
 template <int CIN, int COUT>
 struct DwLines {
   static constexpr int KG = CIN / 8, SEG = 64, PLANE = (SEG + 4) * 16, LINE = KG * PLANE;
@@ -987,7 +1002,7 @@ struct DwLines {
   static constexpr int SMEM = NST * (ABYTES + BBYTES) + TAIL;
   static constexpr int COLS = 3 * NB * COUT <= 128 ? 128 : (3 * NB * COUT <= 256 ? 256 : 512);
 };
-constexpr int DW_TPB = 9 * 32;  // a warp per line
+constexpr int DW_COPY = 9 * 32, DW_TPB = DW_COPY + 32;  // a warp per line, and one that issues the products
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(DW_TPB) k_conv3_dw_lines(int nx, int ny, int nz, const __nv_bfloat16* __restrict__ X,
                                                         const __nv_bfloat16* __restrict__ dZ, float* __restrict__ gW,
@@ -996,7 +1011,7 @@ __global__ void __launch_bounds__(DW_TPB) k_conv3_dw_lines(int nx, int ny, int n
   constexpr int KG = D::KG, SEG = D::SEG, NB = D::NB, NST = D::NST;
   extern __shared__ __align__(1024) uint8_t smem[];  // NST A stages, then NST B stages, then the tail
   uint8_t* const sB = smem + NST * D::ABYTES;
-  __shared__ uint64_t mbar[NST];
+  __shared__ uint64_t full[NST], empty[NST];  // a stage's copies are in; its products are done
   __shared__ uint32_t tslot;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   for (int i = tid; i < NST * D::LINE / 4; i += DW_TPB)  // the lines of ones
@@ -1004,7 +1019,10 @@ __global__ void __launch_bounds__(DW_TPB) k_conv3_dw_lines(int nx, int ny, int n
         0x3f803f80u;
   if (warp == 0) tc05::tmem_alloc(&tslot, D::COLS);
   if (tid == 0) {
-    for (int q = 0; q < NST; ++q) tc05::mbar_init(&mbar[q], 1);
+    for (int q = 0; q < NST; ++q) {
+      tc05::mbar_init(&full[q], DW_COPY);
+      tc05::mbar_init(&empty[q], 1);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   tc05::fence_before_sync();
@@ -1036,23 +1054,34 @@ __global__ void __launch_bounds__(DW_TPB) k_conv3_dw_lines(int nx, int ny, int n
       tc05::cp_async16(dst + p * D::PLANE + q * 16, row + x * CIN + 8 * p);
     }
     const __nv_bfloat16* drow = dZ + ((long long)(z * ny + y) * nx + x0) * COUT;
-    for (int it = tid; it < len * (COUT / 8); it += DW_TPB) {
+    for (int it = tid; it < len * (COUT / 8); it += DW_COPY) {
       const int p = it % (COUT / 8), q = it / (COUT / 8);
       tc05::cp_async16(B + p * D::BPLANE + q * 16, drow + q * COUT + 8 * p);
     }
   };
   bool ok = true;
-  for (int i = 0; i < NST - 1; ++i) {
-    if (i < n) load(i);
-    tc05::cp_async_commit();
-  }
-  for (int i = 0; i < n; ++i) {
-    tc05::cp_async_wait<NST - 2>();
-    tc05::fence_async_smem();
-    tc05::fence_before_sync();
-    __syncthreads();
-    tc05::fence_after_sync();
-    if (tid == 0) {
+  if (warp < 9) {
+    constexpr int LAG = NST - 2;  // units whose copies are under way while the next are started
+    auto publish = [&](int i) {   // this thread's copies of unit i have landed
+      tc05::fence_async_smem();
+      tc05::mbar_arrive(&full[i % NST]);
+    };
+    for (int i = 0; i < n; ++i) {
+      if (i >= NST) ok &= tc05::mbar_wait(&empty[i % NST], (uint32_t)(i / NST - 1) & 1u, WAIT_LIMIT);
+      tc05::fence_after_sync();
+      load(i);
+      tc05::cp_async_commit();
+      if (i >= LAG) {
+        tc05::cp_async_wait<LAG>();
+        publish(i - LAG);
+      }
+    }
+    tc05::cp_async_wait_all();
+    for (int i = n > LAG ? n - LAG : 0; i < n; ++i) publish(i);
+  } else if (lane == 0) {
+    for (int i = 0; i < n; ++i) {
+      ok &= tc05::mbar_wait(&full[i % NST], (uint32_t)(i / NST) & 1u, WAIT_LIMIT);
+      tc05::fence_after_sync();
       const int len = seg_len((int)((u0 + i) % segs));
       // M- and N-major: 8 voxels (K) 128 bytes apart, 8 channels a plane apart
       const uint64_t ad = tc05::desc_noswizzle(tc05::smem_u32(smem + (i % NST) * D::ABYTES), 128, D::PLANE);
@@ -1065,16 +1094,12 @@ __global__ void __launch_bounds__(DW_TPB) k_conv3_dw_lines(int nx, int ny, int n
             tc05::mma_bf16(tmem + (dx * NB + mb) * COUT,
                            ad + ((mb * (128 / CIN) * D::LINE + (16 * kk + dx) * 16) >> 4), bd + ((16 * kk * 16) >> 4),
                            idesc, i > 0 || kk > 0);
-      tc05::mma_commit(&mbar[i % NST]);
+      tc05::mma_commit(&empty[i % NST]);
     }
-    // stage i - 1's products are done: its buffer takes unit i - 1 + NST
-    if (i > 0) ok &= tc05::mbar_wait(&mbar[(i - 1) % NST], (uint32_t)((i - 1) / NST) & 1u, WAIT_LIMIT);
-    tc05::fence_after_sync();
-    if (i > 0 ? i - 1 + NST < n : NST - 1 < n) load(i - 1 + NST);
-    tc05::cp_async_commit();
+    if (n > 0) ok &= tc05::mbar_wait(&empty[(n - 1) % NST], (uint32_t)((n - 1) / NST) & 1u, WAIT_LIMIT);
   }
-  if (n > 0) ok &= tc05::mbar_wait(&mbar[(n - 1) % NST], (uint32_t)((n - 1) / NST) & 1u, WAIT_LIMIT);
-  tc05::cp_async_wait_all();
+  tc05::fence_before_sync();
+  ok = __syncthreads_and(ok);
   tc05::fence_after_sync();
   if (n > 0 && warp < 4) {  // the accumulator's 128 rows
     const int r = warp * 32 + lane, ci = r % CIN;
@@ -1155,6 +1180,8 @@ inline unsigned nblk(long long n, int tpb = 256) {
   const long long b = (n + tpb - 1) / tpb;
   return (unsigned)(b < 1 ? 1 : (b > 65535LL * 8 ? 65535LL * 8 : b));
 }
+
+inline unsigned loss_blocks(long long V) { return (unsigned)std::min<long long>((V + 255) / 256, 152 * 4); }
 
 // Weight and bias gradients of a conv layer: the tensor-core form, or with
 // cuda_cores the CUDA-core form (kept to check the other against).
@@ -1239,6 +1266,10 @@ struct swap_surrogate {
   __nv_bfloat16* d16 = nullptr;            // [V][16]
   float* dy = nullptr;                     // [V][6], the curl loss's e and curl e
   __nv_bfloat16 *dzA = nullptr, *dzB = nullptr;  // [V][32]
+  // the error word, the loss sums and every gradient in one block, laid out as
+  // the host takes it: [0] err, [4..5] acc, then gw[0], gb[0], gw[1], ...
+  float* block = nullptr;
+  std::size_t ngrad = 0;
   float* acc = nullptr;
   int* err = nullptr;
   std::vector<void*> owned;
@@ -1376,10 +1407,7 @@ int backward(swap_surrogate* net, cudaStream_t st) {
 }
 
 int zero_grads(swap_surrogate* net, cudaStream_t st) {
-  for (int l = 0; l < NL; ++l) {
-    SCU(cudaMemsetAsync(net->gw[l], 0, 27 * LCIN[l] * LCOUT[l] * sizeof(float), st));
-    SCU(cudaMemsetAsync(net->gb[l], 0, LCOUT[l] * sizeof(float), st));
-  }
+  SCU(cudaMemsetAsync(net->block + 8, 0, net->ngrad * sizeof(float), st));
   return SWAP_OK;
 }
 
@@ -1406,24 +1434,34 @@ int adam_step(swap_surrogate* net, float lr, cudaStream_t st) {
 }
 
 // Loss of the current x0 against target tgt ([V][3], unnormalised); the
-// output gradient goes to d16.  Returns the sum of squares in *sq.
-int loss_grad(swap_surrogate* net, const float* tgt, float gnorm, double* sq, cudaStream_t st) {
+// output gradient goes to d16, the sums to net->acc (see loss_value).
+int loss_sums(swap_surrogate* net, const float* tgt, float gnorm, cudaStream_t st) {
   SCU(cudaMemsetAsync(net->acc, 0, 2 * sizeof(float), st));
-  const bool curl = net->curl_w > 0.0f && net->kref2 > 0.0;
-  if (curl) {
+  if (net->curl_w > 0.0f && net->kref2 > 0.0) {
     float *e = net->dy, *kap = net->dy + 3 * net->V;
     k_err3<<<nblk(net->V), 256, 0, st>>>(net->V, net->out, tgt, net->on, e);
-    k_curl3<<<nblk(net->V), 256, 0, st>>>(net->nx, net->ny, net->nz, e, kap, net->acc + 1);
-    k_loss_curl<<<nblk(net->V), 256, 0, st>>>(net->nx, net->ny, net->nz, net->out, tgt, net->on, gnorm,
-                                                (float)(3.0 * net->curl_w / net->kref2), kap, net->d16, net->acc);
+    k_curl3<<<loss_blocks(net->V), 256, 0, st>>>(net->nx, net->ny, net->nz, e, kap, net->acc + 1);
+    k_loss_curl<<<loss_blocks(net->V), 256, 0, st>>>(net->nx, net->ny, net->nz, net->out, tgt, net->on, gnorm,
+                                                     (float)(3.0 * net->curl_w / net->kref2), kap, net->d16, net->acc);
   } else {
-    k_loss<<<nblk(net->V), 256, 0, st>>>(net->V, net->out, tgt, net->on, gnorm, net->d16, net->acc);
+    k_loss<<<loss_blocks(net->V), 256, 0, st>>>(net->V, net->out, tgt, net->on, gnorm, net->d16, net->acc);
   }
+  SCU(cudaGetLastError());
+  return SWAP_OK;
+}
+
+// The sum of squares in units of the plain term's sum over V*3 values.
+double loss_value(const swap_surrogate* net, const float* acc) {
+  return acc[0] + (net->curl_w > 0.0f && net->kref2 > 0.0 ? 3.0 * net->curl_w * (double)acc[1] / net->kref2 : 0.0);
+}
+
+int loss_grad(swap_surrogate* net, const float* tgt, float gnorm, double* sq, cudaStream_t st) {
+  const int r = loss_sums(net, tgt, gnorm, st);
+  if (r) return r;
   float h[2] = {0, 0};
   SCU(cudaMemcpyAsync(h, net->acc, sizeof(h), cudaMemcpyDeviceToHost, st));
   SCU(cudaStreamSynchronize(st));
-  // in units of the plain term's sum over V*3 values
-  *sq = h[0] + (curl ? 3.0 * net->curl_w * (double)h[1] / net->kref2 : 0.0);
+  *sq = loss_value(net, h);
   return SWAP_OK;
 }
 
@@ -1491,6 +1529,20 @@ extern "C" int swap_surrogate_create(swap_surrogate** out, uint64_t seed, int32_
   auto* net = new swap_surrogate();
   net->seed = seed;
   net->max_samples = max_samples;
+  for (int l = 0; l < NL; ++l) net->ngrad += (27 * (std::size_t)LCIN[l] + 1) * LCOUT[l];
+  net->block = net->alloc<float>(8 + net->ngrad);
+  if (!net->block) {
+    delete net;
+    return SWAP_ECUDA;
+  }
+  net->err = reinterpret_cast<int*>(net->block);
+  net->acc = net->block + 4;
+  for (int l = 0, o = 8; l < NL; ++l) {
+    net->gw[l] = net->block + o;
+    o += 27 * LCIN[l] * LCOUT[l];
+    net->gb[l] = net->block + o;
+    o += LCOUT[l];
+  }
   std::mt19937_64 rng(seed);
   for (int l = 0; l < NL; ++l) {
     const int ci = LCIN[l], co = LCOUT[l];
@@ -1499,8 +1551,6 @@ extern "C" int swap_surrogate_create(swap_surrogate** out, uint64_t seed, int32_
     net->b[l] = net->alloc<float>(co);
     net->wh[l] = net->alloc<__nv_bfloat16>(nw);
     net->wt[l] = net->alloc<__nv_bfloat16>(nw);
-    net->gw[l] = net->alloc<float>(nw);
-    net->gb[l] = net->alloc<float>(co);
     net->mw[l] = net->alloc<float>(nw);
     net->vw[l] = net->alloc<float>(nw);
     net->mb[l] = net->alloc<float>(co);
@@ -1532,9 +1582,7 @@ extern "C" int swap_surrogate_create(swap_surrogate** out, uint64_t seed, int32_
   }
   net->d_mean = net->alloc<float>(NIN);
   net->d_istd = net->alloc<float>(NIN);
-  net->acc = net->alloc<float>(4);
-  net->err = net->alloc<int>(1);
-  if (!net->d_mean || !net->d_istd || !net->acc || !net->err) {
+  if (!net->d_mean || !net->d_istd) {
     delete net;
     return SWAP_ECUDA;
   }
@@ -1628,20 +1676,17 @@ extern "C" int swap_surrogate_grads(swap_surrogate* net, int32_t nx, int32_t ny,
   cudaStream_t st = nullptr;
   k_norm_inputs<<<nblk(net->V), 256, 0, st>>>(net->V, vin, net->d_mean, net->d_istd, net->x0);
   if ((r = forward(net, true, st))) return r;
-  double sq = 0;
-  if ((r = loss_grad(net, tgt, 1.0f / (3.0f * (float)net->V), &sq, st))) return r;
+  if ((r = loss_sums(net, tgt, 1.0f / (3.0f * (float)net->V), st))) return r;
   if ((r = zero_grads(net, st)) || (r = backward(net, st))) return r;
+  // the error word, the loss and the gradients in one copy
+  std::vector<float> h(8 + net->ngrad);
+  SCU(cudaMemcpyAsync(h.data(), net->block, h.size() * sizeof(float), cudaMemcpyDeviceToHost, st));
   SCU(cudaDeviceSynchronize());
-  if ((r = check_err(net))) return r;
-  *loss = 0.5 * sq / (3.0 * (double)net->V);
-  float* o = grads;
-  for (int l = 0; l < NL; ++l) {
-    const std::size_t nw = 27 * (std::size_t)LCIN[l] * LCOUT[l];
-    SCU(cudaMemcpy(o, net->gw[l], nw * sizeof(float), cudaMemcpyDeviceToHost));
-    o += nw;
-    SCU(cudaMemcpy(o, net->gb[l], LCOUT[l] * sizeof(float), cudaMemcpyDeviceToHost));
-    o += LCOUT[l];
-  }
+  int e = 0;
+  std::memcpy(&e, h.data(), sizeof(e));
+  if (e) return check_err(net);
+  *loss = 0.5 * loss_value(net, h.data() + 4) / (3.0 * (double)net->V);
+  std::copy(h.begin() + 8, h.end(), grads);
   return SWAP_OK;
 }
 
@@ -1689,7 +1734,7 @@ static int fit_norm(swap_surrogate* net) {
     float* e = net->dy;
     SCU(cudaMemsetAsync(net->acc, 0, 2 * sizeof(float), nullptr));
     k_err3<<<nblk(net->V), 256>>>(net->V, nullptr, net->ds_tgt[k], net->on, e);
-    k_curl3<<<nblk(net->V), 256>>>(net->nx, net->ny, net->nz, e, e + 3 * net->V, net->acc + 1);
+    k_curl3<<<loss_blocks(net->V), 256>>>(net->nx, net->ny, net->nz, e, e + 3 * net->V, net->acc + 1);
     float h = 0;
     SCU(cudaMemcpy(&h, net->acc + 1, sizeof(float), cudaMemcpyDeviceToHost));
     k2 += h;
@@ -1709,7 +1754,7 @@ static int pair_k2(swap_surrogate* net) {
     float* e = net->dy;
     SCU(cudaMemsetAsync(net->acc, 0, 2 * sizeof(float), nullptr));
     k_err3<<<nblk(net->V), 256>>>(net->V, nullptr, t, net->on, e);
-    k_curl3<<<nblk(net->V), 256>>>(net->nx, net->ny, net->nz, e, e + 3 * net->V, net->acc + 1);
+    k_curl3<<<loss_blocks(net->V), 256>>>(net->nx, net->ny, net->nz, e, e + 3 * net->V, net->acc + 1);
     float h = 0;
     SCU(cudaMemcpy(&h, net->acc + 1, sizeof(float), cudaMemcpyDeviceToHost));
     net->ds_k2.push_back((double)h / (double)net->V);
