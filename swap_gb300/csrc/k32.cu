@@ -260,6 +260,38 @@ __device__ __forceinline__ void warp_deposit(float (*red)[36], bool live, int t0
   __syncwarp();
 }
 
+// extrapol_up's velocity (gutsp.f:144), rounded the same wherever it is formed.
+__device__ __forceinline__ float extrapolated(float v, float v1) {
+  return __fmaf_rn(1.5f, v, -__fmul_rn(0.5f, v1));
+}
+
+// A crowded brick: carry the low words into the high words (exact: 2^16 low
+// units are one high unit), so that they never wrap.  The whole block calls.
+template <int TNOD>
+__device__ __forceinline__ void carry_tile(unsigned* s_dep) {
+  __syncthreads();
+  for (int t = threadIdx.x; t < 4 * TNOD; t += blockDim.x) {
+    const unsigned lo = s_dep[t];
+    s_dep[t] = lo & 0xFFFFu;
+    s_dep[4 * TNOD + t] += lo >> 16;
+  }
+  __syncthreads();
+}
+
+// The brick's partial tile: FP32, or the node's fixed-point value (high words *
+// 2^16 + low words).
+template <bool EXACT, int TNOD>
+__device__ __forceinline__ void write_tile(const unsigned* s_dep, void* partial, long long b) {
+  if (EXACT) {
+    long long* out = static_cast<long long*>(partial) + b * (4 * TNOD);
+    for (int t = threadIdx.x; t < 4 * TNOD; t += blockDim.x)
+      out[t] = (long long)(int)s_dep[4 * TNOD + t] * 65536LL + (long long)s_dep[t];
+  } else {
+    float* out = static_cast<float*>(partial) + b * (4 * TNOD);
+    for (int t = threadIdx.x; t < 4 * TNOD; t += blockDim.x) out[t] = __uint_as_float(s_dep[t]);
+  }
+}
+
 // One CTA per brick; its particles are the contiguous range of the brick's
 // keys and lie in their key's cell (every move happens in pass 3, after
 // which the sort restores that).
@@ -396,9 +428,9 @@ __global__ void __launch_bounds__(TPB_PASS, PASS == 3 ? 7 : 8) k_pass(G32 g, Par
       if (PASS == 1) {
         if (fresh) p.cell[l] = c & ~CELL_FRESH;
         // extrapol_up (gutsp.f:144)
-        dvx = 1.5f * vx - 0.5f * s_f[u][PASS == 1 ? 6 : 0][threadIdx.x];
-        dvy = 1.5f * vy - 0.5f * s_f[u][PASS == 1 ? 7 : 0][threadIdx.x];
-        dvz = 1.5f * vz - 0.5f * s_f[u][PASS == 1 ? 8 : 0][threadIdx.x];
+        dvx = extrapolated(vx, s_f[u][PASS == 1 ? 6 : 0][threadIdx.x]);
+        dvy = extrapolated(vy, s_f[u][PASS == 1 ? 7 : 0][threadIdx.x]);
+        dvz = extrapolated(vz, s_f[u][PASS == 1 ? 8 : 0][threadIdx.x]);
       } else {
         // trilinear gather of (ajc-upc, btc) at the 8 corners (gutsp.f:217-251)
         const float wxl = 1.0f - ox, wxu = ox, wyl = 1.0f - oy, wyu = oy, wzl = 1.0f - oz, wzu = oz;
@@ -563,17 +595,7 @@ __global__ void __launch_bounds__(TPB_PASS, PASS == 3 ? 7 : 8) k_pass(G32 g, Par
         __syncthreads();
       }
     }
-    if (EXACT && (kc + 1) % CARRY_CHUNKS == 0 && kc + 1 < nchunk) {
-      // a crowded brick: carry the low words into the high words (exact:
-      // 2^16 low units are one high unit), so that they never wrap
-      __syncthreads();
-      for (int t = threadIdx.x; t < 4 * TNOD; t += blockDim.x) {
-        const unsigned lo = s_dep[t];
-        s_dep[t] = lo & 0xFFFFu;
-        s_dep[4 * TNOD + t] += lo >> 16;
-      }
-      __syncthreads();
-    }
+    if (EXACT && (kc + 1) % CARRY_CHUNKS == 0 && kc + 1 < nchunk) carry_tile<TNOD>(s_dep);
   }
   if (EXACT && bad) set_err(err, KERR_RANGE);
   if (CHEX) {
@@ -581,19 +603,111 @@ __global__ void __launch_bounds__(TPB_PASS, PASS == 3 ? 7 : 8) k_pass(G32 g, Par
     if (lane == 0 && n_chex) atomicAdd(sprm.chex_count, (unsigned long long)n_chex);
   }
   __syncthreads();
-  if (EXACT) {  // the node's fixed-point value: high words * 2^16 + low words
-    long long* out = static_cast<long long*>(partial) + b * (4 * TNOD);
-    for (int t = threadIdx.x; t < 4 * TNOD; t += blockDim.x)
-      out[t] = (long long)(int)s_dep[4 * TNOD + t] * 65536LL + (long long)s_dep[t];
-  } else {
-    float* out = static_cast<float*>(partial) + b * (4 * TNOD);
-    for (int t = threadIdx.x; t < 4 * TNOD; t += blockDim.x) out[t] = __uint_as_float(s_dep[t]);
-  }
+  write_tile<EXACT, TNOD>(s_dep, partial, b);
 
   if (PASS == 3 && dep)
     for (int t = threadIdx.x; t < BCELLS * NDIR; t += blockDim.x)  // direction-major: dep[dir][key]
       dep[(long long)(t / BCELLS) * g.nkeys + b * BCELLS + t % BCELLS] =
           (uint16_t)s_rank[(t % BCELLS) * NDIR + t / BCELLS];
+}
+
+// Pass 1 on ions that the last sort has ranked but not moved: perm[l] is the
+// place in src of the ion that belongs at l (~q: new ion q of stage).  Each
+// thread copies its ion's fields into shared memory one chunk ahead (4-byte
+// asynchronous copies; places two chunks ahead), writes them to dst, and
+// deposits them as k_pass<1> does.  The ions so cross HBM once between two
+// steps' pushes (86 B and the 4 B of perm) where the sort's scatter (86 B) and
+// pass 1 (41 B) each read them: 134M ions, 2.41 ms and 0.45 for the places
+// against 2.78 + 1.61.  No thread reads another's copies, so the chunks need
+// no barrier.  (Three buffers instead of two: 3.42 ms.)
+template <bool EXACT>
+__global__ void __launch_bounds__(TPB_PASS, 8) k_pass1_sort(G32 g, Part s, Part n, Part d, Species sp,
+                                                            const int64_t* __restrict__ start,
+                                                            const int32_t* __restrict__ perm,
+                                                            void* __restrict__ partial, int* err) {
+  constexpr int T = TN_IN, TNOD = T * T * T, NF = 10;
+  __shared__ __align__(16) float s_f[2][NF][TPB_PASS];
+  __shared__ unsigned s_dep[(EXACT ? 2 : 1) * 4 * TNOD];
+  __shared__ __align__(16) float s_red[TPB_PASS / 32][12][36];
+  const long long b = blockIdx.x;
+  const int bi = (int)(b % g.nbx), bj = (int)((b / g.nbx) % g.nby), bk = (int)(b / ((long long)g.nbx * g.nby));
+  const int c0x = 4 * bi, c0y = 4 * bj, c0z = 4 * bk;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int t = tid; t < (EXACT ? 2 : 1) * 4 * TNOD; t += TPB_PASS) s_dep[t] = 0u;
+  __syncthreads();
+  const long long first = start[b * BCELLS], last = start[b * BCELLS + BCELLS];
+  const long long a0 = first & ~15LL;  // k_pass<1>'s warps: the same sums, bit for bit
+  const int nchunk = last > first ? (int)((last - a0 + TPB_PASS - 1) / TPB_PASS) : 0;
+  constexpr int32_t NONE = 0x7fffffff;
+  auto place = [&](int k) {
+    const long long l = a0 + (long long)TPB_PASS * k + tid;
+    return k < nchunk && l >= first && l < last ? perm[l] : NONE;
+  };
+  // starts the copies of the ion at place q into buffer u; its species byte
+  auto fetch = [&](int32_t q, int u) -> int {
+    if (q == NONE) return 0;
+    const bool old = q >= 0;
+    const long long i = old ? q : ~q;
+    const void* src[NF] = {old ? (const void*)s.cell : n.cell, old ? s.ox : n.ox, old ? s.oy : n.oy,
+                           old ? s.oz : n.oz, old ? s.vx : n.vx, old ? s.vy : n.vy, old ? s.vz : n.vz,
+                           old ? s.wx : n.wx, old ? s.wy : n.wy, old ? s.wz : n.wz};
+#pragma unroll
+    for (int f = 0; f < NF; ++f) tc05::cp_async4(&s_f[u][f][tid], static_cast<const float*>(src[f]) + i);
+    return (old ? s.sp : n.sp)[i];
+  };
+  unsigned bad = 0;
+  int32_t q0 = place(0), q1 = place(1);
+  int sp0 = fetch(q0, 0), sp1;
+  tc05::cp_async_commit();
+  for (int kc = 0; kc < nchunk; ++kc) {
+    const int u = kc & 1;
+    const int32_t q2 = place(kc + 2);
+    sp1 = fetch(q1, u ^ 1);
+    tc05::cp_async_commit();
+    tc05::cp_async_wait<1>();  // this thread's copies of chunk kc have landed
+    const long long l = a0 + (long long)TPB_PASS * kc + tid;
+    const int32_t c = q0 != NONE ? __float_as_int(s_f[u][0][tid]) & ~CELL_FRESH : CELL_DEAD;
+    bool live = q0 != NONE;
+    int t0 = -1;
+    float w8[8], qdv[4];
+    if (live) {
+      const float ox = s_f[u][1][tid], oy = s_f[u][2][tid], oz = s_f[u][3][tid];
+      const float vx = s_f[u][4][tid], vy = s_f[u][5][tid], vz = s_f[u][6][tid];
+      const float wx = s_f[u][7][tid], wy = s_f[u][8][tid], wz = s_f[u][9][tid];
+      d.cell[l] = c;
+      d.ox[l] = ox; d.oy[l] = oy; d.oz[l] = oz;
+      d.vx[l] = vx; d.vy[l] = vy; d.vz[l] = vz;
+      d.wx[l] = wx; d.wy[l] = wy; d.wz[l] = wz;
+      d.sp[l] = (uint8_t)sp0;
+      const float qw = sp.qw[min(sp0, MAX_SPECIES - 1)];
+      const int rx = pk_i(c) - c0x, ry = pk_j(c) - c0y, rz = pk_k(c) - c0z;
+      if (rx < 0 || rx > 3 || ry < 0 || ry > 3 || rz < 0 || rz > 3) {
+        set_err(err, KERR_MOVE);
+        live = false;
+      } else {
+        t0 = rx + T * (ry + T * rz);
+        const float wxl = 1.0f - ox, wxu = ox, wyl = 1.0f - oy, wyu = oy, wzl = 1.0f - oz, wzu = oz;
+#pragma unroll
+        for (int cc = 0; cc < 8; ++cc)
+          w8[cc] = ((cc & 1) ? wxu : wxl) * (((cc >> 1) & 1) ? wyu : wyl) * ((cc >> 2) ? wzu : wzl);
+        // extrapol_up (gutsp.f:144)
+        qdv[0] = qw;
+        qdv[1] = qw * extrapolated(vx, wx);
+        qdv[2] = qw * extrapolated(vy, wy);
+        qdv[3] = qw * extrapolated(vz, wz);
+      }
+    }
+    if (__any_sync(0xffffffffu, live))
+      warp_deposit<true, T, false, EXACT>(s_red[warp], live, t0, w8, qdv, s_dep, bad, lane);
+    if (EXACT && (kc + 1) % CARRY_CHUNKS == 0 && kc + 1 < nchunk) carry_tile<TNOD>(s_dep);
+    q0 = q1;
+    q1 = q2;
+    sp0 = sp1;
+  }
+  tc05::cp_async_wait_all();
+  if (EXACT && bad) set_err(err, KERR_RANGE);
+  __syncthreads();
+  write_tile<EXACT, TNOD>(s_dep, partial, b);
 }
 
 // Sum, at every interior node, the brick tiles (T nodes per axis) that cover
@@ -1449,6 +1563,88 @@ __global__ void k_new_scatter(G32 g, long long n_host, const int64_t* __restrict
   }
 }
 
+// ---- the sort's moves left to the next step's pass 1 (k_pass1_sort) ----
+
+// perm[dst] = l for the ions the 27-direction sort places (as k_sort_scatter).
+// Four ions per thread: the chain from the ion's words to its key's start and
+// offset is three trips to memory, and with one ion per thread the card held
+// too few of them (134M ions: 0.96 ms, 0.45 this way).
+__global__ void __launch_bounds__(TPB) k_sort_perm(G32 g, long long N, long long cap, const int32_t* __restrict__ cell,
+                                                   const uint32_t* __restrict__ dirrank,
+                                                   const uint16_t* __restrict__ pre,
+                                                   const int64_t* __restrict__ start_new, int32_t* __restrict__ perm,
+                                                   int* err) {
+  const long long l0 = 4 * (blockIdx.x * (long long)TPB + threadIdx.x);
+  if (l0 >= N) return;
+  const bool whole = l0 + 4 <= N;
+  // (the arrays are padded past their last ion)
+  const int4 c4 = *reinterpret_cast<const int4*>(cell + l0);
+  uint4 d4 = make_uint4(DR_DEAD, DR_DEAD, DR_DEAD, DR_DEAD);
+  if (whole) {
+    d4 = *reinterpret_cast<const uint4*>(dirrank + l0);
+  } else {
+    d4.x = dirrank[l0];
+    if (l0 + 1 < N) d4.y = dirrank[l0 + 1];
+    if (l0 + 2 < N) d4.z = dirrank[l0 + 2];
+  }
+  const int32_t c[4] = {c4.x, c4.y, c4.z, c4.w};
+  const uint32_t dr[4] = {d4.x, d4.y, d4.z, d4.w};
+  long long dst[4];
+  bool skip[4], bad = false;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    skip[q] = dr[q] == DR_DEAD || dr[q] == DR_FAR;
+    const int dd = (int)(dr[q] >> 26);
+    if (!skip[q] && dd >= NDIR) {
+      bad = true;
+      skip[q] = true;
+    }
+    dst[q] = 0;
+    if (!skip[q]) {
+      const long long X = key_of(g, pk_i(c[q]), pk_j(c[q]), pk_k(c[q]));
+      dst[q] = start_new[X] + pre[(long long)dd * g.nkeys + X] + (dr[q] & ((1u << 26) - 1u));
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    if (skip[q]) continue;
+    if (dst[q] < 0 || dst[q] >= cap) set_err(err, KERR_CAPACITY);
+    else perm[dst[q]] = (int32_t)(l0 + q);
+  }
+  if (bad) set_err(err, KERR_MOVE);
+}
+
+// perm[dst] = ~q for staged new ion q (as k_new_scatter).
+__global__ void k_new_perm(long long n_host, const int64_t* n_dev, long long n_max, const int32_t* __restrict__ key,
+                           const int32_t* __restrict__ rank, const int32_t* __restrict__ ncount,
+                           const int64_t* __restrict__ start_new, int32_t* __restrict__ perm, long long cap, int* err) {
+  const long long n = n_host + (n_dev ? *n_dev : 0);
+  GSTRIDE(q, n < n_max ? n : n_max) {
+    const long long X = key[q];
+    const long long dst = start_new[X + 1] - ncount[X] + rank[q];
+    if (dst < 0 || dst >= cap) set_err(err, KERR_CAPACITY);
+    else perm[dst] = ~(int32_t)q;
+  }
+}
+
+// The moves alone (a run that ends between the sort and the next pass 1).
+__global__ void k_move_sorted(long long N, const int32_t* __restrict__ perm, Part s, Part n, Part d) {
+  GSTRIDE(l, N) {
+    const int32_t q = perm[l];
+    const Part& a = q >= 0 ? s : n;
+    const long long i = q >= 0 ? q : ~q;
+    const int32_t c = a.cell[i];
+    const float ox = a.ox[i], oy = a.oy[i], oz = a.oz[i], vx = a.vx[i], vy = a.vy[i], vz = a.vz[i], wx = a.wx[i],
+                wy = a.wy[i], wz = a.wz[i];
+    const uint8_t spc = a.sp[i];
+    d.cell[l] = q >= 0 ? c : (c | CELL_FRESH);
+    d.ox[l] = ox; d.oy[l] = oy; d.oz[l] = oz;
+    d.vx[l] = vx; d.vy[l] = vy; d.vz[l] = vz;
+    d.wx[l] = wx; d.wy[l] = wy; d.wz[l] = wz;
+    d.sp[l] = spc;
+  }
+}
+
 // three-phase exclusive scan of int64 (block sums, scan of sums, add)
 constexpr int SCAN_ITEMS = 4;
 constexpr int SCAN_TILE = TPB * SCAN_ITEMS;
@@ -1947,7 +2143,8 @@ __global__ void k_far_count(FarList f, int64_t* __restrict__ count) {
 // (a scan of the whole list: the list is short, and this keeps the order
 // deterministic), then a copy after the near arrivals.
 __global__ void k_far_scatter(G32 g, FarList f, const int32_t* __restrict__ ncount,
-                              const int64_t* __restrict__ start_new, Part s, Part d, long long cap, int* err) {
+                              const int64_t* __restrict__ start_new, Part s, Part d, long long cap,
+                              int32_t* __restrict__ perm, int* err) {
   const int n = min(*f.n, FAR_CAP);
   GSTRIDE(i, n) {
     const long long X = f.key[i];
@@ -1962,6 +2159,10 @@ __global__ void k_far_scatter(G32 g, FarList f, const int32_t* __restrict__ ncou
     const long long dst = start_new[X + 1] - (ncount ? ncount[X] : 0) - cnt + r;
     if (dst < 0 || dst >= cap) {
       set_err(err, KERR_CAPACITY);
+      continue;
+    }
+    if (perm) {  // the move is left to the next pass 1
+      perm[dst] = (int32_t)li;
       continue;
     }
     d.cell[dst] = s.cell[li];
@@ -1980,8 +2181,8 @@ cudaError_t far_count(const FarList& far, int64_t* count, cudaStream_t st) {
   RET((k_far_count<<<64, TPB, 0, st>>>(far, count)));
 }
 cudaError_t far_scatter(const G32& g, const FarList& far, const int32_t* ncount, const int64_t* start_new,
-                        const Part& src, const Part& dst, long long cap, int* err, cudaStream_t st) {
-  RET((k_far_scatter<<<FAR_CAP / TPB, TPB, 0, st>>>(g, far, ncount, start_new, src, dst, cap, err)));
+                        const Part& src, const Part& dst, long long cap, int32_t* perm, int* err, cudaStream_t st) {
+  RET((k_far_scatter<<<FAR_CAP / TPB, TPB, 0, st>>>(g, far, ncount, start_new, src, dst, cap, perm, err)));
 }
 
 cudaError_t sort_prep(const G32& g, const int64_t* start, const int32_t* cell, uint32_t* dirrank, uint16_t* dep,
@@ -2036,6 +2237,29 @@ cudaError_t sort_scatter(const G32& g, long long N, long long cap, const int32_t
                          cudaStream_t st) {
   if (N <= 0) return cudaSuccess;
   RET((k_sort_scatter<<<nblk(N), TPB, 0, st>>>(g, N, cap, cell, dirrank, pre, start_new, src, dst, err)));
+}
+cudaError_t sort_perm(const G32& g, long long N, long long cap, const int32_t* cell, const uint32_t* dirrank,
+                      const uint16_t* pre, const int64_t* start_new, int32_t* perm, int* err, cudaStream_t st) {
+  if (N <= 0) return cudaSuccess;
+  RET((k_sort_perm<<<nblk((N + 3) / 4), TPB, 0, st>>>(g, N, cap, cell, dirrank, pre, start_new, perm, err)));
+}
+cudaError_t new_perm(long long n_host, const int64_t* n_dev, long long n_max, const int32_t* key, const int32_t* rank,
+                     const int32_t* ncount, const int64_t* start_new, int32_t* perm, long long cap, int* err,
+                     cudaStream_t st) {
+  if (n_max <= 0) return cudaSuccess;
+  RET((k_new_perm<<<nblk(n_max), TPB, 0, st>>>(n_host, n_dev, n_max, key, rank, ncount, start_new, perm, cap, err)));
+}
+cudaError_t move_sorted(long long N, const int32_t* perm, const Part& src, const Part& stage, const Part& dst,
+                        cudaStream_t st) {
+  if (N <= 0) return cudaSuccess;
+  RET((k_move_sorted<<<nblk(N), TPB, 0, st>>>(N, perm, src, stage, dst)));
+}
+cudaError_t pass1_sort(const G32& g, const Part& src, const Part& stage, const Part& dst, const Species& sp,
+                       const int64_t* start, const int32_t* perm, void* partial, bool exact, int* err,
+                       cudaStream_t st) {
+  if (exact)
+    RET((k_pass1_sort<true><<<(unsigned)g.nbricks, TPB_PASS, 0, st>>>(g, src, stage, dst, sp, start, perm, partial, err)));
+  RET((k_pass1_sort<false><<<(unsigned)g.nbricks, TPB_PASS, 0, st>>>(g, src, stage, dst, sp, start, perm, partial, err)));
 }
 cudaError_t from_f64(const G32& g, long long N, long long NM, const double* xp, const double* vp, const double* vp1,
                      const double* mrat, const double* beta_p, const Species& sp, Part p, int* err, cudaStream_t st) {

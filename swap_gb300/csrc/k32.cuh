@@ -173,7 +173,7 @@ cudaError_t far_count(const FarList& far, int64_t* count, cudaStream_t st);
 // The far list's survivors to start_new[X+1] - ncount[X] - (far arrivals of
 // X) + (their rank by array index); ncount may be null.
 cudaError_t far_scatter(const G32& g, const FarList& far, const int32_t* ncount, const int64_t* start_new,
-                        const Part& src, const Part& dst, long long cap, int* err, cudaStream_t st);
+                        const Part& src, const Part& dst, long long cap, int32_t* perm, int* err, cudaStream_t st);
 // Sum the brick partial tiles into np and S (interior nodes, (nx,ny,nz) layout).
 // pass: the pass (1-3) whose tiles `partial` holds
 cudaError_t node_sum(const G32& g, int pass, const void* partial, bool exact, float* np, float* S, cudaStream_t st);
@@ -257,6 +257,19 @@ cudaError_t sort_prep(const G32& g, const int64_t* start, const int32_t* cell, u
 // direction-major: pre[dir * nkeys + key].
 cudaError_t sort_count(const G32& g, const uint16_t* dep, const int32_t* ncount, const uint8_t* order,
                        int64_t* count, uint16_t* pre, int* err, cudaStream_t st);
+// The sort's moves left to the next step's pass 1: perm[dst] = the ion's place
+// in the source arrays, or ~q for staged new ion q (with far_scatter's perm).
+cudaError_t sort_perm(const G32& g, long long N, long long cap, const int32_t* cell, const uint32_t* dirrank,
+                      const uint16_t* pre, const int64_t* start_new, int32_t* perm, int* err, cudaStream_t st);
+cudaError_t new_perm(long long n_host, const int64_t* n_dev, long long n_max, const int32_t* key, const int32_t* rank,
+                     const int32_t* ncount, const int64_t* start_new, int32_t* perm, long long cap, int* err,
+                     cudaStream_t st);
+// Pass 1 that makes these moves (src and stage to dst), and the moves alone.
+cudaError_t pass1_sort(const G32& g, const Part& src, const Part& stage, const Part& dst, const Species& sp,
+                       const int64_t* start, const int32_t* perm, void* partial, bool exact, int* err,
+                       cudaStream_t st);
+cudaError_t move_sorted(long long N, const int32_t* perm, const Part& src, const Part& stage, const Part& dst,
+                        cudaStream_t st);
 // Directions by increasing source key for every place in a brick (host).
 void sort_order_table(uint8_t* out);
 cudaError_t scan_exclusive(const int64_t* in, int64_t* out, long long n, int64_t* block_sums, cudaStream_t st);

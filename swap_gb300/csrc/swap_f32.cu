@@ -33,6 +33,11 @@ struct F32State {
   int cur = 0;
   int64_t *start = nullptr, *start_new = nullptr, *count = nullptr, *sums = nullptr;
   uint32_t* dirrank = nullptr;
+  // grids too large for the field loop: between two steps of one run the sort
+  // only ranks, and the next pass 1 moves the ions (perm; move_pending until
+  // then: buf[1 - cur] still holds them, buf[cur] is theirs to be)
+  int32_t* perm = nullptr;
+  bool move_pending = false;
   uint16_t* dep = nullptr;
   uint16_t* pre = nullptr;
   void* partial = nullptr;  // brick partial tiles, 8 bytes per entry (fixed point or FP32)
@@ -199,7 +204,7 @@ struct PreStaged {
 };
 static int side_stream(swap_ctx* c, F32State* s);
 static int sort_step(swap_ctx* c, F32State* s, long long src_step, bool prepared = false,
-                     const PreStaged* pre = nullptr, bool on_side = false);
+                     const PreStaged* pre = nullptr, bool on_side = false, bool defer = false);
 
 // ---------------------------------------------------------------------------
 
@@ -357,6 +362,11 @@ extern "C" int swap_f32_begin(swap_ctx* c) {
   s->count = s->alloc<int64_t>(nk + 1);
   s->sums = s->alloc<int64_t>(nk / 1024 + 16);
   s->dirrank = s->alloc<uint32_t>(NMs);
+  if (!field_loop_fits(g)) {
+    s->perm = s->alloc<int32_t>(NMs);
+    if (!s->perm) return c->fail(SWAP_ECUDA, "FP32 particle allocation failed");
+    CU(cudaMemsetAsync(s->perm, 0, NMs * sizeof(int32_t), c->st));  // always a place inside the arrays
+  }
   s->dep = s->alloc<uint16_t>(nk * NDIR);
   s->pre = s->alloc<uint16_t>(nk * NDIR);
   s->order = s->alloc<uint8_t>(BCELLS * NDIR);
@@ -570,14 +580,14 @@ static int subcycles(swap_ctx* c, F32State* s, float* e_acc = nullptr) {
 // arrivals of their cell, flagged fresh.  prepared: pass 3 already wrote the
 // directions, ranks and per-key counts.
 static int sort_body(swap_ctx* c, F32State* s, long long src_step, bool prepared, const PreStaged* pre,
-                     bool on_side);
+                     bool on_side, bool defer);
 static int side_stream(swap_ctx* c, F32State* s);
 // on_side: the sort goes to the second stream after the main stream's work
 // so far and the staging; sort_join (after the field step) waits for it and
 // takes the new count.
 static int sort_step(swap_ctx* c, F32State* s, long long src_step, bool prepared, const PreStaged* pre,
-                     bool on_side) {
-  if (!on_side) return sort_body(c, s, src_step, prepared, pre, false);
+                     bool on_side, bool defer) {
+  if (!on_side) return sort_body(c, s, src_step, prepared, pre, false, false);
   TRY(side_stream(c, s));
   if (!(pre && pre->valid)) {  // no staging ahead of it: order after the main stream here
     CU(cudaEventRecord(s->ev_main, c->st));
@@ -585,7 +595,7 @@ static int sort_step(swap_ctx* c, F32State* s, long long src_step, bool prepared
   }
   cudaStream_t main = c->st;
   c->st = s->side;
-  const int r = sort_body(c, s, src_step, prepared, pre, true);
+  const int r = sort_body(c, s, src_step, prepared, pre, true, defer);
   c->st = main;
   if (r) return r;
   CU(cudaEventRecord(s->ev_sort, s->side));
@@ -607,7 +617,7 @@ static int sort_join(swap_ctx* c, F32State* s) {
 }
 
 static int sort_body(swap_ctx* c, F32State* s, long long src_step, bool prepared, const PreStaged* pre,
-                     bool on_side) {
+                     bool on_side, bool defer) {
   const G32& g = s->g;
   Part& a = s->buf[s->cur];
   Part& b = s->buf[1 - s->cur];
@@ -628,13 +638,24 @@ static int sort_body(swap_ctx* c, F32State* s, long long src_step, bool prepared
                                   c->d_err, c->st));
   if (prepared) KL("f32_far_count", far_count(s->far, s->count, c->st));
   KLN("f32_sort_scan", 3, scan_exclusive(s->count, s->start_new, g.nkeys, s->sums, c->st));
-  KL("f32_sort_scatter", sort_scatter(g, s->N, cap, a.cell, s->dirrank, s->pre, s->start_new, a, b, c->d_err, c->st));
-  if (prepared)
-    KL("f32_far_scatter", far_scatter(g, s->far, staged ? s->stage.ncount : nullptr, s->start_new, a, b, cap,
+  if (defer) {
+    KL("f32_sort_perm", sort_perm(g, s->N, cap, a.cell, s->dirrank, s->pre, s->start_new, s->perm, c->d_err, c->st));
+    KL("f32_far_scatter", far_scatter(g, s->far, staged ? s->stage.ncount : nullptr, s->start_new, a, b, cap, s->perm,
                                       c->d_err, c->st));
-  if (staged)
-    KL("f32_new_scatter", new_scatter(g, n_host, n_dev, n_max, s->stage.part, s->stage.key, s->stage.rank,
-                                      s->stage.ncount, s->start_new, b, cap, c->d_err, c->st));
+    if (staged)
+      KL("f32_new_scatter", new_perm(n_host, n_dev, n_max, s->stage.key, s->stage.rank, s->stage.ncount,
+                                     s->start_new, s->perm, cap, c->d_err, c->st));
+    s->move_pending = true;
+  } else {
+    KL("f32_sort_scatter",
+       sort_scatter(g, s->N, cap, a.cell, s->dirrank, s->pre, s->start_new, a, b, c->d_err, c->st));
+    if (prepared)
+      KL("f32_far_scatter", far_scatter(g, s->far, staged ? s->stage.ncount : nullptr, s->start_new, a, b, cap,
+                                        nullptr, c->d_err, c->st));
+    if (staged)
+      KL("f32_new_scatter", new_scatter(g, n_host, n_dev, n_max, s->stage.part, s->stage.key, s->stage.rank,
+                                        s->stage.ncount, s->start_new, b, cap, c->d_err, c->st));
+  }
   std::swap(s->start, s->start_new);
   s->cur = 1 - s->cur;
   if (on_side) {  // the count, for sort_join
@@ -794,23 +815,37 @@ static int stage_ahead(swap_ctx* c, F32State* s, long long m, PreStaged* pre) {
   return SWAP_OK;
 }
 
-static int one_step_body(swap_ctx* c, F32State* s);
+static int one_step_body(swap_ctx* c, F32State* s, bool more);
 // A step; after a failure the second stream's work (a sort already queued)
 // is drained, so that nothing of the step runs on when the caller goes on.
-static int one_step(swap_ctx* c, F32State* s) {
-  const int r = one_step_body(c, s);
+// more: another step of the same call follows, whose pass 1 may make this
+// step's sorted moves.
+static int one_step(swap_ctx* c, F32State* s, bool more) {
+  const int r = one_step_body(c, s, more);
   if (r && s->sort_pending) {
     cudaStreamSynchronize(s->side);
     s->sort_pending = false;
   }
+  if (r && s->move_pending) {  // leave the ions where the rest of the state says they are
+    s->move_pending = false;
+    if (s->N <= c->dims.ni_max)
+      move_sorted(s->N, s->perm, s->buf[1 - s->cur], s->stage.part, s->buf[s->cur], c->st);
+  }
   return r;
 }
 
-static int one_step_body(swap_ctx* c, F32State* s) {
+static int one_step_body(swap_ctx* c, F32State* s, bool more) {
   const G32& g = s->g;
   const StepParams sp = step_params(c, s);
   const Part& p = s->buf[s->cur];
-  KL("f32_P1", pass(1, g, p, s->sp, sp, s->start, s->kit, s->partial, nullptr, nullptr, c->d_err, s->exact, c->st));  // :385-387,399
+  // :385-387,399
+  if (s->move_pending) {
+    s->move_pending = false;
+    KL("f32_P1_sort", pass1_sort(g, s->buf[1 - s->cur], s->stage.part, p, s->sp, s->start, s->perm, s->partial,
+                                 s->exact, c->d_err, c->st));
+  } else {
+    KL("f32_P1", pass(1, g, p, s->sp, sp, s->start, s->kit, s->partial, nullptr, nullptr, c->d_err, s->exact, c->st));
+  }
   TRY(deposit_sums(c, s, 1));
   auto kit = [&] {  // :395, :398-400 (curlB, edge_to_center, up and get_Ep's face_to_center)
     return build_kit(g, s->S, s->db1, s->b0c, s->np, (float)c->prm.alpha, s->gp, s->kit, s->kitg, s->far.n, s->d_min,
@@ -835,7 +870,7 @@ static int one_step_body(swap_ctx* c, F32State* s) {
   if (s->src_on) TRY(stage_ahead(c, s, c->src_step + 1, &pre));  // the sources of the next step
   // the sort on the second stream, beside the moments' sums and the field
   // subcycles: it reads pass 3's outputs and the staging, they the grids
-  TRY(sort_step(c, s, c->src_step + 1, true, &pre, true));
+  TRY(sort_step(c, s, c->src_step + 1, true, &pre, true, more && s->perm));
   TRY(deposit_sums(c, s, 3));
   KL("f32_up_courant", up_courant(g, s->np, s->S, s->db1, s->b0c, (float)c->prm.alpha, g.dx, s->up, s->dtn, s->d_min,
                                   c->d_err, c->st));
@@ -851,7 +886,7 @@ extern "C" int swap_f32_run(swap_ctx* c, int32_t nsteps) {
   F32State* s = f32(c);
   if (!s) return c->fail(SWAP_EINVAL, "swap_f32_begin has not been called");
   if (s->ended && s->src_on) return c->fail(SWAP_EINVAL, "call swap_f32_begin again after swap_f32_end");
-  for (int k = 0; k < nsteps; ++k) TRY(one_step(c, s));
+  for (int k = 0; k < nsteps; ++k) TRY(one_step(c, s, k + 1 < nsteps));
   return check_err(c);
 }
 
@@ -1084,7 +1119,7 @@ extern "C" int swap_surrogate_collect(swap_surrogate* net, swap_ctx* c, int32_t 
   if (!s || s->ended) return c->fail(SWAP_EINVAL, "swap_f32_begin has not been called");
   s->collect = net;
   int r = SWAP_OK;
-  for (int k = 0; k < nsteps && !r; ++k) r = one_step(c, s);
+  for (int k = 0; k < nsteps && !r; ++k) r = one_step(c, s, k + 1 < nsteps);
   s->collect = nullptr;
   return r ? r : check_err(c);
 }
