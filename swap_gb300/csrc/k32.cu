@@ -86,37 +86,26 @@ __device__ __forceinline__ void interior_of(const G32& g, long long t, int& i, i
 
 __host__ __device__ __forceinline__ long long n_int(const G32& g) { return (long long)g.ncx * g.ncy * g.ncz; }
 
-// Move one axis of a (cell, offset) position by d cells.  upper_closed:
-// offsets in (0,1] (the '>' cell search of x and z, gutsp.f:1396-1412);
-// otherwise [0,1) (the floor of y, gutsp.f:1404).  Periodic in the cell
-// index (gutsp.f:490-510, one wrap) when wrap; otherwise the cell may leave
-// [0, n).  Returns false on a move that is not finite or spans n - 2 cells
-// or more (one wrap then always lands in [0, n)).
-__device__ __forceinline__ bool move_axis(int& c, float& o, float d, int n, bool upper_closed, bool wrap = true) {
-  if (!(fabsf(d) < (float)(n - 2))) return false;
-  o += d;
-  // carry whole cells: (0,1] keeps o = 1 in the cell, [0,1) moves it up
-  const float k = upper_closed ? ceilf(o) - 1.0f : floorf(o);
+// Move one axis of a (cell, offset) position by d cells; the whole cells
+// carried.  UPPER: offsets in (0,1] (the '>' cell search of x and z,
+// gutsp.f:1396-1412); otherwise [0,1) (the floor of y, gutsp.f:1404).  A move
+// that is not finite or spans n - 2 cells or more is not made and clears ok
+// (below that one wrap always lands in [0, n), gutsp.f:490-510).  No branches,
+// and the caller keeps cells unwrapped and takes its brick and sort steps from
+// the carries: P3 @MOVE@.
+template <bool UPPER>
+__device__ __forceinline__ int half_step(float& o, float d, int n, bool& ok) {
+  const bool fits = fabsf(d) < (float)(n - 2);
+  ok = ok && fits;
+  o += fits ? d : 0.0f;
+  const float k = UPPER ? ceilf(o) - 1.0f : floorf(o);
   o -= k;
-  c += (int)k;
-  if (upper_closed) {  // rounding can leave o at 0 or just above 1
-    if (o <= 0.0f) { o += 1.0f; --c; }
-  } else if (o >= 1.0f) {
-    o -= 1.0f;
-    ++c;
-  }
-  if (wrap) c = c < 0 ? c + n : (c >= n ? c - n : c);
-  return true;
-}
-
-// Offset of a cell from a brick's first cell along one axis, unwrapped
-// across the periodic boundary into the brick tile's window [-1, 4] when
-// one of the periodic images lies there (n >= 8, so at most one does).
-__device__ __forceinline__ int rel_cell(int c, int c0, int n) {
-  int r = c - c0;
-  if (r < -1) r += n;
-  else if (r > 4) r -= n;
-  return r;
+  int c = (int)k;
+  // rounding can leave o at the open end
+  const bool edge = UPPER ? o <= 0.0f : o >= 1.0f;
+  o += edge ? (UPPER ? 1.0f : -1.0f) : 0.0f;
+  c += edge ? (UPPER ? -1 : 1) : 0;
+  return c;
 }
 
 // Step between two cells along one axis, unwrapped into [-1, 1] when one of
@@ -484,22 +473,27 @@ __global__ void __launch_bounds__(TPB_PASS, PASS == 3 ? 7 : 8) k_pass(G32 g, Par
           dvx = vx; dvy = vy; dvz = vz;
           // move_ion_half of maind.f:408 (gutsp.f:473-510): the deposit position
           const float mvx = vx * hdt * g.inv_dx, mvy = vy * hdt * g.inv_dy, mvz = vz * hdt * g.inv_dz;
-          bool ok = move_axis(ci, ox, mvx, g.ncx, true, !sprm.x_open);
-          ok &= move_axis(cj, oy, mvy, g.ncy, false);
-          ok &= move_axis(ck, oz, mvz, g.ncz, true);
-          const bool out1 = ci < 0 || ci >= g.ncx;  // outflow through an open x face
-          rx = rel_cell(ci, c0x, g.ncx); ry = rel_cell(cj, c0y, g.ncy); rz = rel_cell(ck, c0z, g.ncz);
-          float dox = ox, doy = oy, doz = oz;
+          bool ok = true;
+          const int kx = half_step<true>(ox, mvx, g.ncx, ok), ky = half_step<false>(oy, mvy, g.ncy, ok),
+                    kz = half_step<true>(oz, mvz, g.ncz, ok);
+          const int cx1 = ci + kx, cy1 = cj + ky, cz1 = ck + kz;  // not wrapped
+          const bool out1 = sprm.x_open && (cx1 < 0 || cx1 >= g.ncx);  // outflow through an open x face
+          rx += kx; ry += ky; rz += kz;
+          const float dox = ox, doy = oy, doz = oz;
           // move_ion_half of maind.f:479: the stored position
-          int ci2 = ci, cj2 = cj, ck2 = ck;
-          bool out2 = out1;
-          if (!out1) {
-            ok &= move_axis(ci2, ox, mvx, g.ncx, true, !sprm.x_open);
-            ok &= move_axis(cj2, oy, mvy, g.ncy, false);
-            ok &= move_axis(ck2, oz, mvz, g.ncz, true);
-            out2 = ci2 < 0 || ci2 >= g.ncx;
-          }
+          const int lx = half_step<true>(ox, mvx, g.ncx, ok), ly = half_step<false>(oy, mvy, g.ncy, ok),
+                    lz = half_step<true>(oz, mvz, g.ncz, ok);
           if (!ok) set_err(err, KERR_MOVE);
+          const bool out2 = out1 || (sprm.x_open && (cx1 + lx < 0 || cx1 + lx >= g.ncx));
+          // steps from the ion's own cell, for the sort; one wrap brings a
+          // near ion's cell home, a far one's takes one per half move
+          const int sx = kx + lx, sy = ky + ly, sz = kz + lz;
+          const bool near = (unsigned)(sx + 1) <= 2u && (unsigned)(sy + 1) <= 2u && (unsigned)(sz + 1) <= 2u;
+          int ci2 = near ? ci + sx : wrapi(cx1, g.ncx) + lx, cj2 = near ? cj + sy : wrapi(cy1, g.ncy) + ly,
+              ck2 = near ? ck + sz : wrapi(cz1, g.ncz) + lz;
+          ci2 = wrapi(ci2, g.ncx);
+          cj2 = wrapi(cj2, g.ncy);
+          ck2 = wrapi(ck2, g.ncz);
           if (CHEX && !out2 && sprm.heavy_of[s] != s) {
             // res_chex (chem_rates.f:823-840) at the end of the step, FP32
             const float x = (float)g.qx1 + ((float)ci2 + ox) * g.dx - sprm.cloud_x;
@@ -527,12 +521,8 @@ __global__ void __launch_bounds__(TPB_PASS, PASS == 3 ? 7 : 8) k_pass(G32 g, Par
           } else {
             p.cell[l] = pk(ci2, cj2, ck2);
             p.ox[l] = ox; p.oy[l] = oy; p.oz[l] = oz;
-            const int sx = step_cell(ci2, c0x + (kl & 3), g.ncx), sy = step_cell(cj2, c0y + ((kl >> 2) & 3), g.ncy),
-                      sz = step_cell(ck2, c0z + (kl >> 4), g.ncz);
-            if (sx < -1 || sx > 1 || sy < -1 || sy > 1 || sz < -1 || sz > 1)
-              far_ion = true;
-            else
-              grp = kl * NDIR + dir_index(sx, sy, sz);
+            if (near) grp = kl * NDIR + dir_index(sx, sy, sz);
+            else far_ion = true;
           }
           ox = dox; oy = doy; oz = doz;  // the deposit uses the maind.f:408 position
           if (out1) live = false;
@@ -543,7 +533,7 @@ __global__ void __launch_bounds__(TPB_PASS, PASS == 3 ? 7 : 8) k_pass(G32 g, Par
             if (slot < FAR_CAP) {
               far.idx[slot] = l;
               far.key[slot] = out2 ? -1LL : key_of(g, ci2, cj2, ck2);
-              far.dcell[slot] = live ? pk(ci, cj, ck) : -1;
+              far.dcell[slot] = live ? pk(wrapi(cx1, g.ncx), wrapi(cy1, g.ncy), wrapi(cz1, g.ncz)) : -1;
               far.o[slot] = ox; far.o[FAR_CAP + slot] = oy; far.o[2 * FAR_CAP + slot] = oz;
               far.q[slot] = qw; far.q[FAR_CAP + slot] = qw * dvx;
               far.q[2 * FAR_CAP + slot] = qw * dvy; far.q[3 * FAR_CAP + slot] = qw * dvz;
@@ -577,7 +567,8 @@ __global__ void __launch_bounds__(TPB_PASS, PASS == 3 ? 7 : 8) k_pass(G32 g, Par
         qdv[3] = qw * dvz;
       }
     }
-    warp_deposit<PASS != 2, T, PASS == 3, EXACT>(s_red[warp], live, t0, w8, qdv, s_dep, bad, lane, t0o, mover);
+    if (__any_sync(0xffffffffu, live))  // (a brick's last chunk seldom fills its warps)
+      warp_deposit<PASS != 2, T, PASS == 3, EXACT>(s_red[warp], live, t0, w8, qdv, s_dep, bad, lane, t0o, mover);
     if (PASS == 3 && dirrank) {
       // stable ranks per (key, direction): the warps of the CTA take their
       // turn in order, each adding its particles after the earlier ones
