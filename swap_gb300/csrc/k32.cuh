@@ -26,6 +26,7 @@ constexpr int TNODES_IN = TN_IN * TN_IN * TN_IN;  // 125
 // Tile nodes per axis of the passes' deposit tiles (and of k_node_sum).
 __host__ __device__ constexpr int pass_tile(int pass) { return pass == 3 ? TN : TN_IN; }
 constexpr int NDIR = 27;              // displacements in {-1,0,1}^3
+constexpr int SORT_CLASSES = 216;     // a cell's place in its brick and at the seams, 6 per axis
 constexpr int MAX_SPECIES = 16;
 // Inputs per voxel of the field surrogate: B (3), u_p (3), n_p, p_e, E0 (3),
 // and B - b12 (3), the change over the last subcycle (the predictor is a
@@ -253,7 +254,7 @@ cudaError_t join_df(long long n, const float* h, const float* l, double* a, cuda
 cudaError_t sort_prep(const G32& g, const int64_t* start, const int32_t* cell, uint32_t* dirrank, uint16_t* dep,
                       int* err, cudaStream_t st);
 // ncount (may be null): new ions per key, placed after the arrivals.  order:
-// the BCELLS x NDIR table of sort_order_table on the device.  pre is
+// the SORT_CLASSES x NDIR table of sort_order_table on the device.  pre is
 // direction-major: pre[dir * nkeys + key].
 cudaError_t sort_count(const G32& g, const uint16_t* dep, const int32_t* ncount, const uint8_t* order,
                        int64_t* count, uint16_t* pre, int* err, cudaStream_t st);
@@ -270,7 +271,7 @@ cudaError_t pass1_sort(const G32& g, const Part& src, const Part& stage, const P
                        cudaStream_t st);
 cudaError_t move_sorted(long long N, const int32_t* perm, const Part& src, const Part& stage, const Part& dst,
                         cudaStream_t st);
-// Directions by increasing source key for every place in a brick (host).
+// Directions by increasing source key for every class of cell (host).
 void sort_order_table(uint8_t* out);
 cudaError_t scan_exclusive(const int64_t* in, int64_t* out, long long n, int64_t* block_sums, cudaStream_t st);
 // Survivors to start_new[X] + pre + rank; removed ions are skipped; cap = ni_max.

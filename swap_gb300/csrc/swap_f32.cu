@@ -369,9 +369,9 @@ extern "C" int swap_f32_begin(swap_ctx* c) {
   }
   s->dep = s->alloc<uint16_t>(nk * NDIR);
   s->pre = s->alloc<uint16_t>(nk * NDIR);
-  s->order = s->alloc<uint8_t>(BCELLS * NDIR);
+  s->order = s->alloc<uint8_t>(SORT_CLASSES * NDIR);
   {
-    uint8_t ord[BCELLS * NDIR];
+    uint8_t ord[SORT_CLASSES * NDIR];
     sort_order_table(ord);
     if (!s->order || cudaMemcpy(s->order, ord, sizeof(ord), cudaMemcpyHostToDevice) != cudaSuccess)
       return c->fail(SWAP_ECUDA, "sort order table");
