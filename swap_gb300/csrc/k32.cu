@@ -1166,14 +1166,14 @@ __global__ void __launch_bounds__(FBX * FBY) k_bstep(G32 g, const float* __restr
 // meet at the hardware's cluster barrier (0.24 us) -- up to FIELD_CLUSTER *
 // LOOP_TPB nodes.  Otherwise a cooperative launch with a counter in memory
 // (1.2 us at 152 blocks; grid_loop.cuh).
-// A step of 8 ions per cell, loop against launches, in ms: 1.5k nodes 0.234
-// against 0.325, 33k 0.314 against 0.342, 65k 0.341 against 0.408, 131k 0.533
-// against 0.524, 262k 0.887 against 0.791 (one block per SM then hides less
+// A step of 8 ions per cell, loop against launches, in ms: 1.5k nodes 0.183
+// against 0.325, 33k 0.244 against 0.342, 65k 0.272 against 0.408, 131k 0.449
+// against 0.454, 262k 0.726 against 0.682 (one block per SM then hides less
 // latency than full occupancy does): hence FIELD_LOOP_NODES.
 constexpr int LOOP_TPB = 512;
 
 template <bool CLUSTER>
-__global__ void __launch_bounds__(LOOP_TPB, 2) k_field_loop(G32 g, FieldLoop f) {
+__global__ void __launch_bounds__(LOOP_TPB, 1) k_field_loop(G32 g, FieldLoop f) {
   // uniform over the grid (both words are a snapshot that nothing writes
   // now): a failed pass or a Courant violation leaves the state as it is
   if (*f.failed != 0 || (double)*f.courant <= f.courant_floor) return;
@@ -2040,7 +2040,10 @@ cudaError_t field_loop(const G32& g, const FieldLoop& f, cudaStream_t st) {
   G32 gg = g;
   FieldLoop ff = f;
   void* args[] = {&gg, &ff};
-  return loop::launch(reinterpret_cast<const void*>(&k_field_loop<false>), need, LOOP_TPB, args, st);
+  // about the nodes' even share per SM, a block on each; whole groups of four
+  // warps, so that fewer blocks meet at the barrier
+  const long long n = n_int(g), per = ((n + 151) / 152 + 127) / 128 * 128, t = per < LOOP_TPB ? per : LOOP_TPB;
+  return loop::launch(reinterpret_cast<const void*>(&k_field_loop<false>), (n + t - 1) / t, (int)t, args, st);
 }
 cudaError_t b_step_given_e(const G32& g, const float* E, const float* bh, const float* bl, double coef,
                            const float* b0c, float* oh, float* ol, float* dbo, cudaStream_t st) {

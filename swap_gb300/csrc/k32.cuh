@@ -207,7 +207,7 @@ cudaError_t b_step(const G32& g, bool pred, bool write_e, const float* ct, const
 // to the buffers that n rounds of the two launchers above would use.  Nothing
 // is done when *failed is set or *courant (the smallest Courant time) <=
 // courant_floor: the caller looks at both.  Neither word may change meanwhile.
-constexpr long long FIELD_LOOP_NODES = 3 << 15;
+constexpr long long FIELD_LOOP_NODES = 1 << 17;
 constexpr int FIELD_CLUSTER = 8;  // the portable cluster size
 struct FieldLoop {
   int n;

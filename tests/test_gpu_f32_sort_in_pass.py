@@ -9,7 +9,7 @@ import pytest
 from swap_gb300.hybrid import Hybrid, config
 
 pytestmark = pytest.mark.gpu
-CELLS = (64, 48, 36)  # 110592 cells, above FIELD_LOOP_NODES
+CELLS = (64, 60, 40)  # 153600 cells, above FIELD_LOOP_NODES
 
 
 def _make(kind):
