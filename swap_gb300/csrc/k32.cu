@@ -88,27 +88,34 @@ __device__ __forceinline__ void interior_of(const G32& g, long long t, int& i, i
 __host__ __device__ __forceinline__ long long n_int(const G32& g) { return (long long)g.ncx * g.ncy * g.ncz; }
 
 // Move one axis of a (cell, offset) position by d cells; the whole cells
-// carried.  UPPER: offsets in (0,1] (the '>' cell search of x and z,
-// gutsp.f:1396-1412); otherwise [0,1) (the floor of y, gutsp.f:1404).  A move
-// that is not finite or spans n - 2 cells or more is not made and clears ok
-// (below that one wrap always lands in [0, n), gutsp.f:490-510).  No branches,
-// and the caller keeps cells unwrapped and takes its brick and sort steps from
-// the carries: 134M ions,
-// pass 3: 4.10 ms with early returns and steps from wrapped cells, 3.78 so.
+// carried, as a float.  UPPER: offsets in (0,1] (the '>' cell search of x and
+// z, gutsp.f:1396-1412); otherwise [0,1) (the floor of y, gutsp.f:1404).  A
+// move that is not finite or spans n - 2 cells or more is not made and clears
+// ok (below that one wrap always lands in [0, n), gutsp.f:490-510).  No
+// branches, and the caller keeps cells unwrapped and takes its brick and sort
+// steps from the carries.
 template <bool UPPER>
-__device__ __forceinline__ int half_step(float& o, float d, int n, bool& ok) {
+__device__ __forceinline__ float half_step(float& o, float d, int n, bool& ok) {
   const bool fits = fabsf(d) < (float)(n - 2);
   ok = ok && fits;
   o += fits ? d : 0.0f;
-  const float k = UPPER ? ceilf(o) - 1.0f : floorf(o);
+  if (UPPER) {
+    // o - k > 0 holds exactly and so in floats: a difference of two floats
+    // that differ does not round to zero
+    const float k = ceilf(o) - 1.0f;
+    o -= k;
+    return k;
+  }
+  const float k = floorf(o);
   o -= k;
-  int c = (int)k;
-  // rounding can leave o at the open end
-  const bool edge = UPPER ? o <= 0.0f : o >= 1.0f;
-  o += edge ? (UPPER ? 1.0f : -1.0f) : 0.0f;
-  c += edge ? (UPPER ? -1 : 1) : 0;
-  return c;
+  const bool edge = o >= 1.0f;  // a tiny negative o rounds up to the open end
+  o = edge ? 0.0f : o;
+  return edge ? k + 1.0f : k;
 }
+
+// A whole number |x| < 2^22 added to FLOAT_INT is an integer in its low bits.
+constexpr float FLOAT_INT = 12582912.0f;  // 1.5 * 2^23
+__device__ __forceinline__ int float_int(float x) { return __float_as_int(x) - __float_as_int(FLOAT_INT); }
 
 // Step between two cells along one axis, unwrapped into [-1, 1] when one of
 // the periodic images lies there.
@@ -132,7 +139,8 @@ __device__ __forceinline__ int dir_index(int dx, int dy, int dz) { return (dx + 
 // ends known to the whole warp (tested per group of four particles), and adds
 // each run's sum to the brick tile with one shared atomic.  t0: the tile index
 // of the particle's lower corner node, -1 when it deposits nothing.  ALL_Q:
-// every moment (otherwise the density, q = 0, is skipped).
+// every moment (otherwise the density, q = 0, is skipped).  An ion that is not
+// live brings moments of zero.
 // MOVERS (pass 3, which deposits after a half move): the runs follow trun,
 // the particle's cell before the move (sorted, so runs stay long), and the
 // few particles that changed cell (mover) take no part in them; each of
@@ -184,11 +192,10 @@ template <bool ALL_Q, int T, bool MOVERS = false, bool EXACT = true>
 __device__ __forceinline__ void warp_deposit(float (*red)[36], bool live, int t0, const float (&w8)[8],
                                              const float (&qdv)[4], void* tile, unsigned& bad, int lane,
                                              int trun = -1, bool mover = false) {
-  const bool in_runs = live && !(MOVERS && mover);
 #pragma unroll
-  for (int c8 = 0; c8 < 8; ++c8) red[c8][lane] = live ? w8[c8] : 0.0f;
+  for (int c8 = 0; c8 < 8; ++c8) red[c8][lane] = w8[c8];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) red[8 + q][lane] = in_runs ? qdv[q] : 0.0f;
+  for (int q = 0; q < 4; ++q) red[8 + q][lane] = MOVERS && mover ? 0.0f : qdv[q];
   __syncwarp();
   const int key = MOVERS ? trun : t0;
   const int tprev = __shfl_up_sync(0xffffffffu, key, 1);
@@ -256,6 +263,12 @@ __device__ __forceinline__ float extrapolated(float v, float v1) {
   return __fmaf_rn(1.5f, v, -__fmul_rn(0.5f, v1));
 }
 
+__device__ __forceinline__ void corner_weights(float ox, float oy, float oz, float (&w8)[8]) {
+  const float wxl = 1.0f - ox, wyl = 1.0f - oy, wzl = 1.0f - oz;
+#pragma unroll
+  for (int c = 0; c < 8; ++c) w8[c] = ((c & 1) ? ox : wxl) * ((c & 2) ? oy : wyl) * ((c & 4) ? oz : wzl);
+}
+
 // A crowded brick: carry the low words into the high words (exact: 2^16 low
 // units are one high unit), so that they never wrap.  The whole block calls.
 template <int TNOD>
@@ -295,6 +308,15 @@ __device__ __forceinline__ void write_tile(const unsigned* s_dep, void* partial,
 //       res_chex after the second (maind.f:484).  It also prepares the sort:
 //       the direction of every particle's new cell from its key's cell and
 //       its rank among the particles of that key and direction, in order.
+// Bound by issue (77% of the slots in P3, 74% in P2) and by shared memory
+// (59%, 75%): about 760 warp instructions per 32 ions in P3, 475 in P2.  An
+// ion's tile index, key and direction come from its cell word and the whole
+// cells it moves, and wraps, outflow and far moves stand in a branch that
+// bricks away from the faces take for far ions only: 33.5M ions, P3 0.97 ->
+// 0.865 ms (990 instructions when every ion unpacked, wrapped and checked its
+// cells).  The barrier after each warp's turn in the ranks stays: letting the
+// warps run apart (named barriers, or none after the last turn) took P3 to
+// 1.13 and 0.885 ms.
 // PGRAD: the isothermal electron-pressure term in the gathered E (kitg:
 // its face gradient centred per node, as get_Ep's gradient extension).
 template <int PASS, bool CHEX = false, bool EXACT = true, bool PGRAD = false>
@@ -328,6 +350,9 @@ __global__ void __launch_bounds__(TPB_PASS, PASS == 3 ? 7 : 8) k_pass(G32 g, Par
   const long long b = blockIdx.x;
   const int bi = (int)(b % g.nbx), bj = (int)((b / g.nbx) % g.nby), bk = (int)(b / ((long long)g.nbx * g.nby));
   const int c0x = 4 * bi, c0y = 4 * bj, c0z = 4 * bk;
+  const int32_t brick = pk(c0x, c0y, c0z);
+  // a brick at the grid's faces: a step of one cell may wrap or leave there
+  const bool rim = bi == 0 || bj == 0 || bk == 0 || bi == g.nbx - 1 || bj == g.nby - 1 || bk == g.nbz - 1;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (PASS != 1) {
     for (int t = threadIdx.x; t < TNODES_IN; t += blockDim.x) {
@@ -399,25 +424,27 @@ __global__ void __launch_bounds__(TPB_PASS, PASS == 3 ? 7 : 8) k_pass(G32 g, Par
     const int32_t c = mine ? s_c[u][threadIdx.x] : CELL_DEAD;
     bool live = c >= 0;  // outside the range, or removed
     if (PASS == 3 && dirrank && !live && mine) dirrank[l] = DR_DEAD;
+    if (live && (c & ~(pk(3, 3, 3) | CELL_FRESH)) != brick) {  // not sorted
+      set_err(err, KERR_MOVE);
+      if (PASS == 3 && dirrank) dirrank[l] = DR_BAD;
+      live = false;
+    }
     int t0 = -1;
-    int t0o = -1;       // P3: tile index of the cell before the move
-    bool mover = false;  // P3: deposits in another cell than its own
-    int grp = -1;  // P3: local key * NDIR + direction for the sort, -1 when not sorted
-    bool far_ion = false;  // P3: moved more than one cell: placed through the far list
-    float w8[8], qdv[4];
+    int t0o = -1;        // P3: tile index of the cell before the move
+    int dir = 0, grp = -1;  // P3: the sort's direction; local key * NDIR + dir, -1 when not sorted
+    float ox = 0.f, oy = 0.f, oz = 0.f;
+    float qdv[4] = {};
     if (live) {
-      const bool fresh = (c & CELL_FRESH) != 0;
-      int ci = pk_i(c), cj = pk_j(c), ck = pk_k(c);
-      const int kl = (ci & 3) + 4 * (cj & 3) + 16 * (ck & 3);  // local key: the particle is in its key's cell
-      float ox = s_f[u][0][threadIdx.x], oy = s_f[u][1][threadIdx.x], oz = s_f[u][2][threadIdx.x];
+      const int bx4 = pk_i(c) & 3, by4 = pk_j(c) & 3, bz4 = pk_k(c) & 3;  // the ion's cell within the brick
+      ox = s_f[u][0][threadIdx.x]; oy = s_f[u][1][threadIdx.x]; oz = s_f[u][2][threadIdx.x];
       float vx = s_f[u][3][threadIdx.x], vy = s_f[u][4][threadIdx.x], vz = s_f[u][5][threadIdx.x];
       int s = p.sp ? min((int)s_s[u][threadIdx.x], MAX_SPECIES - 1) : 0;
       float mr = sp.mrat[s], qw = sp.qw[s];
       float dvx = 0.f, dvy = 0.f, dvz = 0.f;  // velocity deposited
-      int rx = ci - c0x, ry = cj - c0y, rz = ck - c0z;
-      if (PASS == 3) t0o = (rx + 1) + TN * ((ry + 1) + TN * (rz + 1));
+      t0 = (bx4 + O) + T * ((by4 + O) + T * (bz4 + O));
+      t0o = t0;
       if (PASS == 1) {
-        if (fresh) p.cell[l] = c & ~CELL_FRESH;
+        if (c & CELL_FRESH) p.cell[l] = c & ~CELL_FRESH;
         // extrapol_up (gutsp.f:144)
         dvx = extrapolated(vx, s_f[u][PASS == 1 ? 6 : 0][threadIdx.x]);
         dvy = extrapolated(vy, s_f[u][PASS == 1 ? 7 : 0][threadIdx.x]);
@@ -425,10 +452,7 @@ __global__ void __launch_bounds__(TPB_PASS, PASS == 3 ? 7 : 8) k_pass(G32 g, Par
       } else {
         // trilinear gather of (ajc-upc, btc) at the 8 corners (gutsp.f:217-251)
         const float wxl = 1.0f - ox, wxu = ox, wyl = 1.0f - oy, wyu = oy, wzl = 1.0f - oz, wzu = oz;
-        // (the ion lies in its key's cell; clamped so that a broken sort
-        // cannot index outside the tile: the checks below report it)
-        const int gx = min(max(rx, 0), 3), gy = min(max(ry, 0), 3), gz = min(max(rz, 0), 3);
-        const int tg = gx + TN_IN * (gy + TN_IN * gz);
+        const int tg = bx4 + TN_IN * (by4 + TN_IN * bz4);
         float ax = 0, ay = 0, az = 0, bx = 0, by = 0, bz = 0, qx = 0, qy = 0, qz = 0;
 #pragma unroll
         for (int cz = 0; cz < 2; ++cz)
@@ -476,31 +500,50 @@ __global__ void __launch_bounds__(TPB_PASS, PASS == 3 ? 7 : 8) k_pass(G32 g, Par
           // move_ion_half of maind.f:408 (gutsp.f:473-510): the deposit position
           const float mvx = vx * hdt * g.inv_dx, mvy = vy * hdt * g.inv_dy, mvz = vz * hdt * g.inv_dz;
           bool ok = true;
-          const int kx = half_step<true>(ox, mvx, g.ncx, ok), ky = half_step<false>(oy, mvy, g.ncy, ok),
-                    kz = half_step<true>(oz, mvz, g.ncz, ok);
-          const int cx1 = ci + kx, cy1 = cj + ky, cz1 = ck + kz;  // not wrapped
-          const bool out1 = sprm.x_open && (cx1 < 0 || cx1 >= g.ncx);  // outflow through an open x face
-          rx += kx; ry += ky; rz += kz;
+          const float kx = half_step<true>(ox, mvx, g.ncx, ok), ky = half_step<false>(oy, mvy, g.ncy, ok),
+                      kz = half_step<true>(oz, mvz, g.ncz, ok);
           const float dox = ox, doy = oy, doz = oz;
           // move_ion_half of maind.f:479: the stored position
-          const int lx = half_step<true>(ox, mvx, g.ncx, ok), ly = half_step<false>(oy, mvy, g.ncy, ok),
-                    lz = half_step<true>(oz, mvz, g.ncz, ok);
+          const float lx = half_step<true>(ox, mvx, g.ncx, ok), ly = half_step<false>(oy, mvy, g.ncy, ok),
+                      lz = half_step<true>(oz, mvz, g.ncz, ok);
           if (!ok) set_err(err, KERR_MOVE);
-          const bool out2 = out1 || (sprm.x_open && (cx1 + lx < 0 || cx1 + lx >= g.ncx));
-          // steps from the ion's own cell, for the sort; one wrap brings a
-          // near ion's cell home, a far one's takes one per half move
-          const int sx = kx + lx, sy = ky + ly, sz = kz + lz;
-          const bool near = (unsigned)(sx + 1) <= 2u && (unsigned)(sy + 1) <= 2u && (unsigned)(sz + 1) <= 2u;
-          int ci2 = near ? ci + sx : wrapi(cx1, g.ncx) + lx, cj2 = near ? cj + sy : wrapi(cy1, g.ncy) + ly,
-              ck2 = near ? ck + sz : wrapi(cz1, g.ncz) + lz;
-          ci2 = wrapi(ci2, g.ncx);
-          cj2 = wrapi(cj2, g.ncy);
-          ck2 = wrapi(ck2, g.ncz);
+          // steps from the ion's own cell, of at most one cell per axis for a
+          // near ion: the tile index, the sort's direction and the new cell
+          // word are whole numbers below 2^22 and come straight from floats
+          const float sx = kx + lx, sy = ky + ly, sz = kz + lz;
+          const bool near = fabsf(kx) <= 1.f && fabsf(ky) <= 1.f && fabsf(kz) <= 1.f && fabsf(sx) <= 1.f &&
+                            fabsf(sy) <= 1.f && fabsf(sz) <= 1.f;
+          t0 += float_int(fmaf((float)(T * T), kz, fmaf((float)T, ky, kx + FLOAT_INT)));
+          dir = float_int(fmaf(9.f, sz, fmaf(3.f, sy, sx + (FLOAT_INT + 13.f))));
+          int32_t c2 = (c & ~CELL_FRESH) + float_int(fmaf(1048576.f, sz, fmaf(1024.f, sy, sx + FLOAT_INT)));
+          bool out1 = false, out2 = false;
+          bool far_ion = false;  // moved more than one cell: placed through the far list
+          if (rim || !near) {
+            const int ix = (int)kx, iy = (int)ky, iz = (int)kz;
+            int cx1 = pk_i(c) + ix, cy1 = pk_j(c) + iy, cz1 = pk_k(c) + iz;  // not wrapped
+            const int cx2 = cx1 + (int)lx;
+            // outflow through an open x face
+            out1 = sprm.x_open && (cx1 < 0 || cx1 >= g.ncx);
+            out2 = out1 || (sprm.x_open && (cx2 < 0 || cx2 >= g.ncx));
+            // one wrap brings a near ion's cell home, a far one's takes one
+            // per half move
+            const int ci2 = wrapi(near ? cx2 : wrapi(cx1, g.ncx) + (int)lx, g.ncx),
+                      cj2 = wrapi(near ? cy1 + (int)ly : wrapi(cy1, g.ncy) + (int)ly, g.ncy),
+                      ck2 = wrapi(near ? cz1 + (int)lz : wrapi(cz1, g.ncz) + (int)lz, g.ncz);
+            c2 = pk(ci2, cj2, ck2);
+            if (!near) {
+              const int rx = bx4 + ix, ry = by4 + iy, rz = bz4 + iz;
+              const bool inside = rx >= -1 && rx <= 4 && ry >= -1 && ry <= 4 && rz >= -1 && rz <= 4;
+              t0 = inside ? (rx + O) + T * ((ry + O) + T * (rz + O)) : -1;
+              // a deposit position outside the tile's window takes the far path too
+              far_ion = !out2 || (!out1 && !inside);
+            }
+          }
           if (CHEX && !out2 && sprm.heavy_of[s] != s) {
             // res_chex (chem_rates.f:823-840) at the end of the step, FP32
-            const float x = (float)g.qx1 + ((float)ci2 + ox) * g.dx - sprm.cloud_x;
-            const float y = (float)g.qy1 + ((float)cj2 + oy) * g.dy - sprm.cloud_y;
-            const float z = (float)g.qz1 + ((float)ck2 + oz) * g.dz - sprm.cloud_z;
+            const float x = (float)g.qx1 + ((float)pk_i(c2) + ox) * g.dx - sprm.cloud_x;
+            const float y = (float)g.qy1 + ((float)pk_j(c2) + oy) * g.dy - sprm.cloud_y;
+            const float z = (float)g.qz1 + ((float)pk_k(c2) + oz) * g.dz - sprm.cloud_z;
             const float vrel = sqrtf(vx * vx + vy * vy + vz * vz);
             const float sigma = vrel > 0.f ? sprm.cx_a - sprm.cx_b * logf(vrel) : 0.f;
             if (sigma > 0.f) {
@@ -521,20 +564,18 @@ __global__ void __launch_bounds__(TPB_PASS, PASS == 3 ? 7 : 8) k_pass(G32 g, Par
             p.cell[l] = CELL_DEAD;
             if (dirrank) dirrank[l] = DR_DEAD;
           } else {
-            p.cell[l] = pk(ci2, cj2, ck2);
+            p.cell[l] = c2;
             p.ox[l] = ox; p.oy[l] = oy; p.oz[l] = oz;
-            if (near) grp = kl * NDIR + dir_index(sx, sy, sz);
-            else far_ion = true;
+            if (near) grp = (bx4 + 4 * by4 + 16 * bz4) * NDIR + dir;
           }
           ox = dox; oy = doy; oz = doz;  // the deposit uses the maind.f:408 position
           if (out1) live = false;
-          // a deposit position outside the tile's window also takes the far path
-          if (live && (rx < -1 || rx > 4 || ry < -1 || ry > 4 || rz < -1 || rz > 4)) far_ion = true;
           if (far_ion) {
+            const int cx1 = pk_i(c) + (int)kx, cy1 = pk_j(c) + (int)ky, cz1 = pk_k(c) + (int)kz;
             const int slot = far.n ? atomicAdd(far.n, 1) : FAR_CAP;
             if (slot < FAR_CAP) {
               far.idx[slot] = l;
-              far.key[slot] = out2 ? -1LL : key_of(g, ci2, cj2, ck2);
+              far.key[slot] = out2 ? -1LL : key_of(g, pk_i(c2), pk_j(c2), pk_k(c2));
               far.dcell[slot] = live ? pk(wrapi(cx1, g.ncx), wrapi(cy1, g.ncy), wrapi(cz1, g.ncz)) : -1;
               far.o[slot] = ox; far.o[FAR_CAP + slot] = oy; far.o[2 * FAR_CAP + slot] = oz;
               far.q[slot] = qw; far.q[FAR_CAP + slot] = qw * dvx;
@@ -550,25 +591,18 @@ __global__ void __launch_bounds__(TPB_PASS, PASS == 3 ? 7 : 8) k_pass(G32 g, Par
           }
         }
       }
-      const bool inside = PASS == 3 ? !(rx < -1 || rx > 4 || ry < -1 || ry > 4 || rz < -1 || rz > 4)
-                                    : !(rx < 0 || rx > 3 || ry < 0 || ry > 3 || rz < 0 || rz > 3);
-      if (live && !inside) {
-        set_err(err, KERR_MOVE);
-        live = false;
-      }
       if (live) {
-        t0 = (rx + O) + T * ((ry + O) + T * (rz + O));
-        mover = PASS == 3 && t0 != t0o;
-        const float wxl = 1.0f - ox, wxu = ox, wyl = 1.0f - oy, wyu = oy, wzl = 1.0f - oz, wzu = oz;
-#pragma unroll
-        for (int cc = 0; cc < 8; ++cc)
-          w8[cc] = ((cc & 1) ? wxu : wxl) * (((cc >> 1) & 1) ? wyu : wyl) * ((cc >> 2) ? wzu : wzl);
         qdv[0] = qw;
         qdv[1] = qw * dvx;
         qdv[2] = qw * dvy;
         qdv[3] = qw * dvz;
       }
     }
+    // an ion that deposits nothing: moments zero, no tile index
+    if (!live) t0 = -1;
+    const bool mover = PASS == 3 && t0 != t0o;  // deposits in another cell than its own
+    float w8[8];
+    corner_weights(ox, oy, oz, w8);
     if (__any_sync(0xffffffffu, live))  // (a brick's last chunk seldom fills its warps)
       warp_deposit<PASS != 2, T, PASS == 3, EXACT>(s_red[warp], live, t0, w8, qdv, s_dep, bad, lane, t0o, mover);
     if (PASS == 3 && dirrank) {
@@ -581,7 +615,7 @@ __global__ void __launch_bounds__(TPB_PASS, PASS == 3 ? 7 : 8) k_pass(G32 g, Par
           const unsigned before = grp >= 0 ? s_rank[grp] : 0u;
           __syncwarp();
           if (grp >= 0) {
-            dirrank[l] = ((uint32_t)(grp % NDIR) << 26) | (before + __popc(lt));
+            dirrank[l] = ((uint32_t)dir << 26) | (before + __popc(lt));
             if (lt == 0) s_rank[grp] = (uint16_t)(before + __popc(peers));
           }
         }
@@ -624,7 +658,7 @@ __global__ void __launch_bounds__(TPB_PASS, 8) k_pass1_sort(G32 g, Part s, Part 
   __shared__ __align__(16) float s_red[TPB_PASS / 32][12][36];
   const long long b = blockIdx.x;
   const int bi = (int)(b % g.nbx), bj = (int)((b / g.nbx) % g.nby), bk = (int)(b / ((long long)g.nbx * g.nby));
-  const int c0x = 4 * bi, c0y = 4 * bj, c0z = 4 * bk;
+  const int32_t brick = pk(4 * bi, 4 * bj, 4 * bk);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int t = tid; t < (EXACT ? 2 : 1) * 4 * TNOD; t += TPB_PASS) s_dep[t] = 0u;
   __syncthreads();
@@ -662,9 +696,10 @@ __global__ void __launch_bounds__(TPB_PASS, 8) k_pass1_sort(G32 g, Part s, Part 
     const int32_t c = q0 != NONE ? __float_as_int(s_f[u][0][tid]) & ~CELL_FRESH : CELL_DEAD;
     bool live = q0 != NONE;
     int t0 = -1;
-    float w8[8], qdv[4];
+    float ox = 0.f, oy = 0.f, oz = 0.f;
+    float qdv[4] = {};
     if (live) {
-      const float ox = s_f[u][1][tid], oy = s_f[u][2][tid], oz = s_f[u][3][tid];
+      ox = s_f[u][1][tid]; oy = s_f[u][2][tid]; oz = s_f[u][3][tid];
       const float vx = s_f[u][4][tid], vy = s_f[u][5][tid], vz = s_f[u][6][tid];
       const float wx = s_f[u][7][tid], wy = s_f[u][8][tid], wz = s_f[u][9][tid];
       d.cell[l] = c;
@@ -673,16 +708,11 @@ __global__ void __launch_bounds__(TPB_PASS, 8) k_pass1_sort(G32 g, Part s, Part 
       d.wx[l] = wx; d.wy[l] = wy; d.wz[l] = wz;
       d.sp[l] = (uint8_t)sp0;
       const float qw = sp.qw[min(sp0, MAX_SPECIES - 1)];
-      const int rx = pk_i(c) - c0x, ry = pk_j(c) - c0y, rz = pk_k(c) - c0z;
-      if (rx < 0 || rx > 3 || ry < 0 || ry > 3 || rz < 0 || rz > 3) {
+      if ((c & ~pk(3, 3, 3)) != brick) {  // not sorted
         set_err(err, KERR_MOVE);
         live = false;
       } else {
-        t0 = rx + T * (ry + T * rz);
-        const float wxl = 1.0f - ox, wxu = ox, wyl = 1.0f - oy, wyu = oy, wzl = 1.0f - oz, wzu = oz;
-#pragma unroll
-        for (int cc = 0; cc < 8; ++cc)
-          w8[cc] = ((cc & 1) ? wxu : wxl) * (((cc >> 1) & 1) ? wyu : wyl) * ((cc >> 2) ? wzu : wzl);
+        t0 = (pk_i(c) & 3) + T * ((pk_j(c) & 3) + T * (pk_k(c) & 3));
         // extrapol_up (gutsp.f:144)
         qdv[0] = qw;
         qdv[1] = qw * extrapolated(vx, wx);
@@ -690,6 +720,8 @@ __global__ void __launch_bounds__(TPB_PASS, 8) k_pass1_sort(G32 g, Part s, Part 
         qdv[3] = qw * extrapolated(vz, wz);
       }
     }
+    float w8[8];
+    corner_weights(ox, oy, oz, w8);
     if (__any_sync(0xffffffffu, live))
       warp_deposit<true, T, false, EXACT>(s_red[warp], live, t0, w8, qdv, s_dep, bad, lane);
     if (EXACT && (kc + 1) % CARRY_CHUNKS == 0 && kc + 1 < nchunk) carry_tile<TNOD>(s_dep);
