@@ -809,6 +809,11 @@ __device__ __forceinline__ float gpe_face(const G32& g, const float* np, float g
 
 constexpr int FBX = 32, FBY = 4;
 
+// Bring `bytes` (a multiple of 16) from the 16-byte boundary at or below p to L2.
+__device__ __forceinline__ void prefetch_l2(const float* p, unsigned bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"((unsigned long long)p & ~15ull), "r"(bytes));
+}
+
 #define FIELD_NODE(i, j, k)                                   \
   const int i = blockIdx.x * FBX + threadIdx.x + 2;          \
   const int j = blockIdx.y * FBY + threadIdx.y + 2;          \
@@ -1183,8 +1188,26 @@ __global__ void __launch_bounds__(FBX * FBY) k_bstep(G32 g, const float* __restr
                                                      float* __restrict__ oh, float* __restrict__ ol,
                                                      float* __restrict__ dbo, const float* __restrict__ db1,
                                                      float* __restrict__ dbtp1, float* __restrict__ E,
-                                                     float* __restrict__ e_acc) {
+                                                     float* __restrict__ e_acc, int ahead) {
   FIELD_NODE(i, j, k);
+  // grids that do not fit L2 (ahead > 0): one thread per row asks for the row
+  // that the blocks after the resident ones will read, `ahead` planes up
+  // (whole rows, from the 16-byte boundary below; within the arrays, whose
+  // last plane holds ghosts).  The resident warps' own loads leave HBM idle
+  // while they compute and store: 256x128x128 cells, us per launch, predictor
+  // 74.0 -> 63.5, corrector 79.8 -> 75.6
+  if (blockIdx.x == 0 && threadIdx.x == 0 && ahead && k + ahead <= g.ncz + 1) {
+    const unsigned t = (unsigned)nid(g, i, j, k + ahead), nb = (g.ncx * 4 + 16) & ~15;
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      prefetch_l2(ct + t + g.C * m, nb);
+      prefetch_l2(aj + t + g.C * m, nb);
+      prefetch_l2(bh + t + g.C * m, nb);
+      prefetch_l2(bl + t + g.C * m, nb);
+      if (PRED) prefetch_l2(db1 + t + g.C * m, nb);
+    }
+    prefetch_l2(nu + t, nb);
+  }
   bstep_node<PRED, WRITE_E>(g, ct, nu, aj, gpf, bh, bl, ch, cl, b0c, oh, ol, dbo, db1, dbtp1, E, e_acc, i, j, k);
 }
 
@@ -2039,18 +2062,20 @@ cudaError_t b_step(const G32& g, bool pred, bool write_e, const float* ct, const
                    const float* gpf, const float* bh, const float* bl, double coef, const float* b0c, float* oh,
                    float* ol, float* dbo, const float* db1, float* dbtp1, float* E, float* e_acc, cudaStream_t st) {
   const dim3 grid((g.ncx + FBX - 1) / FBX, (g.ncy + FBY - 1) / FBY, g.ncz), blk(FBX, FBY);
+  // the planes that the resident blocks (about 200k nodes) run ahead; see k_bstep
+  const int plane = g.ncx * g.ncy, ahead = n_int(g) >= B_AHEAD_NODES ? (200000 + plane / 2) / plane + (plane > 400000) : 0;
   const float ch = (float)coef, cl = (float)(coef - (double)ch);
   if (pred && write_e)
     RET((k_bstep<true, true><<<grid, blk, 0, st>>>(g, ct, nu, aj, gpf, bh, bl, ch, cl, b0c, oh, ol, dbo, db1, dbtp1, E,
-                                                   e_acc)));
+                                                   e_acc, ahead)));
   if (pred)
     RET((k_bstep<true, false><<<grid, blk, 0, st>>>(g, ct, nu, aj, gpf, bh, bl, ch, cl, b0c, oh, ol, dbo, db1, dbtp1, E,
-                                                    e_acc)));
+                                                    e_acc, ahead)));
   if (write_e)
     RET((k_bstep<false, true><<<grid, blk, 0, st>>>(g, ct, nu, aj, gpf, bh, bl, ch, cl, b0c, oh, ol, dbo, db1, dbtp1, E,
-                                                    e_acc)));
+                                                    e_acc, ahead)));
   RET((k_bstep<false, false><<<grid, blk, 0, st>>>(g, ct, nu, aj, gpf, bh, bl, ch, cl, b0c, oh, ol, dbo, db1, dbtp1, E,
-                                                   e_acc)));
+                                                   e_acc, ahead)));
 }
 bool field_loop_fits(const G32& g) { return n_int(g) <= FIELD_LOOP_NODES; }
 
