@@ -159,7 +159,7 @@ __device__ __forceinline__ int dir_index(int dx, int dy, int dz) { return (dx + 
 // an ion adds at most once per node, so every CARRY_CHUNKS chunks of a brick
 // the low words carry into the high words and any number of ions fits.
 // Otherwise (plain): FP32 atomics, whose result depends on the order.
-constexpr double FIX_INV = 1.0 / 4294967296.0;  // 2^-32
+constexpr float FIX_INV = 1.0f / 4294967296.0f;  // 2^-32
 constexpr float FIX_MAX = 32768.0f;             // 2^15
 constexpr int CARRY_CHUNKS = 256;               // 32768 ions: the low words stay below 2^32
 
@@ -777,7 +777,10 @@ __global__ void k_node_sum(G32 g, const void* __restrict__ partial, float* __res
       // (plain form: the order of the tiles is x outermost)
 #pragma unroll
       for (int r = 1; r < 8; ++r) s += v[(r >> 2 & 1) | (r & 2) | (r & 1) << 2][q];
-      acc[q] = EXACT ? (float)((double)s * FIX_INV) : (float)s;  // exact: the one rounding of the sum
+      // exact: the one rounding of the sum, from the 64-bit integer (by way of
+      // double the FP64 pipe bound it; 1M nodes, mean of a step's three sums:
+      // 37.4 -> 33.5 us)
+      acc[q] = EXACT ? __ll2float_rn((long long)s) * FIX_INV : (float)s;
     }
     const long long o = nid(g, i, j, k);
     if (NQ == 4) store_img(g, np, i, j, k, acc[0]);  // np with its ghost images
