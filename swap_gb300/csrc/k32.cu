@@ -4,6 +4,7 @@
 #include <type_traits>
 
 #include "grid_loop.cuh"
+#include "launch_next.cuh"
 #include "k32.cuh"
 #include "philox.h"
 #include "swap_dev.cuh"
@@ -744,7 +745,8 @@ __global__ void __launch_bounds__(TPB_PASS, 8) k_pass1_sort(G32 g, Part s, Part 
 // before the first is added: a loop over the tiles that are there left one
 // load in flight per node (256x128x128 cells, ms per step: 0.57 -> 0.36).
 template <int T, int NQ, bool EXACT>
-__global__ void k_node_sum(G32 g, const void* __restrict__ partial, float* __restrict__ np, float* __restrict__ S) {
+__global__ void k_node_sum(G32 g, const void* partial, float* np, float* S) {
+  swapk::after_previous();
   constexpr int O = T == TN ? 1 : 0, TNOD = T * T * T;
   using V = typename std::conditional<EXACT, long long, float>::type;
   GSTRIDE(t, n_int(g)) {
@@ -908,10 +910,11 @@ __device__ __forceinline__ float ct_of(float s, float n) { return n == 0.0f ? 0.
 // the whistler Courant time of check_time_step (gutsf.f:1782-1792) per node,
 // ghosts included, with its smallest value.  look[0]: that value (set large
 // before); look[1]: the error word as it stands (see field_loop).
-__global__ void __launch_bounds__(TPB) k_up_courant(G32 g, const float* __restrict__ np, const float* __restrict__ S,
-                                                    const float* __restrict__ db, const float* __restrict__ b0c,
-                                                    float alpha, float dx, float* __restrict__ up,
-                                                    float* __restrict__ dtn, unsigned* look, const int* err) {
+__global__ void __launch_bounds__(TPB) k_up_courant(G32 g, const float* np, const float* S,
+                                                    const float* db, const float* b0c,
+                                                    float alpha, float dx, float* up,
+                                                    float* dtn, unsigned* look, const int* err) {
+  swapk::after_previous();
   float mn = 3.0e38f;
   if (blockIdx.x == 0 && threadIdx.x == 0) look[1] = (unsigned)*err;
   GSTRIDE(t, n_int(g)) {
@@ -960,10 +963,11 @@ __global__ void __launch_bounds__(TPB) k_up_courant(G32 g, const float* __restri
 // kitg (may be null): the pressure gradient centred like aj, for get_Ep.
 // Thread 0 also resets the far list's count and the Courant word, which the
 // rest of the step writes.
-__global__ void __launch_bounds__(TPB) k_kit(G32 g, const float* __restrict__ S, const float* __restrict__ db,
-                                             const float* __restrict__ b0c, const float* __restrict__ np, float alpha,
-                                             float gp, float4* __restrict__ kit, float4* __restrict__ kitg, int* far_n,
+__global__ void __launch_bounds__(TPB) k_kit(G32 g, const float* S, const float* db,
+                                             const float* b0c, const float* np, float alpha,
+                                             float gp, float4* kit, float4* kitg, int* far_n,
                                              unsigned* look) {
+  swapk::after_previous();
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *far_n = 0;
     look[0] = 0x7f7fffffu;  // FLT_MAX
@@ -1065,10 +1069,11 @@ __device__ __forceinline__ void aj_ct_node(const G32& g, const float* db, const 
 }
 
 template <bool CORR>
-__global__ void __launch_bounds__(FBX * FBY) k_aj_ct(G32 g, const float* __restrict__ db,
-                                                     const float* __restrict__ np, const float* __restrict__ up,
-                                                     const float* __restrict__ b0c, float alpha,
-                                                     float* __restrict__ aj, float* __restrict__ ct) {
+__global__ void __launch_bounds__(FBX * FBY) k_aj_ct(G32 g, const float* db,
+                                                     const float* np, const float* up,
+                                                     const float* b0c, float alpha,
+                                                     float* aj, float* ct) {
+  swapk::after_previous();
   FIELD_NODE(i, j, k);
   aj_ct_node<CORR>(g, db, np, up, b0c, alpha, aj, ct, i, j, k);
 }
@@ -1183,15 +1188,16 @@ __device__ __forceinline__ void bstep_node(const G32& g, const float* ct, const 
 }
 
 template <bool PRED, bool WRITE_E>
-__global__ void __launch_bounds__(FBX * FBY) k_bstep(G32 g, const float* __restrict__ ct,
-                                                     const float* __restrict__ nu, const float* __restrict__ aj,
-                                                     const float* __restrict__ gpf,
-                                                     const float* __restrict__ bh, const float* __restrict__ bl,
-                                                     float ch, float cl, const float* __restrict__ b0c,
-                                                     float* __restrict__ oh, float* __restrict__ ol,
-                                                     float* __restrict__ dbo, const float* __restrict__ db1,
-                                                     float* __restrict__ dbtp1, float* __restrict__ E,
-                                                     float* __restrict__ e_acc, int ahead) {
+__global__ void __launch_bounds__(FBX * FBY) k_bstep(G32 g, const float* ct,
+                                                     const float* nu, const float* aj,
+                                                     const float* gpf,
+                                                     const float* bh, const float* bl,
+                                                     float ch, float cl, const float* b0c,
+                                                     float* oh, float* ol,
+                                                     float* dbo, const float* db1,
+                                                     float* dbtp1, float* E,
+                                                     float* e_acc, int ahead) {
+  swapk::after_previous();
   FIELD_NODE(i, j, k);
   // grids that do not fit L2 (ahead > 0): one thread per row asks for the row
   // that the blocks after the resident ones will read, `ahead` planes up
@@ -1224,10 +1230,11 @@ __global__ void __launch_bounds__(FBX * FBY) k_bstep(G32 g, const float* __restr
 // meet at the hardware's cluster barrier (0.24 us) -- up to FIELD_CLUSTER *
 // LOOP_TPB nodes.  Otherwise a cooperative launch with a counter in memory
 // (1.2 us at 152 blocks; grid_loop.cuh).
-// A step of 8 ions per cell, loop against launches, in ms: 1.5k nodes 0.183
-// against 0.325, 33k 0.244 against 0.342, 65k 0.272 against 0.408, 131k 0.449
-// against 0.454, 262k 0.726 against 0.682 (one block per SM then hides less
-// latency than full occupancy does): hence FIELD_LOOP_NODES.
+// A step of 4 ions per cell, loop against launches, in ms: 33k nodes 0.218
+// against 0.229, 65k 0.245 against 0.258, 78k 0.267 against 0.279, 98k 0.331
+// against 0.300, 131k 0.375 against 0.351 (a second round of nodes per thread
+// costs more than the launches, which overlap: launch_next.cuh): hence
+// FIELD_LOOP_NODES.
 constexpr int LOOP_TPB = 512;
 
 template <bool CLUSTER>
@@ -1283,48 +1290,58 @@ __global__ void __launch_bounds__(LOOP_TPB, 1) k_field_loop(G32 g, FieldLoop f) 
 
 // B_new = base - coef * curl E for a given E (with ghost images), in
 // double-float, with its FP32 dB: the field advance of the surrogate, whose
-// discrete curl keeps div B where it was.
-__global__ void __launch_bounds__(FBX * FBY) k_bstep_given_e(G32 g, const float* __restrict__ E,
-                                                             const float* __restrict__ bh,
-                                                             const float* __restrict__ bl, float ch, float cl,
-                                                             const float* __restrict__ b0c, float* __restrict__ oh,
-                                                             float* __restrict__ ol, float* __restrict__ dbo) {
+// discrete curl keeps div B where it was.  th (may be null): also the B one
+// subcycle before the end of the step, B_new + f * (base - B_new) on hi parts,
+// lo of B_new kept (the predictor's leapfrog base of the next plain subcycle).
+__global__ void __launch_bounds__(FBX * FBY) k_bstep_given_e(G32 g, const float* E, const float* bh, const float* bl,
+                                                             float ch, float cl, const float* b0c, float* oh,
+                                                             float* ol, float* dbo, float f, float* th, float* tl) {
+  swapk::after_previous();
   FIELD_NODE(i, j, k);
-  const long long C = g.C, o = nid(g, i, j, k), sx = 1, sy = g.nx, sz = (long long)g.nx * g.ny;
-  const float* E1 = E;
-  const float* E2 = E + C;
-  const float* E3 = E + 2 * C;
-  const float ce[3] = {(E3[o + sy] - E3[o]) * g.inv_dy + (E2[o] - E2[o + sz]) * g.inv_dz,
-                       (E3[o] - E3[o + sx]) * g.inv_dx + (E1[o + sz] - E1[o]) * g.inv_dz,
-                       (E1[o] - E1[o + sy]) * g.inv_dy + (E2[o + sx] - E2[o]) * g.inv_dx};
+  const Off d = off_of(g, i, j, k);
+  const long long C = g.C;
+  const unsigned o = (unsigned)nid(g, i, j, k);
+  const float *E1 = E, *E2 = E + C, *E3 = E + 2 * C;
+  const float e1 = E1[o], e2 = E2[o], e3 = E3[o], e1y = E1[o + d.yp], e1z = E1[o + d.zp], e2x = E2[o + d.xp],
+              e2z = E2[o + d.zp], e3x = E3[o + d.xp], e3y = E3[o + d.yp];
+  float h[3], l[3], c0[3];
+#pragma unroll
+  for (int m = 0; m < 3; ++m) {
+    h[m] = bh[o + C * m];
+    l[m] = bl[o + C * m];
+    c0[m] = b0c[m];
+  }
+  const float ce[3] = {(e3y - e3) * g.inv_dy + (e2 - e2z) * g.inv_dz, (e3 - e3x) * g.inv_dx + (e1z - e1) * g.inv_dz,
+                       (e1 - e1y) * g.inv_dy + (e2x - e2) * g.inv_dx};
+  float* out[9];
+  float v[9];
+  float* lerp[6];
+  float w[6];
 #pragma unroll
   for (int m = 0; m < 3; ++m) {
     float rh, rl;
-    df_sub_mul(bh[o + C * m], bl[o + C * m], ch, cl, ce[m], rh, rl);
-    store_img(g, oh + C * m, i, j, k, rh);
-    store_img(g, ol + C * m, i, j, k, rl);
-    store_img(g, dbo + C * m, i, j, k, __fadd_rn(__fsub_rn(rh, b0c[m]), rl));
-  }
-}
-
-// b_out = b_new + f * (b_old - b_new) on hi parts, lo of b_new kept: the B
-// one subcycle before the end of a surrogate step (the predictor's leapfrog
-// base of the next plain subcycle).
-__global__ void __launch_bounds__(FBX * FBY) k_df_lerp(G32 g, const float* __restrict__ nh,
-                                                       const float* __restrict__ nl, const float* __restrict__ oh,
-                                                       float f, float* __restrict__ rh, float* __restrict__ rl) {
-  FIELD_NODE(i, j, k);
-  const long long C = g.C, o = nid(g, i, j, k);
-#pragma unroll
-  for (int m = 0; m < 3; ++m) {
-    const float d = f * (oh[o + C * m] - nh[o + C * m]);
+    df_sub_mul(h[m], l[m], ch, cl, ce[m], rh, rl);
+    out[m] = oh + C * m;
+    v[m] = rh;
+    out[3 + m] = ol + C * m;
+    v[3 + m] = rl;
+    out[6 + m] = dbo + C * m;
+    v[6 + m] = __fadd_rn(__fsub_rn(rh, c0[m]), rl);
     float s, e;
-    two_sum(nh[o + C * m], d, s, e);
-    e = __fadd_rn(e, nl[o + C * m]);
-    const float h = __fadd_rn(s, e);
-    store_img(g, rh + C * m, i, j, k, h);
-    store_img(g, rl + C * m, i, j, k, __fsub_rn(e, __fsub_rn(h, s)));
+    two_sum(rh, f * (h[m] - rh), s, e);
+    e = __fadd_rn(e, rl);
+    lerp[m] = th + C * m;
+    w[m] = __fadd_rn(s, e);
+    lerp[3 + m] = tl + C * m;
+    w[3 + m] = __fsub_rn(e, __fsub_rn(w[m], s));
   }
+#pragma unroll
+  for (int q = 0; q < 9; ++q) out[q][o] = v[q];
+  ghost_images(g, i, j, k, out, v);
+  if (!th) return;
+#pragma unroll
+  for (int q = 0; q < 6; ++q) lerp[q][o] = w[q];
+  ghost_images(g, i, j, k, lerp, w);
 }
 
 // Block sum (thread 0 holds the result; every thread of the block calls it).
@@ -1375,39 +1392,50 @@ __global__ void k_judge(G32 g, const float* __restrict__ ah, const float* __rest
 // [V][SUR_NIN]: B = dB + b0, u_p, n_p, p_e = te * n_p, and E0 = ct + nu aj at
 // the faces (the plain E of get_E from the predictor's aj and ct; zero when
 // ct is null).
-__global__ void k_grid_to_voxels(G32 g, const float* __restrict__ db, const float* __restrict__ b0c,
-                                 const float* __restrict__ up, const float* __restrict__ np, float te,
-                                 const float* __restrict__ ct, const float* __restrict__ aj,
-                                 const float* __restrict__ nu, const float* __restrict__ gpf,
-                                 const float* __restrict__ b1h, const float* __restrict__ b1l,
-                                 const float* __restrict__ b12h, const float* __restrict__ b12l,
-                                 float* __restrict__ out) {
-  GSTRIDE(v, n_int(g)) {
-    int i, j, k;
-    interior_of(g, v, i, j, k);
-    const long long C = g.C, o = nid(g, i, j, k);
-    float* r = out + v * SUR_NIN;
-    r[0] = db[o] + b0c[0];
-    r[1] = db[o + C] + b0c[1];
-    r[2] = db[o + 2 * C] + b0c[2];
-    r[3] = up[o];
-    r[4] = up[o + C];
-    r[5] = up[o + 2 * C];
-    r[6] = np[o];
-    r[7] = te * np[o];
-    r[8] = ct ? e_o<0>(g, ct, nu, aj, gpf, o) : 0.0f;
-    r[9] = ct ? e_o<1>(g, ct, nu, aj, gpf, o) : 0.0f;
-    r[10] = ct ? e_o<2>(g, ct, nu, aj, gpf, o) : 0.0f;
+// A block's voxels go out through shared memory as whole lines: stores of 14
+// floats a thread apart cost 28 us for 262k voxels, these 13.
+__global__ void __launch_bounds__(TPB) k_grid_to_voxels(G32 g, const float* db, const float* b0c, const float* up,
+                                                        const float* np, float te, const float* ct, const float* aj,
+                                                        const float* nu, const float* gpf, const float* b1h,
+                                                        const float* b1l, const float* b12h, const float* b12l,
+                                                        float* out) {
+  __shared__ float s_out[TPB * SUR_NIN];
+  swapk::after_previous();
+  const long long V = n_int(g);
+  for (long long v0 = blockIdx.x * (long long)TPB; v0 < V; v0 += (long long)gridDim.x * TPB) {
+    const long long v = v0 + threadIdx.x;
+    if (v < V) {
+      int i, j, k;
+      interior_of(g, v, i, j, k);
+      const long long C = g.C, o = nid(g, i, j, k);
+      float* r = s_out + threadIdx.x * SUR_NIN;
+      r[0] = db[o] + b0c[0];
+      r[1] = db[o + C] + b0c[1];
+      r[2] = db[o + 2 * C] + b0c[2];
+      r[3] = up[o];
+      r[4] = up[o + C];
+      r[5] = up[o + 2 * C];
+      r[6] = np[o];
+      r[7] = te * np[o];
+      r[8] = ct ? e_o<0>(g, ct, nu, aj, gpf, o) : 0.0f;
+      r[9] = ct ? e_o<1>(g, ct, nu, aj, gpf, o) : 0.0f;
+      r[10] = ct ? e_o<2>(g, ct, nu, aj, gpf, o) : 0.0f;
 #pragma unroll
-    for (int m = 0; m < 3; ++m)
-      r[11 + m] = b12h ? (b1h[o + C * m] - b12h[o + C * m]) + (b1l[o + C * m] - b12l[o + C * m]) : 0.0f;
+      for (int m = 0; m < 3; ++m)
+        r[11 + m] = b12h ? (b1h[o + C * m] - b12h[o + C * m]) + (b1l[o + C * m] - b12l[o + C * m]) : 0.0f;
+    }
+    __syncthreads();
+    const int n = (int)(V - v0 < TPB ? V - v0 : TPB) * SUR_NIN;
+    for (int q = threadIdx.x; q < n; q += TPB) out[v0 * SUR_NIN + q] = s_out[q];
+    __syncthreads();
   }
 }
 
 // E = E0 + the predicted correction ([V][3]) into the field layout with ghost
 // images (E0 from the inputs vin, none when vin is null).
-__global__ void k_voxels_to_grid(G32 g, const float* __restrict__ ev, const float* __restrict__ vin,
-                                 float* __restrict__ E) {
+__global__ void k_voxels_to_grid(G32 g, const float* ev, const float* vin,
+                                 float* E) {
+  swapk::after_previous();
   GSTRIDE(v, n_int(g)) {
     int i, j, k;
     interior_of(g, v, i, j, k);
@@ -2024,23 +2052,23 @@ cudaError_t pass(int which, const G32& g, const Part& p, const Species& sp, cons
 cudaError_t node_sum(const G32& g, int pass, const void* partial, bool exact, float* np, float* S, cudaStream_t st) {
   const unsigned nb = nblk(n_int(g));
   // pass 2 deposits no density
-  if (pass == 3 && exact) RET((k_node_sum<TN, 4, true><<<nb, TPB, 0, st>>>(g, partial, np, S)));
-  if (pass == 3) RET((k_node_sum<TN, 4, false><<<nb, TPB, 0, st>>>(g, partial, np, S)));
-  if (pass == 2 && exact) RET((k_node_sum<TN_IN, 3, true><<<nb, TPB, 0, st>>>(g, partial, np, S)));
-  if (pass == 2) RET((k_node_sum<TN_IN, 3, false><<<nb, TPB, 0, st>>>(g, partial, np, S)));
-  if (exact) RET((k_node_sum<TN_IN, 4, true><<<nb, TPB, 0, st>>>(g, partial, np, S)));
-  RET((k_node_sum<TN_IN, 4, false><<<nb, TPB, 0, st>>>(g, partial, np, S)));
+  if (pass == 3 && exact) return swapk::launch_next(k_node_sum<TN, 4, true>, nb, TPB, st, g, partial, np, S);
+  if (pass == 3) return swapk::launch_next(k_node_sum<TN, 4, false>, nb, TPB, st, g, partial, np, S);
+  if (pass == 2 && exact) return swapk::launch_next(k_node_sum<TN_IN, 3, true>, nb, TPB, st, g, partial, np, S);
+  if (pass == 2) return swapk::launch_next(k_node_sum<TN_IN, 3, false>, nb, TPB, st, g, partial, np, S);
+  if (exact) return swapk::launch_next(k_node_sum<TN_IN, 4, true>, nb, TPB, st, g, partial, np, S);
+  return swapk::launch_next(k_node_sum<TN_IN, 4, false>, nb, TPB, st, g, partial, np, S);
 }
 cudaError_t up_courant(const G32& g, const float* np, const float* S, const float* db, const float* b0c, float alpha,
                        float dx, float* up, float* dtn, float* look, const int* err, cudaStream_t st) {
   const unsigned nb = nblk(n_int(g)) < 152u * 8u ? nblk(n_int(g)) : 152u * 8u;
-  RET((k_up_courant<<<nb, TPB, 0, st>>>(g, np, S, db, b0c, alpha, dx, up, dtn, reinterpret_cast<unsigned*>(look),
-                                        err)));
+  return swapk::launch_next(k_up_courant, nb, TPB, st, g, np, S, db, b0c, alpha, dx, up, dtn,
+                            reinterpret_cast<unsigned*>(look), err);
 }
 cudaError_t build_kit(const G32& g, const float* S, const float* db, const float* b0c, const float* np, float alpha,
                       float gp, float4* kit, float4* kitg, int* far_n, float* look, cudaStream_t st) {
-  RET((k_kit<<<nblk(n_int(g)), TPB, 0, st>>>(g, S, db, b0c, np, alpha, gp, kit, kitg, far_n,
-                                             reinterpret_cast<unsigned*>(look))));
+  return swapk::launch_next(k_kit, nblk(n_int(g)), TPB, st, g, S, db, b0c, np, alpha, gp, kit, kitg, far_n,
+                            reinterpret_cast<unsigned*>(look));
 }
 __global__ void k_gpe(G32 g, const float* __restrict__ np, float gp, float* __restrict__ gpf) {
   GSTRIDE(t, n_int(g)) {
@@ -2058,8 +2086,7 @@ cudaError_t gpe_faces(const G32& g, const float* np, float gp, float* gpf, cudaS
 cudaError_t aj_ct(const G32& g, bool corr, const float* db, const float* np, const float* up, const float* b0c,
                   float alpha, float* aj, float* ct, cudaStream_t st) {
   const dim3 grid((g.ncx + FBX - 1) / FBX, (g.ncy + FBY - 1) / FBY, g.ncz), blk(FBX, FBY);
-  if (corr) RET((k_aj_ct<true><<<grid, blk, 0, st>>>(g, db, np, up, b0c, alpha, aj, ct)));
-  RET((k_aj_ct<false><<<grid, blk, 0, st>>>(g, db, np, up, b0c, alpha, aj, ct)));
+  return swapk::launch_next(corr ? k_aj_ct<true> : k_aj_ct<false>, grid, blk, st, g, db, np, up, b0c, alpha, aj, ct);
 }
 cudaError_t b_step(const G32& g, bool pred, bool write_e, const float* ct, const float* nu, const float* aj,
                    const float* gpf, const float* bh, const float* bl, double coef, const float* b0c, float* oh,
@@ -2068,17 +2095,10 @@ cudaError_t b_step(const G32& g, bool pred, bool write_e, const float* ct, const
   // the planes that the resident blocks (about 200k nodes) run ahead; see k_bstep
   const int plane = g.ncx * g.ncy, ahead = n_int(g) >= B_AHEAD_NODES ? (200000 + plane / 2) / plane + (plane > 400000) : 0;
   const float ch = (float)coef, cl = (float)(coef - (double)ch);
-  if (pred && write_e)
-    RET((k_bstep<true, true><<<grid, blk, 0, st>>>(g, ct, nu, aj, gpf, bh, bl, ch, cl, b0c, oh, ol, dbo, db1, dbtp1, E,
-                                                   e_acc, ahead)));
-  if (pred)
-    RET((k_bstep<true, false><<<grid, blk, 0, st>>>(g, ct, nu, aj, gpf, bh, bl, ch, cl, b0c, oh, ol, dbo, db1, dbtp1, E,
-                                                    e_acc, ahead)));
-  if (write_e)
-    RET((k_bstep<false, true><<<grid, blk, 0, st>>>(g, ct, nu, aj, gpf, bh, bl, ch, cl, b0c, oh, ol, dbo, db1, dbtp1, E,
-                                                    e_acc, ahead)));
-  RET((k_bstep<false, false><<<grid, blk, 0, st>>>(g, ct, nu, aj, gpf, bh, bl, ch, cl, b0c, oh, ol, dbo, db1, dbtp1, E,
-                                                   e_acc, ahead)));
+  const auto k = pred ? (write_e ? k_bstep<true, true> : k_bstep<true, false>)
+                      : (write_e ? k_bstep<false, true> : k_bstep<false, false>);
+  return swapk::launch_next(k, grid, blk, st, g, ct, nu, aj, gpf, bh, bl, ch, cl, b0c, oh, ol, dbo, db1, dbtp1, E,
+                            e_acc, ahead);
 }
 bool field_loop_fits(const G32& g) { return n_int(g) <= FIELD_LOOP_NODES; }
 
@@ -2100,28 +2120,25 @@ cudaError_t field_loop(const G32& g, const FieldLoop& f, cudaStream_t st) {
   G32 gg = g;
   FieldLoop ff = f;
   void* args[] = {&gg, &ff};
-  // about the nodes' even share per SM, a block on each; whole groups of four
-  // warps, so that fewer blocks meet at the barrier
-  const long long n = n_int(g), per = ((n + 151) / 152 + 127) / 128 * 128, t = per < LOOP_TPB ? per : LOOP_TPB;
+  // the nodes evenly over the SMs, a block on each, and over the rounds of
+  // its threads (whole groups of four warps: fewer blocks meet at the barrier)
+  const long long n = n_int(g), per = (n + 151) / 152, rounds = (per + LOOP_TPB - 1) / LOOP_TPB,
+                  t = ((per + rounds - 1) / rounds + 127) / 128 * 128;
   return loop::launch(reinterpret_cast<const void*>(&k_field_loop<false>), (n + t - 1) / t, (int)t, args, st);
 }
 cudaError_t b_step_given_e(const G32& g, const float* E, const float* bh, const float* bl, double coef,
-                           const float* b0c, float* oh, float* ol, float* dbo, cudaStream_t st) {
+                           const float* b0c, float* oh, float* ol, float* dbo, float f, float* th, float* tl,
+                           cudaStream_t st) {
   const dim3 grid((g.ncx + FBX - 1) / FBX, (g.ncy + FBY - 1) / FBY, g.ncz), blk(FBX, FBY);
   const float ch = (float)coef, cl = (float)(coef - (double)ch);
-  RET((k_bstep_given_e<<<grid, blk, 0, st>>>(g, E, bh, bl, ch, cl, b0c, oh, ol, dbo)));
-}
-cudaError_t df_lerp(const G32& g, const float* nh, const float* nl, const float* oh, float f, float* rh, float* rl,
-                    cudaStream_t st) {
-  const dim3 grid((g.ncx + FBX - 1) / FBX, (g.ncy + FBY - 1) / FBY, g.ncz), blk(FBX, FBY);
-  RET((k_df_lerp<<<grid, blk, 0, st>>>(g, nh, nl, oh, f, rh, rl)));
+  return swapk::launch_next(k_bstep_given_e, grid, blk, st, g, E, bh, bl, ch, cl, b0c, oh, ol, dbo, f, th, tl);
 }
 cudaError_t grid_to_voxels(const G32& g, const float* db, const float* b0c, const float* up, const float* np,
                            float te, const float* ct, const float* aj, const float* nu, const float* gpf,
                            const float* b1h, const float* b1l, const float* b12h, const float* b12l, float* out,
                            cudaStream_t st) {
-  RET((k_grid_to_voxels<<<nblk(n_int(g)), TPB, 0, st>>>(g, db, b0c, up, np, te, ct, aj, nu, gpf, b1h, b1l, b12h,
-                                                         b12l, out)));
+  return swapk::launch_next(k_grid_to_voxels, nblk(n_int(g)), TPB, st, g, db, b0c, up, np, te, ct, aj, nu, gpf, b1h, b1l, b12h,
+                                                         b12l, out);
 }
 cudaError_t judge_sums(const G32& g, const float* ah, const float* al, const float* bh, const float* bl,
                        const float* b0c, double* acc3, cudaStream_t st) {
@@ -2131,7 +2148,7 @@ cudaError_t judge_sums(const G32& g, const float* ah, const float* al, const flo
   RET((k_judge<<<nb, TPB, 0, st>>>(g, ah, al, bh, bl, b0c, acc3)));
 }
 cudaError_t voxels_to_grid(const G32& g, const float* ev, const float* vin, float* E, cudaStream_t st) {
-  RET((k_voxels_to_grid<<<nblk(n_int(g)), TPB, 0, st>>>(g, ev, vin, E)));
+  return swapk::launch_next(k_voxels_to_grid, nblk(n_int(g)), TPB, st, g, ev, vin, E);
 }
 cudaError_t grid_e_to_voxels(const G32& g, const float* E, float f, const float* vin, float* ev, cudaStream_t st) {
   RET((k_grid_e_to_voxels<<<nblk(n_int(g)), TPB, 0, st>>>(g, E, f, vin, ev)));
@@ -2150,7 +2167,8 @@ cudaError_t join_df(long long n, const float* h, const float* l, double* a, cuda
 // of its deposit cell's brick, as that tile would hold a run of one ion
 // (fixed point: 64-bit integer adds, exact and order-independent).
 template <bool EXACT>
-__global__ void k_far_deposit(G32 g, FarList f, void* __restrict__ partial, int* err) {
+__global__ void k_far_deposit(G32 g, FarList f, void* partial, int* err) {
+  swapk::after_previous();
   const int n = min(*f.n, FAR_CAP);
   unsigned bad = 0;
   GSTRIDE(i, n) {
@@ -2227,8 +2245,8 @@ __global__ void k_far_scatter(G32 g, FarList f, const int32_t* __restrict__ ncou
 }
 
 cudaError_t far_deposit(const G32& g, const FarList& far, void* partial, bool exact, int* err, cudaStream_t st) {
-  if (exact) RET((k_far_deposit<true><<<64, TPB, 0, st>>>(g, far, partial, err)));
-  RET((k_far_deposit<false><<<64, TPB, 0, st>>>(g, far, partial, err)));
+  if (exact) return swapk::launch_next(k_far_deposit<true>, 64, TPB, st, g, far, partial, err);
+  return swapk::launch_next(k_far_deposit<false>, 64, TPB, st, g, far, partial, err);
 }
 cudaError_t far_count(const FarList& far, int64_t* count, cudaStream_t st) {
   RET((k_far_count<<<64, TPB, 0, st>>>(far, count)));

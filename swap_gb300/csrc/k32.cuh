@@ -210,7 +210,7 @@ cudaError_t b_step(const G32& g, bool pred, bool write_e, const float* ct, const
 // to the buffers that n rounds of the two launchers above would use.  Nothing
 // is done when *failed is set or *courant (the smallest Courant time) <=
 // courant_floor: the caller looks at both.  Neither word may change meanwhile.
-constexpr long long FIELD_LOOP_NODES = 1 << 17;
+constexpr long long FIELD_LOOP_NODES = 152 * 512;  // a node per thread
 constexpr int FIELD_CLUSTER = 8;  // the portable cluster size
 struct FieldLoop {
   int n;
@@ -228,12 +228,11 @@ struct FieldLoop {
 };
 bool field_loop_fits(const G32& g);
 cudaError_t field_loop(const G32& g, const FieldLoop& f, cudaStream_t st);
-// The surrogate's field advance: B_new = base - coef * curl E for a given E.
+// The surrogate's field advance: B_new = base - coef * curl E for a given E;
+// with (th, tl), also r = B_new + f * (base - B_new) (hi parts of base).
 cudaError_t b_step_given_e(const G32& g, const float* E, const float* bh, const float* bl, double coef,
-                           const float* b0c, float* oh, float* ol, float* dbo, cudaStream_t st);
-// r = b_new + f*(b_old - b_new) (double-float, hi parts of b_old).
-cudaError_t df_lerp(const G32& g, const float* nh, const float* nl, const float* oh, float f, float* rh, float* rl,
-                    cudaStream_t st);
+                           const float* b0c, float* oh, float* ol, float* dbo, float f, float* th, float* tl,
+                           cudaStream_t st);
 // Surrogate inputs per interior node, FP32 [V][SUR_NIN]: B, u_p, n_p,
 // te*n_p, E0 = ct + nu aj (zero when ct is null) and B - b12 from the
 // double-float levels (b1h, b1l) and (b12h, b12l) (zero when b12h is null).

@@ -26,6 +26,7 @@
 // device 0.74 -> 0.36 ms (18x11x14: 0.355 -> 0.211 ms).
 #include "k64.cuh"
 #include "grid_loop.cuh"
+#include "launch_next.cuh"
 #include "k64_dev.cuh"
 
 namespace swapk {
@@ -294,9 +295,10 @@ __device__ __forceinline__ void b_node(const Geo& g, const Node& n, const Nbr& d
 // curlB; FILL: b's ghosts too (curlB begins with periodic(b)).  btc (not
 // null): edge_to_center of b at the interior nodes, for the corrector.
 template <int SP>
-__global__ void __launch_bounds__(TPB) k_curlB(Geo g, double* b, const double* __restrict__ np,
-                                               const double* __restrict__ den, double alpha,
-                                               double* __restrict__ aj, double* __restrict__ btc, bool fill) {
+__global__ void __launch_bounds__(TPB) k_curlB(Geo g, double* b, const double* np,
+                                               const double* den, double alpha,
+                                               double* aj, double* btc, bool fill) {
+  after_previous();
   NODES(n, d);
   curlB_node<SP>(g, n, d, b, np, den, alpha, aj);
   if (btc) {
@@ -311,8 +313,9 @@ __global__ void __launch_bounds__(TPB) k_curlB(Geo g, double* b, const double* _
 
 // The divisors of curlB and their reciprocals: once per field step, where each
 // of its 20 curls divided anew (nine operations a quotient).
-__global__ void __launch_bounds__(TPB) k_face_density(Geo g, const double* __restrict__ np, double alpha,
-                                                      double* __restrict__ den) {
+__global__ void __launch_bounds__(TPB) k_face_density(Geo g, const double* np, double alpha,
+                                                      double* den) {
+  after_previous();
   const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (unsigned)n_interior(g)) return;
   const unsigned o = node_of(g, t).o;
@@ -326,32 +329,36 @@ __global__ void __launch_bounds__(TPB) k_face_density(Geo g, const double* __res
 }
 
 template <bool CORR>
-__global__ void __launch_bounds__(TPB) k_ct(Geo g, const double* __restrict__ aj, const double* __restrict__ up,
-                                            double* b, double* __restrict__ ct, bool fill) {
+__global__ void __launch_bounds__(TPB) k_ct(Geo g, const double* aj, const double* up,
+                                            double* b, double* ct, bool fill) {
+  after_previous();
   NODES(n, d);
   ct_node<CORR>(g, n, d, aj, up, b, ct);
   if (fill) fill3(g, n, b);
 }
 
-__global__ void __launch_bounds__(TPB) k_E(Geo g, const double* __restrict__ ct, const double* __restrict__ nu,
-                                           const double* __restrict__ aj, const double* __restrict__ np, double gp,
-                                           double* __restrict__ E) {
+__global__ void __launch_bounds__(TPB) k_E(Geo g, const double* ct, const double* nu,
+                                           const double* aj, const double* np, double gp,
+                                           double* E) {
+  after_previous();
   NODES(n, d);
   e_node(g, n, d, ct, nu, aj, np, gp, E);
 }
 
 template <int SP>
-__global__ void __launch_bounds__(TPB) k_B(Geo g, const double* __restrict__ E, const double* __restrict__ base,
-                                           double coef, double* __restrict__ b1p2, const double* __restrict__ b1,
-                                           double* __restrict__ half) {
+__global__ void __launch_bounds__(TPB) k_B(Geo g, const double* E, const double* base,
+                                           double coef, double* b1p2, const double* b1,
+                                           double* half) {
+  after_previous();
   NODES(n, d);
   b_node<SP>(g, n, d, E, base, coef, b1p2, b1, half);
 }
 
 // 0.5*(a + b) at the interior nodes (gutsf.f:1210-1219); the consumers read
 // ghosts at their images.
-__global__ void __launch_bounds__(TPB) k_half(Geo g, const double* __restrict__ a, const double* __restrict__ b,
-                                              double* __restrict__ out) {
+__global__ void __launch_bounds__(TPB) k_half(Geo g, const double* a, const double* b,
+                                              double* out) {
+  after_previous();
   const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (unsigned)n_interior(g)) return;
   const unsigned o = node_of(g, t).o;
@@ -359,7 +366,8 @@ __global__ void __launch_bounds__(TPB) k_half(Geo g, const double* __restrict__ 
 }
 
 // edge_to_center (grid_interp.f:10-62): bt's and btc's ghosts too.
-__global__ void __launch_bounds__(TPB) k_edge_to_center(Geo g, double* bt, double* __restrict__ btc) {
+__global__ void __launch_bounds__(TPB) k_edge_to_center(Geo g, double* bt, double* btc) {
+  after_previous();
   NODES(n, d);
   double c[3];
   e2c_node(g, n, d, bt, c);
@@ -372,8 +380,9 @@ __global__ void __launch_bounds__(TPB) k_edge_to_center(Geo g, double* bt, doubl
 
 // face_to_center (grid_interp.f:136-176) of v, and of w when given: the
 // ghosts of inputs and outputs too.
-__global__ void __launch_bounds__(TPB) k_face_to_center(Geo g, double* v, double* __restrict__ vc, double* w,
-                                                        double* __restrict__ wc) {
+__global__ void __launch_bounds__(TPB) k_face_to_center(Geo g, double* v, double* vc, double* w,
+                                                        double* wc) {
+  after_previous();
   NODES(n, d);
   const long long C = g.C;
   const unsigned o = n.o;
@@ -395,13 +404,13 @@ __global__ void __launch_bounds__(TPB) k_face_to_center(Geo g, double* v, double
 // The end of update_up (gutsp.f:1825-1839): ct = S/np at the interior (zero
 // where no particle deposits, as in the reference) and its face average, with
 // up's ghosts.
-__device__ __forceinline__ double ct_at(const double* __restrict__ S, const double* __restrict__ np, unsigned o,
-                                        long long cm) {
+__device__ __forceinline__ double ct_at(const double* S, const double* np, unsigned o, long long cm) {
   const double n = np[o];
   return n == 0.0 ? 0.0 : S[o + cm] / n;
 }
-__global__ void __launch_bounds__(TPB) k_up(Geo g, const double* __restrict__ S, double* np,
-                                            double* __restrict__ up, bool fill_np) {
+__global__ void __launch_bounds__(TPB) k_up(Geo g, const double* S, double* np,
+                                            double* up, bool fill_np) {
+  after_previous();
   NODES(n, d);
   const long long C = g.C;
   const unsigned o = n.o;
@@ -420,9 +429,10 @@ __global__ void __launch_bounds__(TPB) k_up(Geo g, const double* __restrict__ S,
 // table keeps it).  FULL also stores btc and fills aj's ghosts, as the
 // operators it stands for do (edge_to_center, get_Ep's face_to_center(aj)).
 template <bool FULL>
-__global__ void __launch_bounds__(TPB) k_kit(Geo g, double* aj, const double* __restrict__ up,
-                                             const double* __restrict__ bt, double* __restrict__ btc,
-                                             double* __restrict__ kit) {
+__global__ void __launch_bounds__(TPB) k_kit(Geo g, double* aj, const double* up,
+                                             const double* bt, double* btc,
+                                             double* kit) {
+  after_previous();
   NODES(n, d);
   const long long C = g.C;
   const unsigned o = n.o;
@@ -459,10 +469,10 @@ __global__ void __launch_bounds__(TPB) k_kit(Geo g, double* aj, const double* __
 // blocks meet at a barrier (1.2 us) instead of in a launch: below
 // FIELD_LOOP_NODES a phase's FP64 work is about as long as a launch and the
 // ramp of its loads.  The same node functions on the same operands: the same
-// bits.  A step of 4 ions per cell, loop against launches, in ms: 960 nodes
-// 0.42 against 0.54, 33k 0.58 against 0.76, 65k 0.84 against 0.98, 131k 1.48
-// against 1.53, 262k 2.63 against 2.54 (16 warps per SM then hide less than a
-// full SM): hence FIELD_LOOP_NODES.
+// bits.  A step of 4 ions per cell, loop against launches, in ms: 33k nodes
+// 0.58 against 0.78, 65k 0.84 against 1.00, 98k 1.17 against 1.26, 131k 1.41
+// against 1.63, 164k 1.74 against 1.76, 262k 2.48 against 2.40 (16 warps per SM
+// then hide less than a full SM): hence FIELD_LOOP_NODES.
 constexpr int LOOP_TPB = 512;
 template <int SP>
 __global__ void __launch_bounds__(LOOP_TPB) k_field_loop(Geo g, FieldLoop64 f) {
@@ -523,15 +533,16 @@ cudaError_t field_loop(const Geo& g, const FieldLoop64& f, cudaStream_t st) {
   const void* k = g.spacing == SPACING_UNIT ? reinterpret_cast<const void*>(&k_field_loop<SPACING_UNIT>)
                   : g.spacing == SPACING_P2 ? reinterpret_cast<const void*>(&k_field_loop<SPACING_P2>)
                                             : reinterpret_cast<const void*>(&k_field_loop<SPACING_ANY>);
-  // the nodes evenly over the SMs, a block on each
-  const long long n = n_interior(g), per = ((n + 151) / 152 + 31) / 32 * 32, t = per < LOOP_TPB ? per : LOOP_TPB;
+  // the nodes evenly over the SMs, a block on each, and over the rounds of
+  // its threads
+  const long long n = n_interior(g), per = (n + 151) / 152, rounds = (per + LOOP_TPB - 1) / LOOP_TPB,
+                  t = ((per + rounds - 1) / rounds + 31) / 32 * 32;
   return loop::launch(k, (n + t - 1) / t, (int)t, args, st);
 }
 
 #define FL(kern, ...)                                                 \
   do {                                                                \
-    kern<<<nblocks(n_interior(g)), threads_for(n_interior(g)), 0, st>>>(__VA_ARGS__);        \
-    return cudaGetLastError();                                        \
+    return launch_next(kern, nblocks(n_interior(g)), threads_for(n_interior(g)), st, __VA_ARGS__); \
   } while (0)
 
 cudaError_t curlB(const Geo& g, double* b, const double* np, const double* den, double alpha, double* aj,

@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/swap_gpu.h"
+#include "launch_next.cuh"
 #include "tc05.cuh"
 
 namespace {
@@ -153,8 +154,27 @@ __device__ __forceinline__ void conv_store(const ConvArgs& a, long long vo, int 
   }
 }
 
+// The weights into the K-major core layout, one B operand (COUT x CIN) per
+// tap: 8 values along CIN are 16 contiguous bytes on both sides (W itself may
+// start anywhere when a caller brings it).
+template <int CIN, int COUT, int THREADS>
+__device__ __forceinline__ void load_weights(const __nv_bfloat16* W, uint8_t* sW) {
+  constexpr int KG = CIN / 8;
+  for (int i = threadIdx.x; i < 27 * COUT * KG; i += THREADS) {
+    const int t = i / (COUT * KG), r = i % (COUT * KG), n = r / KG, k = 8 * (r % KG);
+    uint4 w;
+    if ((reinterpret_cast<uintptr_t>(W) & 15) == 0) {
+      w = reinterpret_cast<const uint4*>(W)[i];
+    } else {
+      for (int e = 0; e < 8; ++e) reinterpret_cast<__nv_bfloat16*>(&w)[e] = W[8 * i + e];
+    }
+    *reinterpret_cast<uint4*>(sW + t * (COUT * CIN * 2) + tc05::core_offset(n, k, COUT)) = w;
+  }
+}
+
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(128) k_conv3(ConvArgs a) {
+  swapk::after_previous();
   static_assert(CIN % 16 == 0 && (COUT == 16 || COUT == 32), "operand shapes");
   constexpr int WBYTES = 27 * COUT * CIN * 2, ABYTES = 128 * CIN * 2;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -164,11 +184,7 @@ __global__ void __launch_bounds__(128) k_conv3(ConvArgs a) {
   __shared__ uint32_t tslot;
   __shared__ float sbias[COUT];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // weights into the K-major core layout, one B operand (COUT x CIN) per tap
-  for (int i = tid; i < 27 * COUT * CIN; i += 128) {
-    const int t = i / (COUT * CIN), r = i % (COUT * CIN), n = r / CIN, k = r % CIN;
-    *reinterpret_cast<__nv_bfloat16*>(sW + t * (COUT * CIN * 2) + tc05::core_offset(n, k, COUT)) = a.W[i];
-  }
+  load_weights<CIN, COUT, 128>(a.W, sW);
   if (tid < COUT) sbias[tid] = a.bias ? a.bias[tid] : 0.0f;
   if (warp == 0) tc05::tmem_alloc(&tslot, 32);
   if (tid == 0) {
@@ -261,6 +277,7 @@ __global__ void __launch_bounds__(128) k_conv3(ConvArgs a) {
 // columns.
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(256) k_conv3r(ConvArgs a, int ychunk) {
+  swapk::after_previous();
   static_assert(CIN % 16 == 0 && (COUT == 16 || COUT == 32), "operand shapes");
   constexpr int KG = CIN / 8;                // channel groups (16 bytes each)
   constexpr int RP = KG == 2 ? 132 : 130;    // rows per plane; the padding spreads the copies over the banks
@@ -275,10 +292,7 @@ __global__ void __launch_bounds__(256) k_conv3r(ConvArgs a, int ychunk) {
   __shared__ uint32_t tslot;
   __shared__ float sbias[COUT];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  for (int i = tid; i < 27 * COUT * CIN; i += 256) {
-    const int t = i / (COUT * CIN), r = i % (COUT * CIN), n = r / CIN, k = r % CIN;
-    *reinterpret_cast<__nv_bfloat16*>(sW + t * (COUT * CIN * 2) + tc05::core_offset(n, k, COUT)) = a.W[i];
-  }
+  load_weights<CIN, COUT, 256>(a.W, sW);
   if (tid < COUT) sbias[tid] = a.bias ? a.bias[tid] : 0.0f;
   if (warp == 0) tc05::tmem_alloc(&tslot, 64);
   if (tid == 0) {
@@ -414,6 +428,7 @@ __global__ void __launch_bounds__(256) k_conv3r(ConvArgs a, int ychunk) {
 // multiplied in the same order as in the other forms: the same bits.
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(128) k_conv3t(ConvArgs a) {
+  swapk::after_previous();
   static_assert(CIN % 16 == 0 && (COUT == 16 || COUT == 32), "operand shapes");
   constexpr int KG = CIN / 8, WBYTES = 27 * COUT * CIN * 2, ABYTES = 128 * CIN * 2, SBYTES = 9 * ABYTES;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -423,11 +438,7 @@ __global__ void __launch_bounds__(128) k_conv3t(ConvArgs a) {
   __shared__ uint32_t tslot;
   __shared__ float sbias[COUT];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  for (int i = tid; i < 27 * COUT * KG; i += 128) {
-    const int t = i / (COUT * KG), r = i % (COUT * KG), n = r / KG, k = 8 * (r % KG);
-    *reinterpret_cast<uint4*>(sW + t * (COUT * CIN * 2) + tc05::core_offset(n, k, COUT)) =
-        reinterpret_cast<const uint4*>(a.W)[i];
-  }
+  load_weights<CIN, COUT, 128>(a.W, sW);
   if (tid < COUT) sbias[tid] = a.bias ? a.bias[tid] : 0.0f;
   if (warp == 0) tc05::tmem_alloc(&tslot, 64);
   if (tid == 0) {
@@ -541,8 +552,7 @@ cudaError_t launch_conv3t(const ConvArgs& a, int nsm, cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(k_conv3t<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   const long long ntiles = a.V / 128, most = (CIN == 16 ? 2LL : 1LL) * nsm;  // blocks that fit in shared memory
-  k_conv3t<CIN, COUT><<<(unsigned)(ntiles < most ? ntiles : most), 128, smem, st>>>(a);
-  return cudaGetLastError();
+  return swapk::launch_next_smem(k_conv3t<CIN, COUT>, (unsigned)(ntiles < most ? ntiles : most), 128, smem, st, a);
 }
 
 template <int CIN, int COUT>
@@ -561,8 +571,7 @@ cudaError_t launch_conv3r(const ConvArgs& a, int nsm, cudaStream_t st) {
   while (ychunk > 8 && cols * ((a.ny + ychunk - 1) / ychunk) < 4 * blocks) ychunk = (ychunk + 1) / 2;
   const long long units = cols * ((a.ny + ychunk - 1) / ychunk);
   const int grid = (int)(units < blocks ? units : blocks);
-  k_conv3r<CIN, COUT><<<grid, 256, smem, st>>>(a, ychunk);
-  return cudaGetLastError();
+  return swapk::launch_next_smem(k_conv3r<CIN, COUT>, grid, 256, smem, st, a, ychunk);
 }
 
 template <int CIN, int COUT>
@@ -574,8 +583,7 @@ cudaError_t launch_conv3(const ConvArgs& a, int nsm, cudaStream_t st) {
   if (e != cudaSuccess) return e;
   const long long ntiles = a.V / 128;
   const int grid = (int)(ntiles < 2LL * nsm ? ntiles : 2LL * nsm);
-  k_conv3<CIN, COUT><<<grid, 128, smem, st>>>(a);
-  return cudaGetLastError();
+  return swapk::launch_next_smem(k_conv3<CIN, COUT>, grid, 128, smem, st, a);
 }
 
 cudaError_t conv3(int cin, int cout, const ConvArgs& a, cudaStream_t st) {
@@ -684,15 +692,25 @@ constexpr int NIN = 14, NOUT = 3;
 static_assert(NIN <= 16, "the first layer's input is padded to 16 channels");
 
 // Normalised BF16 inputs [V][16] from FP32 [V][NIN].
-__global__ void k_norm_inputs(long long V, const float* __restrict__ in, const float* __restrict__ mean,
-                              const float* __restrict__ inv_std, __nv_bfloat16* __restrict__ x) {
-  for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < V; v += (long long)gridDim.x * blockDim.x) {
-    alignas(16) __nv_bfloat16 h[16];
+// (a block's voxels come in through shared memory as whole lines)
+__global__ void __launch_bounds__(256) k_norm_inputs(long long V, const float* in, const float* mean,
+                                                     const float* inv_std, __nv_bfloat16* x) {
+  __shared__ float s_in[256 * NIN];
+  swapk::after_previous();
+  for (long long v0 = blockIdx.x * 256LL; v0 < V; v0 += gridDim.x * 256LL) {
+    const int n = (int)(V - v0 < 256 ? V - v0 : 256);
+    for (int q = threadIdx.x; q < n * NIN; q += 256) s_in[q] = in[v0 * NIN + q];
+    __syncthreads();
+    if ((int)threadIdx.x < n) {
+      alignas(16) __nv_bfloat16 h[16];
 #pragma unroll
-    for (int c = 0; c < 16; ++c) h[c] = __float2bfloat16(c < NIN ? (in[v * NIN + c] - mean[c]) * inv_std[c] : 0.0f);
-    uint4* dst = reinterpret_cast<uint4*>(x + v * 16);
-    dst[0] = reinterpret_cast<const uint4*>(h)[0];
-    dst[1] = reinterpret_cast<const uint4*>(h)[1];
+      for (int c = 0; c < 16; ++c)
+        h[c] = __float2bfloat16(c < NIN ? (s_in[threadIdx.x * NIN + c] - mean[c]) * inv_std[c] : 0.0f);
+      uint4* dst = reinterpret_cast<uint4*>(x + (v0 + threadIdx.x) * 16);
+      dst[0] = reinterpret_cast<const uint4*>(h)[0];
+      dst[1] = reinterpret_cast<const uint4*>(h)[1];
+    }
+    __syncthreads();
   }
 }
 
@@ -1170,7 +1188,8 @@ __global__ void k_flip_t(int cin, int cout, const __nv_bfloat16* __restrict__ W,
 }
 
 // E [V][3] from the network's normalised output.
-__global__ void k_denorm(long long V, const float* __restrict__ out, OutNorm on, float* __restrict__ ve) {
+__global__ void k_denorm(long long V, const float* out, OutNorm on, float* ve) {
+  swapk::after_previous();
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < V; v += (long long)gridDim.x * blockDim.x)
 #pragma unroll
     for (int c = 0; c < NOUT; ++c) ve[v * NOUT + c] = fmaf(out[v * NOUT + c], on.std[c], on.mean[c]);
@@ -1484,11 +1503,10 @@ int predict_e(swap_surrogate* net, int nx, int ny, int nz, const float* vin, flo
   if (!net->normed) return fail(net, SWAP_EINVAL, "the surrogate has not been trained");
   int r = ensure_shape(net, nx, ny, nz);
   if (r) return r;
-  k_norm_inputs<<<nblk(net->V), 256, 0, st>>>(net->V, vin, net->d_mean, net->d_istd, net->x0);
+  SCU(swapk::launch_next(k_norm_inputs, nblk(net->V), 256, st, net->V, vin, net->d_mean, net->d_istd, net->x0));
   r = forward(net, false, st);
   if (r) return r;
-  k_denorm<<<nblk(net->V), 256, 0, st>>>(net->V, net->out, net->on, ve);
-  SCU(cudaGetLastError());
+  SCU(swapk::launch_next(k_denorm, nblk(net->V), 256, st, net->V, net->out, net->on, ve));
   return SWAP_OK;
 }
 

@@ -725,8 +725,10 @@ static int sur_inputs(swap_ctx* c, F32State* s) {
 
 // The network's field advance from the state at the start of the subcycles:
 // E = E0 + the predicted correction per node, B into (oh, ol) and its dB
-// into odb as B - dt curl E.  The inputs are in s->vin.
-static int sur_predict(swap_ctx* c, F32State* s, float* oh, float* ol, float* odb) {
+// into odb as B - dt curl E.  The inputs are in s->vin.  back (may be null):
+// B one subcycle before the end of the step, the leapfrog base of the next
+// predictor.
+static int sur_predict(swap_ctx* c, F32State* s, float* oh, float* ol, float* odb, const F32State::DF* back) {
   const G32& g = s->g;
   {
     ProfScope ps(c, "f32_sur_net", c->st, 6);  // the network's own launches (normalise, 4 convs, scale)
@@ -734,7 +736,9 @@ static int sur_predict(swap_ctx* c, F32State* s, float* oh, float* ol, float* od
       return c->fail(SWAP_EINVAL, std::string("surrogate: ") + surr::last_error(s->sur));
   }
   KL("f32_sur_E", voxels_to_grid(g, s->ve, s->vin, s->E, c->st));
-  KL("f32_sur_B", b_step_given_e(g, s->E, s->b1.h, s->b1.l, c->prm.dt, s->b0c, oh, ol, odb, c->st));
+  KL("f32_sur_B", b_step_given_e(g, s->E, s->b1.h, s->b1.l, c->prm.dt, s->b0c, oh, ol, odb,
+                                      1.0f / (float)c->prm.ntsub, back ? back->h : nullptr, back ? back->l : nullptr,
+                                      c->st));
   return SWAP_OK;
 }
 
@@ -751,10 +755,7 @@ static int field_step(swap_ctx* c, F32State* s) {
   if (use_net) {
     TRY(sur_buffers(c, s));
     TRY(sur_inputs(c, s));
-    TRY(sur_predict(c, s, s->b1p2.h, s->b1p2.l, s->db1p2));
-    // b12: B one subcycle before the end of the step, the leapfrog base of the next predictor
-    KL("f32_sur_B", df_lerp(g, s->b1p2.h, s->b1p2.l, s->b1.h, 1.0f / (float)c->prm.ntsub, s->b12.h, s->b12.l,
-                            c->st));
+    TRY(sur_predict(c, s, s->b1p2.h, s->b1p2.l, s->db1p2, &s->b12));
     std::swap(s->b1, s->b1p2);
     std::swap(s->db1, s->db1p2);
     ++s->sur_used;
@@ -766,7 +767,7 @@ static int field_step(swap_ctx* c, F32State* s) {
     CU(cudaMemsetAsync(s->e_sum, 0, 3 * (std::size_t)g.C * sizeof(float), c->st));
   }
   if (collect || judge) TRY(sur_inputs(c, s));
-  if (judge) TRY(sur_predict(c, s, s->jh, s->jl, s->jdb));
+  if (judge) TRY(sur_predict(c, s, s->jh, s->jl, s->jdb, nullptr));
   TRY(subcycles(c, s, (collect || judge) ? s->e_sum : nullptr));
   if (collect) {
     KL("f32_sur_target", grid_e_to_voxels(g, s->e_sum, (float)(1.0 / s->last_ntf), s->vin, s->ve, c->st));

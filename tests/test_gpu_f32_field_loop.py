@@ -14,7 +14,7 @@ from helpers import make_hybrid, oracle_for
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("cells", [(8, 8, 8), (16, 16, 16), (20, 16, 16), (64, 64, 32), (68, 64, 32)])
+@pytest.mark.parametrize("cells", [(8, 8, 8), (16, 16, 16), (20, 16, 16), (76, 32, 32), (80, 32, 32)])
 def test_step_against_the_oracle_and_itself(cells):
     h = make_hybrid(cells=cells, ppc=6, seed=9, db=0.03)
     o = oracle_for(h, nthreads=8)
