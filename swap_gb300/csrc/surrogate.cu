@@ -735,8 +735,9 @@ __device__ __forceinline__ void add_block_sum(float s, float* acc) {
 
 // Loss 0.5*mean (out - (tgt - mean)/std)^2 over V*3 values, its gradient as
 // BF16 [V][16] (channels 3..15 zero); the sum of squares goes to *acc.
-__global__ void k_loss(long long V, const float* __restrict__ out, const float* __restrict__ tgt, OutNorm on,
-                       float gscale, __nv_bfloat16* __restrict__ d16, float* acc) {
+__global__ void k_loss(long long V, const float* out, const float* tgt, OutNorm on,
+                       float gscale, __nv_bfloat16* d16, float* acc) {
+  swapk::after_previous();
   float s = 0.0f;
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < V; v += (long long)gridDim.x * blockDim.x) {
     alignas(16) __nv_bfloat16 h[16];
@@ -760,8 +761,9 @@ __global__ void k_loss(long long V, const float* __restrict__ out, const float* 
 // add lam * 0.5 sum |curl e|^2 of the physical error e = out*std + mean - tgt
 // (forward differences on the periodic voxel grid, as the B update's curl,
 // in voxel units).  k_err3: e [V][3].
-__global__ void k_err3(long long V, const float* __restrict__ out, const float* __restrict__ tgt, OutNorm on,
-                       float* __restrict__ e) {
+__global__ void k_err3(long long V, const float* out, const float* tgt, OutNorm on,
+                       float* e) {
+  swapk::after_previous();
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < V; v += (long long)gridDim.x * blockDim.x)
 #pragma unroll
     for (int c = 0; c < NOUT; ++c)
@@ -777,7 +779,8 @@ __device__ __forceinline__ unsigned vox(int i, int j, int k, int nx, int ny, int
 
 // kap = curl e (forward differences): kap_x = Dy e3 - Dz e2, kap_y = Dz e1 -
 // Dx e3, kap_z = Dx e2 - Dy e1; the sum of |kap|^2 into *acc.
-__global__ void k_curl3(int nx, int ny, int nz, const float* __restrict__ e, float* __restrict__ kap, float* acc) {
+__global__ void k_curl3(int nx, int ny, int nz, const float* e, float* kap, float* acc) {
+  swapk::after_previous();
   const unsigned V = (unsigned)(nx * ny * nz);  // the work buffers hold far fewer than 2^31 voxels
   float s = 0.0f;
   for (unsigned v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
@@ -797,9 +800,10 @@ __global__ void k_curl3(int nx, int ny, int nz, const float* __restrict__ e, flo
 
 // The plain loss of k_loss plus lam * std_c * (curl^T kap)_c in the output
 // gradient (D_a^T g = g[o - s_a] - g[o]); the plain sum of squares to *acc.
-__global__ void k_loss_curl(int nx, int ny, int nz, const float* __restrict__ out, const float* __restrict__ tgt,
-                            OutNorm on, float gscale, float lam, const float* __restrict__ kap,
-                            __nv_bfloat16* __restrict__ d16, float* acc) {
+__global__ void k_loss_curl(int nx, int ny, int nz, const float* out, const float* tgt,
+                            OutNorm on, float gscale, float lam, const float* kap,
+                            __nv_bfloat16* d16, float* acc) {
+  swapk::after_previous();
   const unsigned V = (unsigned)(nx * ny * nz);  // the work buffers hold far fewer than 2^31 voxels
   float s = 0.0f;
   for (unsigned v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
@@ -1022,9 +1026,10 @@ struct DwLines {
 };
 constexpr int DW_COPY = 9 * 32, DW_TPB = DW_COPY + 32;  // a warp per line, and one that issues the products
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(DW_TPB) k_conv3_dw_lines(int nx, int ny, int nz, const __nv_bfloat16* __restrict__ X,
-                                                        const __nv_bfloat16* __restrict__ dZ, float* __restrict__ gW,
-                                                        float* __restrict__ gb, int units_per_block, int* err) {
+__global__ void __launch_bounds__(DW_TPB) k_conv3_dw_lines(int nx, int ny, int nz, const __nv_bfloat16* X,
+                                                        const __nv_bfloat16* dZ, float* gW,
+                                                        float* gb, int units_per_block, int* err) {
+  swapk::after_previous();
   using D = DwLines<CIN, COUT>;
   constexpr int KG = D::KG, SEG = D::SEG, NB = D::NB, NST = D::NST;
   extern __shared__ __align__(1024) uint8_t smem[];  // NST A stages, then NST B stages, then the tail
@@ -1222,9 +1227,8 @@ cudaError_t conv3_dw(int nx, int ny, int nz, long long V, const __nv_bfloat16* X
     if (e != cudaSuccess) return e;
     const long long units = (long long)((nx + D::SEG - 1) / D::SEG) * ny * nz;
     const long long per = (units + 151) / 152;
-    k_conv3_dw_lines<CIN, COUT><<<(unsigned)((units + per - 1) / per), DW_TPB, D::SMEM, st>>>(nx, ny, nz, X, dZ, gW, gb,
-                                                                                          (int)per, err);
-    return cudaGetLastError();
+    return swapk::launch_next_smem(k_conv3_dw_lines<CIN, COUT>, (unsigned)((units + per - 1) / per), DW_TPB, D::SMEM,
+                                   st, nx, ny, nz, X, dZ, gW, gb, (int)per, err);
   }
   // voxel chunks of a multiple of 64 (V is a multiple of 128), about 152 x 4
   // blocks over all tap groups
@@ -1458,14 +1462,15 @@ int loss_sums(swap_surrogate* net, const float* tgt, float gnorm, cudaStream_t s
   SCU(cudaMemsetAsync(net->acc, 0, 2 * sizeof(float), st));
   if (net->curl_w > 0.0f && net->kref2 > 0.0) {
     float *e = net->dy, *kap = net->dy + 3 * net->V;
-    k_err3<<<nblk(net->V), 256, 0, st>>>(net->V, net->out, tgt, net->on, e);
-    k_curl3<<<loss_blocks(net->V), 256, 0, st>>>(net->nx, net->ny, net->nz, e, kap, net->acc + 1);
-    k_loss_curl<<<loss_blocks(net->V), 256, 0, st>>>(net->nx, net->ny, net->nz, net->out, tgt, net->on, gnorm,
-                                                     (float)(3.0 * net->curl_w / net->kref2), kap, net->d16, net->acc);
+    SCU(swapk::launch_next(k_err3, nblk(net->V), 256, st, net->V, net->out, tgt, net->on, e));
+    SCU(swapk::launch_next(k_curl3, loss_blocks(net->V), 256, st, net->nx, net->ny, net->nz, e, kap, net->acc + 1));
+    SCU(swapk::launch_next(k_loss_curl, loss_blocks(net->V), 256, st, net->nx, net->ny, net->nz,
+                           net->out, tgt, net->on, gnorm, (float)(3.0 * net->curl_w / net->kref2), kap, net->d16,
+                           net->acc));
   } else {
-    k_loss<<<loss_blocks(net->V), 256, 0, st>>>(net->V, net->out, tgt, net->on, gnorm, net->d16, net->acc);
+    SCU(swapk::launch_next(k_loss, loss_blocks(net->V), 256, st, net->V, net->out, tgt, net->on, gnorm, net->d16,
+                           net->acc));
   }
-  SCU(cudaGetLastError());
   return SWAP_OK;
 }
 
@@ -1692,7 +1697,7 @@ extern "C" int swap_surrogate_grads(swap_surrogate* net, int32_t nx, int32_t ny,
   int r = ensure_shape(net, nx, ny, nz);
   if (r) return r;
   cudaStream_t st = nullptr;
-  k_norm_inputs<<<nblk(net->V), 256, 0, st>>>(net->V, vin, net->d_mean, net->d_istd, net->x0);
+  SCU(swapk::launch_next(k_norm_inputs, nblk(net->V), 256, st, net->V, vin, net->d_mean, net->d_istd, net->x0));
   if ((r = forward(net, true, st))) return r;
   if ((r = loss_sums(net, tgt, 1.0f / (3.0f * (float)net->V), st))) return r;
   if ((r = zero_grads(net, st)) || (r = backward(net, st))) return r;
