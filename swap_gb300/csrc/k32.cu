@@ -316,8 +316,8 @@ __device__ __forceinline__ void write_tile(const unsigned* s_dep, void* partial,
 // bricks away from the faces take for far ions only: 33.5M ions, P3 0.97 ->
 // 0.865 ms (990 instructions when every ion unpacked, wrapped and checked its
 // cells).  The barrier after each warp's turn in the ranks stays: letting the
-// warps run apart (named barriers, or none after the last turn) took P3 to
-// 1.13 and 0.885 ms.
+// warps run apart (a named barrier to the next warp, or no barrier after the
+// last turn) took P3 to 0.91 and 0.885 ms.
 // PGRAD: the isothermal electron-pressure term in the gathered E (kitg:
 // its face gradient centred per node, as get_Ep's gradient extension).
 template <int PASS, bool CHEX = false, bool EXACT = true, bool PGRAD = false>
