@@ -834,14 +834,30 @@ __device__ __forceinline__ void prefetch_l2(const float* p, unsigned bytes) {
 // cells 338 against 331; in the field loop below 307 us a step of 64x32x32
 // cells against 182.)
 
+// Offsets are in bytes and 32 bits wide (a component is below 4 GB), beside
+// bases that the whole grid shares: the address of a load is then its base
+// and one register (64-bit element indices: 56 registers instead of 44 in the
+// correctors; 20 steps of 128x64x64 cells 16.2 ms against 16.0).
 struct Off {
   int xm, xp, ym, yp, zm, zp;
 };
+struct In {
+  const float* p;
+  __device__ __forceinline__ float operator[](unsigned at) const {
+    return *reinterpret_cast<const float*>(reinterpret_cast<const char*>(p) + at);
+  }
+};
+__device__ __forceinline__ void put(float* p, unsigned at, float v) {
+  *reinterpret_cast<float*>(reinterpret_cast<char*>(p) + at) = v;
+}
+__device__ __forceinline__ unsigned at_node(const G32& g, int i, int j, int k) {
+  return 4u * ((unsigned)(i - 1) + (unsigned)g.nx * ((unsigned)(j - 1) + (unsigned)g.ny * (unsigned)(k - 1)));
+}
 __device__ __forceinline__ Off off_of(const G32& g, int i, int j, int k) {
-  const int sy = g.nx, sz = g.nx * g.ny;
+  const int sy = 4 * g.nx, sz = 4 * g.nx * g.ny;
   Off d;
-  d.xm = i == 2 ? g.ncx - 1 : -1;
-  d.xp = i == g.nx - 1 ? 1 - g.ncx : 1;
+  d.xm = i == 2 ? 4 * (g.ncx - 1) : -4;
+  d.xp = i == g.nx - 1 ? 4 * (1 - g.ncx) : 4;
   d.ym = j == 2 ? (g.ncy - 1) * sy : -sy;
   d.yp = j == g.ny - 1 ? (1 - g.ncy) * sy : sy;
   d.zm = k == 2 ? (g.ncz - 1) * sz : -sz;
@@ -874,7 +890,7 @@ struct Stencil {
   float b1, b1y, b1z, b1yz, b2, b2x, b2z, b2xz, b3, b3x, b3y, b3xy;
 };
 __device__ __forceinline__ Stencil stencil_of(const G32& g, const float* db, unsigned o, const Off& d) {
-  const float *B1 = db, *B2 = db + g.C, *B3 = db + 2 * g.C;
+  const In B1{db}, B2{db + g.C}, B3{db + 2 * g.C};
   return Stencil{B1[o], B1[o + d.ym], B1[o + d.zm], B1[o + d.ym + d.zm], B2[o], B2[o + d.xm], B2[o + d.zm],
                  B2[o + d.xm + d.zm], B3[o], B3[o + d.xm], B3[o + d.ym], B3[o + d.xm + d.ym]};
 }
@@ -922,11 +938,11 @@ __global__ void __launch_bounds__(TPB) k_up_courant(G32 g, const float* np, cons
     interior_of(g, t, i, j, k);
     const Off d = off_of(g, i, j, k);
     const long long C = g.C;
-    const unsigned o = (unsigned)nid(g, i, j, k);
-    const float *s1 = S, *s2 = S + C, *s3 = S + 2 * C;
-    const float n = np[o], nx = np[o + d.xp], ny = np[o + d.yp], nz = np[o + d.zp];
+    const unsigned o = at_node(g, i, j, k);
+    const In s1{S}, s2{S + C}, s3{S + 2 * C}, N{np}, D1{db}, D2{db + C}, D3{db + 2 * C};
+    const float n = N[o], nx = N[o + d.xp], ny = N[o + d.yp], nz = N[o + d.zp];
     const float a0 = s1[o], a1 = s1[o + d.xp], c0 = s2[o], c1 = s2[o + d.yp], e0 = s3[o], e1 = s3[o + d.zp];
-    const float b1 = db[o] + b0c[0], b2 = db[o + C] + b0c[1], b3 = db[o + 2 * C] + b0c[2];
+    const float b1 = D1[o] + b0c[0], b2 = D2[o] + b0c[1], b3 = D3[o] + b0c[2];
     const float btot = sqrtf(b1 * b1 + b2 * b2 + b3 * b3);
     const float ak = 2.0f / dx;
     const float q1 = ak * ak * btot / (alpha * n);
@@ -938,7 +954,7 @@ __global__ void __launch_bounds__(TPB) k_up_courant(G32 g, const float* np, cons
     const float v[4] = {0.5f * (ct_of(a0, n) + ct_of(a1, nx)), 0.5f * (ct_of(c0, n) + ct_of(c1, ny)),
                         0.5f * (ct_of(e0, n) + ct_of(e1, nz)), dt};
 #pragma unroll
-    for (int q = 0; q < 4; ++q) f[q][o] = v[q];
+    for (int q = 0; q < 4; ++q) put(f[q], o, v[q]);
     ghost_images(g, i, j, k, f, v);
   }
   // one atomic per block (a grid of a few per SM): atomics from every warp to
@@ -977,11 +993,11 @@ __global__ void __launch_bounds__(TPB) k_kit(G32 g, const float* S, const float*
     interior_of(g, t, i, j, k);
     const Off d = off_of(g, i, j, k);
     const long long C = g.C;
-    const unsigned o = (unsigned)nid(g, i, j, k);
+    const unsigned o = at_node(g, i, j, k);
     const Stencil s = stencil_of(g, db, o, d);
-    const float n0 = np[o], nxm = np[o + d.xm], nxp = np[o + d.xp], nym = np[o + d.ym], nyp = np[o + d.yp],
-                nzm = np[o + d.zm], nzp = np[o + d.zp];
-    const float *s1 = S, *s2 = S + C, *s3 = S + 2 * C;
+    const In N{np}, s1{S}, s2{S + C}, s3{S + 2 * C};
+    const float n0 = N[o], nxm = N[o + d.xm], nxp = N[o + d.xp], nym = N[o + d.ym], nyp = N[o + d.yp],
+                nzm = N[o + d.zm], nzp = N[o + d.zp];
     const float x0 = ct_of(s1[o], n0), xm = ct_of(s1[o + d.xm], nxm), xp = ct_of(s1[o + d.xp], nxp);
     const float y0 = ct_of(s2[o], n0), ym = ct_of(s2[o + d.ym], nym), yp = ct_of(s2[o + d.yp], nyp);
     const float z0 = ct_of(s3[o], n0), zm = ct_of(s3[o + d.zm], nzm), zp = ct_of(s3[o + d.zp], nzp);
@@ -995,10 +1011,10 @@ __global__ void __launch_bounds__(TPB) k_kit(G32 g, const float* S, const float*
     kit[2 * t + 1] = make_float4(centre(s.b2, s.b2x, s.b2z, s.b2xz) + b0c[1],
                                  centre(s.b3, s.b3y, s.b3x, s.b3xy) + b0c[2], 0.0f, 0.0f);
     if (kitg) {
-      const unsigned sy = (unsigned)g.nx, sz = (unsigned)(g.nx * g.ny);
-      kitg[t] = make_float4(0.5f * (gpe_face<0>(g, np, gp, o) + gpe_face<0>(g, np, gp, o - 1u)),
-                            0.5f * (gpe_face<1>(g, np, gp, o) + gpe_face<1>(g, np, gp, o - sy)),
-                            0.5f * (gpe_face<2>(g, np, gp, o) + gpe_face<2>(g, np, gp, o - sz)), 0.0f);
+      const unsigned n = o / 4, sy = (unsigned)g.nx, sz = (unsigned)(g.nx * g.ny);
+      kitg[t] = make_float4(0.5f * (gpe_face<0>(g, np, gp, n) + gpe_face<0>(g, np, gp, n - 1u)),
+                            0.5f * (gpe_face<1>(g, np, gp, n) + gpe_face<1>(g, np, gp, n - sy)),
+                            0.5f * (gpe_face<2>(g, np, gp, n) + gpe_face<2>(g, np, gp, n - sz)), 0.0f);
     }
   }
 }
@@ -1016,11 +1032,11 @@ __device__ __forceinline__ void aj_ct_node(const G32& g, const float* db, const 
                                            const float* b0c, float alpha, float* aj, float* ct, int i, int j, int k) {
   const Off d = off_of(g, i, j, k);
   const long long C = g.C;
-  const unsigned o = (unsigned)nid(g, i, j, k);
-  const float *u1 = up, *u2 = up + C, *u3 = up + 2 * C;
+  const unsigned o = at_node(g, i, j, k);
+  const In u1{up}, u2{up + C}, u3{up + 2 * C}, N{np};
   const Stencil s = stencil_of(g, db, o, d);
-  const float n0 = np[o], nxm = np[o + d.xm], nxp = np[o + d.xp], nym = np[o + d.ym], nyp = np[o + d.yp],
-              nzm = np[o + d.zm], nzp = np[o + d.zp];
+  const float n0 = N[o], nxm = N[o + d.xm], nxp = N[o + d.xp], nym = N[o + d.ym], nyp = N[o + d.yp],
+              nzm = N[o + d.zm], nzp = N[o + d.zp];
   const float ux = u1[o], uxm = u1[o + d.xm], uy = u2[o], uym = u2[o + d.ym], uz = u3[o], uzm = u3[o + d.zm];
   // the same four values one step down and up the component's own axis
   float m[3][4], p[3][4];
@@ -1029,7 +1045,7 @@ __device__ __forceinline__ void aj_ct_node(const G32& g, const float* db, const 
     const int lo[3] = {d.xm, d.ym, d.zm}, hi[3] = {d.xp, d.yp, d.zp};
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-      const float* B = db + C * q;
+      const In B{db + C * q};
       const unsigned a = o + lo[q], b = o + hi[q];
       m[q][0] = B[a]; m[q][1] = B[a + e[q][1]]; m[q][2] = B[a + e[q][2]]; m[q][3] = B[a + e[q][1] + e[q][2]];
       p[q][0] = B[b]; p[q][1] = B[b + e[q][1]]; p[q][2] = B[b + e[q][2]]; p[q][3] = B[b + e[q][1] + e[q][2]];
@@ -1064,7 +1080,7 @@ __device__ __forceinline__ void aj_ct_node(const G32& g, const float* db, const 
   float* const f[6] = {aj, aj + C, aj + 2 * C, ct, ct + C, ct + 2 * C};
   const float v[6] = {a1, a2, a3, ay * bz - az * by, az * bx - ax * bz, ax * by - ay * bx};
 #pragma unroll
-  for (int q = 0; q < 6; ++q) f[q][o] = v[q];
+  for (int q = 0; q < 6; ++q) put(f[q], o, v[q]);
   ghost_images(g, i, j, k, f, v);
 }
 
@@ -1072,9 +1088,22 @@ template <bool CORR>
 __global__ void __launch_bounds__(FBX * FBY) k_aj_ct(G32 g, const float* db,
                                                      const float* np, const float* up,
                                                      const float* b0c, float alpha,
-                                                     float* aj, float* ct) {
+                                                     float* aj, float* ct, int ahead) {
   swapk::after_previous();
   FIELD_NODE(i, j, k);
+  // rows of later planes, as in k_bstep; the predictor's kernel runs further
+  // ahead, having the least to do per node.  With the addresses above, us per
+  // launch, predictor and corrector: 256x128x128 cells 55.8 -> 51.7 and 73.9 ->
+  // 65.8, 512x256x128 195 -> 175 and 274 -> 220
+  if (blockIdx.x == 0 && threadIdx.x == 0 && ahead && k + ahead <= g.ncz + 1) {
+    const unsigned t = (unsigned)nid(g, i, j, k + ahead), nb = (g.ncx * 4 + 16) & ~15;
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      prefetch_l2(db + t + g.C * m, nb);
+      prefetch_l2(up + t + g.C * m, nb);
+    }
+    prefetch_l2(np + t, nb);
+  }
   aj_ct_node<CORR>(g, db, np, up, b0c, alpha, aj, ct, i, j, k);
 }
 
@@ -1126,9 +1155,9 @@ __device__ __forceinline__ void bstep_node(const G32& g, const float* ct, const 
                                            float* dbtp1, float* E, float* e_acc, int i, int j, int k) {
   const Off d = off_of(g, i, j, k);
   const long long C = g.C;
-  const unsigned o = (unsigned)nid(g, i, j, k), ox = o + d.xp, oy = o + d.yp, oz = o + d.zp;
-  const float *c1 = ct, *c2 = ct + C, *c3 = ct + 2 * C, *j1 = aj, *j2 = aj + C, *j3 = aj + 2 * C;
-  const float n0 = nu[o], nx = nu[ox], ny = nu[oy], nz = nu[oz];
+  const unsigned o = at_node(g, i, j, k), ox = o + d.xp, oy = o + d.yp, oz = o + d.zp;
+  const In c1{ct}, c2{ct + C}, c3{ct + 2 * C}, j1{aj}, j2{aj + C}, j3{aj + 2 * C}, nus{nu};
+  const float n0 = nus[o], nx = nus[ox], ny = nus[oy], nz = nus[oz];
   float e1 = 0.5f * (c1[o] + c1[ox]) + n0 * j1[o], e1y = 0.5f * (c1[oy] + c1[oy + d.xp]) + ny * j1[oy],
         e1z = 0.5f * (c1[oz] + c1[oz + d.xp]) + nz * j1[oz];
   float e2 = 0.5f * (c2[o] + c2[oy]) + n0 * j2[o], e2x = 0.5f * (c2[ox] + c2[ox + d.yp]) + nx * j2[ox],
@@ -1138,13 +1167,13 @@ __device__ __forceinline__ void bstep_node(const G32& g, const float* ct, const 
   float h[3], l[3], c0[3], old[3];
 #pragma unroll
   for (int m = 0; m < 3; ++m) {
-    h[m] = bh[o + C * m];
-    l[m] = bl[o + C * m];
+    h[m] = In{bh + C * m}[o];
+    l[m] = In{bl + C * m}[o];
     c0[m] = b0c[m];
-    old[m] = PRED ? db1[o + C * m] : 0.0f;
+    old[m] = PRED ? In{db1 + C * m}[o] : 0.0f;
   }
   if (gpf) {
-    const float *g1 = gpf, *g2 = gpf + C, *g3 = gpf + 2 * C;
+    const In g1{gpf}, g2{gpf + C}, g3{gpf + 2 * C};
     e1 -= g1[o]; e1y -= g1[oy]; e1z -= g1[oz];
     e2 -= g2[o]; e2x -= g2[ox]; e2z -= g2[oz];
     e3 -= g3[o]; e3x -= g3[ox]; e3y -= g3[oy];
@@ -1177,13 +1206,13 @@ __device__ __forceinline__ void bstep_node(const G32& g, const float* ct, const 
     v[N - 3] = e1; v[N - 2] = e2; v[N - 1] = e3;
   }
 #pragma unroll
-  for (int q = 0; q < N; ++q) f[q][o] = v[q];
+  for (int q = 0; q < N; ++q) put(f[q], o, v[q]);
   float* const(&cf)[N] = f;
   ghost_images(g, i, j, k, cf, v);
   if (e_acc) {
-    e_acc[o] += e1;
-    e_acc[o + C] += e2;
-    e_acc[o + 2 * C] += e3;
+    put(e_acc, o, In{e_acc}[o] + e1);
+    put(e_acc + C, o, In{e_acc + C}[o] + e2);
+    put(e_acc + 2 * C, o, In{e_acc + 2 * C}[o] + e3);
   }
 }
 
@@ -1300,15 +1329,15 @@ __global__ void __launch_bounds__(FBX * FBY) k_bstep_given_e(G32 g, const float*
   FIELD_NODE(i, j, k);
   const Off d = off_of(g, i, j, k);
   const long long C = g.C;
-  const unsigned o = (unsigned)nid(g, i, j, k);
-  const float *E1 = E, *E2 = E + C, *E3 = E + 2 * C;
+  const unsigned o = at_node(g, i, j, k);
+  const In E1{E}, E2{E + C}, E3{E + 2 * C};
   const float e1 = E1[o], e2 = E2[o], e3 = E3[o], e1y = E1[o + d.yp], e1z = E1[o + d.zp], e2x = E2[o + d.xp],
               e2z = E2[o + d.zp], e3x = E3[o + d.xp], e3y = E3[o + d.yp];
   float h[3], l[3], c0[3];
 #pragma unroll
   for (int m = 0; m < 3; ++m) {
-    h[m] = bh[o + C * m];
-    l[m] = bl[o + C * m];
+    h[m] = In{bh + C * m}[o];
+    l[m] = In{bl + C * m}[o];
     c0[m] = b0c[m];
   }
   const float ce[3] = {(e3y - e3) * g.inv_dy + (e2 - e2z) * g.inv_dz, (e3 - e3x) * g.inv_dx + (e1z - e1) * g.inv_dz,
@@ -1336,11 +1365,11 @@ __global__ void __launch_bounds__(FBX * FBY) k_bstep_given_e(G32 g, const float*
     w[3 + m] = __fsub_rn(e, __fsub_rn(w[m], s));
   }
 #pragma unroll
-  for (int q = 0; q < 9; ++q) out[q][o] = v[q];
+  for (int q = 0; q < 9; ++q) put(out[q], o, v[q]);
   ghost_images(g, i, j, k, out, v);
   if (!th) return;
 #pragma unroll
-  for (int q = 0; q < 6; ++q) lerp[q][o] = w[q];
+  for (int q = 0; q < 6; ++q) put(lerp[q], o, w[q]);
   ghost_images(g, i, j, k, lerp, w);
 }
 
@@ -2083,22 +2112,26 @@ __global__ void k_gpe(G32 g, const float* __restrict__ np, float gp, float* __re
 cudaError_t gpe_faces(const G32& g, const float* np, float gp, float* gpf, cudaStream_t st) {
   RET((k_gpe<<<nblk(n_int(g)), TPB, 0, st>>>(g, np, gp, gpf)));
 }
+// How far ahead of its blocks a field kernel asks for rows, in planes.
+static int planes_ahead(const G32& g, int nodes) {
+  const int plane = g.ncx * g.ncy;
+  return n_int(g) >= B_AHEAD_NODES ? std::max(1, (nodes + plane / 2) / plane) : 0;
+}
 cudaError_t aj_ct(const G32& g, bool corr, const float* db, const float* np, const float* up, const float* b0c,
                   float alpha, float* aj, float* ct, cudaStream_t st) {
   const dim3 grid((g.ncx + FBX - 1) / FBX, (g.ncy + FBY - 1) / FBY, g.ncz), blk(FBX, FBY);
-  return swapk::launch_next(corr ? k_aj_ct<true> : k_aj_ct<false>, grid, blk, st, g, db, np, up, b0c, alpha, aj, ct);
+  return swapk::launch_next(corr ? k_aj_ct<true> : k_aj_ct<false>, grid, blk, st, g, db, np, up, b0c, alpha, aj, ct,
+                            planes_ahead(g, corr ? 200000 : 400000));
 }
 cudaError_t b_step(const G32& g, bool pred, bool write_e, const float* ct, const float* nu, const float* aj,
                    const float* gpf, const float* bh, const float* bl, double coef, const float* b0c, float* oh,
                    float* ol, float* dbo, const float* db1, float* dbtp1, float* E, float* e_acc, cudaStream_t st) {
   const dim3 grid((g.ncx + FBX - 1) / FBX, (g.ncy + FBY - 1) / FBY, g.ncz), blk(FBX, FBY);
-  // the planes that the resident blocks (about 200k nodes) run ahead; see k_bstep
-  const int plane = g.ncx * g.ncy, ahead = n_int(g) >= B_AHEAD_NODES ? (200000 + plane / 2) / plane + (plane > 400000) : 0;
   const float ch = (float)coef, cl = (float)(coef - (double)ch);
   const auto k = pred ? (write_e ? k_bstep<true, true> : k_bstep<true, false>)
                       : (write_e ? k_bstep<false, true> : k_bstep<false, false>);
   return swapk::launch_next(k, grid, blk, st, g, ct, nu, aj, gpf, bh, bl, ch, cl, b0c, oh, ol, dbo, db1, dbtp1, E,
-                            e_acc, ahead);
+                            e_acc, planes_ahead(g, 200000));
 }
 bool field_loop_fits(const G32& g) { return n_int(g) <= FIELD_LOOP_NODES; }
 

@@ -200,8 +200,8 @@ cudaError_t aj_ct(const G32& g, bool corr, const float* db, const float* np, con
                   float alpha, float* aj, float* ct, cudaStream_t st);
 // e_acc (may be null): the step's E summed over the correctors.
 // gpf (may be null): the electron-pressure face gradient E subtracts.
-// From this many nodes on, the 19 to 22 arrays of b_step do not stay in L2
-// (129 MB) and it prefetches.
+// From this many nodes on, the 13 to 22 arrays of a field kernel do not stay
+// in L2 (129 MB) and it prefetches.
 constexpr long long B_AHEAD_NODES = 1 << 21;
 cudaError_t b_step(const G32& g, bool pred, bool write_e, const float* ct, const float* nu, const float* aj,
                    const float* gpf, const float* bh, const float* bl, double coef, const float* b0c, float* oh,
