@@ -52,11 +52,6 @@ __device__ __forceinline__ int wrapi(int i, int n) { return i < 0 ? i + n : (i >
 __device__ __forceinline__ long long nid(const G32& g, int i, int j, int k) {
   return (long long)(i - 1) + (long long)g.nx * ((long long)(j - 1) + (long long)g.ny * (long long)(k - 1));
 }
-// node index of physical node (p,q,r), p in [0,ncx): 1-based i = p + 2
-__device__ __forceinline__ long long pid(const G32& g, int p, int q, int r) { return nid(g, p + 2, q + 2, r + 2); }
-// interior image of a 1-based node index (ghost 1 -> n-1, ghost n -> 2)
-__device__ __forceinline__ int img(int i, int n) { return i == 1 ? n - 1 : (i == n ? 2 : i); }
-
 // Store v at interior node (i,j,k) and at every ghost node whose image it
 // is: the periodic fill of boundary.f:9-52 fused into the producer.
 template <class T>
@@ -1828,21 +1823,84 @@ __global__ void k_scan_apply(const int64_t* __restrict__ in, long long n, const 
 // conversions and diagnostics
 // ---------------------------------------------------------------------------
 
-__global__ void k_from_f64(G32 g, long long N, long long NM, const double* __restrict__ xp,
+// The conversion to the FP32 form is bound by the FP64 pipe (a divide holds it
+// 135 clocks, any other operation or conversion 16), so what can goes through
+// integers.  The bits are those of split_axis and of casts.  f32_begin of 134M
+// ions: 20.2 -> 12.9 ms; f32_end 6.2 -> 3.6.
+
+// (float)x rounded to nearest even; what is no normal float by the conversion
+// (a call, or it would be made every time and selected).
+__device__ __noinline__ float narrow_any(double x) { return (float)x; }
+__device__ __forceinline__ float narrow(double x) {
+  const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x), m = h & 0x7fffffffu;
+  if (m - 0x38100000u >= 0x0fd00000u) return narrow_any(x);  // exponents -126 to 126
+  const unsigned b = (m - 0x38000000u) << 3 | l >> 29;
+  const unsigned rest = (l << 3) | (b & 1u);  // above one half, or one half and odd: up
+  return __uint_as_float((h & 0x80000000u) | (b + (rest > 0x80000000u ? 1u : 0u)));
+}
+
+// split_axis with the reciprocal r of d (1/d rounded; UNIT: d is one): the
+// quotient from one product and its exact remainder (Markstein 1990), the
+// nearest whole number by adding 1.5 * 2^52.  What that does not cover
+// (differences of 2^15 and more, tiny or zero ones, NaN) goes to split_axis.
+struct Spacing {
+  double d[3], r[3];
+};
+template <bool UPPER, bool UNIT>
+__device__ __forceinline__ bool split_fast(double x, double q1, double d, double r, int n, int& c, float& o) {
+  const double a = x - q1;
+  const unsigned ha = (unsigned)__double2hiint(a) & 0x7fffffffu;
+  if (ha - 0x20000000u >= 0x20e00000u) return split_axis(x, q1, d, n, UPPER, c, o);  // |a| outside [2^-511, 2^15)
+  double u = a;
+  if (!UNIT) {
+    u = a * r;
+    u = __fma_rn(__fma_rn(-u, d, a), r, u);
+  }
+  constexpr double M = 6755399441055744.0;
+  const double t = u + M;
+  int i = __double2loint(t);
+  double f = u - (t - M);  // in [-1/2, 1/2], exact
+  const int h = __double2hiint(f);
+  // (f is no negative zero: u is not zero)
+  if (UPPER ? h < 0 || (h | __double2loint(f)) == 0 : h < 0) {
+    f += 1.0;
+    --i;
+  }
+  if (i < 0 || i >= n) return false;
+  c = i;
+  o = narrow(f);
+  if (UPPER && o <= 0.0f) o = 1e-7f;
+  if (!UPPER && o >= 1.0f) o = 0.99999994f;
+  return true;
+}
+// (double)x; zeros, denormals, infinities and NaN by the conversion itself.
+__device__ __noinline__ double widen_any(float x) { return (double)x; }
+__device__ __forceinline__ double widen(float x) {
+  const unsigned b = __float_as_uint(x);
+  if (((b + 0x00800000u) & 0x7fffffffu) < 0x01000000u) return widen_any(x);
+  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
+}
+// q1 + (c + o) * d, c a cell index
+__device__ __forceinline__ double position(double q1, int c, float o, double d) {
+  return q1 + ((__hiloint2double(0x43300000, c) - 4503599627370496.0) + widen(o)) * d;
+}
+
+template <bool UNIT>
+__global__ void k_from_f64(G32 g, Spacing sp3, long long N, long long NM, const double* __restrict__ xp,
                            const double* __restrict__ vp, const double* __restrict__ vp1,
                            const double* __restrict__ mrat, const double* __restrict__ beta_p, Species sp, Part p,
                            int* err) {
   GSTRIDE(l, N) {
     int ci = 0, cj = 0, ck = 0;
     float ox = 0.5f, oy = 0.5f, oz = 0.5f;
-    const bool ok = split_axis(xp[l], g.qx1, g.dx, g.ncx, true, ci, ox) &&
-                    split_axis(xp[l + NM], g.qy1, g.dy, g.ncy, false, cj, oy) &&
-                    split_axis(xp[l + 2 * NM], g.qz1, g.dz, g.ncz, true, ck, oz);
+    const bool ok = split_fast<true, UNIT>(xp[l], g.qx1, sp3.d[0], sp3.r[0], g.ncx, ci, ox) &&
+                    split_fast<false, UNIT>(xp[l + NM], g.qy1, sp3.d[1], sp3.r[1], g.ncy, cj, oy) &&
+                    split_fast<true, UNIT>(xp[l + 2 * NM], g.qz1, sp3.d[2], sp3.r[2], g.ncz, ck, oz);
     if (!ok) set_err(err, KERR_DOMAIN);
     p.cell[l] = pk(ci, cj, ck);
     p.ox[l] = ox; p.oy[l] = oy; p.oz[l] = oz;
-    p.vx[l] = (float)vp[l]; p.vy[l] = (float)vp[l + NM]; p.vz[l] = (float)vp[l + 2 * NM];
-    p.wx[l] = (float)vp1[l]; p.wy[l] = (float)vp1[l + NM]; p.wz[l] = (float)vp1[l + 2 * NM];
+    p.vx[l] = narrow(vp[l]); p.vy[l] = narrow(vp[l + NM]); p.vz[l] = narrow(vp[l + 2 * NM]);
+    p.wx[l] = narrow(vp1[l]); p.wy[l] = narrow(vp1[l + NM]); p.wz[l] = narrow(vp1[l + 2 * NM]);
   }
 }
 
@@ -1861,15 +1919,15 @@ __global__ void k_assign_species(long long N, const double* __restrict__ mrat, c
   }
 }
 
-__global__ void k_to_f64(G32 g, long long N, long long NM, Part p, double* __restrict__ xp, double* __restrict__ vp,
+__global__ void k_to_f64(G32 g, double3 d3, long long N, long long NM, Part p, double* __restrict__ xp, double* __restrict__ vp,
                          double* __restrict__ vp1) {
   GSTRIDE(l, N) {
     const int32_t c = p.cell[l];
-    xp[l] = g.qx1 + ((double)pk_i(c) + (double)p.ox[l]) * (double)g.dx;
-    xp[l + NM] = g.qy1 + ((double)pk_j(c) + (double)p.oy[l]) * (double)g.dy;
-    xp[l + 2 * NM] = g.qz1 + ((double)pk_k(c) + (double)p.oz[l]) * (double)g.dz;
-    vp[l] = p.vx[l]; vp[l + NM] = p.vy[l]; vp[l + 2 * NM] = p.vz[l];
-    vp1[l] = p.wx[l]; vp1[l + NM] = p.wy[l]; vp1[l + 2 * NM] = p.wz[l];
+    xp[l] = position(g.qx1, pk_i(c), p.ox[l], d3.x);
+    xp[l + NM] = position(g.qy1, pk_j(c), p.oy[l], d3.y);
+    xp[l + 2 * NM] = position(g.qz1, pk_k(c), p.oz[l], d3.z);
+    vp[l] = widen(p.vx[l]); vp[l + NM] = widen(p.vy[l]); vp[l + 2 * NM] = widen(p.vz[l]);
+    vp1[l] = widen(p.wx[l]); vp1[l + NM] = widen(p.wy[l]); vp1[l + 2 * NM] = widen(p.wz[l]);
   }
 }
 
@@ -1901,29 +1959,57 @@ __global__ void k_keep_count(long long N, const int32_t* __restrict__ cell, int6
   if (threadIdx.x == 0) bcount[blockIdx.x] = tot;
 }
 
-__global__ void k_to_f64_kept(G32 g, long long N, long long NM, Part p, const int64_t* __restrict__ bstart,
+__global__ void __launch_bounds__(TPB) k_to_f64_kept(G32 g, double3 d3, long long N, long long NM, Part p, const int64_t* __restrict__ bstart,
                               const double* __restrict__ tm, const double* __restrict__ tb, double* __restrict__ xp,
                               double* __restrict__ vp, double* __restrict__ vp1, double* __restrict__ mrat,
                               double* __restrict__ beta_p) {
-  __shared__ int64_t sh[32];
+  // the kept ions' places in the tile, all at once: a scan per 256 ions left
+  // their loads one behind the other (16.8M ions: 699 us, this way 391)
+  constexpr int ROUNDS = KEEP_TILE / TPB, WARPS = TPB / 32;
+  __shared__ int at[ROUNDS * WARPS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long base = (long long)blockIdx.x * KEEP_TILE;
-  int64_t run = bstart[blockIdx.x];
-  for (int q = 0; q < KEEP_TILE / TPB; ++q) {
+  int32_t c[ROUNDS];
+  int d[ROUNDS];
+#pragma unroll
+  for (int q = 0; q < ROUNDS; ++q) {
     const long long l = base + q * TPB + threadIdx.x;
-    const int32_t c = l < N ? p.cell[l] : CELL_DEAD;
-    const bool k = kept(c);
-    int64_t tot;
-    const long long d = run + block_excl_scan(k ? 1 : 0, sh, tot);
-    run += tot;
-    if (!k) continue;
-    xp[d] = g.qx1 + ((double)pk_i(c) + (double)p.ox[l]) * (double)g.dx;
-    xp[d + NM] = g.qy1 + ((double)pk_j(c) + (double)p.oy[l]) * (double)g.dy;
-    xp[d + 2 * NM] = g.qz1 + ((double)pk_k(c) + (double)p.oz[l]) * (double)g.dz;
-    vp[d] = p.vx[l]; vp[d + NM] = p.vy[l]; vp[d + 2 * NM] = p.vz[l];
-    vp1[d] = p.wx[l]; vp1[d + NM] = p.wy[l]; vp1[d + 2 * NM] = p.wz[l];
+    c[q] = l < N ? p.cell[l] : CELL_DEAD;
+  }
+#pragma unroll
+  for (int q = 0; q < ROUNDS; ++q) {
+    const unsigned m = __ballot_sync(0xffffffffu, kept(c[q]));
+    d[q] = __popc(m & ((1u << lane) - 1u));
+    if (lane == 0) at[q * WARPS + warp] = __popc(m);
+  }
+  __syncthreads();
+  static_assert(ROUNDS * WARPS == 64, "two counts a lane");
+  if (warp == 0) {
+    const int n0 = at[2 * lane], n1 = at[2 * lane + 1];
+    int sum = n0 + n1;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int below = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += below;
+    }
+    at[2 * lane] = sum - n1 - n0;
+    at[2 * lane + 1] = sum - n1;
+  }
+  __syncthreads();
+  const long long first = bstart[blockIdx.x];
+#pragma unroll
+  for (int q = 0; q < ROUNDS; ++q) {
+    if (!kept(c[q])) continue;
+    const long long l = base + q * TPB + threadIdx.x, t = first + at[q * WARPS + warp] + d[q];
+    const float ox = p.ox[l], oy = p.oy[l], oz = p.oz[l], vx = p.vx[l], vy = p.vy[l], vz = p.vz[l], wx = p.wx[l],
+                wy = p.wy[l], wz = p.wz[l];
     const int s = p.sp ? min((int)p.sp[l], MAX_SPECIES - 1) : 0;
-    mrat[d] = tm[s];
-    beta_p[d] = tb[s];
+    xp[t] = position(g.qx1, pk_i(c[q]), ox, d3.x);
+    xp[t + NM] = position(g.qy1, pk_j(c[q]), oy, d3.y);
+    xp[t + 2 * NM] = position(g.qz1, pk_k(c[q]), oz, d3.z);
+    vp[t] = widen(vx); vp[t + NM] = widen(vy); vp[t + 2 * NM] = widen(vz);
+    vp1[t] = widen(wx); vp1[t + NM] = widen(wy); vp1[t + 2 * NM] = widen(wz);
+    mrat[t] = tm[s];
+    beta_p[t] = tb[s];
   }
 }
 
@@ -2370,7 +2456,10 @@ cudaError_t pass1_sort(const G32& g, const Part& src, const Part& stage, const P
 cudaError_t from_f64(const G32& g, long long N, long long NM, const double* xp, const double* vp, const double* vp1,
                      const double* mrat, const double* beta_p, const Species& sp, Part p, int* err, cudaStream_t st) {
   if (N <= 0) return cudaSuccess;
-  RET((k_from_f64<<<nblk(N), TPB, 0, st>>>(g, N, NM, xp, vp, vp1, mrat, beta_p, sp, p, err)));
+  const Spacing sp3{{g.dx, g.dy, g.dz}, {1.0 / (double)g.dx, 1.0 / (double)g.dy, 1.0 / (double)g.dz}};
+  if (g.dx == 1.0f && g.dy == 1.0f && g.dz == 1.0f)
+    RET((k_from_f64<true><<<nblk(N), TPB, 0, st>>>(g, sp3, N, NM, xp, vp, vp1, mrat, beta_p, sp, p, err)));
+  RET((k_from_f64<false><<<nblk(N), TPB, 0, st>>>(g, sp3, N, NM, xp, vp, vp1, mrat, beta_p, sp, p, err)));
 }
 cudaError_t assign_species(long long N, const double* mrat, const double* beta_p, const double* tab_mrat,
                            const double* tab_bp, int n, uint8_t* spid, int* miss, cudaStream_t st) {
@@ -2388,7 +2477,7 @@ cudaError_t not_uniform(long long C, const double* b, int* flag, cudaStream_t st
 cudaError_t to_f64(const G32& g, long long N, long long NM, const Part& p, double* xp, double* vp, double* vp1,
                    cudaStream_t st) {
   if (N <= 0) return cudaSuccess;
-  RET((k_to_f64<<<nblk(N), TPB, 0, st>>>(g, N, NM, p, xp, vp, vp1)));
+  RET((k_to_f64<<<nblk(N), TPB, 0, st>>>(g, make_double3(g.dx, g.dy, g.dz), N, NM, p, xp, vp, vp1)));
 }
 cudaError_t species_to_f64(long long N, const uint8_t* spid, const double* tab_mrat, const double* tab_bp,
                            double* mrat, double* beta_p, cudaStream_t st) {
@@ -2405,7 +2494,7 @@ cudaError_t to_f64_kept(const G32& g, long long N, long long NM, const Part& p, 
   k_keep_count<<<(unsigned)nb, TPB, 0, st>>>(N, p.cell, bcount);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if ((e = scan_exclusive(bcount, bstart, nb, sums, st)) != cudaSuccess) return e;
-  k_to_f64_kept<<<(unsigned)nb, TPB, 0, st>>>(g, N, NM, p, bstart, tab_mrat, tab_bp, xp, vp, vp1, mrat, beta_p);
+  k_to_f64_kept<<<(unsigned)nb, TPB, 0, st>>>(g, make_double3(g.dx, g.dy, g.dz), N, NM, p, bstart, tab_mrat, tab_bp, xp, vp, vp1, mrat, beta_p);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   int64_t n = 0;
   if ((e = cudaMemcpyAsync(&n, bstart + nb, sizeof(int64_t), cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
