@@ -870,6 +870,12 @@ __device__ __forceinline__ void ghost_images(const G32& g, int i, int j, int k, 
   if (!(di | dj | dk)) return;
   const long long o = nid(g, i, j, k);
   const int x = di, y = dj * g.nx, z = dk * g.nx * g.ny;
+  if ((di != 0) + (dj != 0) + (dk != 0) == 1) {  // a face: one image
+    const long long t = o + x + y + z;
+#pragma unroll
+    for (int q = 0; q < N; ++q) f[q][t] = v[q];
+    return;
+  }
 #pragma unroll 1
   for (int c = 1; c < 8; ++c) {
     if (((c & 1) && !x) || ((c & 2) && !y) || ((c & 4) && !z)) continue;
@@ -909,13 +915,20 @@ __device__ __forceinline__ float curl_down(const G32& g, const Stencil& s) {
 // Cell-centre B from the edge field's values at the node, one step down two
 // axes, and both (edge_to_center, grid_interp.f:35-51, with ratios 1/2).
 __device__ __forceinline__ float centre(float v, float v1, float v2, float v12) {
-  const float h2 = 0.5f * (v + v1), h1 = 0.5f * (v2 + v12);
-  return 0.5f * (h1 + h2);
+  return 0.25f * ((v2 + v12) + (v + v1));  // (the halvings of each average are exact)
 }
 
 // ct = S/np (zero where no ion deposits; the fast divide, two ulps: n is a
 // density, far from where it loses accuracy).
 __device__ __forceinline__ float ct_of(float s, float n) { return n == 0.0f ? 0.0f : __fdividef(s, n); }
+
+// a / b for a normal b: the product with the approximate reciprocal, without
+// the scaling that __fdividef keeps for denormals.
+__device__ __forceinline__ float over(float a, float b) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+  return a * r;
+}
 
 // update_up's face average (gutsp.f:1825-1836) of ct, with ghost images, and
 // the whistler Courant time of check_time_step (gutsf.f:1782-1792) per node,
@@ -1022,6 +1035,11 @@ __global__ void __launch_bounds__(TPB) k_kit(G32 g, const float* S, const float*
 // average along axis m of edge_to_center.  The divide is the fast one (two
 // ulps): the denominator, a density times alpha, is far from the range where
 // it loses accuracy.
+// Bound by issue (ncu, 4.2M nodes: 86 and 89% of the slots in the predictor and
+// the corrector, b_step 79 and 66%), so the halvings are folded, the quotient
+// is two instructions and a face node stores its one image without the loop
+// over all seven: 20 steps of 4 ions a cell, 64x64x64 9.91 -> 9.28 ms,
+// 128x64x64 15.97 -> 15.27, 256x128x128 105.5 -> 103.4; the same bits.
 template <bool CORR>
 __device__ __forceinline__ void aj_ct_node(const G32& g, const float* db, const float* np, const float* up,
                                            const float* b0c, float alpha, float* aj, float* ct, int i, int j, int k) {
@@ -1046,13 +1064,13 @@ __device__ __forceinline__ void aj_ct_node(const G32& g, const float* db, const 
       p[q][0] = B[b]; p[q][1] = B[b + e[q][1]]; p[q][2] = B[b + e[q][2]]; p[q][3] = B[b + e[q][1] + e[q][2]];
     }
   }
-  const float c0x = b0c[0], c0y = b0c[1], c0z = b0c[2];
-  const float a1 = __fdividef(curl_at<0>(g, s), 0.5f * (n0 + nxp) * alpha);
-  const float a2 = __fdividef(curl_at<1>(g, s), 0.5f * (n0 + nyp) * alpha);
-  const float a3 = __fdividef(curl_at<2>(g, s), 0.5f * (n0 + nzp) * alpha);
-  const float a1m = __fdividef(curl_down<0>(g, s), 0.5f * (nxm + n0) * alpha);
-  const float a2m = __fdividef(curl_down<1>(g, s), 0.5f * (nym + n0) * alpha);
-  const float a3m = __fdividef(curl_down<2>(g, s), 0.5f * (nzm + n0) * alpha);
+  const float ha = 0.5f * alpha, c0x = b0c[0], c0y = b0c[1], c0z = b0c[2];
+  const float a1 = over(curl_at<0>(g, s), (n0 + nxp) * ha);
+  const float a2 = over(curl_at<1>(g, s), (n0 + nyp) * ha);
+  const float a3 = over(curl_at<2>(g, s), (n0 + nzp) * ha);
+  const float a1m = over(curl_down<0>(g, s), (nxm + n0) * ha);
+  const float a2m = over(curl_down<1>(g, s), (nym + n0) * ha);
+  const float a3m = over(curl_down<2>(g, s), (nzm + n0) * ha);
   const float ax = 0.5f * ((a1 - ux) + (a1m - uxm));
   const float ay = 0.5f * ((a2 - uy) + (a2m - uym));
   const float az = 0.5f * ((a3 - uz) + (a3m - uzm));
