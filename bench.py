@@ -145,6 +145,10 @@ KERNEL_BYTES_F64 = {
     "vplus_vminus": 12 + 64 + 8 + 24 + 24 + 48,  # + Ep, vp; write v+, v-
     "vp_final": 24 + 24 + 24 + 48,
     "move_half": 24 + 24 + 24,
+    # the fused step's passes
+    "pass1": 24 + 24 + 24 + 8 + 12 + 64,                # read xp, vp, vp1, beta_p; write ijk, wght
+    "pass2": 12 + 64 + 24 + 8 + 8 + 24,                 # read ijk, wght, vp, mrat, beta_p; write B
+    "pass3": 12 + 64 + 24 + 24 + 24 + 8 + 8 + 72 + 76,  # + B, xp; write xp, vp, vp1, ijk, wght
 }
 
 
@@ -154,6 +158,8 @@ KERNEL_BYTES_F32 = {
     "f32_P1": 41,                # read state (deposit only)
     "f32_P2": 29,                # read cell, offsets, v, species
     "f32_P3": 29 + 40 + 4,       # + write v, vp1, cell, offsets and the sort's direction/rank
+    "f32_P1_sort": 4 + 41 + 41,  # read the place and the state, write the state in order
+    "f32_sort_perm": 4 + 4 + 4,  # read cell and sort word, write the place
     "f32_sort_scatter": 41 + 4 + 41,
     "f32_sort_prep": 4 + 4,
 }
@@ -164,14 +170,13 @@ KERNEL_BYTES_F32 = {
 KERNEL_TRAFFIC_F32 = {"f32_P1": 44.4, "f32_P2": 34.1, "f32_P3": 70.5, "f32_sort_scatter": 86.0}
 # per interior node (FP32 fields, double-float B levels of 8 B per component)
 NODE_BYTES_F32 = {
-    "f32_curlB": 12 + 4 + 12,
     "f32_aj_ct_pred": 12 + 4 + 12 + 12 + 12,        # read dB, np, up; write aj, ct
     "f32_aj_ct_corr": 12 + 4 + 12 + 12 + 12,
     "f32_bstep_pred": 12 + 12 + 4 + 24 + 12 + 12,  # read ct, aj, nu, B, dB1; write dB(m+1/2)
     "f32_bstep_corr": 12 + 12 + 4 + 24 + 24 + 12,    # read ct, aj, nu, B; write B, dB
-    "f32_kit": 36 + 32,
+    "f32_kit": 12 + 12 + 4 + 32,                     # read S, dB, np; write the table
     "f32_node_sum": 16 * 2 + 16,
-    "f32_ct_up": 16 + 12,
+    "f32_up_courant": 4 + 12 + 12 + 12 + 4,          # read np, S, dB; write up, the Courant times
 }
 
 
@@ -365,7 +370,7 @@ def run_surrogate(h, args, N, ws, net, info):
     n = C.c_int32()
     lib.swap_profile_read(ctx, 64, names, tot, cnt, C.byref(n))
     field = {names[i].decode(): tot[i] / args.steps for i in range(min(n.value, 64))
-             if names[i].decode().startswith(("f32_sur", "f32_aj_ct", "f32_bstep", "f32_courant"))}
+             if names[i].decode().startswith(("f32_sur", "f32_aj_ct", "f32_bstep", "f32_field_loop", "f32_up_courant"))}
     attach_surrogate(h, None)
     h.f32_end()
     return dict(info, ms_per_step=t_ms / args.steps, value=N * args.steps * ws / (t_ms / 1e3), unit=UNIT,
