@@ -1271,10 +1271,10 @@ __global__ void __launch_bounds__(FBX * FBY) k_bstep(G32 g, const float* ct,
 // operands.  Two forms.  CLUSTER: one cluster of FIELD_CLUSTER blocks, which
 // meet at the hardware's cluster barrier (0.24 us) -- up to FIELD_CLUSTER *
 // LOOP_TPB nodes.  Otherwise a cooperative launch with a counter in memory
-// (1.2 us at 152 blocks; grid_loop.cuh).
-// A step of 4 ions per cell, loop against launches, in ms: 33k nodes 0.218
-// against 0.229, 65k 0.245 against 0.258, 78k 0.267 against 0.279, 98k 0.331
-// against 0.300, 131k 0.375 against 0.351 (a second round of nodes per thread
+// (0.9 us at 152 blocks; grid_loop.cuh).
+// A step of 4 ions per cell, loop against launches, in ms: 33k nodes 0.189
+// against 0.213, 65k 0.226 against 0.253, 78k 0.258 against 0.262, 98k 0.317
+// against 0.289, 131k 0.362 against 0.336 (a second round of nodes per thread
 // costs more than the launches, which overlap: launch_next.cuh): hence
 // FIELD_LOOP_NODES.
 constexpr int LOOP_TPB = 512;

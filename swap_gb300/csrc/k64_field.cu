@@ -466,13 +466,14 @@ __global__ void __launch_bounds__(TPB) k_kit(Geo g, double* aj, const double* up
 // ---- the whole field step of a small grid in one launch ----
 //
 // The eight kernels of a subcycle as phases of one cooperative kernel, whose
-// blocks meet at a barrier (1.2 us) instead of in a launch: below
+// blocks meet at a barrier (0.9 us) instead of in a launch: below
 // FIELD_LOOP_NODES a phase's FP64 work is about as long as a launch and the
 // ramp of its loads.  The same node functions on the same operands: the same
-// bits.  A step of 4 ions per cell, loop against launches, in ms: 33k nodes
-// 0.58 against 0.78, 65k 0.84 against 1.00, 98k 1.17 against 1.26, 131k 1.41
-// against 1.63, 164k 1.74 against 1.76, 262k 2.48 against 2.40 (16 warps per SM
-// then hide less than a full SM): hence FIELD_LOOP_NODES.
+// bits.  A step of 4 ions per cell, loop against launches, in ms: 1k nodes
+// 0.390 against 0.396, 33k 0.56 against 0.79, 65k 0.82 against 1.01, 98k 1.14
+// against 1.27, 131k 1.38 against 1.64, 164k 1.70 against 1.77, 262k 2.46
+// against 2.41 (16 warps per SM then hide less than a full SM): hence
+// FIELD_LOOP_NODES.
 constexpr int LOOP_TPB = 512;
 template <int SP>
 __global__ void __launch_bounds__(LOOP_TPB) k_field_loop(Geo g, FieldLoop64 f) {
