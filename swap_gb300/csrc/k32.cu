@@ -922,12 +922,12 @@ __device__ __forceinline__ float centre(float v, float v1, float v2, float v12) 
 // density, far from where it loses accuracy).
 __device__ __forceinline__ float ct_of(float s, float n) { return n == 0.0f ? 0.0f : __fdividef(s, n); }
 
-// a / b for a normal b: the product with the approximate reciprocal, without
-// the scaling that __fdividef keeps for denormals.
-__device__ __forceinline__ float over(float a, float b) {
+// The approximate reciprocal of a normal number: a times it is the fast divide
+// without the scaling that __fdividef keeps for denormals.
+__device__ __forceinline__ float reciprocal(float x) {
   float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
-  return a * r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
 }
 
 // update_up's face average (gutsp.f:1825-1836) of ct, with ghost images, and
@@ -1040,17 +1040,33 @@ __global__ void __launch_bounds__(TPB) k_kit(G32 g, const float* S, const float*
 // is two instructions and a face node stores its one image without the loop
 // over all seven: 20 steps of 4 ions a cell, 64x64x64 9.91 -> 9.28 ms,
 // 128x64x64 15.97 -> 15.27, 256x128x128 105.5 -> 103.4; the same bits.
+// FaceTerms: what the density and up give there, the same in every subcycle:
+// the reciprocals of the face densities times alpha at the node (r) and one
+// step down each axis (rm), and up there.
+struct FaceTerms {
+  float r1, r2, r3, r1m, r2m, r3m, ux, uxm, uy, uym, uz, uzm;
+};
+__device__ __forceinline__ FaceTerms face_terms(const G32& g, const float* np, const float* up, float alpha, int i,
+                                                int j, int k) {
+  const Off d = off_of(g, i, j, k);
+  const unsigned o = at_node(g, i, j, k);
+  const In u1{up}, u2{up + g.C}, u3{up + 2 * g.C}, N{np};
+  const float n0 = N[o], nxm = N[o + d.xm], nxp = N[o + d.xp], nym = N[o + d.ym], nyp = N[o + d.yp],
+              nzm = N[o + d.zm], nzp = N[o + d.zp];
+  FaceTerms f;
+  f.ux = u1[o]; f.uxm = u1[o + d.xm]; f.uy = u2[o]; f.uym = u2[o + d.ym]; f.uz = u3[o]; f.uzm = u3[o + d.zm];
+  const float ha = 0.5f * alpha;
+  f.r1 = reciprocal((n0 + nxp) * ha); f.r2 = reciprocal((n0 + nyp) * ha); f.r3 = reciprocal((n0 + nzp) * ha);
+  f.r1m = reciprocal((nxm + n0) * ha); f.r2m = reciprocal((nym + n0) * ha); f.r3m = reciprocal((nzm + n0) * ha);
+  return f;
+}
 template <bool CORR>
-__device__ __forceinline__ void aj_ct_node(const G32& g, const float* db, const float* np, const float* up,
-                                           const float* b0c, float alpha, float* aj, float* ct, int i, int j, int k) {
+__device__ __forceinline__ void aj_ct_node(const G32& g, const float* db, const FaceTerms& ft, const float* b0c,
+                                           float* aj, float* ct, int i, int j, int k) {
   const Off d = off_of(g, i, j, k);
   const long long C = g.C;
   const unsigned o = at_node(g, i, j, k);
-  const In u1{up}, u2{up + C}, u3{up + 2 * C}, N{np};
   const Stencil s = stencil_of(g, db, o, d);
-  const float n0 = N[o], nxm = N[o + d.xm], nxp = N[o + d.xp], nym = N[o + d.ym], nyp = N[o + d.yp],
-              nzm = N[o + d.zm], nzp = N[o + d.zp];
-  const float ux = u1[o], uxm = u1[o + d.xm], uy = u2[o], uym = u2[o + d.ym], uz = u3[o], uzm = u3[o + d.zm];
   // the same four values one step down and up the component's own axis
   float m[3][4], p[3][4];
   if (CORR) {
@@ -1064,16 +1080,16 @@ __device__ __forceinline__ void aj_ct_node(const G32& g, const float* db, const 
       p[q][0] = B[b]; p[q][1] = B[b + e[q][1]]; p[q][2] = B[b + e[q][2]]; p[q][3] = B[b + e[q][1] + e[q][2]];
     }
   }
-  const float ha = 0.5f * alpha, c0x = b0c[0], c0y = b0c[1], c0z = b0c[2];
-  const float a1 = over(curl_at<0>(g, s), (n0 + nxp) * ha);
-  const float a2 = over(curl_at<1>(g, s), (n0 + nyp) * ha);
-  const float a3 = over(curl_at<2>(g, s), (n0 + nzp) * ha);
-  const float a1m = over(curl_down<0>(g, s), (nxm + n0) * ha);
-  const float a2m = over(curl_down<1>(g, s), (nym + n0) * ha);
-  const float a3m = over(curl_down<2>(g, s), (nzm + n0) * ha);
-  const float ax = 0.5f * ((a1 - ux) + (a1m - uxm));
-  const float ay = 0.5f * ((a2 - uy) + (a2m - uym));
-  const float az = 0.5f * ((a3 - uz) + (a3m - uzm));
+  const float c0x = b0c[0], c0y = b0c[1], c0z = b0c[2];
+  const float a1 = curl_at<0>(g, s) * ft.r1;
+  const float a2 = curl_at<1>(g, s) * ft.r2;
+  const float a3 = curl_at<2>(g, s) * ft.r3;
+  const float a1m = curl_down<0>(g, s) * ft.r1m;
+  const float a2m = curl_down<1>(g, s) * ft.r2m;
+  const float a3m = curl_down<2>(g, s) * ft.r3m;
+  const float ax = 0.5f * ((a1 - ft.ux) + (a1m - ft.uxm));
+  const float ay = 0.5f * ((a2 - ft.uy) + (a2m - ft.uym));
+  const float az = 0.5f * ((a3 - ft.uz) + (a3m - ft.uzm));
   float bx = centre(s.b1, s.b1y, s.b1z, s.b1yz), by = centre(s.b2, s.b2x, s.b2z, s.b2xz),
         bz = centre(s.b3, s.b3y, s.b3x, s.b3xy);
   if (CORR) {
@@ -1117,7 +1133,7 @@ __global__ void __launch_bounds__(FBX * FBY) k_aj_ct(G32 g, const float* db,
     }
     prefetch_l2(np + t, nb);
   }
-  aj_ct_node<CORR>(g, db, np, up, b0c, alpha, aj, ct, i, j, k);
+  aj_ct_node<CORR>(g, db, face_terms(g, np, up, alpha, i, j, k), b0c, aj, ct, i, j, k);
 }
 
 // Component m of E = face average of ct + nu*aj at node (i,j,k) (gutsf.f:
@@ -1272,11 +1288,12 @@ __global__ void __launch_bounds__(FBX * FBY) k_bstep(G32 g, const float* ct,
 // meet at the hardware's cluster barrier (0.24 us) -- up to FIELD_CLUSTER *
 // LOOP_TPB nodes.  Otherwise a cooperative launch with a counter in memory
 // (0.9 us at 152 blocks; grid_loop.cuh).
-// A step of 4 ions per cell, loop against launches, in ms: 33k nodes 0.189
-// against 0.213, 65k 0.226 against 0.253, 78k 0.258 against 0.262, 98k 0.317
-// against 0.289, 131k 0.362 against 0.336 (a second round of nodes per thread
-// costs more than the launches, which overlap: launch_next.cuh): hence
-// FIELD_LOOP_NODES.
+// A step of 4 ions per cell, loop against launches, in ms: 33k nodes 0.179
+// against 0.21, 65k 0.215 against 0.25, 78k 0.242 against 0.26; with two nodes
+// per thread 98k 0.317 against 0.289, 131k 0.362 against 0.336 (the launches
+// overlap: launch_next.cuh): hence FIELD_LOOP_NODES, a node per thread.  Its
+// place and what the subcycles share are then found once (20 steps of 64x32x32
+// cells 5.40 -> 5.19 ms, of 16x8x12 3.32 -> 3.13).
 constexpr int LOOP_TPB = 512;
 
 template <bool CLUSTER>
@@ -1285,20 +1302,21 @@ __global__ void __launch_bounds__(LOOP_TPB, 1) k_field_loop(G32 g, FieldLoop f) 
   // now): a failed pass or a Courant violation leaves the state as it is
   if (*f.failed != 0 || (double)*f.courant <= f.courant_floor) return;
   loop::Barrier bar{f.bar, f.polls, 0u, true};
-  const unsigned n = (unsigned)n_int(g), t0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  // a node per thread (field_loop_fits), and what its subcycles share, found once
+  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool mine = t < (unsigned)n_int(g);
+  int i = 2, j = 2, k = 2;
+  if (mine) interior_of(g, t, i, j, k);
+  const FaceTerms ft = face_terms(g, f.np, f.up, f.alpha, i, j, k);
   float *b1h = f.b1h, *b1l = f.b1l, *b12h = f.b12h, *b12l = f.b12l, *bph = f.bph, *bpl = f.bpl, *db1 = f.db1,
         *dbp = f.dbp;
   auto each = [&](auto&& node) {
-    for (unsigned t = t0; t < n; t += step) {
-      int i, j, k;
-      interior_of(g, t, i, j, k);
-      node(i, j, k);
-    }
+    if (mine) node(i, j, k);
     return bar.template sync<CLUSTER>();
   };
   for (int s = 0; s < f.n; ++s) {
     if (!each([&](int i, int j, int k) {
-          aj_ct_node<false>(g, db1, f.np, f.up, f.b0c, f.alpha, f.aj, f.ct, i, j, k);
+          aj_ct_node<false>(g, db1, ft, f.b0c, f.aj, f.ct, i, j, k);
         }))
       break;
     if (!each([&](int i, int j, int k) {
@@ -1307,7 +1325,7 @@ __global__ void __launch_bounds__(LOOP_TPB, 1) k_field_loop(G32 g, FieldLoop f) 
         }))
       break;
     if (!each([&](int i, int j, int k) {
-          aj_ct_node<true>(g, f.dbt, f.np, f.up, f.b0c, f.alpha, f.aj, f.ct, i, j, k);
+          aj_ct_node<true>(g, f.dbt, ft, f.b0c, f.aj, f.ct, i, j, k);
         }))
       break;
     const bool last = s + 1 == f.n;
@@ -2237,14 +2255,22 @@ cudaError_t b_step(const G32& g, bool pred, bool write_e, const float* ct, const
   return swapk::launch_next(k, grid, blk, st, g, ct, nu, aj, gpf, bh, bl, ch, cl, b0c, oh, ol, dbo, db1, dbtp1, E,
                             e_acc, planes_ahead(g, 200000));
 }
-bool field_loop_fits(const G32& g) { return n_int(g) <= FIELD_LOOP_NODES; }
+static int sm_count() {
+  int dev = 0, sms = 0;
+  const bool ok = cudaGetDevice(&dev) == cudaSuccess &&
+                  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess;
+  return ok ? sms : 0;
+}
+bool field_loop_fits(const G32& g) {
+  return n_int(g) <= FIELD_LOOP_NODES && n_int(g) <= (long long)sm_count() * LOOP_TPB;
+}
 
 cudaError_t field_loop(const G32& g, const FieldLoop& f, cudaStream_t st) {
   const long long need = (n_int(g) + LOOP_TPB - 1) / LOOP_TPB;
   if (need <= FIELD_CLUSTER) {  // always the whole cluster: fewer warps share an SM's load path
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(FIELD_CLUSTER);
-    cfg.blockDim = dim3((unsigned)((n_int(g) / FIELD_CLUSTER + 31) / 32 * 32));
+    cfg.blockDim = dim3((unsigned)(((n_int(g) + FIELD_CLUSTER - 1) / FIELD_CLUSTER + 31) / 32 * 32));
     cfg.stream = st;
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeClusterDimension;
@@ -2257,10 +2283,9 @@ cudaError_t field_loop(const G32& g, const FieldLoop& f, cudaStream_t st) {
   G32 gg = g;
   FieldLoop ff = f;
   void* args[] = {&gg, &ff};
-  // the nodes evenly over the SMs, a block on each, and over the rounds of
-  // its threads (whole groups of four warps: fewer blocks meet at the barrier)
-  const long long n = n_int(g), per = (n + 151) / 152, rounds = (per + LOOP_TPB - 1) / LOOP_TPB,
-                  t = ((per + rounds - 1) / rounds + 127) / 128 * 128;
+  // the nodes evenly over the SMs, a block on each (whole groups of four
+  // warps: fewer blocks meet at the barrier)
+  const long long n = n_int(g), sms = sm_count(), t = ((n + sms - 1) / sms + 127) / 128 * 128;
   return loop::launch(reinterpret_cast<const void*>(&k_field_loop<false>), (n + t - 1) / t, (int)t, args, st);
 }
 cudaError_t b_step_given_e(const G32& g, const float* E, const float* bh, const float* bl, double coef,
