@@ -70,10 +70,13 @@ cudaError_t edge_to_center(const Geo& g, double* bt, double* btc, cudaStream_t s
 cudaError_t face_to_center(const Geo& g, double* v, double* vc, double* w, double* wc, cudaStream_t st);
 // up = face average of S/np (zero where np is zero); fill_np: np's ghosts too.
 cudaError_t up_from_sums(const Geo& g, const double* S, double* np, double* up, bool fill_np, cudaStream_t st);
+// n values from one array to two others.
+cudaError_t copy_both(long long n, const double* from, double* a, double* b, cudaStream_t st);
 // The particle passes' gather table, [C][6]: face_to_center(aj - up) and, when
-// full, edge_to_center(bt), with btc and aj's ghosts.
+// full, edge_to_center(bt), with btc and aj's ghosts.  Clears S and, when given,
+// np at the interior nodes, for the next pass's deposit.
 cudaError_t gather_kit(const Geo& g, bool full, double* aj, const double* up, const double* bt, double* btc,
-                       double* kit, cudaStream_t st);
+                       double* kit, double* S, double* np, cudaStream_t st);
 
 // The Courant time per node, and the bits of the smallest into *least.
 cudaError_t deltat_all(const Geo& g, const double* bt, const double* np, double alpha, double dx, double* dtn,

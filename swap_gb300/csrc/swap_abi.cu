@@ -349,8 +349,7 @@ int field_step(swap_ctx* c, double* b1, double* b12, double* b1p2, double* bt, d
   auto copy = [&](double* d, const double* from) {
     return cudaMemcpyAsync(d, from, bytes, cudaMemcpyDeviceToDevice, c->st);
   };
-  KL("cudaMemcpyAsync", copy(b1p2, now));
-  KL("cudaMemcpyAsync", copy(bt, now));
+  KL("copy_both", copy_both(3 * c->g.C, now, b1p2, bt, c->st));
   if (now != b1) {  // an odd count: the levels sit in each other's memory
     KL("cudaMemcpyAsync", copy(b12, b1));
     KL("cudaMemcpyAsync", copy(b1, b1p2));
@@ -1167,13 +1166,10 @@ int step_passes(swap_ctx* c, Bound& b, bool final_move) {
   KL("pass1", particle_pass(1, a, c->st));                                      // :385-386, :399
   KL("up_from_sums", up_from_sums(c->g, c->s_S, b.np, b.up, true, c->st));
   TRY(ops::curlB(c, b.bt, b.np, b.aj));                                         // :395
-  KL("gather_kit", gather_kit(c->g, true, b.aj, b.up, b.bt, b.btc, c->s_kit, c->st));  // :398, :400
-  KL("cudaMemsetAsync", cudaMemsetAsync(c->s_S, 0, 3 * bC, c->st));
+  KL("gather_kit", gather_kit(c->g, true, b.aj, b.up, b.bt, b.btc, c->s_kit, c->s_S, nullptr, c->st));  // :398, :400
   KL("pass2", particle_pass(2, a, c->st));                                      // :400-402
   KL("up_from_sums", up_from_sums(c->g, c->s_S, b.np, b.up, false, c->st));
-  KL("gather_kit", gather_kit(c->g, false, b.aj, b.up, b.bt, b.btc, c->s_kit, c->st));  // :404
-  KL("cudaMemsetAsync", cudaMemsetAsync(b.np, 0, bC, c->st));
-  KL("cudaMemsetAsync", cudaMemsetAsync(c->s_S, 0, 3 * bC, c->st));
+  KL("gather_kit", gather_kit(c->g, false, b.aj, b.up, b.bt, b.btc, c->s_kit, c->s_S, b.np, c->st));  // :404
   KL("pass3", particle_pass(3, a, c->st));                                      // :404-413
   KL("up_from_sums", up_from_sums(c->g, c->s_S, b.np, b.up, true, c->st));
   c->weights_valid = true;
