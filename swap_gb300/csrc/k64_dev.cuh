@@ -62,11 +62,12 @@ __device__ __forceinline__ long long ordered(double x) {
 // when x is outside (q(1), q(n)] or not a number.  An FP32 guess from the
 // uniform spacing is corrected against the node array itself by integer
 // comparisons, so the result is the reference's linear search for any
-// monotone q.
+// monotone q.  The guess is bounded while it is a float: of a position far
+// outside the conversion alone is the largest int, and one more overflows.
 __device__ __forceinline__ int find_cell(const double* __restrict__ q, int n, double x, float q1, float inv_d) {
   const long long xb = ordered(x);
-  int i = (int)((__double2float_rn(x) - q1) * inv_d) + 1;
-  i = i < 1 ? 1 : (i > n - 1 ? n - 1 : i);
+  int i = (int)fminf(fmaxf((__double2float_rn(x) - q1) * inv_d, 0.0f), 1.0e9f) + 1;
+  i = i > n - 1 ? n - 1 : i;
   while (i > 1 && !(xb > ordered(q[i]))) --i;
   while (i < n - 1 && xb > ordered(q[i + 1])) ++i;
   return xb > ordered(q[i]) && xb <= ordered(q[i + 1]) ? i : 0;
