@@ -1186,7 +1186,7 @@ int step_pre(swap_ctx* c, Bound& b, bool final_move = false, bool* moved = nullp
     if (moved) *moved = final_move;
     // an ion that left in the first half move goes on outwards in the second:
     // one removal after both takes the same ions
-    return final_move ? SWAP_OK : srcops::after_move(c, b.xp, b.vp, b.vp1);
+    return final_move ? SWAP_OK : srcops::after_move(c, b.xp, b.vp, b.vp1, srcops::Weights::Keep);
   }
   TRY(push_array(c, &c->w_Ep));
   TRY(push_array(c, &c->w_vplus));
@@ -1204,7 +1204,7 @@ int step_pre(swap_ctx* c, Bound& b, bool final_move = false, bool* moved = nullp
   TRY(ops::vpm(c, c->w_Ep, b.btc, b.vp, c->w_vplus, c->w_vminus));           // :405
   TRY(ops::vp_final(c, c->w_Ep, b.vp, b.vp1, c->w_vplus));                   // :406
   TRY(ops::move_ion_half(c, b.xp, b.vp));                                    // :408
-  TRY(srcops::after_move(c, b.xp, b.vp, b.vp1));                             // outflow
+  TRY(srcops::after_move(c, b.xp, b.vp, b.vp1, srcops::Weights::Drop));      // outflow
   TRY(ops::get_interp_weights(c, b.xp));                                     // :411
   TRY(ops::update_np(c, b.np));                                              // :412
   TRY(ops::update_up_mode(c, 0, b.vp, nullptr, nullptr, b.np, b.up));        // :413
@@ -1223,7 +1223,7 @@ int subcycles(swap_ctx* c, Bound& b) {
 // maind.f:479 and the sinks after it (res_chex, maind.f:484).
 int step_post(swap_ctx* c, Bound& b, bool moved = false) {
   if (!moved) TRY(ops::move_ion_half(c, b.xp, b.vp));
-  TRY(srcops::after_move(c, b.xp, b.vp, b.vp1));
+  TRY(srcops::after_move(c, b.xp, b.vp, b.vp1, moved ? srcops::Weights::KeepIfNoneLate : srcops::Weights::Drop));
   TRY(srcops::step_end(c, b.xp, b.vp, b.vp1));
   return SWAP_OK;
 }

@@ -23,8 +23,13 @@ namespace srcops {
 bool x_open(const swap_ctx* c);
 // Start of a fused step: ionization, cloud ionization, inflow.
 int step_begin(swap_ctx* c, double* xp, double* vp, double* vp1);
+// What an outflow removal does with the ions' cells and weights: they are
+// stale after it; they were formed at the present positions and are kept for
+// the ions that stay; or they are of a whole step's pass 3 (formed between its
+// half moves), and kept when no ion left in the second one.
+enum class Weights { Drop, Keep, KeepIfNoneLate };
 // After each half move: outflow removal when x is open.
-int after_move(swap_ctx* c, double* xp, double* vp, double* vp1);
+int after_move(swap_ctx* c, double* xp, double* vp, double* vp1, Weights w);
 // End of a fused step: res_chex, then the step counter advances.
 int step_end(swap_ctx* c, double* xp, double* vp, double* vp1);
 void free_all(swap_ctx* c);

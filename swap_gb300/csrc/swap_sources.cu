@@ -125,9 +125,19 @@ __global__ void k_chex(PView p, long long N, swap_sources s, long long step, dou
   if (mine) atomicAdd(count, mine);
 }
 
-__global__ void k_outflow_flags(Geo g, const double* xp, long long N, int64_t* keep) {
-  for (long long l = blockIdx.x * (long long)blockDim.x + threadIdx.x; l < N; l += (long long)gridDim.x * blockDim.x)
-    keep[l] = (xp[l] > g.qx[1] && !(xp[l] > g.qx[g.nx - 1])) ? 1 : 0;
+// late (may be null): counts the ions outside that have weights (pass 3 of a
+// whole step leaves those that its first half move took out without).
+__global__ void k_outflow_flags(Geo g, const double* xp, long long N, int64_t* keep, const double* wght, long long NM,
+                                unsigned long long* late) {
+  for (long long l = blockIdx.x * (long long)blockDim.x + threadIdx.x; l < N; l += (long long)gridDim.x * blockDim.x) {
+    const bool in = xp[l] > g.qx[1] && !(xp[l] > g.qx[g.nx - 1]);
+    keep[l] = in ? 1 : 0;
+    if (!in && late) {
+      bool has = false;
+      for (int c = 0; c < 8; ++c) has = has || wght[l + c * NM] != 0.0;
+      if (has) atomicAdd(late, 1ull);
+    }
+  }
 }
 
 __global__ void k_keep_all_but(long long N, long long drop, int64_t* keep) {
@@ -320,9 +330,10 @@ int compact_one(swap_ctx* c, T* a, long long N, long long kept) {
 
 // Stable removal of the particles whose src_flag is 0 from xp, vp, vp1, mrat
 // and beta_p: the bulk form of remove_ion's shift (gutsp.f:29-41).  With
-// keep_weights the device ijkp/wght are shifted too (gutsp.f:33,37-39);
-// otherwise they are marked stale.
-int compact_particles(swap_ctx* c, double* xp, double* vp, double* vp1, bool keep_weights) {
+// keep_weights (looked at once the stream has been waited for) the device
+// ijkp/wght are shifted too (gutsp.f:33,37-39); otherwise they are marked stale.
+template <class Keep>
+int compact_particles(swap_ctx* c, double* xp, double* vp, double* vp1, Keep&& keep_weights) {
   const long long N = c->ntot(), NM = c->dims.ni_max;
   long long kept = 0;
   TRY(scan_count(c, N, &kept));
@@ -334,7 +345,7 @@ int compact_particles(swap_ctx* c, double* xp, double* vp, double* vp1, bool kee
   }
   TRY(compact_one(c, c->d_mrat, N, kept));
   TRY(compact_one(c, c->d_beta_p, N, kept));
-  if (keep_weights && c->weights_valid && c->weights_n >= N) {
+  if (keep_weights() && c->weights_valid && c->weights_n >= N) {
     for (int m = 0; m < 3; ++m) TRY(compact_one(c, c->d_ijk + m * NM, N, kept));
     for (int m = 0; m < 8; ++m) TRY(compact_one(c, c->d_wght + m * NM, N, kept));
     c->weights_n = kept;
@@ -422,16 +433,23 @@ int src_cloud(swap_ctx* c, double* xp, double* vp, double* vp1, long long m) {
   return SWAP_OK;
 }
 
-int src_outflow(swap_ctx* c, double* xp, double* vp, double* vp1, bool keep_weights) {
+int src_outflow(swap_ctx* c, double* xp, double* vp, double* vp1, srcops::Weights w) {
   const long long N = c->ntot();
   if (N <= 0) return SWAP_OK;
   TRY(src_scratch(c, N));
+  const bool count = w == srcops::Weights::KeepIfNoneLate && c->weights_valid && c->weights_n >= N;
+  unsigned long long* late = count ? c->src_cnt + 2 : nullptr;
+  if (count) CU(cudaMemsetAsync(late, 0, sizeof(*late), c->st));
   {
     ProfScope ps(c, "src_outflow", c->st);
-    k_outflow_flags<<<nb(N), TPB, 0, c->st>>>(c->g, xp, N, c->src_flag);
+    k_outflow_flags<<<nb(N), TPB, 0, c->st>>>(c->g, xp, N, c->src_flag, c->d_wght, c->dims.ni_max, late);
   }
   CU(cudaGetLastError());
-  return compact_particles(c, xp, vp, vp1, keep_weights);
+  if (count)
+    CU(cudaMemcpyAsync(&c->pinned->late, late, sizeof(*late), cudaMemcpyDeviceToHost, c->st));
+  return compact_particles(c, xp, vp, vp1, [&] {
+    return w == srcops::Weights::Keep || (count && c->pinned->late == 0);
+  });
 }
 
 // res_chex over the live particles; the count of this call goes to
@@ -479,9 +497,9 @@ int step_begin(swap_ctx* c, double* xp, double* vp, double* vp1) {
   return SWAP_OK;
 }
 
-int after_move(swap_ctx* c, double* xp, double* vp, double* vp1) {
+int after_move(swap_ctx* c, double* xp, double* vp, double* vp1, Weights w) {
   if (!x_open(c)) return SWAP_OK;
-  return src_outflow(c, xp, vp, vp1, false);
+  return src_outflow(c, xp, vp, vp1, w);
 }
 
 int step_end(swap_ctx* c, double* xp, double* vp, double* vp1) {
@@ -701,7 +719,7 @@ extern "C" int swap_remove_outflow_x(swap_ctx* c) {
   TRY(touch_scalars(c));
   double *dxp, *dvp, *dvp1;
   TRY(bound_particles(c, &dxp, &dvp, &dvp1));
-  TRY(src_outflow(c, dxp, dvp, dvp1, true));
+  TRY(src_outflow(c, dxp, dvp, dvp1, srcops::Weights::Keep));
   return c->finish();
 }
 
@@ -718,7 +736,7 @@ extern "C" int swap_remove_ion(swap_ctx* c, double* xp, double* vp, double* vp1,
   TRY(src_scratch(c, N));
   k_keep_all_but<<<nb(N), TPB, 0, c->st>>>(N, (long long)ion_l - 1, c->src_flag);
   CU(cudaGetLastError());
-  TRY(compact_particles(c, dxp, dvp, dvp1, true));
+  TRY(compact_particles(c, dxp, dvp, dvp1, [] { return true; }));
   return c->finish();
 }
 
