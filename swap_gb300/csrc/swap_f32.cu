@@ -38,6 +38,7 @@ struct F32State {
   // then: buf[1 - cur] still holds them, buf[cur] is theirs to be)
   int32_t* perm = nullptr;
   bool move_pending = false;
+  bool over = false;  // start[] counts more ions than the arrays hold, or a step failed half-way: no pass may run
   uint16_t* dep = nullptr;
   uint16_t* pre = nullptr;
   void* partial = nullptr;  // brick partial tiles, 8 bytes per entry (fixed point or FP32)
@@ -666,7 +667,8 @@ static int sort_body(swap_ctx* c, F32State* s, long long src_step, bool prepared
     int64_t n = 0;
     CU(cudaMemcpyAsync(&n, s->start + g.nkeys, sizeof(int64_t), cudaMemcpyDeviceToHost, c->st));
     CU(cudaStreamSynchronize(c->st));
-    if (n > cap) return c->fail(SWAP_ECAPACITY, "Ni_max exceeded by new ions");
+    s->over = n > cap;
+    if (s->over) return c->fail(SWAP_ECAPACITY, "Ni_max exceeded by new ions");
     s->N = n;
   }
   return SWAP_OK;
@@ -817,22 +819,39 @@ static int stage_ahead(swap_ctx* c, F32State* s, long long m, PreStaged* pre) {
 }
 
 static int one_step_body(swap_ctx* c, F32State* s, bool more);
-// A step; after a failure the second stream's work (a sort already queued)
-// is drained, so that nothing of the step runs on when the caller goes on.
+// After a failed step: the second stream's work (a sort already queued) is
+// drained, so that nothing of the step runs on when the caller goes on, and
+// the state is made whole: the ions that start[] counts (the sort's count where
+// sources change it, as many as there is room for) lie where it says.
+static int settle(swap_ctx* c, F32State* s) {
+  s->sort_pending = false;
+  const bool moves = s->move_pending;
+  s->move_pending = false;
+  CU(cudaStreamSynchronize(s->side));
+  if (s->src_on) {
+    int64_t n = 0;
+    CU(cudaMemcpyAsync(&n, s->start + s->g.nkeys, sizeof(n), cudaMemcpyDeviceToHost, c->st));
+    CU(cudaStreamSynchronize(c->st));
+    s->over = n > c->dims.ni_max;
+    s->N = std::min<int64_t>(n, c->dims.ni_max);
+  }
+  if (moves) CU(move_sorted(s->N, s->perm, s->buf[1 - s->cur], s->stage.part, s->buf[s->cur], c->st));
+  CU(cudaStreamSynchronize(c->st));
+  return SWAP_OK;
+}
 // more: another step of the same call follows, whose pass 1 may make this
 // step's sorted moves.
 static int one_step(swap_ctx* c, F32State* s, bool more) {
   const int r = one_step_body(c, s, more);
-  if (r && s->sort_pending) {
-    cudaStreamSynchronize(s->side);
-    s->sort_pending = false;
-  }
-  if (r && s->move_pending) {  // leave the ions where the rest of the state says they are
-    s->move_pending = false;
-    if (s->N <= c->dims.ni_max)
-      move_sorted(s->N, s->perm, s->buf[1 - s->cur], s->stage.part, s->buf[s->cur], c->st);
-  }
+  if (!r) return SWAP_OK;
+  const std::string why = c->err;  // of the step, also when settling fails
+  if (settle(c, s)) s->over = true;
+  c->err = why;
   return r;
+}
+// Whether the passes may run: start[] counts no more ions than there is room for.
+static int whole(swap_ctx* c, const F32State* s) {
+  return s->over ? c->fail(SWAP_ECAPACITY, "the last step left no room for its ions, or stopped half-way: call swap_f32_begin again") : SWAP_OK;
 }
 
 static int one_step_body(swap_ctx* c, F32State* s, bool more) {
@@ -841,9 +860,9 @@ static int one_step_body(swap_ctx* c, F32State* s, bool more) {
   const Part& p = s->buf[s->cur];
   // :385-387,399
   if (s->move_pending) {
-    s->move_pending = false;
     KL("f32_P1_sort", pass1_sort(g, s->buf[1 - s->cur], s->stage.part, p, s->sp, s->start, s->perm, s->partial,
                                  s->exact, c->d_err, c->st));
+    s->move_pending = false;
   } else {
     KL("f32_P1", pass(1, g, p, s->sp, sp, s->start, s->kit, s->partial, nullptr, nullptr, c->d_err, s->exact, c->st));
   }
@@ -887,6 +906,7 @@ extern "C" int swap_f32_run(swap_ctx* c, int32_t nsteps) {
   F32State* s = f32(c);
   if (!s) return c->fail(SWAP_EINVAL, "swap_f32_begin has not been called");
   if (s->ended && s->src_on) return c->fail(SWAP_EINVAL, "call swap_f32_begin again after swap_f32_end");
+  TRY(whole(c, s));
   for (int k = 0; k < nsteps; ++k) TRY(one_step(c, s, k + 1 < nsteps));
   return check_err(c);
 }
@@ -1020,6 +1040,7 @@ extern "C" int swap_f32_displace_resort(swap_ctx* c, int64_t n, const int64_t* i
   if (!c || n < 0 || (n > 0 && (!idx || !dcell))) return SWAP_EINVAL;
   F32State* s = f32(c);
   if (!s) return c->fail(SWAP_EINVAL, "swap_f32_begin has not been called");
+  TRY(whole(c, s));
   for (int64_t q = 0; q < n; ++q) {
     if (idx[q] < 0 || idx[q] >= s->N) return c->fail(SWAP_EINVAL, "particle index out of range");
     if (pk_i(dcell[q]) > 2 || pk_j(dcell[q]) > 2 || pk_k(dcell[q]) > 2 || (dcell[q] >> 30))
@@ -1106,7 +1127,7 @@ int swap_f32_checkpoint(swap_ctx* c, std::FILE* f, bool write) {
       if (bl.bytes) CU(cudaMemcpy(bl.dev, buf.data(), bl.bytes, cudaMemcpyHostToDevice));
     }
   }
-  if (!write) s->ended = false;
+  if (!write) s->ended = s->over = false;
   return SWAP_OK;
 }
 
@@ -1118,6 +1139,7 @@ extern "C" int swap_surrogate_collect(swap_surrogate* net, swap_ctx* c, int32_t 
   if (!net || !c || nsteps < 0) return SWAP_EINVAL;
   F32State* s = f32(c);
   if (!s || s->ended) return c->fail(SWAP_EINVAL, "swap_f32_begin has not been called");
+  TRY(whole(c, s));
   s->collect = net;
   int r = SWAP_OK;
   for (int k = 0; k < nsteps && !r; ++k) r = one_step(c, s, k + 1 < nsteps);
