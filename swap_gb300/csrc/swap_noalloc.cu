@@ -148,9 +148,12 @@ extern "C" int swap_update_up_noalloc(const swap_dims* dims, const swap_params* 
   g.inv_dx = 1.0 / (coords->qx[1] - coords->qx[0]);
   g.inv_dz = 1.0 / (coords->qz[1] - coords->qz[0]);
   swapk::set_cell_constants(g, coords->qx, coords->qy, coords->qz, nullptr, nullptr, nullptr);
-  if (ni_tot > 0)
-    k_na_deposit<<<(unsigned)((ni_tot + 127) / 128), 128, 0, st>>>(g, xp, vp, beta_p, ni_tot, dims->ni_max,
-                                                                   params->beta, S, flag);
+  if (ni_tot > 0) {
+    const long long blocks = (ni_tot + 127) / 128;
+    if (blocks > 0x7fffffffLL) return fail_after_enqueue();  // the unsigned conversion must not wrap
+    k_na_deposit<<<(unsigned)blocks, 128, 0, st>>>(g, xp, vp, beta_p, ni_tot, dims->ni_max, params->beta, S, flag);
+    if (cudaGetLastError() != cudaSuccess) return fail_after_enqueue();
+  }
   // the face average of S/np (gutsp.f:1825-1839) with up's ghosts; np is only read
   if (swapk::up_from_sums(g, S, const_cast<double*>(np), up, false, st) != cudaSuccess) return fail_after_enqueue();
   int hflag = 0;
