@@ -1878,7 +1878,8 @@ __device__ __forceinline__ float narrow(double x) {
 // split_axis with the reciprocal r of d (1/d rounded; UNIT: d is one): the
 // quotient from one product and its exact remainder (Markstein 1990), the
 // nearest whole number by adding 1.5 * 2^52.  What that does not cover
-// (differences of 2^15 and more, tiny or zero ones, NaN) goes to split_axis.
+// (differences or quotients of 2^15 and more -- a quotient beyond 2^31 would wrap
+// in the low word --, tiny or zero differences, NaN) goes to split_axis.
 struct Spacing {
   double d[3], r[3];
 };
@@ -1891,6 +1892,7 @@ __device__ __forceinline__ bool split_fast(double x, double q1, double d, double
   if (!UNIT) {
     u = a * r;
     u = __fma_rn(__fma_rn(-u, d, a), r, u);
+    if (((unsigned)__double2hiint(u) & 0x7fffffffu) >= 0x40e00000u) return split_axis(x, q1, d, n, UPPER, c, o);
   }
   constexpr double M = 6755399441055744.0;
   const double t = u + M;
