@@ -49,12 +49,12 @@ __device__ __forceinline__ double reciprocal(double d) {
   return e - 963u <= 120u && !ones ? 1.0 / d : 0.0;
 }
 
-// The bits of a double as an integer that orders like it (NaN beyond the
-// infinities): a comparison costs a few integer instructions instead of one
-// of the FP64 pipe's 16-clock slots.
+// The bits of a double as an integer that orders like it (the two zeros alike,
+// NaN beyond the infinities): a comparison costs a few integer instructions
+// instead of one of the FP64 pipe's 16-clock slots.
 __device__ __forceinline__ long long ordered(double x) {
-  const long long b = __double_as_longlong(x);
-  return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+  const long long b = __double_as_longlong(x), m = b >> 63;
+  return (b ^ (m & 0x7fffffffffffffffLL)) - m;
 }
 
 // Cell search of get_interp_weights (gutsp.f:1396-1401): the index i with
