@@ -822,7 +822,8 @@ static int one_step_body(swap_ctx* c, F32State* s, bool more);
 // After a failed step: the second stream's work (a sort already queued) is
 // drained, so that nothing of the step runs on when the caller goes on, and
 // the state is made whole: the ions that start[] counts (the sort's count where
-// sources change it, as many as there is room for) lie where it says.
+// sources change it, as many as there is room for) lie where it says.  The step's
+// failure is reported already: its error word does not fail the next entry.
 static int settle(swap_ctx* c, F32State* s) {
   s->sort_pending = false;
   const bool moves = s->move_pending;
@@ -836,6 +837,8 @@ static int settle(swap_ctx* c, F32State* s) {
     s->N = std::min<int64_t>(n, c->dims.ni_max);
   }
   if (moves) CU(move_sorted(s->N, s->perm, s->buf[1 - s->cur], s->stage.part, s->buf[s->cur], c->st));
+  CU(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->st));
+  CU(cudaMemsetAsync(s->loop_bar, 0, 2 * sizeof(unsigned), c->st));
   CU(cudaStreamSynchronize(c->st));
   return SWAP_OK;
 }
