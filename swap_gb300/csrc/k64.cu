@@ -106,6 +106,14 @@ __global__ void k_weights(Geo g, PartDev p, long long N, int* err) {
   }
 }
 
+// The cells to another ijkp array; an entry that failed leaves it as it was.
+__global__ void k_copy_cells(PartDev p, long long N, int32_t* __restrict__ ijkp, const int* err) {
+  if (*err) return;
+  GRID_STRIDE(l, N) {
+    for (int m = 0; m < 3; ++m) ijkp[l + m * p.NM] = p.ijk[l + m * p.NM];
+  }
+}
+
 // A cell index triple is usable for node addressing only inside
 // [1,n-1] on every axis; anything else is reported and skipped.
 __device__ __forceinline__ bool cell_ok(const Geo& g, int i, int j, int k) {
@@ -569,6 +577,10 @@ cudaError_t deltat_all(const Geo& g, const double* bt, const double* np, double 
 cudaError_t interp_weights(const Geo& g, const PartDev& p, long long N, int* err, cudaStream_t st) {
   if (N <= 0) return cudaSuccess;
   LAUNCH_P(k_weights, N, g, p, N, err);
+}
+cudaError_t copy_cells(const PartDev& p, long long N, int32_t* ijkp, const int* err, cudaStream_t st) {
+  if (N <= 0) return cudaSuccess;
+  LAUNCH_P(k_copy_cells, N, p, N, ijkp, err);
 }
 cudaError_t deposit_np(const Geo& g, const PartDev& p, long long N, double beta, double* np, int* err,
                        cudaStream_t st, Fix64 fix) {

@@ -85,6 +85,8 @@ cudaError_t grad_pe_face_int(const Geo& g, const double* np, double grad_pe, dou
 
 // gutsp.f particle operators
 cudaError_t interp_weights(const Geo& g, const PartDev& p, long long N, int* err, cudaStream_t st);
+// The cells of the first N particles to another ijkp array, unless *err is set.
+cudaError_t copy_cells(const PartDev& p, long long N, int32_t* ijkp, const int* err, cudaStream_t st);
 // Deterministic deposits: each added value x goes into a 128-bit fixed-point
 // sum in units of 2^-60, as floor(x * 2^28) into a signed 64-bit word (h)
 // and the rest * 2^32, rounded, into an unsigned one (l).  Integer adds are

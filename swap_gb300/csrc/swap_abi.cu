@@ -833,16 +833,9 @@ extern "C" int swap_get_interp_weights(swap_ctx* c, const double* xp) {
   TRY(c->use(xp, Access::In, &dxp));
   TRY(ops::get_interp_weights(c, dxp));
   Mirror* m = c->h_ijkp ? c->find(c->h_ijkp) : nullptr;
-  cudaError_t e = cudaSuccess;
-  if (m) {  // the COMMON ijkp mirror takes the new indices
-    const std::size_t NM = (std::size_t)c->dims.ni_max;
-    for (int k = 0; k < 3 && e == cudaSuccess && c->ntot() > 0; ++k)
-      e = cudaMemcpyAsync(static_cast<int32_t*>(m->dev) + k * NM, c->d_ijk + k * NM, (std::size_t)c->ntot() * 4,
-                          cudaMemcpyDeviceToDevice, c->st);
-  }
-  const int r = c->finish();  // also after a failed copy: nothing stays queued
-  if (r) return r;
-  if (e != cudaSuccess) return c->cuda_fail(e, "ijkp mirror");
+  // the COMMON ijkp mirror takes the new indices, unless a particle lies outside
+  if (m) KL("copy_cells", copy_cells(c->part_view(), c->ntot(), static_cast<int32_t*>(m->dev), c->d_err, c->st));
+  TRY(c->finish());
   if (m) {
     m->dev_valid = true;
     m->host_valid = false;

@@ -94,3 +94,26 @@ def test_a_move_onto_a_face_at_minus_zero():
         got.append(h.xp[3].copy())
         h.close()
     assert np.array_equal(got[0], got[1]) and got[0][0] == 7.0 and got[0][2] == 6.0
+
+
+def test_a_refused_call_leaves_the_cells_of_the_one_before():
+    h = _make()
+    n = int(h.ni_tot[0])
+    h.get_interp_weights(h.xp)
+    h.sync_to_host(h.ijkp)
+    had = h.ijkp[:n].copy()
+    h.get_interp_weights(h.xp)  # current on the device alone
+    keep = h.xp.copy(order="F")
+    h.xp[:n] = h.xp[:n][::-1].copy()
+    h.xp[n // 2, 2] = 1e9
+    h.mark_host_dirty(h.xp)
+    with pytest.raises(abi.SwapError, match="EDOMAIN"):
+        h.get_interp_weights(h.xp)
+    h.sync_to_host(h.ijkp)
+    assert np.array_equal(h.ijkp[:n], had)
+    h.xp[:n] = keep[:n][::-1].copy()
+    h.mark_host_dirty(h.xp)
+    h.get_interp_weights(h.xp)
+    h.sync_to_host(h.ijkp)
+    assert np.array_equal(h.ijkp[:n], had[::-1])
+    h.close()
