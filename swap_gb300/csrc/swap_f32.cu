@@ -35,8 +35,10 @@ struct F32State {
   uint32_t* dirrank = nullptr;
   // grids too large for the field loop: between two steps of one run the sort
   // only ranks, and the next pass 1 moves the ions (perm; move_pending until
-  // then: buf[1 - cur] still holds them, buf[cur] is theirs to be)
+  // then: buf[1 - cur] still holds them, buf[cur] is theirs to be).  Made by
+  // the first run of several steps; without room for it the sort moves them.
   int32_t* perm = nullptr;
+  bool perm_tried = false;
   bool move_pending = false;
   bool over = false;  // start[] counts more ions than the arrays hold, or a step failed half-way: no pass may run
   uint16_t* dep = nullptr;
@@ -363,11 +365,6 @@ extern "C" int swap_f32_begin(swap_ctx* c) {
   s->count = s->alloc<int64_t>(nk + 1);
   s->sums = s->alloc<int64_t>(nk / 1024 + 16);
   s->dirrank = s->alloc<uint32_t>(NMs);
-  if (!field_loop_fits(g)) {
-    s->perm = s->alloc<int32_t>(NMs);
-    if (!s->perm) return c->fail(SWAP_ECUDA, "FP32 particle allocation failed");
-    CU(cudaMemsetAsync(s->perm, 0, NMs * sizeof(int32_t), c->st));  // always a place inside the arrays
-  }
   s->dep = s->alloc<uint16_t>(nk * NDIR);
   s->pre = s->alloc<uint16_t>(nk * NDIR);
   s->order = s->alloc<uint8_t>(SORT_CLASSES * NDIR);
@@ -842,9 +839,24 @@ static int settle(swap_ctx* c, F32State* s) {
   CU(cudaStreamSynchronize(c->st));
   return SWAP_OK;
 }
+// perm, when this run of several steps is the first (see F32State).
+static int reserve_perm(swap_ctx* c, F32State* s) {
+  if (s->perm_tried || field_loop_fits(s->g)) return SWAP_OK;
+  s->perm_tried = true;
+  const std::size_t n = (std::size_t)std::max<long long>(c->dims.ni_max, 1);
+  int32_t* p = s->alloc<int32_t>(n);
+  if (!p) {
+    cudaGetLastError();  // not the next launch's
+    return SWAP_OK;
+  }
+  CU(cudaMemsetAsync(p, 0, n * sizeof(int32_t), c->st));  // always a place inside the arrays
+  s->perm = p;
+  return SWAP_OK;
+}
 // more: another step of the same call follows, whose pass 1 may make this
 // step's sorted moves.
 static int one_step(swap_ctx* c, F32State* s, bool more) {
+  if (more) TRY(reserve_perm(c, s));
   const int r = one_step_body(c, s, more);
   if (!r) return SWAP_OK;
   const std::string why = c->err;  // of the step, also when settling fails
