@@ -291,7 +291,8 @@ int swap_checkpoint_read(swap_ctx* ctx, const char* path);
  * 48 significant bits: GB300's FP64 rate is a small fraction of its FP32
  * rate).  The sources and sinks of swap_set_sources apply, with new ions
  * drawn as in the FP64 path and charge exchange drawn per sorted ion.  Needs a uniform grid with
- * 8..1024 physical cells per axis in multiples of 4, a uniform b0, at most 16
+ * 8..1024 physical cells per axis in multiples of 4 and fewer than 2^29 nodes in
+ * all, a uniform b0, at most 16
  * (mrat, beta_p) species.  An ion that moves more than one cell per axis in
  * a step takes a slower path (listed by pass 3, deposited and sorted apart,
  * at most 65536 per step); a half move that spans the grid less two cells,

@@ -820,7 +820,7 @@ __device__ __forceinline__ void prefetch_l2(const float* p, unsigned bytes) {
   const int k = blockIdx.z + 2;                              \
   if (i > g.ncx + 1 || j > g.ncy + 1) return
 
-// Neighbours by 32-bit offsets (3 C < 2^32), at the periodic image where the
+// Neighbours by 32-bit offsets, at the periodic image where the
 // neighbour is a ghost.  Every load of a node stands before its first store:
 // one round trip to memory per node, also on the boundary; and the ghost
 // images of all outputs are stored together.  (A separate path for boundary
@@ -829,7 +829,7 @@ __device__ __forceinline__ void prefetch_l2(const float* p, unsigned bytes) {
 // cells 338 against 331; in the field loop below 307 us a step of 64x32x32
 // cells against 182.)
 
-// Offsets are in bytes and 32 bits wide (a component is below 4 GB), beside
+// Offsets are in bytes and 32 bits wide (addressable(), k32.cuh), beside
 // bases that the whole grid shares: the address of a load is then its base
 // and one register (20 steps of 128x64x64 cells with 64-bit element indices
 // 16.2 ms against 16.0).

@@ -28,6 +28,12 @@ __host__ __device__ constexpr int pass_tile(int pass) { return pass == 3 ? TN : 
 constexpr int NDIR = 27;              // displacements in {-1,0,1}^3
 constexpr int SORT_CLASSES = 216;     // a cell's place in its brick and at the seams, 6 per axis
 constexpr int MAX_SPECIES = 16;
+// The field kernels address a component by 32-bit byte offsets, with the sign
+// of a step to a neighbour: a component stays below 2^31 bytes.  (All the arrays
+// of a context and its FP32 form take about 1 kB a node, so no grid that fits
+// 288 GB comes near.)
+constexpr bool addressable(long long nx, long long ny, long long nz) { return 4 * nx * ny * nz < (1LL << 31); }
+static_assert(addressable(1026, 514, 1010) && !addressable(1026, 1026, 1026) && !addressable(1026, 1026, 514));
 // Inputs per voxel of the field surrogate: B (3), u_p (3), n_p, p_e, E0 (3),
 // and B - b12 (3), the change over the last subcycle (the predictor is a
 // leapfrog from b12, so the subcycles depend on it as well as on B).

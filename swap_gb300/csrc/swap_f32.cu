@@ -219,6 +219,7 @@ extern "C" int swap_f32_begin(swap_ctx* c) {
   const int ncx = nx - 2, ncy = ny - 2, ncz = nz - 2;
   if (ncx % 4 || ncy % 4 || ncz % 4 || ncx < 8 || ncy < 8 || ncz < 8 || ncx > 1024 || ncy > 1024 || ncz > 1024)
     return c->fail(SWAP_EINVAL, "the FP32 form needs 8..1024 physical cells per axis, multiples of 4");
+  if (!addressable(nx, ny, nz)) return c->fail(SWAP_EINVAL, "the FP32 form's grid must stay below 2^29 nodes");
   // uniform spacing per axis
   auto uniform = [](const std::vector<double>& q) {
     const double d = q[1] - q[0];
