@@ -92,8 +92,10 @@ void grd7(Mesh<R>& g, int nx, int ny, int nz, R dx, R dy, R delz, R xsf = 0, R z
     // initial.f:175-191 (x) and 211-231 (z)
     for (int i = rc; i <= rc + nrgrd; ++i)
       if (i >= 1 && i <= n) d[i] = base;
+    // (n = rc + nrgrd + 1: the stretched part is the one node where it starts, 0/0 as written)
+    const int span = n - (rc + nrgrd + 1);
     for (int i = rc + nrgrd + 1; i <= n; ++i)
-      if (i >= 1) d[i] = base + sf * base * R(i - (rc + nrgrd + 1)) / R(n - (rc + nrgrd + 1));
+      if (i >= 1) d[i] = span == 0 ? base : base + sf * base * R(i - (rc + nrgrd + 1)) / R(span);
     for (int i = rc - nrgrd; i <= rc - 1; ++i)
       if (i >= 1 && i <= n) d[i] = base;
     for (int i = 1; i <= rc - nrgrd - 1; ++i) {
