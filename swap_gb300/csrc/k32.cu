@@ -113,6 +113,16 @@ __device__ __forceinline__ float half_step(float& o, float d, int n, bool& ok) {
 constexpr float FLOAT_INT = 12582912.0f;  // 1.5 * 2^23
 __device__ __forceinline__ int float_int(float x) { return __float_as_int(x) - __float_as_int(FLOAT_INT); }
 
+// Offset of a cell from a brick's first cell along one axis, unwrapped across
+// the periodic boundary into the brick tile's window [-1, 4] when one of the
+// periodic images lies there (n >= 8, so at most one does).
+__device__ __forceinline__ int rel_cell(int c, int c0, int n) {
+  int r = c - c0;
+  if (r < -1) r += n;
+  else if (r > 4) r -= n;
+  return r;
+}
+
 // Step between two cells along one axis, unwrapped into [-1, 1] when one of
 // the periodic images lies there.
 __device__ __forceinline__ int step_cell(int c, int c0, int n) {
@@ -514,6 +524,7 @@ __global__ void __launch_bounds__(TPB_PASS, PASS == 3 ? 7 : 8) k_pass(G32 g, Par
           int32_t c2 = (c & ~CELL_FRESH) + float_int(fmaf(1048576.f, sz, fmaf(1024.f, sy, sx + FLOAT_INT)));
           bool out1 = false, out2 = false;
           bool far_ion = false;  // moved more than one cell: placed through the far list
+          bool beside = near;    // ends in its own cell or next to it
           if (rim || !near) {
             const int ix = (int)kx, iy = (int)ky, iz = (int)kz;
             int cx1 = pk_i(c) + ix, cy1 = pk_j(c) + iy, cz1 = pk_k(c) + iz;  // not wrapped
@@ -528,11 +539,18 @@ __global__ void __launch_bounds__(TPB_PASS, PASS == 3 ? 7 : 8) k_pass(G32 g, Par
                       ck2 = wrapi(near ? cz1 + (int)lz : wrapi(cz1, g.ncz) + (int)lz, g.ncz);
             c2 = pk(ci2, cj2, ck2);
             if (!near) {
-              const int rx = bx4 + ix, ry = by4 + iy, rz = bz4 + iz;
+              // the periodic image in the tile's window, and next to the ion's
+              // own cell, counts: a move about once around the box
+              const int rx = rel_cell(wrapi(cx1, g.ncx), c0x, g.ncx), ry = rel_cell(wrapi(cy1, g.ncy), c0y, g.ncy),
+                        rz = rel_cell(wrapi(cz1, g.ncz), c0z, g.ncz);
               const bool inside = rx >= -1 && rx <= 4 && ry >= -1 && ry <= 4 && rz >= -1 && rz <= 4;
               t0 = inside ? (rx + O) + T * ((ry + O) + T * (rz + O)) : -1;
+              const int wx = step_cell(ci2, pk_i(c), g.ncx), wy = step_cell(cj2, pk_j(c), g.ncy),
+                        wz = step_cell(ck2, pk_k(c), g.ncz);
+              beside = wx >= -1 && wx <= 1 && wy >= -1 && wy <= 1 && wz >= -1 && wz <= 1;
+              dir = dir_index(wx, wy, wz);
               // a deposit position outside the tile's window takes the far path too
-              far_ion = !out2 || (!out1 && !inside);
+              far_ion = (!out2 && !beside) || (!out1 && !inside);
             }
           }
           if (CHEX && !out2 && sprm.heavy_of[s] != s) {
@@ -562,7 +580,7 @@ __global__ void __launch_bounds__(TPB_PASS, PASS == 3 ? 7 : 8) k_pass(G32 g, Par
           } else {
             p.cell[l] = c2;
             p.ox[l] = ox; p.oy[l] = oy; p.oz[l] = oz;
-            if (near) grp = (bx4 + 4 * by4 + 16 * bz4) * NDIR + dir;
+            if (beside) grp = (bx4 + 4 * by4 + 16 * bz4) * NDIR + dir;
           }
           ox = dox; oy = doy; oz = doz;  // the deposit uses the maind.f:408 position
           if (out1) live = false;
