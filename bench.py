@@ -165,9 +165,10 @@ KERNEL_BYTES_F32 = {
 }
 # DRAM bytes per particle that ncu measured for these kernels
 # (dram__bytes_read.sum + dram__bytes_write.sum over one launch at 128x64x64
-# cells, 16 ppc, 8.4M particles); the roofline's traffic is this figure times
-# the particles of a launch.
-KERNEL_TRAFFIC_F32 = {"f32_P1": 44.4, "f32_P2": 34.1, "f32_P3": 70.5, "f32_sort_scatter": 86.0}
+# cells, 16 ppc, 8.4M particles; profiles/k_pass_fp32_128x64x64_16ppc.md); the
+# roofline's traffic is this figure times the particles of a launch.
+KERNEL_TRAFFIC_F32 = {"f32_P1": 44.1, "f32_P2": 33.7, "f32_P3": 70.0, "f32_P1_sort": 85.0, "f32_sort_perm": 10.0,
+                      "f32_sort_scatter": 84.8}
 # per interior node (FP32 fields, double-float B levels of 8 B per component)
 NODE_BYTES_F32 = {
     "f32_aj_ct_pred": 12 + 4 + 12 + 12 + 12,        # read dB, np, up; write aj, ct
