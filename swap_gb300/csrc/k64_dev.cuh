@@ -52,12 +52,18 @@ __device__ __forceinline__ double reciprocal(double d) {
   return e - 963u <= 120u && !ones ? 1.0 / d : 0.0;
 }
 
-// The bits of a double as an integer that orders like it (the two zeros alike,
+// The bits of a double as an integer that orders like it (-0.0 just below 0.0,
 // NaN beyond the infinities): a comparison costs a few integer instructions
 // instead of one of the FP64 pipe's 16-clock slots.
 __device__ __forceinline__ long long ordered(double x) {
-  const long long b = __double_as_longlong(x), m = b >> 63;
-  return (b ^ (m & 0x7fffffffffffffffLL)) - m;
+  const long long b = __double_as_longlong(x);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+}
+// The same of a position, to be held against ordered() nodes by > and <= alone:
+// a zero of either sign as -0.0, so that it is not above a node at -0.0 or 0.0.
+__device__ __forceinline__ long long ordered_position(double x) {
+  const long long o = ordered(x);
+  return o == 0 ? -1 : o;
 }
 
 // Cell search of get_interp_weights (gutsp.f:1396-1401): the index i with
@@ -68,7 +74,7 @@ __device__ __forceinline__ long long ordered(double x) {
 // monotone q.  The guess is bounded while it is a float: of a position far
 // outside the conversion alone is the largest int, and one more overflows.
 __device__ __forceinline__ int find_cell(const double* __restrict__ q, int n, double x, float q1, float inv_d) {
-  const long long xb = ordered(x);
+  const long long xb = ordered_position(x);
   int i = (int)fminf(fmaxf((__double2float_rn(x) - q1) * inv_d, 0.0f), 1.0e9f) + 1;
   i = i > n - 1 ? n - 1 : i;
   while (i > 1 && !(xb > ordered(q[i]))) --i;

@@ -54,7 +54,7 @@ __device__ __forceinline__ bool locate(const PassArgs& a, long long l, double x,
 __device__ __forceinline__ double half_move(double x, double v, double dth, double q1, double qn, bool wrap) {
   x = x + dth * v;
   if (wrap) {
-    const long long b = ordered(x);
+    const long long b = ordered_position(x);
     if (b > ordered(qn)) x = q1 + (x - qn);
     else if (b <= ordered(q1)) x = qn - (q1 - x);
   }
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(TPB, 4) k_pass(PassArgs a) {
         double x = half_move(p.xp[l], vn[0], dth, qx1, qxn, !a.x_open);
         double y = half_move(p.xp[l + NM], vn[1], dth, qy1, qyn, true);
         double z = half_move(p.xp[l + 2 * NM], vn[2], dth, qz1, qzn, true);
-        const bool out = a.x_open && !(ordered(x) > ordered(qx1) && ordered(x) <= ordered(qxn));
+        const bool out = a.x_open && !(ordered_position(x) > ordered(qx1) && ordered_position(x) <= ordered(qxn));
         if (out) {  // removed by the caller; its weights are those of no cell
           p.ijk[l] = p.ijk[l + NM] = p.ijk[l + 2 * NM] = 1;
 #pragma unroll
