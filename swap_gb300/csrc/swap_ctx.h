@@ -42,11 +42,9 @@ struct swap_ctx {
   cudaStream_t st = nullptr;
   int* d_err = nullptr;
   // what the host reads back, in page-locked memory: the error word at the
-  // last finish(), the smallest Courant time once ev_look has passed, the ions
-  // that left in a whole step's second half move
+  // last finish(), the smallest Courant time once ev_look has passed
   struct Pinned {
     double courant;
-    unsigned long long late;
     int err;
   };
   Pinned* pinned = nullptr;
@@ -116,7 +114,7 @@ struct swap_ctx {
   long long src_cap = 0;                     // capacity of the scan scratch
   int64_t *src_flag = nullptr, *src_pos = nullptr, *src_sums = nullptr;
   void* src_tmp = nullptr;                   // ni_max elements of 8 bytes
-  unsigned long long* src_cnt = nullptr;     // [0] last res_chex, [1] fused-step total, [2] ions that left late
+  unsigned long long* src_cnt = nullptr;     // [0] last res_chex, [1] fused-step total
 
   cudaEvent_t t0 = nullptr, t1 = nullptr;
 

@@ -125,18 +125,18 @@ __global__ void k_chex(PView p, long long N, swap_sources s, long long step, dou
   if (mine) atomicAdd(count, mine);
 }
 
-// late (may be null): counts the ions outside that have weights (pass 3 of a
-// whole step leaves those that its first half move took out without).
-__global__ void k_outflow_flags(Geo g, const double* xp, long long N, int64_t* keep, const double* wght, long long NM,
-                                unsigned long long* late) {
+// wght (may be null): an ion outside that has weights (pass 3 of a whole step
+// leaves those that its first half move took out without) is flagged LATE, so
+// that the scan of the flags counts the two kinds in the halves of one word.
+constexpr int64_t LATE = 1LL << 32;
+__global__ void k_outflow_flags(Geo g, const double* xp, long long N, int64_t* keep, const double* wght,
+                                long long NM) {
   for (long long l = blockIdx.x * (long long)blockDim.x + threadIdx.x; l < N; l += (long long)gridDim.x * blockDim.x) {
     const bool in = xp[l] > g.qx[1] && !(xp[l] > g.qx[g.nx - 1]);
-    keep[l] = in ? 1 : 0;
-    if (!in && late) {
-      bool has = false;
+    bool has = false;
+    if (!in && wght)
       for (int c = 0; c < 8; ++c) has = has || wght[l + c * NM] != 0.0;
-      if (has) atomicAdd(late, 1ull);
-    }
+    keep[l] = in ? 1 : (has ? LATE : 0);
   }
 }
 
@@ -150,7 +150,7 @@ template <class T>
 __global__ void k_compact(const T* __restrict__ src, T* __restrict__ dst, long long N, const int64_t* __restrict__ keep,
                           const int64_t* __restrict__ pos) {
   for (long long l = blockIdx.x * (long long)blockDim.x + threadIdx.x; l < N; l += (long long)gridDim.x * blockDim.x)
-    if (keep[l]) dst[pos[l]] = src[l];
+    if (keep[l] == 1) dst[(uint32_t)pos[l]] = src[l];  // (the upper half counts LATE ones)
 }
 
 // ---- the FP32 form: new ions staged for the sort ----
@@ -328,15 +328,15 @@ int compact_one(swap_ctx* c, T* a, long long N, long long kept) {
   return SWAP_OK;
 }
 
-// Stable removal of the particles whose src_flag is 0 from xp, vp, vp1, mrat
+// Stable removal of the particles whose src_flag is not 1 from xp, vp, vp1, mrat
 // and beta_p: the bulk form of remove_ion's shift (gutsp.f:29-41).  With
-// keep_weights (looked at once the stream has been waited for) the device
-// ijkp/wght are shifted too (gutsp.f:33,37-39); otherwise they are marked stale.
-template <class Keep>
-int compact_particles(swap_ctx* c, double* xp, double* vp, double* vp1, Keep&& keep_weights) {
+// keep_weights the device ijkp/wght are shifted too (gutsp.f:33,37-39), unless
+// one of the removed is LATE; otherwise they are marked stale.
+int compact_particles(swap_ctx* c, double* xp, double* vp, double* vp1, bool keep_weights) {
   const long long N = c->ntot(), NM = c->dims.ni_max;
-  long long kept = 0;
-  TRY(scan_count(c, N, &kept));
+  long long sum = 0;
+  TRY(scan_count(c, N, &sum));
+  const long long kept = sum & (LATE - 1), late = sum / LATE;
   if (kept == N) return SWAP_OK;
   for (int m = 0; m < 3; ++m) {
     TRY(compact_one(c, xp + m * NM, N, kept));
@@ -345,7 +345,7 @@ int compact_particles(swap_ctx* c, double* xp, double* vp, double* vp1, Keep&& k
   }
   TRY(compact_one(c, c->d_mrat, N, kept));
   TRY(compact_one(c, c->d_beta_p, N, kept));
-  if (keep_weights() && c->weights_valid && c->weights_n >= N) {
+  if (keep_weights && late == 0 && c->weights_valid && c->weights_n >= N) {
     for (int m = 0; m < 3; ++m) TRY(compact_one(c, c->d_ijk + m * NM, N, kept));
     for (int m = 0; m < 8; ++m) TRY(compact_one(c, c->d_wght + m * NM, N, kept));
     c->weights_n = kept;
@@ -437,19 +437,13 @@ int src_outflow(swap_ctx* c, double* xp, double* vp, double* vp1, srcops::Weight
   const long long N = c->ntot();
   if (N <= 0) return SWAP_OK;
   TRY(src_scratch(c, N));
-  const bool count = w == srcops::Weights::KeepIfNoneLate && c->weights_valid && c->weights_n >= N;
-  unsigned long long* late = count ? c->src_cnt + 2 : nullptr;
-  if (count) CU(cudaMemsetAsync(late, 0, sizeof(*late), c->st));
+  const bool look = w == srcops::Weights::KeepIfNoneLate && c->weights_valid && c->weights_n >= N;
   {
     ProfScope ps(c, "src_outflow", c->st);
-    k_outflow_flags<<<nb(N), TPB, 0, c->st>>>(c->g, xp, N, c->src_flag, c->d_wght, c->dims.ni_max, late);
+    k_outflow_flags<<<nb(N), TPB, 0, c->st>>>(c->g, xp, N, c->src_flag, look ? c->d_wght : nullptr, c->dims.ni_max);
   }
   CU(cudaGetLastError());
-  if (count)
-    CU(cudaMemcpyAsync(&c->pinned->late, late, sizeof(*late), cudaMemcpyDeviceToHost, c->st));
-  return compact_particles(c, xp, vp, vp1, [&] {
-    return w == srcops::Weights::Keep || (count && c->pinned->late == 0);
-  });
+  return compact_particles(c, xp, vp, vp1, look || w == srcops::Weights::Keep);
 }
 
 // res_chex over the live particles; the count of this call goes to
@@ -736,7 +730,7 @@ extern "C" int swap_remove_ion(swap_ctx* c, double* xp, double* vp, double* vp1,
   TRY(src_scratch(c, N));
   k_keep_all_but<<<nb(N), TPB, 0, c->st>>>(N, (long long)ion_l - 1, c->src_flag);
   CU(cudaGetLastError());
-  TRY(compact_particles(c, dxp, dvp, dvp1, [] { return true; }));
+  TRY(compact_particles(c, dxp, dvp, dvp1, true));
   return c->finish();
 }
 
